@@ -174,10 +174,20 @@ __device__ __forceinline__ void ag_mover(const AgGemmArgs& a, uint8_t* smem_raw)
   gin_barrier(h, a.channel, blockIdx.x);  // nobody overwrites a shard that a peer is still reading
 }
 
-template <int BN, bool B_MN, class Epi>
+// The epilogue of an ag_gemm kernel: SwiGLU (activation and, if wanted, the raw pair) or a plain store.
+template <bool SWIGLU>
+__device__ __forceinline__ auto ag_epilogue(const CUtensorMap* tmC, const CUtensorMap* tmAct, int keep_c) {
+  if constexpr (SWIGLU)
+    return SwiGluEpilogue{tmAct, tmC, keep_c, {}};
+  else
+    return StoreEpilogue<__nv_bfloat16>{tmC, nullptr, 0, 0, {}};
+}
+
+template <int BN, bool B_MN, bool SWIGLU>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-    ag_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmShape shape,
-                   AgGemmArgs args, Epi epi, int gate_on_b) {
+    ag_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAct, GemmShape shape,
+                   AgGemmArgs args, int keep_c, int gate_on_b) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (static_cast<int>(blockIdx.x) < args.n_movers) {
     ag_mover(args, smem_raw);
@@ -185,15 +195,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   }
   ChunkGate gate{reinterpret_cast<const uint32_t*>(args.h.pad[args.h.rank] + TP_READY_OFF), args.epoch,
                  args.chunks_per_shard, args.h.rank, gate_on_b, args.h.wait_limit_ns};
+  auto epi = ag_epilogue<SWIGLU>(&tmC, &tmAct, keep_c);
+  epi.slab.init(smem_raw, GemmSmem<BN>::EPI_OFF);
   gemm_mainloop<BN, false, B_MN>(&tmA, &tmB, shape, epi, gate, args.h.status, smem_raw);
 }
 
 // The same kernel on CTA pairs (256-row cluster tiles, tcgen05.mma.cta_group::2). Movers come in
 // pairs too (n_movers is even), so every cluster is either two movers or two GEMM CTAs.
-template <bool B_MN, class Epi>
+template <bool B_MN, bool SWIGLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-    ag_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmShape shape,
-                        AgGemmArgs args, Epi epi, int gate_on_b) {
+    ag_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                        const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAct, GemmShape shape,
+                        AgGemmArgs args, int keep_c, int gate_on_b) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (static_cast<int>(blockIdx.x) < args.n_movers) {
     ag_mover(args, smem_raw);
@@ -201,6 +214,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   }
   ChunkGate gate{reinterpret_cast<const uint32_t*>(args.h.pad[args.h.rank] + TP_READY_OFF), args.epoch,
                  args.chunks_per_shard, args.h.rank, gate_on_b, args.h.wait_limit_ns};
+  auto epi = ag_epilogue<SWIGLU>(&tmC, &tmAct, keep_c);
+  epi.slab.init(smem_raw, Gemm2Smem<256>::EPI_OFF);
   gemm_mainloop_2cta<256, false, B_MN>(&tmA, &tmB, shape, epi, gate, args.h.status, smem_raw);
 }
 
@@ -248,6 +263,7 @@ struct RingEpilogue {
   int step, row_base, tile_in_shard;
   bool have_in;
 
+  __device__ __forceinline__ void drain() {}
   __device__ __forceinline__ size_t slot_elems() const { return static_cast<size_t>(a.rows_per_shard) * N; }
   __device__ __forceinline__ __nv_bfloat16* staging(int rank, int slot) const {
     const size_t parity_elems = static_cast<size_t>(a.h.nranks - 1) * slot_elems();
@@ -460,7 +476,7 @@ int b200_ag_gemm(int comm, size_t gathered_off, int gather_b, int M, int N, int 
       shape.m_major = gm >= shape.tiles_m ? 1 : 0;
     }
   }
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC, tmAct;
   int rc;
   const void* gathered = h.window[h.rank] + gathered_off;
   const int b_box_rows = pairs ? BN / 2 : BN;
@@ -475,34 +491,39 @@ int b200_ag_gemm(int comm, size_t gathered_off, int gather_b, int M, int N, int 
               : make_tmap_2d(&tmB, other, N, K, ld_other, b_box_rows, GEMM_BK, 2, true);
   }
   if (rc) return rc;
+  // what the epilogue stores: boxes of 32 rows x 128 bytes, the activation 32 rows x 64 bytes; a map
+  // that is not used stays a copy of the other
+  if (C && (rc = make_tmap_2d(&tmC, C, M, N, ldc, 32, 64, 2, true))) return rc;
+  if (epilogue == 1 && (rc = make_tmap_2d(&tmAct, act, M, N / 2, ld_act, 32, 32, 2, true, true))) return rc;
+  if (!C) tmC = tmAct;
+  if (epilogue != 1) tmAct = tmC;
   AgGemmArgs args{h, gathered_off, shard_bytes, static_cast<size_t>(gather_b ? BN : GEMM_BM) * K * 2, chunks_per_shard,
                   n_movers, channel, ++g_ag_epoch[comm]};
   const int grid = n_movers + shape.num_ctas;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int smem = pairs ? Gemm2Smem<BN>::TOTAL : GemmSmem<BN>::TOTAL;
-#define B200_AG_LAUNCH(KERNEL, EPI)                                             \
-  do {                                                                          \
-    auto k = KERNEL;                                                            \
-    if (set_smem(k, smem)) return B200_ERR_BAD_ARG;                             \
-    k<<<grid, GEMM_THREADS, smem, s>>>(tmA, tmB, shape, args, EPI, gather_b);   \
+  const int smem = pairs ? Gemm2Smem<BN>::TOTAL_EPI : GemmSmem<BN>::TOTAL_EPI;
+  const int keep_c = C != nullptr;
+#define B200_AG_LAUNCH(KERNEL)                                                                        \
+  do {                                                                                                \
+    auto k = KERNEL;                                                                                  \
+    if (set_smem(k, smem)) return B200_ERR_BAD_ARG;                                                   \
+    k<<<grid, GEMM_THREADS, smem, s>>>(tmA, tmB, tmC, tmAct, shape, args, keep_c, gather_b);          \
   } while (0)
   if (epilogue == 1) {
-    SwiGluEpilogue epi{static_cast<__nv_bfloat16*>(act), ld_act, static_cast<__nv_bfloat16*>(C), ldc};
     if (pairs) {
-      if (b_mn) B200_AG_LAUNCH((ag_gemm_pair_kernel<true, SwiGluEpilogue>), epi);
-      else B200_AG_LAUNCH((ag_gemm_pair_kernel<false, SwiGluEpilogue>), epi);
+      if (b_mn) B200_AG_LAUNCH((ag_gemm_pair_kernel<true, true>));
+      else B200_AG_LAUNCH((ag_gemm_pair_kernel<false, true>));
     } else {
-      if (b_mn) B200_AG_LAUNCH((ag_gemm_kernel<BN, true, SwiGluEpilogue>), epi);
-      else B200_AG_LAUNCH((ag_gemm_kernel<BN, false, SwiGluEpilogue>), epi);
+      if (b_mn) B200_AG_LAUNCH((ag_gemm_kernel<BN, true, true>));
+      else B200_AG_LAUNCH((ag_gemm_kernel<BN, false, true>));
     }
   } else {
-    StoreEpilogue<__nv_bfloat16> epi{static_cast<__nv_bfloat16*>(C), ldc, 0};
     if (pairs) {
-      if (b_mn) B200_AG_LAUNCH((ag_gemm_pair_kernel<true, StoreEpilogue<__nv_bfloat16>>), epi);
-      else B200_AG_LAUNCH((ag_gemm_pair_kernel<false, StoreEpilogue<__nv_bfloat16>>), epi);
+      if (b_mn) B200_AG_LAUNCH((ag_gemm_pair_kernel<true, false>));
+      else B200_AG_LAUNCH((ag_gemm_pair_kernel<false, false>));
     } else {
-      if (b_mn) B200_AG_LAUNCH((ag_gemm_kernel<BN, true, StoreEpilogue<__nv_bfloat16>>), epi);
-      else B200_AG_LAUNCH((ag_gemm_kernel<BN, false, StoreEpilogue<__nv_bfloat16>>), epi);
+      if (b_mn) B200_AG_LAUNCH((ag_gemm_kernel<BN, true, false>));
+      else B200_AG_LAUNCH((ag_gemm_kernel<BN, false, false>));
     }
   }
 #undef B200_AG_LAUNCH

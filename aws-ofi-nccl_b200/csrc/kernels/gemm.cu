@@ -28,12 +28,21 @@ int* device_status_word() {
   return words[dev];
 }
 
+// C as the epilogues store it: boxes of 32 rows x 128 bytes.
+template <typename OutT>
+static int make_tmap_out(CUtensorMap* tm, const void* C, int M, int N, int64_t ldc) {
+  if (M == 1) ldc = (static_cast<int64_t>(N) + 7) / 8 * 8;   // a single row may come with any pitch
+  return make_tmap_2d(tm, C, M, N, ldc, 32, 128 / sizeof(OutT), sizeof(OutT), true);
+}
+
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-    gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OutT* C,
-                     int64_t ldc, GemmShape shape, int accumulate, int* err_word) {
+    gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ CUtensorMap tmC, const OutT* C, int64_t ldc, GemmShape shape, int accumulate,
+                     int* err_word) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  StoreEpilogue<OutT> epi{C, ldc, accumulate};
+  StoreEpilogue<OutT> epi{&tmC, C, ldc, accumulate, {}};
+  epi.slab.init(smem_raw, GemmSmem<BN>::EPI_OFF);
   NoGate gate;
   gemm_mainloop<BN, A_MN, B_MN>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
 }
@@ -54,7 +63,7 @@ static int gemm_group_m(int bn) {
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                        int64_t ldc, int accumulate, int max_ctas, cudaStream_t stream) {
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC;
   int rc;
   if (!A_MN)
     rc = make_tmap_2d(&tmA, A, M, K, lda, GEMM_BM, GEMM_BK, 2, true);
@@ -66,12 +75,13 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   else
     rc = make_tmap_2d(&tmB, B, K, N, ldb, GEMM_BK, 64, 2, true);
   if (rc) return rc;
+  if ((rc = make_tmap_out<OutT>(&tmC, C, M, N, ldc))) return rc;
   GemmShape shape{M, N, K, (M + GEMM_BM - 1) / GEMM_BM, (N + BN - 1) / BN};
   shape.group_m = gemm_group_m(BN);
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, OutT>;
   static bool attr_set = false;
   if (!attr_set) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL));
+    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL_EPI));
     attr_set = true;
   }
   int grid = shape.tiles_m * shape.tiles_n;
@@ -79,8 +89,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
   if (grid > cap) grid = cap;
   int* err = device_status_word();
-  kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(tmA, tmB, static_cast<OutT*>(C), ldc, shape, accumulate,
-                                                           err);
+  kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<const OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -88,10 +97,12 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
 // ---------------------------------------------------------------- CTA-pair variant (256 x 256 tile per cluster)
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-    gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OutT* C,
-                          int64_t ldc, GemmShape shape, int accumulate, int* err_word) {
+    gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                          const __grid_constant__ CUtensorMap tmC, const OutT* C, int64_t ldc, GemmShape shape, int accumulate,
+                          int* err_word) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  StoreEpilogue<OutT> epi{C, ldc, accumulate};
+  StoreEpilogue<OutT> epi{&tmC, C, ldc, accumulate, {}};
+  epi.slab.init(smem_raw, Gemm2Smem<BN>::EPI_OFF);
   NoGate gate;
   gemm_mainloop_2cta<BN, A_MN, B_MN>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
 }
@@ -99,7 +110,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                             int64_t ldc, int accumulate, int max_ctas, cudaStream_t stream) {
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC;
   int rc;
   // every CTA loads 128 rows of A and BN/2 rows (its half) of B per k-block
   if (!A_MN)
@@ -112,12 +123,13 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
   else
     rc = make_tmap_2d(&tmB, B, K, N, ldb, GEMM_BK, 64, 2, true);
   if (rc) return rc;
+  if ((rc = make_tmap_out<OutT>(&tmC, C, M, N, ldc))) return rc;
   GemmShape shape{M, N, K, (M + GEMM2_BM - 1) / GEMM2_BM, (N + BN - 1) / BN};
   shape.group_m = (gemm_group_m(BN) + 1) / 2;
   auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, OutT>;
   static bool attr_set = false;
   if (!attr_set) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL));
+    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
     attr_set = true;
   }
   int cap = sm_count();
@@ -125,7 +137,7 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
   int grid = 2 * shape.tiles_m * shape.tiles_n;
   if (grid > cap) grid = cap & ~1;
   int* err = device_status_word();
-  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL, stream>>>(tmA, tmB, static_cast<OutT*>(C), ldc, shape, accumulate, err);
+  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<const OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -143,8 +155,11 @@ static int dispatch_major_2cta(const void* A, const void* B, void* C, int M, int
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                         ScaledStoreEpilogue epi, GemmShape shape, int* err_word) {
+                         const __grid_constant__ CUtensorMap tmC, const float* row_scale, const float* col_scale, GemmShape shape,
+                         int* err_word) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  ScaledStoreEpilogue epi{&tmC, row_scale, col_scale, {}};
+  epi.slab.init(smem_raw, Gemm2Smem<BN>::EPI_OFF);
   NoGate gate;
   gemm_mainloop_2cta<BN, false, false, ScaledStoreEpilogue, NoGate, true>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
 }
@@ -152,24 +167,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 template <int BN>
 static int launch_gemm_fp8(const void* A, const void* B, const float* a_scale, const float* b_scale, void* C, int M, int N,
                            int K, int64_t lda, int64_t ldb, int64_t ldc, cudaStream_t stream) {
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC;
   int rc = make_tmap_2d(&tmA, A, M, K, lda, 128, 2 * GEMM_BK, 1, true);   // 128 one-byte elements = 128 B per row
   if (rc) return rc;
   rc = make_tmap_2d(&tmB, B, N, K, ldb, BN / 2, 2 * GEMM_BK, 1, true);
   if (rc) return rc;
+  if ((rc = make_tmap_out<__nv_bfloat16>(&tmC, C, M, N, ldc))) return rc;
   GemmShape shape{M, N, K, (M + GEMM2_BM - 1) / GEMM2_BM, (N + BN - 1) / BN};
   shape.group_m = (gemm_group_m(BN) + 1) / 2;
   auto kern = gemm_fp8_2cta_kernel<BN>;
   static bool attr_set = false;
   if (!attr_set) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL));
+    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
     attr_set = true;
   }
   int grid = 2 * shape.tiles_m * shape.tiles_n;
   const int cap = sm_count() & ~1;
   if (grid > cap) grid = cap;
-  ScaledStoreEpilogue epi{static_cast<__nv_bfloat16*>(C), ldc, a_scale, b_scale};
-  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL, stream>>>(tmA, tmB, epi, shape, device_status_word());
+  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, a_scale, b_scale, shape, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

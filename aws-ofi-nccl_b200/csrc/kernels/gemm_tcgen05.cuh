@@ -13,6 +13,8 @@ namespace b200 {
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int GEMM_THREADS = 192;
+constexpr int GEMM_EPI_WARP_BYTES = 8192;                    // output staging per epilogue warp: two 4 KiB buffers
+constexpr int GEMM_EPI_BYTES = 4 * GEMM_EPI_WARP_BYTES;
 constexpr uint64_t GEMM_WAIT_LIMIT_NS = 2000000000ull;  // 2 s per wait, then the kernel gives up
 
 template <int BN>
@@ -23,6 +25,9 @@ struct GemmSmem {
   static constexpr int STAGES = (BN == 256) ? 4 : 6;
   static constexpr int BAR_BYTES = 256;
   static constexpr int TOTAL = 1024 + STAGES * STAGE_BYTES + BAR_BYTES;
+  // with the output staging buffers of the epilogue warps (1024-byte aligned, behind the barriers)
+  static constexpr int EPI_OFF = STAGES * STAGE_BYTES + 1024;
+  static constexpr int TOTAL_EPI = 1024 + EPI_OFF + GEMM_EPI_BYTES;
 };
 
 struct GemmShape {
@@ -66,7 +71,8 @@ __device__ __forceinline__ void tile_coords(const GemmShape& s, int tile, int& t
 // Epilogue functor contract:
 //   __device__ void operator()(int row, int col0, const uint32_t (&acc)[32], const GemmShape&)
 // called by one thread per accumulator row for 32 consecutive columns starting at col0 (fp32 bits).
-// Optional hooks: tile_begin(tm, tn) / tile_end(tm, tn) called by every epilogue thread.
+// Hooks: tile_begin(tm, tn) / tile_end(tm, tn) and, after the last tile, drain(), called by every
+// epilogue thread.
 
 template <int BN, bool A_MN, bool B_MN, class Epilogue, class LoadGate>
 __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUtensorMap* tmB, GemmShape shape,
@@ -238,6 +244,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
       acc_buf ^= 1;
       if (acc_buf == 0) acc_phase ^= 1;
     }
+    epi.drain();
   }
 
   // ------------------------------------------------------------ teardown

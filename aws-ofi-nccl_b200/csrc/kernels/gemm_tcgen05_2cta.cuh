@@ -27,6 +27,8 @@ struct Gemm2Smem {
   static constexpr int STAGES = (BN == 256) ? 6 : 8;
   static constexpr int BAR_BYTES = 256;
   static constexpr int TOTAL = 1024 + STAGES * STAGE_BYTES + BAR_BYTES;
+  static constexpr int EPI_OFF = STAGES * STAGE_BYTES + 1024;
+  static constexpr int TOTAL_EPI = 1024 + EPI_OFF + GEMM_EPI_BYTES;
 };
 constexpr int GEMM2_BM = 256;  // rows per cluster tile
 
@@ -286,6 +288,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
       acc_buf ^= 1;
       if (acc_buf == 0) acc_phase ^= 1;
     }
+    epi.drain();
   }
 
   // ------------------------------------------------------------ teardown

@@ -42,9 +42,10 @@ inline EncodeTiledFn get_encode_tiled() {
 }
 
 // 2-D row-major tensor [rows][cols] of `elem_bytes` elements, row pitch `ld` elements.
-// Box = [box_rows][box_cols]; box_cols * elem_bytes must equal the swizzle span (128 B) when swizzled.
+// Box = [box_rows][box_cols]; when swizzled, box_cols * elem_bytes must equal the swizzle span: 128 B,
+// or 64 B with `span64`.
 inline int make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                        uint32_t box_rows, uint32_t box_cols, int elem_bytes, bool swizzle128) {
+                        uint32_t box_rows, uint32_t box_cols, int elem_bytes, bool swizzle, bool span64 = false) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return B200_ERR_NO_DRIVER;
   cuuint64_t dims[2] = {cols, rows};
@@ -55,7 +56,7 @@ inline int make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint6
                            : elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                              : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   CUresult r = enc(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                   !swizzle ? CU_TENSOR_MAP_SWIZZLE_NONE : span64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr, "[b200ops] cuTensorMapEncodeTiled failed: %d (base=%p rows=%llu cols=%llu ld=%llu box=%ux%u)\n",

@@ -1,0 +1,50 @@
+"""The edges of the tiles that the GEMM epilogues store, against a product in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# edges of the 64-column and 32-row slabs that the epilogue stores
+WHOLE = [(33, 72, 64), (129, 200, 136), (257, 328, 72), (2000, 1032, 128)]
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K", WHOLE)
+def test_product_and_accumulation(M, N, K, out_dtype, a_mn, b_mn):
+    from aws_ofi_nccl_b200.ops.gemm import gemm
+
+    if a_mn:
+        M = (M + 7) // 8 * 8   # the pitch of a transposed operand is a multiple of 16 bytes
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N * 3 + K)
+    a = torch.randn((K, M) if a_mn else (M, K), device="cuda", generator=g).bfloat16()
+    b = torch.randn((K, N) if b_mn else (N, K), device="cuda", generator=g).bfloat16()
+    A, B = (a.T if a_mn else a).double(), (b if b_mn else b.T).double()
+    ref, mag = A @ B, A.abs() @ B.abs()
+    # the output lies in a larger buffer whose other elements must stay as they were
+    pad = torch.full((M + 1, (N + 15) // 8 * 8), 7.0, device="cuda", dtype=out_dtype)
+    out = pad[:M, :N]
+    step = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -24
+    # fp32 sums of K exact products in any order: K ulp of the sum of their magnitudes, far from reached
+    bound = K * 2.0 ** -24 * mag + step * ref.abs()
+    gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out)
+    assert ((out.double() - ref).abs() <= bound).all()
+    first = out.double()
+    gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, accumulate=True)
+    want = first + ref
+    assert ((out.double() - want).abs() <= bound + step * want.abs() + 2.0 ** -24 * (first.abs() + mag)).all()
+    assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 132, 128), (300, 200, 144), (257, 1000, 272)])
+def test_fp8_product_at_ragged_edges(M, N, K):
+    from aws_ofi_nccl_b200.ops.gemm import gemm_fp8, quantize_rows_fp8
+
+    N = N // 8 * 8
+    xq, xs = quantize_rows_fp8(torch.randn(M, K, device="cuda").bfloat16())
+    wq, ws = quantize_rows_fp8(torch.randn(N, K, device="cuda").bfloat16())
+    X, W = xq.double() * xs.double()[:, None], wq.double() * ws.double()[:, None]
+    ref, mag = X @ W.T, X.abs() @ W.T.abs()
+    out = gemm_fp8(xq, wq, xs, ws)
+    # bf16 rounding of the result, two fp32 roundings of the scales, fp32 sums
+    assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (K + 4) * 2.0 ** -24 * mag).all()
