@@ -438,6 +438,9 @@ int b200_ag_gemm(int comm, size_t gathered_off, int gather_b, int M, int N, int 
   if (chunks_total > TP_MAX_CHUNKS) return B200_ERR_TOO_LARGE;
   if (n_movers <= 0) n_movers = 16;
   if (n_movers > chunks_per_shard) n_movers = chunks_per_shard;
+  // One rank has nothing to fetch, and a mover's SM multiplies nothing: with the default of 16 movers
+  // 8192 x 16384 x 2048 + SwiGLU took 451 us on 132 SMs, 399 on all 148.
+  if (h.nranks == 1) n_movers = 0;
   const int sms = sm_count();
   shape.cta_first = n_movers;
   shape.num_ctas = sms - n_movers;
