@@ -10,6 +10,7 @@
 #include <cuda_fp8.h>
 
 #include "gemm_epilogues.cuh"
+#include "gemm_splitk.h"
 #include "gemm_tcgen05.cuh"
 #include "gemm_tcgen05_2cta.cuh"
 #include "host_util.h"
@@ -271,6 +272,12 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
     const double eff256 = static_cast<double>(t256) / (((t256 + units - 1) / units) * units);
     const double eff128 = static_cast<double>(t128) / (((t128 + units - 1) / units) * units);
     bn = (N >= 256 && eff256 + 0.08 >= eff128) ? 256 : 128;
+    // Few tiles and a long K: the chip is filled by splitting K over clusters.
+    if (max_ctas == 0) {
+      const SplitkPlan plan = plan_splitk(M, N, K, pairs, bn);
+      if (plan.slices > 1)
+        return launch_splitk({A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate}, pairs, plan, s);
+    }
   }
   if (pairs) {
     if (bn == 256)

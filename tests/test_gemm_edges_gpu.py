@@ -1,16 +1,19 @@
-"""The edges of the tiles that the GEMM epilogues store, against a product in 64 bits."""
+"""Products with few output tiles and a long reduction (cluster split-K) and the edges of the stored
+tiles, against a product in 64 bits."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-# edges of the 64-column and 32-row slabs that the epilogue stores
+# one 128-row tile / ragged rows and columns; both tile widths; 256-row tiles on CTA pairs; K with a tail
+SPLIT = [(1, 8, 4096), (16, 72, 2056), (128, 4096, 14336), (130, 264, 8200), (256, 128, 4096), (300, 520, 8248), (512, 768, 16384)]
+# no split: edges of the 64-column and 32-row slabs that the epilogue stores
 WHOLE = [(33, 72, 64), (129, 200, 136), (257, 328, 72), (2000, 1032, 128)]
 
 
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("M,N,K", WHOLE)
+@pytest.mark.parametrize("M,N,K", SPLIT + WHOLE)
 def test_product_and_accumulation(M, N, K, out_dtype, a_mn, b_mn):
     from aws_ofi_nccl_b200.ops.gemm import gemm
 
@@ -34,6 +37,21 @@ def test_product_and_accumulation(M, N, K, out_dtype, a_mn, b_mn):
     want = first + ref
     assert ((out.double() - want).abs() <= bound + step * want.abs() + 2.0 ** -24 * (first.abs() + mag)).all()
     assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
+
+
+def test_split_sums_are_the_same_every_time_and_on_two_streams():
+    from aws_ofi_nccl_b200.ops.gemm import gemm
+
+    a = torch.randn(128, 14336, device="cuda").bfloat16()
+    b = torch.randn(4096, 14336, device="cuda").bfloat16()
+    want = gemm(a, b)
+    torch.cuda.synchronize()
+    streams, outs = [torch.cuda.Stream() for _ in range(2)], []
+    for i in range(6):
+        with torch.cuda.stream(streams[i % 2]):
+            outs.append(gemm(a, b))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs)
 
 
 @pytest.mark.parametrize("M,N,K", [(256, 132, 128), (300, 200, 144), (257, 1000, 272)])
