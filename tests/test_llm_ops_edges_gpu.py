@@ -1,0 +1,42 @@
+"""The bandwidth kernels at the sizes where their work splits change: widths around the threads-per-row
+steps, token counts around a CTA's rows, vector counts around an unrolled pass."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _within(got, ref, rel, abs_):
+    """|got - ref| <= rel * |ref| + abs_, element by element, against 64 bits."""
+    err = (got.double() - ref).abs()
+    assert (err <= rel * ref.abs() + abs_).all(), (err - rel * ref.abs()).max().item()
+
+
+BF = 2.0 ** -8   # one rounding to bf16, as a relative error (half an ulp is 2^-9; a tie in the fp32 value may add one)
+
+
+@pytest.mark.parametrize("T,H", [(1, 8), (9, 256), (7, 264), (17, 520), (5, 1032), (600, 2048), (3, 2056), (299, 4096), (4, 4104),
+                                 (5, 6152), (301, 8192)])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_rmsnorm(T, H, with_res):
+    from aws_ofi_nccl_b200.ops import llm
+
+    g = torch.Generator(device="cuda").manual_seed(T * 31 + H)
+    x, r, dy, dh = (torch.randn(T, H, device="cuda", generator=g).bfloat16() for _ in range(4))
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16()
+    x.requires_grad_(True), r.requires_grad_(True), w.requires_grad_(True)
+    y, h = llm.rmsnorm(x, w, 1e-5, residual=r if with_res else None)
+    got = torch.autograd.grad((y, h) if with_res else y, (x, w) + ((r,) if with_res else ()), (dy, dh) if with_res else dy)
+    hq = h.detach().double()   # the kernel normalises the rounded sum
+    rstd = torch.rsqrt(hq.pow(2).mean(-1, keepdim=True) + 1e-5)
+    W, D = w.detach().double(), dy.double()
+    _within(y.detach(), hq * rstd * W, 2 * BF, 1e-6)
+    gw = D * W
+    dx = rstd * (gw - hq * rstd ** 2 * (gw * hq).mean(-1, keepdim=True)) + (dh.double() if with_res else 0)
+    _within(got[0], dx, 2 * BF, 1e-4)
+    terms = D * hq * rstd
+    _within(got[1], terms.sum(0), 2 * BF, 2.0 ** -20 * math.sqrt(T) * terms.abs().max().item() + 1e-6)
+    if with_res:
+        assert torch.equal(got[0], got[2])
