@@ -40,3 +40,20 @@ def test_rmsnorm(T, H, with_res):
     _within(got[1], terms.sum(0), 2 * BF, 2.0 ** -20 * math.sqrt(T) * terms.abs().max().item() + 1e-6)
     if with_res:
         assert torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("T,F", [(1, 8), (3, 72), (257, 520), (1000, 2056), (4096, 1376)])
+def test_swiglu(T, F):
+    from aws_ofi_nccl_b200.ops import llm
+
+    gu = (torch.randn(T, 2 * F, device="cuda") * 3).bfloat16()
+    gu[0, :4] = torch.tensor([-100.0, 100.0, -88.0, 0.0], device="cuda")   # both ends of the exponential
+    gu.requires_grad_(True)
+    d = torch.randn(T, F, device="cuda").bfloat16()
+    out = llm.swiglu(gu)
+    (dgu,) = torch.autograd.grad(out, (gu,), d)
+    g, u = gu.detach().double().split(F, -1)
+    s = torch.sigmoid(g)
+    _within(out.detach(), g * s * u, 2 * BF, 1e-35)
+    D = d.double()
+    _within(dgu, torch.cat((D * u * s * (1 + g * (1 - s)), D * g * s), -1), 2 * BF, 2.0 ** -20 * (D.abs() * u.abs()).max().item())
