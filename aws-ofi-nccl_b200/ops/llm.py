@@ -149,13 +149,18 @@ class _CrossEntropy(torch.autograd.Function):
                                                   logits.stride(0), 1.0 / T, _lib.stream_ptr()), "cross_entropy")
         ctx.save_for_backward(logits)
         ctx.mark_dirty(logits)
+        # nobody differentiates through the overwritten logits: no zero-filled [T, V] gradient for them
+        ctx.set_materialize_grads(False)
         return loss.mean(), logits
 
     @staticmethod
     def backward(ctx, dloss, _unused):
         (dlogits,) = ctx.saved_tensors
+        unit = getattr(_CrossEntropy, "assume_unit_grad", True)
+        if dloss is None:   # only the logits output was differentiated
+            return (dlogits if unit else torch.zeros_like(dlogits)), None
         # dloss is 1.0 in the training loop; avoid a 1 GB multiply in that case
-        if dloss.numel() == 1 and getattr(_CrossEntropy, "assume_unit_grad", True):
+        if dloss.numel() == 1 and unit:
             return dlogits, None
         return dlogits * dloss, None
 
