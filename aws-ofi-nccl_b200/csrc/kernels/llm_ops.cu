@@ -408,6 +408,63 @@ __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cs, 
   }
 }
 
+// Rotary embedding between the fused projection [T][pitch] (q heads, k heads, v heads of `hd` elements
+// each) and the three tensors that attention takes, in one pass: forward reads the projection and
+// writes q, k (rotated) and v; backward reads the three gradients, undoes the rotation and writes the
+// projection's gradient, in place of a zero-filled slice per tensor and two sums over all of it.
+// Element (t, h, i) of q lies at q + (t / seq) * batch + (t % seq) * tok + h * head + i. A thread moves
+// V elements of a head's lower half and the V that they rotate with; V = 8 needs 16-byte aligned rows
+// and hd % 16 == 0.
+struct HeadsView {
+  bf16* p;
+  int64_t batch, tok, head;
+};
+template <int V>
+struct alignas(2 * V) Bf16Vec {
+  bf162 v[V / 2];
+};
+template <int V, bool BACKWARD>
+__global__ void __launch_bounds__(256)
+    rope_qkv_kernel(bf16* __restrict__ qkv, int64_t pitch, HeadsView q, HeadsView k, HeadsView v, const float* __restrict__ cs,
+                    const float* __restrict__ sn, int64_t T, int nq, int nkv, int hd, int seq) {
+  using Vec = Bf16Vec<V>;
+  const int half = hd / 2, per_head = half / V;
+  const int heads = nq + 2 * nkv;
+  const int64_t total = T * heads * per_head;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t th = i / per_head;
+    const int c = static_cast<int>(i - th * per_head) * V;   // first element of the lower half's piece
+    const int64_t t = th / heads;
+    int h = static_cast<int>(th - t * heads);
+    const int64_t b = t / seq;
+    const int pos = static_cast<int>(t - b * seq);
+    bf16* fused = qkv + t * pitch + static_cast<int64_t>(h) * hd + c;
+    const bool rotate = h < nq + nkv;
+    const HeadsView& view = h < nq ? q : h < nq + nkv ? k : v;
+    h -= h < nq ? 0 : h < nq + nkv ? nq : nq + nkv;
+    bf16* part = view.p + b * view.batch + pos * view.tok + h * view.head + c;
+    const bf16* src = BACKWARD ? part : fused;
+    bf16* dst = BACKWARD ? fused : part;
+    Vec lo = *reinterpret_cast<const Vec*>(src), hi = *reinterpret_cast<const Vec*>(src + half);
+    if (rotate) {
+      const float* cp = cs + static_cast<int64_t>(pos) * half + c;
+      const float* sp = sn + static_cast<int64_t>(pos) * half + c;
+#pragma unroll
+      for (int j = 0; j < V / 2; ++j) {
+        const float2 co = *reinterpret_cast<const float2*>(cp + 2 * j);
+        float2 si = *reinterpret_cast<const float2*>(sp + 2 * j);
+        if (BACKWARD) si = make_float2(-si.x, -si.y);
+        const float a0 = __low2float(lo.v[j]), a1 = __high2float(lo.v[j]), b0 = __low2float(hi.v[j]), b1 = __high2float(hi.v[j]);
+        lo.v[j] = __floats2bfloat162_rn(a0 * co.x - b0 * si.x, a1 * co.y - b1 * si.y);
+        hi.v[j] = __floats2bfloat162_rn(b0 * co.x + a0 * si.x, b1 * co.y + a1 * si.y);
+      }
+    }
+    *reinterpret_cast<Vec*>(dst) = lo;
+    *reinterpret_cast<Vec*>(dst + half) = hi;
+  }
+}
+
 // ------------------------------------------------------------------ softmax cross-entropy, forward + backward fused
 // One CTA per token row. Pass 1: online max/sum. Pass 2: overwrite the logits with
 // dlogits = (softmax - onehot) * grad_scale. loss[row] = logsumexp - logit[target].
@@ -669,6 +726,31 @@ int b200_rope(void* x, const float* cs, const float* sn, long long T, int nheads
   if (hd % 4) return B200_ERR_BAD_ARG;
   rope_kernel<<<grid_for(T * nheads * (hd / 4), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<bf16*>(x), cs, sn, T, nheads, hd, pitch, seq, backward ? -1.f : 1.f);
+  B200_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// q, k, v: element strides (batch, token, head) in `strides` as {q.batch, q.tok, q.head, k..., v...}; cs, sn
+// [>= seq][hd / 2]; T = batches * seq rows of the fused projection. hd must be a multiple of 4.
+int b200_rope_qkv(void* qkv, long long pitch, void* q, void* k, void* v, const long long* strides, const float* cs,
+                  const float* sn, long long T, int nq, int nkv, int hd, int seq, int backward, void* stream) {
+  b200::ensure_context();
+  if (hd % 4 || T <= 0 || seq <= 0 || nq <= 0 || nkv <= 0) return B200_ERR_BAD_ARG;
+  HeadsView w[3];
+  bf16* base[3] = {static_cast<bf16*>(q), static_cast<bf16*>(k), static_cast<bf16*>(v)};
+  uint64_t ptrs = reinterpret_cast<uint64_t>(qkv), steps = static_cast<uint64_t>(pitch);
+  for (int i = 0; i < 3; ++i) {
+    w[i] = HeadsView{base[i], strides[3 * i], strides[3 * i + 1], strides[3 * i + 2]};
+    ptrs |= reinterpret_cast<uint64_t>(base[i]);
+    steps |= static_cast<uint64_t>(w[i].batch) | static_cast<uint64_t>(w[i].tok) | static_cast<uint64_t>(w[i].head);
+  }
+  if (ptrs % 4 || steps % 2) return B200_ERR_BAD_ARG;
+  const bool wide = hd % 16 == 0 && ptrs % 16 == 0 && steps % 8 == 0;
+  const int grid = grid_for(T * (nq + 2 * nkv) * (hd / 2 / (wide ? 8 : 2)), 256);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  auto kern = wide ? (backward ? rope_qkv_kernel<8, true> : rope_qkv_kernel<8, false>)
+                   : (backward ? rope_qkv_kernel<2, true> : rope_qkv_kernel<2, false>);
+  kern<<<grid, 256, 0, s>>>(static_cast<bf16*>(qkv), pitch, w[0], w[1], w[2], cs, sn, T, nq, nkv, hd, seq);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -61,32 +61,6 @@ class LlamaConfig:
         return sum(math.prod(s) for _, s in self.param_shapes())
 
 
-class _QKRope(torch.autograd.Function):
-    """Rotary embedding applied in place to the q and k heads of a fused [T, (nq+2nkv)*hd] tensor."""
-
-    @staticmethod
-    def forward(ctx, qkv, cos, sin, n_rot_heads, hd, seq):
-        T = qkv.shape[0]
-        view = qkv.as_strided((T, n_rot_heads, hd), (qkv.stride(0), hd, 1))
-        from ..ops import _lib
-        _lib.check(_lib.load().b200_rope(view.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, n_rot_heads, hd,
-                                         qkv.stride(0), seq, 0, _lib.stream_ptr()), "rope")
-        ctx.save_for_backward(cos, sin)
-        ctx.meta = (n_rot_heads, hd, seq)
-        ctx.mark_dirty(qkv)
-        return qkv
-
-    @staticmethod
-    def backward(ctx, d):
-        from ..ops import _lib
-        cos, sin = ctx.saved_tensors
-        n_rot_heads, hd, seq = ctx.meta
-        d = d.clone(memory_format=torch.contiguous_format)
-        _lib.check(_lib.load().b200_rope(d.data_ptr(), cos.data_ptr(), sin.data_ptr(), d.shape[0], n_rot_heads, hd,
-                                         d.stride(0), seq, 1, _lib.stream_ptr()), "rope_bwd")
-        return d, None, None, None, None, None
-
-
 class Llama:
     """Functional model over a flat parameter buffer (no nn.Module: the buffers are the state)."""
 
@@ -136,10 +110,8 @@ class Llama:
     def _attention(self, qkv: torch.Tensor, B: int, S: int) -> torch.Tensor:
         cfg = self.cfg
         hd, nq, nkv = cfg.head_dim, cfg.n_heads, cfg.n_kv_heads
-        qkv = _QKRope.apply(qkv, self.cos, self.sin, nq + nkv, hd, S)
-        q = qkv[:, : nq * hd].view(B, S, nq, hd).transpose(1, 2)
-        k = qkv[:, nq * hd:(nq + nkv) * hd].view(B, S, nkv, hd).transpose(1, 2)
-        v = qkv[:, (nq + nkv) * hd:].view(B, S, nkv, hd).transpose(1, 2)
+        q, k, v = llm_ops.rope_qkv(qkv, self.cos, self.sin, B, S, nq, nkv, hd)
+        q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=(nq != nkv))
         return o.transpose(1, 2).reshape(B * S, nq * hd)
 

@@ -1,6 +1,8 @@
 """Autograd wrappers of the bandwidth-bound Llama kernels (csrc/kernels/llm_ops.cu)."""
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -134,6 +136,45 @@ class _RoPE(torch.autograd.Function):
 
 def rope_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, seq: int) -> torch.Tensor:
     return _RoPE.apply(x, cos, sin, seq)
+
+
+class _RopeQKV(torch.autograd.Function):
+    """The fused projection split into q, k (rotated) and v, each a tensor of its own; one kernel each way."""
+
+    @staticmethod
+    def _launch(qkv, parts, cos, sin, seq, backward):
+        strides = (ctypes.c_longlong * 9)(*(s for p in parts for s in p.stride()[:3]))
+        q, k, v = parts
+        _lib.check(_lib.load().b200_rope_qkv(qkv.data_ptr(), qkv.stride(0), q.data_ptr(), k.data_ptr(), v.data_ptr(), strides,
+                                             cos.data_ptr(), sin.data_ptr(), qkv.shape[0], q.shape[2], k.shape[2], q.shape[3], seq,
+                                             backward, _lib.stream_ptr()), "rope_qkv")
+
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, batch, seq, nq, nkv, hd):
+        assert qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.shape == (batch * seq, (nq + 2 * nkv) * hd) and qkv.stride(1) == 1
+        assert cos.is_contiguous() and sin.is_contiguous() and cos.shape[0] >= seq and cos.shape == sin.shape and cos.shape[1] == hd // 2
+        parts = [torch.empty((batch, seq, n, hd), device=qkv.device, dtype=qkv.dtype) for n in (nq, nkv, nkv)]
+        _RopeQKV._launch(qkv, parts, cos, sin, seq, 0)
+        ctx.save_for_backward(cos, sin)
+        return tuple(parts)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        cos, sin = ctx.saved_tensors
+        # attention returns its gradients as transposed views: any layout with contiguous heads is read in place
+        grads = [g if g.stride(3) == 1 and not any(s % 8 for s in g.stride()[:3]) and g.data_ptr() % 16 == 0 else g.contiguous()
+                 for g in grads]
+        batch, seq, _, hd = grads[0].shape
+        d = torch.empty((batch * seq, sum(g.shape[2] for g in grads) * hd), device=grads[0].device, dtype=grads[0].dtype)
+        _RopeQKV._launch(d, grads, cos, sin, seq, 1)
+        return d, None, None, None, None, None, None, None
+
+
+def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, seq: int, n_heads: int, n_kv_heads: int,
+             head_dim: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """Rotated q and k, and v, as [batch, seq, heads, head_dim] tensors of their own from the fused
+    projection [batch * seq, (n_heads + 2 * n_kv_heads) * head_dim]."""
+    return _RopeQKV.apply(qkv, cos, sin, batch, seq, n_heads, n_kv_heads, head_dim)
 
 
 class _CrossEntropy(torch.autograd.Function):

@@ -57,3 +57,30 @@ def test_swiglu(T, F):
     _within(out.detach(), g * s * u, 2 * BF, 1e-35)
     D = d.double()
     _within(dgu, torch.cat((D * u * s * (1 + g * (1 - s)), D * g * s), -1), 2 * BF, 2.0 ** -20 * (D.abs() * u.abs()).max().item())
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 4, 2), (128, 3, 1), (20, 2, 1), (40, 2, 2)])
+@pytest.mark.parametrize("layout", ["tokens", "heads"])
+def test_rope_qkv(hd, nq, nkv, layout):
+    from aws_ofi_nccl_b200.ops import llm
+
+    B, S = 2, 37
+    qkv = torch.randn(B * S, (nq + 2 * nkv) * hd, device="cuda").bfloat16().requires_grad_(True)
+    ang = torch.rand(S + 3, hd // 2, device="cuda") * 6
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    outs = llm.rope_qkv(qkv, cos, sin, B, S, nq, nkv, hd)
+    c, s = cos[:S].double().view(1, S, 1, -1), sin[:S].double().view(1, S, 1, -1)
+
+    def turn(t, sign):
+        a, b = t.double().split(hd // 2, -1)
+        return torch.cat((a * c - sign * b * s, b * c + sign * a * s), -1)
+
+    parts = qkv.detach().view(B, S, nq + 2 * nkv, hd).split((nq, nkv, nkv), 2)
+    for got, part, rotated in zip(outs, parts, (True, True, False)):
+        _within(got.detach(), turn(part, 1) if rotated else part.double(), BF, 2.0 ** -7)
+    grads = [torch.randn_like(o) for o in outs]
+    if layout == "heads":   # as attention returns them: a transposed [B, heads, S, hd]
+        grads = [g.transpose(1, 2).contiguous().transpose(1, 2) for g in grads]
+    (d,) = torch.autograd.grad(outs, (qkv,), grads)
+    want = torch.cat((turn(grads[0], -1), turn(grads[1], -1), grads[2].double()), 2).view(B * S, -1)
+    _within(d, want, BF, 2.0 ** -7)   # the two products of a rotation cancel: an error of one bf16 step of them
