@@ -6,6 +6,7 @@ stale; ``build_all(force=True)`` rebuilds everything.
 
 Targets
   libb200ops.so            CUDA kernels (GEMM, collectives, GIN device API users, model ops)
+  _b200torch.so            the differentiable layers on those kernels (a Python extension module)
   libnccl-net-ofi-b200.so  ncclNet / ncclTuner / GIN / RMA plugin (also installed under the
                            names NCCL searches for: libnccl-net.so, libnccl-tuner-ofi-b200.so)
   unit test executables    csrc/tests/*.cpp -> lib/tests/<name>
@@ -87,6 +88,24 @@ def build_kernels(force: bool = False, extra_flags: list[str] | None = None) -> 
     if force or jobs or not out.exists():
         _run([NVCC, "-shared", "-o", str(out), *map(str, objs), "-cudart", "static",
               "-gencode", "arch=compute_100a,code=sm_100a"])
+    return out
+
+
+def build_torch_ops(force: bool = False) -> Path:
+    """csrc/kernels/torch_ops.cpp -> lib/_b200torch.so: the differentiable layers, linked against torch
+    and against libb200ops.so next to it."""
+    src, out = CSRC / "kernels" / "torch_ops.cpp", LIB / "_b200torch.so"
+    if force or _stale(out, [src]):
+        import sysconfig
+
+        import torch
+
+        root = Path(torch.__file__).resolve().parent
+        _run([CXX, "-std=c++17", "-O2", "-fPIC", "-shared", "-Wall", "-DTORCH_EXTENSION_NAME=_b200torch",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", str(root / "include"),
+              "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-I", sysconfig.get_paths()["include"],
+              "-I", f"{CUDA_HOME}/include", str(src), "-o", str(out), "-L", str(root / "lib"), "-ltorch", "-ltorch_cpu", "-lc10",
+              "-lc10_cuda", "-ltorch_python", "-L", str(LIB), "-lb200ops", "-Wl,-rpath,$ORIGIN"])
     return out
 
 
@@ -224,6 +243,7 @@ def build_fake_cuda(force: bool = False, sanitize: str | None = None) -> Path:
 
 def build_all(force: bool = False) -> None:
     build_kernels(force)
+    build_torch_ops(force)
     build_host(force)
     build_tests(force)
     build_cuda_tests(force)

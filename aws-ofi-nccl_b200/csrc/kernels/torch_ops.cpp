@@ -1,0 +1,293 @@
+// The differentiable layers of the training path (linear, RMSNorm, SwiGLU, rotary split of the fused
+// projection) as autograd functions in native code: shape checks, output allocation, the calls into
+// libb200ops.so and the weight-gradient hand-over run without the interpreter. A layer's launches are
+// a few microseconds of device time each at small sizes, and the interpreter's share of a forward and
+// backward call was several times that.
+//
+// Weight gradients follow the convention of the Python side: a parameter that carries `main_grad` (a
+// view of the flat gradient buffer) has its gradient written there, `grad_written` is set, and the
+// parameter's `grad_ready` hook is called; other parameters receive an ordinary gradient.
+#include <torch/extension.h>
+
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+
+#include <atomic>
+
+extern "C" {
+int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
+                   int a_mn, int b_mn, int out_fp32, int accumulate, int bn, int max_ctas, void* stream);
+int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w, void* y, float* rstd, int T, int H, float eps,
+                     void* stream);
+int b200_rmsnorm_bwd_partial_rows();
+int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
+                     float* dw_partial, void* dw, int accumulate_dw, int T, int H, void* stream);
+int b200_swiglu_fwd(const void* gu, void* out, long long T, int F, void* stream);
+int b200_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, int F, void* stream);
+int b200_rope_qkv(void* qkv, long long pitch, void* q, void* k, void* v, const long long* strides, const float* cs,
+                  const float* sn, long long T, int nq, int nkv, int hd, int seq, int backward, void* stream);
+}
+
+namespace {
+
+namespace py = pybind11;
+using torch::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+
+std::atomic<int64_t> g_launches{0};
+
+// Raises a Python exception from either side: in a call from Python (the GIL is held) it travels as
+// error_already_set; on an autograd thread torch's own carrier takes it to the caller of backward().
+[[noreturn]] void raise(PyObject* type, const std::string& what) {
+  if (PyGILState_Check()) {
+    PyErr_SetString(type, what.c_str());
+    throw py::error_already_set();
+  }
+  py::gil_scoped_acquire gil;
+  PyErr_SetString(type, what.c_str());
+  python_error err;
+  err.persist();
+  throw err;
+}
+void require(bool ok, const char* what) {
+  if (!ok) raise(PyExc_AssertionError, what);
+}
+void check(int rc, const char* what) {
+  if (rc == 0) return;
+  PyObject* type = PyExc_RuntimeError;
+  {
+    py::gil_scoped_acquire gil;
+    // the package's own class (a RuntimeError); it lives as long as the module
+    static PyObject* own = py::object(py::module_::import("aws_ofi_nccl_b200.ops._lib").attr("B200OpsError")).release().ptr();
+    type = own;
+  }
+  raise(type, std::string(what) + " failed with code " + std::to_string(rc));
+}
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+// C[M,N] (+)= op(A) op(B); the checks of ops.gemm.gemm
+void gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const Tensor& out, bool accumulate) {
+  require(a.is_cuda() && b.is_cuda() && a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16,
+          "operands are bfloat16 CUDA tensors");
+  require(a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1, "operands are matrices with contiguous rows");
+  const int64_t M = a.size(a_mn ? 1 : 0), K = a.size(a_mn ? 0 : 1), N = b.size(b_mn ? 1 : 0);
+  require(b.size(b_mn ? 0 : 1) == K, "reduction dims differ");
+  require(out.dim() == 2 && out.size(0) == M && out.size(1) == N && out.stride(1) == 1 &&
+              (out.scalar_type() == at::kBFloat16 || out.scalar_type() == at::kFloat),
+          "the output is an [M, N] bfloat16 or float32 matrix with contiguous rows");
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  check(b200_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), static_cast<int>(M), static_cast<int>(N), static_cast<int>(K),
+                       a.stride(0), b.stride(0), out.stride(0), a_mn, b_mn, out.scalar_type() == at::kFloat, accumulate, 0, 0,
+                       stream()),
+        "b200_gemm_bf16");
+}
+
+PyObject* interned(const char* name) { return PyUnicode_InternFromString(name); }
+
+// Runs produce(out, accumulate) into weight.main_grad when the parameter has one (and returns an
+// undefined tensor), else into a new tensor of the weight's shape.
+template <class Produce>
+Tensor write_param_grad(const Tensor& weight, Produce produce) {
+  {
+    py::gil_scoped_acquire gil;
+    static PyObject* const kMain = interned("main_grad");
+    static PyObject* const kWritten = interned("grad_written");
+    static PyObject* const kReady = interned("grad_ready");
+    const py::object w = py::reinterpret_steal<py::object>(THPVariable_Wrap(weight));
+    auto attribute = [&](PyObject* name) {
+      PyObject* v = PyObject_GetAttr(w.ptr(), name);
+      if (!v) {
+        if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw py::error_already_set();
+        PyErr_Clear();
+      }
+      return py::reinterpret_steal<py::object>(v);
+    };
+    const py::object main = attribute(kMain);
+    if (main && !main.is_none()) {
+      const py::object written = attribute(kWritten);
+      const bool accumulate = written && PyObject_IsTrue(written.ptr()) == 1;
+      produce(main.cast<Tensor>(), accumulate);
+      if (PyObject_SetAttr(w.ptr(), kWritten, Py_True) != 0) throw py::error_already_set();
+      const py::object ready = attribute(kReady);
+      if (ready && !ready.is_none()) ready(w);
+      return {};
+    }
+  }
+  Tensor dw = at::empty_like(weight);
+  produce(dw, false);
+  return dw;
+}
+
+// pybind's exception cannot cross the autograd engine's threads; torch's carrier can.
+template <class F>
+auto on_engine_thread(F f) {
+  try {
+    return f();
+  } catch (py::error_already_set& e) {
+    py::gil_scoped_acquire gil;
+    e.restore();
+    python_error err;
+    err.persist();
+    throw err;
+  }
+}
+
+// y = x W^T
+struct Linear : public Function<Linear> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight) {
+    ctx->save_for_backward({x, weight});
+    require(x.dim() >= 1 && weight.dim() == 2, "x has a last dimension and the weight is a matrix");
+    auto shape = x.sizes().vec();
+    shape.back() = weight.size(0);
+    // allocated with the final shape: a custom function must not return a view that it made, or later
+    // in-place ops on the output are refused
+    Tensor y = at::empty(shape, x.options().dtype(at::kBFloat16));
+    gemm(x.reshape({-1, x.size(-1)}), weight, false, false, y.view({-1, weight.size(0)}), false);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return on_engine_thread([&]() -> variable_list {
+      const auto saved = ctx->get_saved_variables();
+      const Tensor &x = saved[0], &weight = saved[1];
+      const Tensor dy = grads[0].reshape({-1, grads[0].size(-1)}).contiguous();
+      const Tensor x2 = x.reshape({-1, x.size(-1)});
+      Tensor dx, dw;
+      if (ctx->needs_input_grad(0)) {
+        dx = at::empty_like(x2, x2.options(), at::MemoryFormat::Contiguous);
+        gemm(dy, weight, false, true, dx, false);
+        dx = dx.view(x.sizes());
+      }
+      if (ctx->needs_input_grad(1))
+        dw = write_param_grad(weight, [&](const Tensor& out, bool accumulate) { gemm(dy, x2, true, true, out, accumulate); });
+      return {dx, dw};
+    });
+  }
+};
+
+// y = rmsnorm(h) * w with h = x (+ res), h a new tensor when there is a residual
+struct RMSNorm : public Function<RMSNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const c10::optional<Tensor>& res, const Tensor& weight,
+                               double eps) {
+    require(x.is_contiguous() && (!res || res->is_contiguous()), "x and the residual are contiguous");
+    const int64_t H = x.size(-1), T = x.numel() / H;
+    Tensor y = at::empty_like(x), h = res ? at::empty_like(x) : x;
+    Tensor rstd = at::empty({T}, x.options().dtype(at::kFloat));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    check(b200_rmsnorm_fwd(x.data_ptr(), res ? res->data_ptr() : nullptr, res ? h.data_ptr() : nullptr, weight.data_ptr(),
+                           y.data_ptr(), rstd.data_ptr<float>(), static_cast<int>(T), static_cast<int>(H),
+                           static_cast<float>(eps), stream()),
+          "b200_rmsnorm_fwd");
+    ctx->save_for_backward({h, weight, rstd});
+    ctx->saved_data["res"] = res.has_value();
+    if (res) return {y, h};
+    return {y};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return on_engine_thread([&]() -> variable_list {
+      const auto saved = ctx->get_saved_variables();
+      const Tensor &x = saved[0], &weight = saved[1], &rstd = saved[2];
+      const bool has_res = ctx->saved_data["res"].toBool();
+      const int64_t H = x.size(-1), T = x.numel() / H;
+      const Tensor dy = grads[0].contiguous();
+      const Tensor dres = has_res ? grads[1].contiguous() : Tensor();
+      Tensor dx = at::empty_like(x);
+      const Tensor partial = at::empty({b200_rmsnorm_bwd_partial_rows(), H}, rstd.options());
+      const Tensor dw = write_param_grad(weight, [&](const Tensor& out, bool accumulate) {
+        g_launches.fetch_add(2, std::memory_order_relaxed);
+        check(b200_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), weight.data_ptr(), rstd.data_ptr<float>(),
+                               has_res ? dres.data_ptr() : nullptr, dx.data_ptr(), partial.data_ptr<float>(), out.data_ptr(),
+                               accumulate, static_cast<int>(T), static_cast<int>(H), stream()),
+              "b200_rmsnorm_bwd");
+      });
+      return {dx, has_res ? dx : Tensor(), dw, Tensor()};
+    });
+  }
+};
+
+// silu(gate) * up of a [..., 2F] tensor laid out as gate | up
+struct SwiGLU : public Function<SwiGLU> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& gu) {
+    const int64_t F = gu.size(-1) / 2, T = gu.numel() / (2 * F);
+    require(gu.is_contiguous(), "gate_up is contiguous");
+    auto shape = gu.sizes().vec();
+    shape.back() = F;
+    Tensor out = at::empty(shape, gu.options());
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    check(b200_swiglu_fwd(gu.data_ptr(), out.data_ptr(), T, static_cast<int>(F), stream()), "swiglu_fwd");
+    ctx->save_for_backward({gu});
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return on_engine_thread([&]() -> variable_list {
+      const auto saved = ctx->get_saved_variables();
+      const Tensor& gu = saved[0];
+      const int64_t F = gu.size(-1) / 2, T = gu.numel() / (2 * F);
+      const Tensor dout = grads[0].contiguous();
+      Tensor dgu = at::empty_like(gu);
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+      check(b200_swiglu_bwd(dout.data_ptr(), gu.data_ptr(), dgu.data_ptr(), T, static_cast<int>(F), stream()), "swiglu_bwd");
+      return {dgu};
+    });
+  }
+};
+
+// q, k (rotated) and v as [B, S, heads, hd] tensors of their own from the fused projection [B*S, (nq+2nkv)*hd]
+struct RopeQKV : public Function<RopeQKV> {
+  static void launch(const Tensor& qkv, const Tensor (&part)[3], const Tensor& cos, const Tensor& sin, int64_t S, bool backward) {
+    long long strides[9];
+    for (int i = 0; i < 3; ++i)
+      for (int d = 0; d < 3; ++d) strides[3 * i + d] = part[i].stride(d);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    check(b200_rope_qkv(qkv.data_ptr(), qkv.stride(0), part[0].data_ptr(), part[1].data_ptr(), part[2].data_ptr(), strides,
+                        cos.data_ptr<float>(), sin.data_ptr<float>(), qkv.size(0), static_cast<int>(part[0].size(2)),
+                        static_cast<int>(part[1].size(2)), static_cast<int>(part[0].size(3)), static_cast<int>(S), backward,
+                        stream()),
+          "rope_qkv");
+  }
+  static variable_list forward(AutogradContext* ctx, const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S,
+                               int64_t nq, int64_t nkv, int64_t hd) {
+    require(qkv.is_cuda() && qkv.scalar_type() == at::kBFloat16 && qkv.dim() == 2 && qkv.stride(1) == 1 && qkv.size(0) == B * S &&
+                qkv.size(1) == (nq + 2 * nkv) * hd,
+            "the projection is a [B*S, (nq+2nkv)*hd] bfloat16 CUDA matrix");
+    require(cos.is_contiguous() && sin.is_contiguous() && cos.size(0) >= S && sin.size(0) >= S && cos.size(-1) == hd / 2 &&
+                sin.size(-1) == hd / 2,
+            "cos and sin are [>= S, hd/2] tables");
+    const Tensor part[3] = {at::empty({B, S, nq, hd}, qkv.options()), at::empty({B, S, nkv, hd}, qkv.options()),
+                            at::empty({B, S, nkv, hd}, qkv.options())};
+    launch(qkv, part, cos, sin, S, false);
+    ctx->save_for_backward({cos, sin});
+    return {part[0], part[1], part[2]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return on_engine_thread([&]() -> variable_list {
+      const auto saved = ctx->get_saved_variables();
+      // attention returns its gradients as transposed views: any layout with contiguous heads is read in place
+      auto rows = [](const Tensor& g) {
+        const bool fits = g.stride(3) == 1 && g.stride(0) % 8 == 0 && g.stride(1) % 8 == 0 && g.stride(2) % 8 == 0 &&
+                          reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
+        return fits ? g : g.contiguous();
+      };
+      const Tensor part[3] = {rows(grads[0]), rows(grads[1]), rows(grads[2])};
+      const int64_t B = part[0].size(0), S = part[0].size(1), hd = part[0].size(3);
+      Tensor d = at::empty({B * S, (part[0].size(2) + 2 * part[1].size(2)) * hd}, part[0].options());
+      launch(d, part, saved[0], saved[1], S, true);
+      return {d, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    });
+  }
+};
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("linear", [](const Tensor& x, const Tensor& w) { return Linear::apply(x, w); });
+  m.def("rmsnorm", [](const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
+    return RMSNorm::apply(x, res, w, eps);
+  });
+  m.def("swiglu", [](const Tensor& gu) { return SwiGLU::apply(gu); });
+  m.def("rope_qkv", [](const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S, int64_t nq, int64_t nkv,
+                       int64_t hd) { return RopeQKV::apply(qkv, cos, sin, B, S, nq, nkv, hd); });
+  m.def("launches", [] { return g_launches.load(std::memory_order_relaxed); });
+}

@@ -26,7 +26,6 @@ _SIGNATURES = {
     "b200_swiglu_bwd": ([_vp, _vp, _vp, _ll, _i, _vp], _i),
     "b200_swiglu_bwd_interleaved": ([_vp, _vp, _vp, _ll, _i, _vp], _i),
     "b200_rope": ([_vp, _vp, _vp, _ll, _i, _i, _ll, _i, _i, _vp], _i),
-    "b200_rope_qkv": ([_vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _i, _vp], _i),
     "b200_cross_entropy": ([_vp, _vp, _vp, _i, _i, _ll, _f, _vp], _i),
     "b200_embedding_fwd": ([_vp, _vp, _vp, _ll, _i, _vp], _i),
     "b200_embedding_bwd": ([_vp, _vp, _vp, _ll, _i, _vp], _i),
@@ -47,9 +46,16 @@ def register(name: str, argtypes, restype=_i) -> None:
         fn.argtypes, fn.restype = argtypes, restype
 
 
-# kernels launched per library call (default 1); used for the launch counter
+# kernels launched per ctypes call (default 1); used for the launch counter
 _KERNELS_PER_CALL = {"b200_rmsnorm_bwd": 2, "b200_read_status": 0, "b200_rmsnorm_bwd_partial_rows": 0}
-launch_count = 0
+_launched = 0
+
+
+def __getattr__(name):
+    """``launch_count``: kernels launched so far, by ctypes calls and by the native layers."""
+    if name == "launch_count":
+        return _launched + (_native.launches() if _native is not None else 0)
+    raise AttributeError(name)
 
 
 class _CountingLib:
@@ -67,8 +73,8 @@ class _CountingLib:
             k = _KERNELS_PER_CALL.get(name, 1)
 
             def w(*args, _fn=fn, _k=k):
-                global launch_count
-                launch_count += _k
+                global _launched
+                _launched += _k
                 return _fn(*args)
 
             cache[name] = w
@@ -76,6 +82,26 @@ class _CountingLib:
 
 
 _proxy = None
+_native = None
+
+
+def native():
+    """The extension module with the differentiable layers (csrc/kernels/torch_ops.cpp)."""
+    global _native
+    if _native is None:
+        load()   # the kernel library it calls into
+        path = _LIB_DIR / "_b200torch.so"
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: run `python -m aws_ofi_nccl_b200.build`")
+        import importlib.util
+
+        import torch  # noqa: F401  (the module links against torch's libraries)
+
+        spec = importlib.util.spec_from_file_location("_b200torch", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _native = module
+    return _native
 
 
 def load():

@@ -1,4 +1,4 @@
-"""tcgen05 GEMM bindings and the autograd ``linear`` built on them.
+"""tcgen05 GEMM bindings and the differentiable ``linear`` built on them.
 
 ``gemm`` exposes the kernel's storage flags directly (see csrc/kernels/gemm.cu); ``linear`` maps
 a linear layer's forward, input-gradient and weight-gradient products onto them so no transpose
@@ -70,45 +70,8 @@ def gemm_fp8(a8: torch.Tensor, b8: torch.Tensor, a_scale: torch.Tensor, b_scale:
     return out
 
 
-class _Linear(torch.autograd.Function):
+def linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """y = x W^T.  The weight gradient is written straight into ``weight.main_grad`` when the
     parameter has one (a view of the flat gradient buffer), and the ``grad_ready`` hook of the
     parameter is called so a data-parallel engine can start reducing that bucket at once."""
-
-    @staticmethod
-    def forward(ctx, x, weight):
-        ctx.save_for_backward(x, weight)
-        x2 = x.reshape(-1, x.shape[-1])
-        # allocate with the final shape: a custom Function must not return a view it created,
-        # or later in-place ops on the output (RoPE) are refused by autograd
-        y = torch.empty((*x.shape[:-1], weight.shape[0]), device=x.device, dtype=torch.bfloat16)
-        gemm(x2, weight, out=y.view(-1, weight.shape[0]))
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, weight = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1])
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
-        x2 = x.reshape(-1, x.shape[-1])
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, weight, b_mn=True).view_as(x)
-        dw = None
-        if ctx.needs_input_grad[1]:
-            main_grad = getattr(weight, "main_grad", None)
-            if main_grad is not None:
-                fresh = not getattr(weight, "grad_written", False)
-                gemm(dy2, x2, a_mn=True, b_mn=True, out=main_grad, accumulate=not fresh)
-                weight.grad_written = True
-                hook = getattr(weight, "grad_ready", None)
-                if hook is not None:
-                    hook(weight)
-            else:
-                dw = gemm(dy2, x2, a_mn=True, b_mn=True)
-        return dx, dw
-
-
-def linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    return _Linear.apply(x, weight)
+    return _lib.native().linear(x, weight)

@@ -1,23 +1,9 @@
 """Autograd wrappers of the bandwidth-bound Llama kernels (csrc/kernels/llm_ops.cu)."""
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from . import _lib
-
-_scratch: dict = {}
-
-
-def _dw_partial(device, H: int) -> torch.Tensor:
-    rows = _lib.load().b200_rmsnorm_bwd_partial_rows()
-    key = (device, H)
-    buf = _scratch.get(key)
-    if buf is None or buf.shape[0] < rows:
-        buf = torch.empty((rows, H), device=device, dtype=torch.float32)
-        _scratch[key] = buf
-    return buf
 
 
 def _write_param_grad(weight: torch.Tensor, producer) -> torch.Tensor | None:
@@ -35,79 +21,23 @@ def _write_param_grad(weight: torch.Tensor, producer) -> torch.Tensor | None:
     return out
 
 
-class _RMSNorm(torch.autograd.Function):
-    """y = rmsnorm(h) * w with h = x (+ res).  Returns (y, h); with a residual, h is a new tensor
-    produced in the same pass as the normalisation."""
-
-    @staticmethod
-    def forward(ctx, x, res, weight, eps):
-        H = x.shape[-1]
-        T = x.numel() // H
-        assert x.is_contiguous() and (res is None or res.is_contiguous())
-        y = torch.empty_like(x)
-        h = torch.empty_like(x) if res is not None else x
-        rstd = torch.empty(T, device=x.device, dtype=torch.float32)
-        rc = _lib.load().b200_rmsnorm_fwd(x.data_ptr(), res.data_ptr() if res is not None else None,
-                                          h.data_ptr() if res is not None else None, weight.data_ptr(),
-                                          y.data_ptr(), rstd.data_ptr(), T, H, eps, _lib.stream_ptr())
-        _lib.check(rc, "b200_rmsnorm_fwd")
-        ctx.save_for_backward(h, weight, rstd)
-        ctx.has_res = res is not None
-        return y, (h if res is not None else None)
-
-    @staticmethod
-    def backward(ctx, dy, dh):
-        x, weight, rstd = ctx.saved_tensors
-        H = x.shape[-1]
-        T = x.numel() // H
-        dy = dy.contiguous()
-        dx = torch.empty_like(x)
-        dres_in = dh.contiguous() if dh is not None else None
-        partial = _dw_partial(x.device, H)
-        lib = _lib.load()
-
-        def produce(out, acc):
-            rc = lib.b200_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), weight.data_ptr(), rstd.data_ptr(),
-                                      dres_in.data_ptr() if dres_in is not None else None, dx.data_ptr(),
-                                      partial.data_ptr(), out.data_ptr(), int(acc), T, H, _lib.stream_ptr())
-            _lib.check(rc, "b200_rmsnorm_bwd")
-
-        dw = _write_param_grad(weight, produce)
-        return dx, (dx if ctx.has_res else None), dw, None
-
-
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, residual: torch.Tensor | None = None):
-    """Returns (normed, h) where h = x + residual (or x itself when residual is None)."""
-    y, h = _RMSNorm.apply(x, residual, weight, eps)
-    return y, (h if residual is not None else x)
-
-
-class _SwiGLU(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, gu):
-        F = gu.shape[-1] // 2
-        T = gu.numel() // (2 * F)
-        assert gu.is_contiguous()
-        out = torch.empty((*gu.shape[:-1], F), device=gu.device, dtype=gu.dtype)
-        _lib.check(_lib.load().b200_swiglu_fwd(gu.data_ptr(), out.data_ptr(), T, F, _lib.stream_ptr()), "swiglu_fwd")
-        ctx.save_for_backward(gu)
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        (gu,) = ctx.saved_tensors
-        F = gu.shape[-1] // 2
-        T = gu.numel() // (2 * F)
-        dout = dout.contiguous()
-        dgu = torch.empty_like(gu)
-        _lib.check(_lib.load().b200_swiglu_bwd(dout.data_ptr(), gu.data_ptr(), dgu.data_ptr(), T, F,
-                                               _lib.stream_ptr()), "swiglu_bwd")
-        return dgu
+    """Returns (normed, h) where h = x + residual (or x itself when residual is None); with a residual,
+    h is a new tensor produced in the same pass as the normalisation."""
+    out = _lib.native().rmsnorm(x, residual, weight, eps)
+    return out[0], (out[1] if residual is not None else x)
 
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """silu(gate) * up for a fused [..., 2F] tensor laid out as gate | up."""
-    return _SwiGLU.apply(gate_up)
+    return _lib.native().swiglu(gate_up)
+
+
+def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, seq: int, n_heads: int, n_kv_heads: int,
+             head_dim: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """Rotated q and k, and v, as [batch, seq, heads, head_dim] tensors of their own from the fused
+    projection [batch * seq, (n_heads + 2 * n_kv_heads) * head_dim]."""
+    return tuple(_lib.native().rope_qkv(qkv, cos, sin, batch, seq, n_heads, n_kv_heads, head_dim))
 
 
 class _RoPE(torch.autograd.Function):
@@ -136,45 +66,6 @@ class _RoPE(torch.autograd.Function):
 
 def rope_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, seq: int) -> torch.Tensor:
     return _RoPE.apply(x, cos, sin, seq)
-
-
-class _RopeQKV(torch.autograd.Function):
-    """The fused projection split into q, k (rotated) and v, each a tensor of its own; one kernel each way."""
-
-    @staticmethod
-    def _launch(qkv, parts, cos, sin, seq, backward):
-        strides = (ctypes.c_longlong * 9)(*(s for p in parts for s in p.stride()[:3]))
-        q, k, v = parts
-        _lib.check(_lib.load().b200_rope_qkv(qkv.data_ptr(), qkv.stride(0), q.data_ptr(), k.data_ptr(), v.data_ptr(), strides,
-                                             cos.data_ptr(), sin.data_ptr(), qkv.shape[0], q.shape[2], k.shape[2], q.shape[3], seq,
-                                             backward, _lib.stream_ptr()), "rope_qkv")
-
-    @staticmethod
-    def forward(ctx, qkv, cos, sin, batch, seq, nq, nkv, hd):
-        assert qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.shape == (batch * seq, (nq + 2 * nkv) * hd) and qkv.stride(1) == 1
-        assert cos.is_contiguous() and sin.is_contiguous() and cos.shape[0] >= seq and cos.shape == sin.shape and cos.shape[1] == hd // 2
-        parts = [torch.empty((batch, seq, n, hd), device=qkv.device, dtype=qkv.dtype) for n in (nq, nkv, nkv)]
-        _RopeQKV._launch(qkv, parts, cos, sin, seq, 0)
-        ctx.save_for_backward(cos, sin)
-        return tuple(parts)
-
-    @staticmethod
-    def backward(ctx, *grads):
-        cos, sin = ctx.saved_tensors
-        # attention returns its gradients as transposed views: any layout with contiguous heads is read in place
-        grads = [g if g.stride(3) == 1 and not any(s % 8 for s in g.stride()[:3]) and g.data_ptr() % 16 == 0 else g.contiguous()
-                 for g in grads]
-        batch, seq, _, hd = grads[0].shape
-        d = torch.empty((batch * seq, sum(g.shape[2] for g in grads) * hd), device=grads[0].device, dtype=grads[0].dtype)
-        _RopeQKV._launch(d, grads, cos, sin, seq, 1)
-        return d, None, None, None, None, None, None, None
-
-
-def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, seq: int, n_heads: int, n_kv_heads: int,
-             head_dim: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    """Rotated q and k, and v, as [batch, seq, heads, head_dim] tensors of their own from the fused
-    projection [batch * seq, (n_heads + 2 * n_kv_heads) * head_dim]."""
-    return _RopeQKV.apply(qkv, cos, sin, batch, seq, n_heads, n_kv_heads, head_dim)
 
 
 class _CrossEntropy(torch.autograd.Function):
