@@ -13,6 +13,10 @@
 //  moe_combine  : every expert-output row travels back to its source token's (token, slot) cell;
 //                 when all ranks have delivered, the source sums its k cells, gate-weighted.
 //
+// Rows that stay on their rank need no mailbox: dispatch can store them straight into the tensor that
+// the experts read (moe_collect_rows adds what came through the window), and combine sums them from
+// the expert outputs.
+//
 // The reference moves such traffic as host-proxied RDMA writes with immediate data and signal
 // atomics (reference: src/rdma/gin/nccl_ofi_gin.cpp, nccl_ofi_gin_resources.cpp); here the GPU
 // threads that produce the bytes also put them.
@@ -136,6 +140,8 @@ struct DispatchArgs {
   const int32_t* dest_base;  // [E]
   int32_t* cursor;           // [E]
   int32_t* row_of;           // [T][k] receive-buffer row of every (token, slot); -1 = dropped
+  int32_t* local_row;        // [T][k] the same row where this rank owns the expert, else -1 (written with row_of)
+  __nv_bfloat16* local_out;  // bf16 payload: rows of this rank's own tokens go here instead of the window, or null
   size_t recv_off, scale_off, meta_off;  // window offsets on the receiving side
   int capacity_rows;
   unsigned int* done;
@@ -192,6 +198,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
             my_row = -1;
           }
           a.row_of[t * a.k + lane] = my_row;
+          a.local_row[t * a.k + lane] = my_rank == h.rank ? my_row : -1;
         }
         if (my_row >= 0) {
           MoeMeta m{t, lane, my_w, h.rank};
@@ -200,12 +207,18 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
         }
       } else if (!a.use_saved_rows) {
         a.row_of[t * a.k + lane] = -1;
+        a.local_row[t * a.k + lane] = -1;
       }
     }
     // ---- the row itself, 256 elements (two scale groups) per pass; an unweighted row is
     // quantised once and stored k times, a weighted one is scaled and quantised per slot
     const uint4* src = reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(t) * a.H);
     const bool weighted = a.scale_by_weight != 0;
+    // first byte of the row of slot s, for every lane
+    auto row_base = [&](int drank, int drow) {
+      return a.local_out && drank == h.rank ? reinterpret_cast<uint8_t*>(a.local_out) + static_cast<size_t>(drow) * row_bytes
+                                            : h.window[drank] + a.recv_off + static_cast<size_t>(drow) * row_bytes;
+    };
     for (int c = 0; c < chunks; ++c) {
       const uint4 raw = src[c * 32 + lane];
       const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -226,7 +239,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
         const int drow = __shfl_sync(0xffffffffu, my_row, s);
         const float w = __shfl_sync(0xffffffffu, my_w, s);
         if (drow < 0) continue;  // uniform over the warp
-        uint8_t* dst = h.window[drank] + a.recv_off + static_cast<size_t>(drow) * row_bytes;
+        uint8_t* dst = row_base(drank, drow);
         if (a.fp8) {
           if (weighted) {
             q = quantize8(v, w, scale);
@@ -265,6 +278,38 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
   moe_wait_all(h, 1, a.epoch);
 }
 
+// What dispatch left in the window (rows from other ranks' tokens) -> out; rows past the last received
+// one are zeroed. With `local_in_place` this rank's own rows are in `out` already, stored there by dispatch:
+// 6 us for 32768 rows that are all local, where a copy of the window took 146.
+__global__ void __launch_bounds__(MOE_THREADS)
+    moe_collect_rows_kernel(GinDevHandle h, const int32_t* rows_ptr, size_t recv_off, size_t meta_off, int capacity_rows, int H,
+                            int local_in_place, __nv_bfloat16* out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int rows = min(*rows_ptr, capacity_rows);
+  const int vec = H / 8;
+  const MoeMeta* meta = reinterpret_cast<const MoeMeta*>(h.window[h.rank] + meta_off);
+  const uint4* recv = reinterpret_cast<const uint4*>(h.window[h.rank] + recv_off);
+  for (int r = blockIdx.x * warps + warp; r < capacity_rows; r += gridDim.x * warps) {
+    uint4* dst = reinterpret_cast<uint4*>(out) + static_cast<size_t>(r) * vec;
+    if (r >= rows) {
+      for (int v = lane; v < vec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    if (local_in_place && meta[r].src_rank == h.rank) continue;
+    const uint4* src = recv + static_cast<size_t>(r) * vec;
+    constexpr int U = 4;
+    for (int v0 = lane; v0 < vec; v0 += 32 * U) {
+      uint4 tmp[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (v0 + 32 * u < vec) tmp[u] = src[v0 + 32 * u];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (v0 + 32 * u < vec) dst[v0 + 32 * u] = tmp[u];
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------ combine
 struct CombineArgs {
   GinDevHandle h;
@@ -274,13 +319,16 @@ struct CombineArgs {
   size_t meta_off, comb_off;       // window offsets: MoeMeta [rows] (local), bf16 [T][k][H] (on the source)
   const float* topk_w;             // [T][k] on the source, or null for an unweighted sum
   const int32_t* row_of;           // [T][k] on the source: cells whose row is < 0 were never sent
+  const int32_t* local_row;        // [T][k] row of y for the cells whose expert is on the source itself, else -1
+  int keep_cells;                  // 1: the window's cells of those rows are filled too
+  __nv_bfloat16* cells_out;        // [T][k][H] a copy of every sent cell, or null
   int T, k, H;
   __nv_bfloat16* out;              // [T][H]
   unsigned int* done;
   uint64_t epoch;
 };
 
-__global__ void __launch_bounds__(MOE_THREADS) moe_combine_kernel(CombineArgs a) {
+__global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs a) {
   const GinDevHandle& h = a.h;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int rows = a.expert_offsets[a.experts_local];
@@ -292,6 +340,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_combine_kernel(CombineArgs a)
       if (lane == 0) gin_record_error(h, DEV_ERR_BOUNDS);
       continue;
     }
+    if (m.src_rank == h.rank) continue;   // summed from y below
     const uint4* src = reinterpret_cast<const uint4*>(a.y + static_cast<size_t>(r) * a.H);
     uint4* dst = reinterpret_cast<uint4*>(h.window[m.src_rank] + a.comb_off) +
                  (static_cast<size_t>(m.token) * a.k + m.slot) * vec;
@@ -315,31 +364,60 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_combine_kernel(CombineArgs a)
   }
   // ---- ... and every CTA waits for all ranks' rows before it reduces its share of the tokens
   if (!moe_wait_all(h, 2, a.epoch)) return;
-  const uint4* comb = reinterpret_cast<const uint4*>(h.window[h.rank] + a.comb_off);
-  for (int t = blockIdx.x * warps + warp; t < a.T; t += gridDim.x * warps) {
-    float w = 0.f;
-    int live = 0;
-    if (lane < a.k) {
-      live = a.row_of[t * a.k + lane] >= 0;
-      w = a.topk_w ? a.topk_w[t * a.k + lane] : 1.f;
+  // One CTA per token: its threads read 4 KiB of each of the token's rows at a time. With a warp per
+  // token every row is visited 512 bytes at a time by thousands of warps at once: 4096 tokens x 7168,
+  // top-8, one rank took 194 us that way (314 with eight loads in flight per warp instead of four)
+  // and take 138 now, on average over the forward call, which copies the cells, and the backward call,
+  // which does not; 299 when every row went through its cell in the window. Four cells' loads are issued
+  // together and added in the order of the slots.
+  uint4* comb = reinterpret_cast<uint4*>(h.window[h.rank] + a.comb_off);
+  __shared__ float slot_w[MOE_MAX_TOPK];
+  __shared__ int slot_row[MOE_MAX_TOPK];   // row of y, -1: the cell in the window, -2: never sent
+  for (int t = blockIdx.x; t < a.T; t += gridDim.x) {
+    __syncthreads();   // the slots of the token before have been read
+    if (static_cast<int>(threadIdx.x) < a.k) {
+      const int i = t * a.k + threadIdx.x;
+      int row = a.row_of[i] < 0 ? -2 : a.local_row[i];
+      if (row >= rows) {
+        gin_record_error(h, DEV_ERR_BOUNDS);
+        row = -2;
+      }
+      slot_row[threadIdx.x] = row;
+      slot_w[threadIdx.x] = a.topk_w ? a.topk_w[i] : 1.f;
     }
-    for (int v0 = lane; v0 < vec; v0 += 32) {
+    __syncthreads();
+    constexpr int U = 4;
+    for (int v = threadIdx.x; v < vec; v += MOE_THREADS) {
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (int s = 0; s < a.k; ++s) {
-        const float ws = __shfl_sync(0xffffffffu, w, s);
-        if (!__shfl_sync(0xffffffffu, live, s)) continue;
-        const uint4 q = comb[(static_cast<size_t>(t) * a.k + s) * vec + v0];
-        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q);
+      for (int s0 = 0; s0 < a.k; s0 += U) {
+        uint4 q[U];
+        int row[U];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[2 * j] += ws * __low2float(p[j]);
-          acc[2 * j + 1] += ws * __high2float(p[j]);
+        for (int u = 0; u < U; ++u) {
+          row[u] = s0 + u < a.k ? slot_row[s0 + u] : -2;
+          if (row[u] == -2) continue;
+          q[u] = row[u] >= 0 ? reinterpret_cast<const uint4*>(a.y)[static_cast<size_t>(row[u]) * vec + v]
+                             : comb[(static_cast<size_t>(t) * a.k + s0 + u) * vec + v];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (row[u] == -2) continue;
+          const size_t cell = (static_cast<size_t>(t) * a.k + s0 + u) * vec + v;
+          if (row[u] >= 0 && a.keep_cells) comb[cell] = q[u];
+          if (a.cells_out) reinterpret_cast<uint4*>(a.cells_out)[cell] = q[u];
+          const float ws = slot_w[s0 + u];
+          const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q[u]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            acc[2 * j] += ws * __low2float(p[j]);
+            acc[2 * j + 1] += ws * __high2float(p[j]);
+          }
         }
       }
       __nv_bfloat162 o[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) o[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-      reinterpret_cast<uint4*>(a.out + static_cast<size_t>(t) * a.H)[v0] = *reinterpret_cast<const uint4*>(o);
+      reinterpret_cast<uint4*>(a.out + static_cast<size_t>(t) * a.H)[v] = *reinterpret_cast<const uint4*>(o);
     }
   }
 }
@@ -356,13 +434,24 @@ __global__ void __launch_bounds__(MOE_THREADS)
     if (row_of[i] >= 0) {
       const uint4* a = reinterpret_cast<const uint4*>(dout + static_cast<size_t>(t) * H);
       const uint4* b = reinterpret_cast<const uint4*>(comb + static_cast<size_t>(i) * H);
-      for (int v = lane; v < vec; v += 32) {
-        const uint4 x = a[v], y = b[v];
-        const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&x);
-        const __nv_bfloat162* py = reinterpret_cast<const __nv_bfloat162*>(&y);
+      constexpr int U = 4;
+      for (int v0 = lane; v0 < vec; v0 += 32 * U) {
+        uint4 x[U], y[U];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc += __low2float(px[j]) * __low2float(py[j]) + __high2float(px[j]) * __high2float(py[j]);
+        for (int u = 0; u < U; ++u)
+          if (v0 + 32 * u < vec) {
+            x[u] = a[v0 + 32 * u];
+            y[u] = b[v0 + 32 * u];
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (v0 + 32 * u >= vec) break;
+          const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&x[u]);
+          const __nv_bfloat162* py = reinterpret_cast<const __nv_bfloat162*>(&y[u]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            acc += __low2float(px[j]) * __low2float(py[j]) + __high2float(px[j]) * __high2float(py[j]);
+        }
       }
     }
 #pragma unroll
@@ -371,29 +460,48 @@ __global__ void __launch_bounds__(MOE_THREADS)
   }
 }
 
-// fp8 (e4m3) rows with one fp32 scale per 128 elements -> bf16.
+// fp8 (e4m3) rows with one fp32 scale per 128 elements -> bf16. One warp per row; a lane takes 8 values
+// at a time, so that the warp's stores are 512 consecutive bytes, and four such loads are in flight: 32768 x
+// 7168 in 125 us (5.6 TB/s), 175 with a grid-stride loop over single vectors. With zero_tail the rows past
+// the last received one are written as zeros, in place of a fill of the whole output before (120 us).
 __global__ void __launch_bounds__(MOE_THREADS)
     fp8_dequant_rows_kernel(const uint8_t* q, const float* scales, __nv_bfloat16* out, const int32_t* rows_ptr, int rows_max,
-                            int H) {
+                            int H, int zero_tail) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int rows = rows_ptr ? min(*rows_ptr, rows_max) : rows_max;
-  const int64_t nvec = static_cast<int64_t>(rows) * H / 8;
-  const int groups = H / 128;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < nvec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t e0 = i * 8;
-    const int64_t r = e0 / H;
-    const int g = static_cast<int>((e0 - r * H) / 128);
-    const float s = scales[r * groups + g];
-    const uint2 raw = reinterpret_cast<const uint2*>(q)[i];
-    const __nv_fp8x2_storage_t* p = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw);
-    __nv_bfloat162 o[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[j], __NV_E4M3);
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
-      o[j] = __floats2bfloat162_rn(f.x * s, f.y * s);
+  const int vec = H / 8, groups = H / 128;
+  for (int r = blockIdx.x * warps + warp; r < (zero_tail ? rows_max : rows); r += gridDim.x * warps) {
+    uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(r) * H);
+    if (r >= rows) {
+      for (int v = lane; v < vec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
+      continue;
     }
-    reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(o);
+    const uint2* src = reinterpret_cast<const uint2*>(q + static_cast<size_t>(r) * H);
+    const float* sc = scales + static_cast<size_t>(r) * groups;
+    constexpr int U = 4;
+    for (int v0 = lane; v0 < vec; v0 += 32 * U) {
+      uint2 raw[U];
+      float s[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (v0 + 32 * u < vec) {
+          raw[u] = src[v0 + 32 * u];
+          s[u] = sc[(v0 + 32 * u) / 16];
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (v0 + 32 * u >= vec) break;
+        const __nv_fp8x2_storage_t* p = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw[u]);
+        __nv_bfloat162 o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[j], __NV_E4M3);
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+          o[j] = __floats2bfloat162_rn(f.x * s[u], f.y * s[u]);
+        }
+        dst[v0 + 32 * u] = *reinterpret_cast<const uint4*>(o);
+      }
+    }
   }
 }
 
@@ -435,8 +543,8 @@ int b200_moe_route(int comm, const void* topk_idx, int T, int k, int E, size_t c
 // Collective. Window layout on every rank: payload rows at recv_off (H bytes per row for fp8, 2H
 // for bf16), fp32 scales at scale_off (H/128 per row, fp8 only), 16-byte records at meta_off.
 int b200_moe_dispatch(int comm, const void* x, const void* topk_idx, const void* topk_w, int T, int k, int H, int E, int fp8,
-                      int use_saved_rows, int scale_by_weight, const void* dest_base, void* cursor, void* row_of,
-                      size_t recv_off, size_t scale_off, size_t meta_off, int capacity_rows, void* done, void* stream) {
+                      int use_saved_rows, int scale_by_weight, const void* dest_base, void* cursor, void* row_of, void* local_row,
+                      void* local_out, size_t recv_off, size_t scale_off, size_t meta_off, int capacity_rows, void* done, void* stream) {
   ensure_context();
   const GinDevHandle* hp = comm_handle(comm);
   if (!hp || comm < 0 || comm >= 64) return B200_ERR_BAD_ARG;
@@ -445,14 +553,30 @@ int b200_moe_dispatch(int comm, const void* x, const void* topk_idx, const void*
   if (H / 128 > 64) return B200_ERR_TOO_LARGE;
   const size_t row_bytes = fp8 ? static_cast<size_t>(H) : static_cast<size_t>(H) * 2;
   if (recv_off % 16 || meta_off % 16 || scale_off % 16) return B200_ERR_BAD_ARG;
+  if (!local_row || (local_out && (fp8 || reinterpret_cast<uintptr_t>(local_out) % 16))) return B200_ERR_BAD_ARG;
   if (recv_off + row_bytes * capacity_rows > h.window_bytes || meta_off + 16ull * capacity_rows > h.window_bytes ||
       (fp8 && scale_off + 4ull * (H / 128) * capacity_rows > h.window_bytes))
     return B200_ERR_BAD_ARG;
   DispatchArgs a{h, static_cast<const __nv_bfloat16*>(x), static_cast<const int32_t*>(topk_idx),
                  static_cast<const float*>(topk_w), T, k, H, E, fp8, use_saved_rows, scale_by_weight,
                  static_cast<const int32_t*>(dest_base), static_cast<int32_t*>(cursor), static_cast<int32_t*>(row_of),
-                 recv_off, scale_off, meta_off, capacity_rows, static_cast<unsigned int*>(done), ++g_moe_epoch[comm][1]};
+                 static_cast<int32_t*>(local_row), static_cast<__nv_bfloat16*>(local_out), recv_off, scale_off, meta_off, capacity_rows, static_cast<unsigned int*>(done), ++g_moe_epoch[comm][1]};
   moe_dispatch_kernel<<<moe_grid(T), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  B200_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// Rows of the last dispatch (bf16 payload) -> out[capacity_rows][H], see moe_collect_rows_kernel.
+int b200_moe_collect_rows(int comm, const void* rows_ptr, size_t recv_off, size_t meta_off, int capacity_rows, int H,
+                          int local_in_place, void* out, void* stream) {
+  ensure_context();
+  const GinDevHandle* hp = comm_handle(comm);
+  if (!hp || !rows_ptr || !out || H % 8 || capacity_rows <= 0 || recv_off % 16 || meta_off % 16) return B200_ERR_BAD_ARG;
+  if (recv_off + 2ull * H * capacity_rows > hp->window_bytes || meta_off + 16ull * capacity_rows > hp->window_bytes)
+    return B200_ERR_BAD_ARG;
+  moe_collect_rows_kernel<<<moe_grid(capacity_rows), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      *hp, static_cast<const int32_t*>(rows_ptr), recv_off, meta_off, capacity_rows, H, local_in_place,
+      static_cast<__nv_bfloat16*>(out));
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -460,15 +584,17 @@ int b200_moe_dispatch(int comm, const void* x, const void* topk_idx, const void*
 // Collective. Every CTA of this kernel waits for the other ranks, so the grid is limited to what
 // is resident at once.
 int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int experts_local, size_t meta_off, size_t comb_off,
-                     const void* topk_w, const void* row_of, int T, int k, int H, void* out, void* done, void* stream) {
+                     const void* topk_w, const void* row_of, const void* local_row, int keep_cells, void* cells_out, int T, int k,
+                     int H, void* out, void* done, void* stream) {
   ensure_context();
   const GinDevHandle* hp = comm_handle(comm);
   if (!hp || comm < 0 || comm >= 64) return B200_ERR_BAD_ARG;
   GinDevHandle h = *hp;
-  if (H % 8 || k <= 0 || k > MOE_MAX_TOPK || T <= 0) return B200_ERR_BAD_ARG;
+  if (H % 8 || k <= 0 || k > MOE_MAX_TOPK || T <= 0 || !local_row) return B200_ERR_BAD_ARG;
   if (comb_off % 16 || comb_off + static_cast<size_t>(T) * k * H * 2 > h.window_bytes) return B200_ERR_BAD_ARG;
   CombineArgs a{h, static_cast<const __nv_bfloat16*>(y), static_cast<const int32_t*>(expert_offsets), experts_local, meta_off,
-                comb_off, static_cast<const float*>(topk_w), static_cast<const int32_t*>(row_of), T, k, H,
+                comb_off, static_cast<const float*>(topk_w), static_cast<const int32_t*>(row_of),
+                static_cast<const int32_t*>(local_row), keep_cells, static_cast<__nv_bfloat16*>(cells_out), T, k, H,
                 static_cast<__nv_bfloat16*>(out), static_cast<unsigned int*>(done), ++g_moe_epoch[comm][2]};
   int per_sm = 0;
   B200_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_combine_kernel, MOE_THREADS, 0));
@@ -489,14 +615,15 @@ int b200_moe_combine_wgrad(const void* dout, const void* comb, const void* row_o
   return 0;
 }
 
-// rows_ptr (device int32, may be null) limits the work to the rows actually received.
-int b200_fp8_dequant_rows(const void* q, const void* scales, void* out, const void* rows_ptr, int rows_max, int H, void* stream) {
+// rows_ptr (device int32, may be null) limits the work to the rows actually received; with zero_tail the
+// others are written as zeros.
+int b200_fp8_dequant_rows(const void* q, const void* scales, void* out, const void* rows_ptr, int rows_max, int H, int zero_tail,
+                          void* stream) {
   ensure_context();
   if (H % 128) return B200_ERR_BAD_ARG;
-  int grid = sm_count() * 8;
-  fp8_dequant_rows_kernel<<<grid, MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+  fp8_dequant_rows_kernel<<<moe_grid(rows_max), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint8_t*>(q), static_cast<const float*>(scales), static_cast<__nv_bfloat16*>(out),
-      static_cast<const int32_t*>(rows_ptr), rows_max, H);
+      static_cast<const int32_t*>(rows_ptr), rows_max, H, zero_tail);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -25,11 +25,12 @@ from .symm import Communicator
 
 _vp, _i, _sz = C.c_void_p, C.c_int, C.c_size_t
 _lib.register("b200_moe_route", [_i, _vp, _i, _i, _i, _sz, _vp, _vp, _vp, _vp, _vp, _vp], _i)
-_lib.register("b200_moe_dispatch", [_i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _sz, _sz, _sz, _i, _vp,
-                                    _vp], _i)
-_lib.register("b200_moe_combine", [_i, _vp, _vp, _i, _sz, _sz, _vp, _vp, _i, _i, _i, _vp, _vp, _vp], _i)
+_lib.register("b200_moe_dispatch", [_i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _sz, _sz, _sz,
+                                    _i, _vp, _vp], _i)
+_lib.register("b200_moe_collect_rows", [_i, _vp, _sz, _sz, _i, _i, _i, _vp, _vp], _i)
+_lib.register("b200_moe_combine", [_i, _vp, _vp, _i, _sz, _sz, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _vp, _vp, _vp], _i)
 _lib.register("b200_moe_combine_wgrad", [_vp, _vp, _vp, _vp, _i, _i, _i, _vp], _i)
-_lib.register("b200_fp8_dequant_rows", [_vp, _vp, _vp, _vp, _i, _i, _vp], _i)
+_lib.register("b200_fp8_dequant_rows", [_vp, _vp, _vp, _vp, _i, _i, _i, _vp], _i)
 
 
 def _align(x: int, a: int = 1024) -> int:
@@ -60,6 +61,7 @@ class ExpertParallel:
         self.cursor = torch.zeros(experts, device=dev, dtype=torch.int32)
         self.expert_offsets = torch.zeros(self.experts_local + 1, device=dev, dtype=torch.int32)
         self.row_of = torch.full((tokens, topk), -1, device=dev, dtype=torch.int32)
+        self.local_row = torch.full((tokens, topk), -1, device=dev, dtype=torch.int32)   # row_of where this rank owns the expert
         self._done = torch.zeros(4, device=dev, dtype=torch.int32)
         self._last_topk_idx = None
 
@@ -97,31 +99,54 @@ class ExpertParallel:
         return self.expert_offsets
 
     def dispatch_raw(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.Tensor | None, *, fp8: bool,
-                     use_saved_rows: bool = False, scale_by_weight: bool = False) -> None:
+                     use_saved_rows: bool = False, scale_by_weight: bool = False,
+                     local_out: torch.Tensor | None = None) -> None:
+        """With ``local_out`` (bf16 payload, [capacity, H]) the rows of this rank's own tokens are stored
+        there instead of in the window; ``collect`` adds the others."""
         assert x.shape == (self.T, self.H) and x.dtype == torch.bfloat16 and x.is_contiguous()
         rc = _lib.load().b200_moe_dispatch(
             self.comm.id, x.data_ptr(), topk_idx.data_ptr(), topk_w.data_ptr() if topk_w is not None else None,
             self.T, self.k, self.H, self.E, int(fp8), int(use_saved_rows), int(scale_by_weight),
-            self.dest_base.data_ptr(), self.cursor.data_ptr(), self.row_of.data_ptr(), self.recv_off, self.scale_off,
-            self.meta_off, self.capacity, self._done[1:].data_ptr(), _lib.stream_ptr())
+            self.dest_base.data_ptr(), self.cursor.data_ptr(), self.row_of.data_ptr(), self.local_row.data_ptr(),
+            local_out.data_ptr() if local_out is not None else None, self.recv_off, self.scale_off, self.meta_off, self.capacity, self._done[1:].data_ptr(), _lib.stream_ptr())
         _lib.check(rc, "b200_moe_dispatch")
 
-    def combine_raw(self, y_rows: torch.Tensor, topk_w: torch.Tensor | None, out: torch.Tensor) -> None:
+    def collect(self, out: torch.Tensor, local_in_place: bool) -> torch.Tensor:
+        """The bf16 rows of the last dispatch -> ``out`` [capacity, H]: all of them, or (``local_in_place``)
+        those that dispatch did not store there itself.  Rows past the last received one become zeros."""
+        rc = _lib.load().b200_moe_collect_rows(self.comm.id, self.expert_offsets[self.experts_local:].data_ptr(), self.recv_off,
+                                               self.meta_off, self.capacity, self.H, int(local_in_place), out.data_ptr(),
+                                               _lib.stream_ptr())
+        _lib.check(rc, "b200_moe_collect_rows")
+        return out
+
+    def _dispatch_rows(self, x, topk_idx, topk_w, **kw) -> torch.Tensor:
+        """bf16 dispatch into a tensor of its own: no row is copied that need not cross to another rank."""
+        rows = torch.empty(self.capacity, self.H, device=x.device, dtype=torch.bfloat16)
+        self.dispatch_raw(x, topk_idx, topk_w, fp8=False, local_out=rows, **kw)
+        return self.collect(rows, True)
+
+    def combine_raw(self, y_rows: torch.Tensor, topk_w: torch.Tensor | None, out: torch.Tensor,
+                    cells_out: torch.Tensor | None = None, keep_cells: bool = True) -> None:
+        """``cells_out`` [T, k, H] receives a copy of every sent cell; without ``keep_cells`` the window's
+        combine cells are filled only where the expert is on another rank."""
         assert y_rows.dtype == torch.bfloat16 and y_rows.is_contiguous() and y_rows.shape[1] == self.H
         assert out.shape == (self.T, self.H) and out.dtype == torch.bfloat16 and out.is_contiguous()
         rc = _lib.load().b200_moe_combine(
             self.comm.id, y_rows.data_ptr(), self.expert_offsets.data_ptr(), self.experts_local, self.meta_off,
-            self.comb_off, topk_w.data_ptr() if topk_w is not None else None, self.row_of.data_ptr(), self.T, self.k,
+            self.comb_off, topk_w.data_ptr() if topk_w is not None else None, self.row_of.data_ptr(),
+            self.local_row.data_ptr(), int(keep_cells), cells_out.data_ptr() if cells_out is not None else None, self.T, self.k,
             self.H, out.data_ptr(), self._done[2:].data_ptr(), _lib.stream_ptr())
         _lib.check(rc, "b200_moe_combine")
 
     def dequant(self, out: torch.Tensor | None = None) -> torch.Tensor:
         """fp8 receive rows + scales -> bf16 [capacity, H] (only the rows actually received are written)."""
-        if out is None:
-            out = torch.zeros(self.capacity, self.H, device=self.comm.device, dtype=torch.bfloat16)
+        fresh = out is None
+        if fresh:   # the kernel writes the zeros of the rows that nobody sent
+            out = torch.empty(self.capacity, self.H, device=self.comm.device, dtype=torch.bfloat16)
         rc = _lib.load().b200_fp8_dequant_rows(self.recv_rows(True).data_ptr(), self.recv_scales().data_ptr(),
                                                out.data_ptr(), self.expert_offsets[self.experts_local:].data_ptr(),
-                                               self.capacity, self.H, _lib.stream_ptr())
+                                               self.capacity, self.H, int(fresh), _lib.stream_ptr())
         _lib.check(rc, "b200_fp8_dequant_rows")
         return out
 
@@ -139,18 +164,18 @@ class _Dispatch(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, ep, topk_idx, topk_w, fp8):
         ep.route(topk_idx)
-        ep.dispatch_raw(x.contiguous(), topk_idx, topk_w, fp8=fp8)
         ep._last_topk_idx = topk_idx
         ctx.ep = ep
         if fp8:
+            ep.dispatch_raw(x.contiguous(), topk_idx, topk_w, fp8=True)
             return ep.dequant()
-        return ep.recv_rows(False).clone()
+        return ep._dispatch_rows(x.contiguous(), topk_idx, topk_w)
 
     @staticmethod
     def backward(ctx, d_rows):
         ep = ctx.ep
         dx = torch.empty(ep.T, ep.H, device=d_rows.device, dtype=torch.bfloat16)
-        ep.combine_raw(d_rows.contiguous(), None, dx)   # unweighted sum of the k row gradients of each token
+        ep.combine_raw(d_rows.contiguous(), None, dx, keep_cells=False)   # unweighted sum of the k row gradients of each token
         return dx, None, None, None, None
 
 
@@ -159,10 +184,11 @@ class _Combine(torch.autograd.Function):
     def forward(ctx, y_rows, topk_w, ep):
         out = torch.empty(ep.T, ep.H, device=y_rows.device, dtype=torch.bfloat16)
         w = topk_w.detach().float().contiguous()
-        ep.combine_raw(y_rows.contiguous(), w, out)
+        cells = torch.empty(ep.T, ep.k, ep.H, device=y_rows.device, dtype=torch.bfloat16)
+        ep.combine_raw(y_rows.contiguous(), w, out, cells_out=cells, keep_cells=False)
         ctx.ep = ep
         ctx.n_rows = y_rows.shape[0]
-        ctx.save_for_backward(w, ep.combine_cells().clone())
+        ctx.save_for_backward(w, cells)
         return out
 
     @staticmethod
@@ -175,6 +201,5 @@ class _Combine(torch.autograd.Function):
                                                       dw.data_ptr(), ep.T, ep.k, ep.H, _lib.stream_ptr()),
                    "b200_moe_combine_wgrad")
         # d(y_row) = weight * d_out[token]: the forward dispatch again, on the same rows, weighted
-        idx = ep._last_topk_idx
-        ep.dispatch_raw(d_out, idx, w, fp8=False, use_saved_rows=True, scale_by_weight=True)
-        return ep.recv_rows(False)[:ctx.n_rows].clone(), dw, None
+        d_rows = ep._dispatch_rows(d_out, ep._last_topk_idx, w, use_saved_rows=True, scale_by_weight=True)
+        return d_rows[:ctx.n_rows], dw, None
