@@ -264,14 +264,25 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
   const bool pairs = gemm_pair_mode() != 0 && M >= 256 && N >= 128 && (max_ctas == 0 || max_ctas >= 2);
   if (bn == 0) {
     // Wider tiles re-read A less; fall back to the narrower tile when that fills the SMs better.
-    // With CTA pairs the tile is 256 rows tall and a wave is one tile per pair of SMs.
     const int units = pairs ? sm_count() / 2 : sm_count();
     const long rows = pairs ? (M + 255) / 256 : (M + 127) / 128;
     const long t256 = rows * ((N + 255) / 256);
     const long t128 = rows * ((N + 127) / 128);
-    const double eff256 = static_cast<double>(t256) / (((t256 + units - 1) / units) * units);
-    const double eff128 = static_cast<double>(t128) / (((t128 + units - 1) / units) * units);
-    bn = (N >= 256 && eff256 + 0.08 >= eff128) ? 256 : 128;
+    const long w256 = (t256 + units - 1) / units, w128 = (t128 + units - 1) / units;
+    if (pairs) {
+      // With CTA pairs the tile is 256 rows tall and a wave is one tile per pair of SMs. A wave of narrow
+      // tiles costs about 0.56 of one of wide tiles (4096 x 4096 x 14336: seven waves 408 us, four wide ones
+      // 444), but nearly as much where the 128-byte rows of the operand boxes straddle cache lines and L2
+      // delivers the operands late (1000 x 5160 x 2568: three waves 46 us, two wide ones 41;
+      // 4096 x 4096 x 16040: seven 660 us, four wide ones 436).
+      const bool aligned = lda % 64 == 0 && ldb % 64 == 0 &&
+                           ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 127) == 0;
+      bn = (N >= 256 && w256 <= (aligned ? 0.56 : 0.85) * w128) ? 256 : 128;
+    } else {
+      const double eff256 = static_cast<double>(t256) / (w256 * units);
+      const double eff128 = static_cast<double>(t128) / (w128 * units);
+      bn = (N >= 256 && eff256 + 0.08 >= eff128) ? 256 : 128;
+    }
     // Few tiles and a long K: the chip is filled by splitting K over clusters.
     if (max_ctas == 0) {
       const SplitkPlan plan = plan_splitk(M, N, K, pairs, bn);
