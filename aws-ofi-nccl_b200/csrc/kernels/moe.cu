@@ -7,7 +7,7 @@
 //                 each (source rank, expert) segment starts in the owner's receive buffer. The
 //                 receive buffer therefore comes out packed expert-major with no padding and is
 //                 directly usable as the row-segmented operand of the expert GEMMs.
-//  moe_dispatch : one warp per token: quantise (or copy) the row once, then store it into the
+//  moe_dispatch : a team of warps per token: quantise (or copy) the row once, then store it into the
 //                 receive buffer of every rank that owns one of its k experts, with its scales
 //                 and a 16-byte record (token, slot, weight, source rank) used on the way back.
 //  moe_combine  : every expert-output row travels back to its source token's (token, slot) cell;
@@ -156,6 +156,27 @@ __device__ __forceinline__ float warp_half_max(float v) {  // max over each grou
 
 constexpr int MOE_MAX_TOPK = 16;
 
+// How the warps of a CTA share tokens in dispatch and in combine's sum: the smallest power of two of
+// warps that covers a row of H elements, 256 per warp, works on one token (a whole CTA from 2048
+// elements on), so that a wide row moves in pieces of several KiB and a narrow one leaves no warp idle.
+struct TokenTeam {
+  static constexpr int WARPS = MOE_THREADS / 32;
+  int warps, teams;   // warps of a team, teams of the CTA
+  int team, warp;     // this thread's team and its warp in the team
+  __host__ __device__ static int warps_for(int H) {
+    int w = 1;
+    while (w < WARPS && w * 256 < H) w *= 2;
+    return w;
+  }
+  __device__ __forceinline__ explicit TokenTeam(int H) {
+    warps = warps_for(H);
+    teams = WARPS / warps;
+    team = static_cast<int>(threadIdx.x >> 5) / warps;
+    warp = static_cast<int>(threadIdx.x >> 5) % warps;
+  }
+  __device__ __forceinline__ int thread() const { return warp * 32 + static_cast<int>(threadIdx.x & 31); }
+};
+
 // Eight values of one lane (16 lanes share a 128-element scale group) -> eight e4m3 bytes.
 __device__ __forceinline__ uint2 quantize8(const float (&v)[8], float w, float& scale) {
   float amax = 0.f;
@@ -172,55 +193,74 @@ __device__ __forceinline__ uint2 quantize8(const float (&v)[8], float w, float& 
   return q;
 }
 
+// A team per token: from 2048 elements on it writes one destination row 2 KiB (fp8) or 4 KiB (bf16) at a time,
+// where a warp per token left every row 256 or 512 bytes at a time among thousands of others (4096 tokens x
+// 7168, top-8: 92 us on average over the fp8 and the weighted bf16 call, 86 now).
 __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs a) {
   const GinDevHandle& h = a.h;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const TokenTeam team(a.H);
+  const int lane = threadIdx.x & 31;
   const int el = a.E / h.nranks;
   const int chunks = a.H / 256;      // 256 elements (two scale groups) per warp pass
   const int groups = a.H / 128;
   const size_t row_bytes = a.fp8 ? static_cast<size_t>(a.H) : static_cast<size_t>(a.H) * 2;
-  __shared__ float scale_buf[MOE_THREADS / 32][64];
-  for (int t = blockIdx.x * warps + warp; t < a.T; t += gridDim.x * warps) {
-    // ---- where do the k copies go
-    int my_rank = -1, my_row = -1;   // lane s (< k) holds the destination of slot s
-    float my_w = 0.f;
-    if (lane < a.k) {
-      const int e = a.topk_idx[t * a.k + lane];
-      my_w = a.topk_w ? a.topk_w[t * a.k + lane] : 1.f;
+  const bool weighted = a.scale_by_weight != 0;
+  constexpr int MAX_PASSES = 4;      // H / 128 <= 64 (the launcher checks): at most 32 chunks
+  __shared__ float team_scale[TokenTeam::WARPS][64];
+  __shared__ int team_rank[TokenTeam::WARPS][MOE_MAX_TOPK], team_row[TokenTeam::WARPS][MOE_MAX_TOPK];   // row < 0: goes nowhere
+  __shared__ float team_w[TokenTeam::WARPS][MOE_MAX_TOPK];
+  float* scale_buf = team_scale[team.team];
+  int *slot_rank = team_rank[team.team], *slot_row = team_row[team.team];
+  float* slot_w = team_w[team.team];
+  for (int t0 = blockIdx.x * team.teams; t0 < a.T; t0 += gridDim.x * team.teams) {
+    const int t = t0 + team.team;
+    const bool live = t < a.T;
+    // the token's row is on its way while the k copies find their places
+    const uint4* src = reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(t) * a.H);
+    uint4 raws[MAX_PASSES];
+#pragma unroll
+    for (int i = 0; i < MAX_PASSES; ++i)
+      if (live && team.warp + i * team.warps < chunks) raws[i] = src[(team.warp + i * team.warps) * 32 + lane];
+    __syncthreads();   // the slots and scales of the token before have been read
+    if (live && team.thread() < a.k) {
+      const int slot = team.thread();
+      int my_rank = 0, my_row = -1;
+      const int e = a.topk_idx[t * a.k + slot];
+      const float my_w = a.topk_w ? a.topk_w[t * a.k + slot] : 1.f;
       if (e >= 0 && e < a.E) {
         my_rank = e / el;
         if (a.use_saved_rows) {
-          my_row = a.row_of[t * a.k + lane];
+          my_row = a.row_of[t * a.k + slot];
         } else {
           my_row = a.dest_base[e] + atomicAdd(&a.cursor[e], 1);
           if (my_row >= a.capacity_rows) {
             gin_record_error(h, DEV_ERR_CAPACITY);
             my_row = -1;
           }
-          a.row_of[t * a.k + lane] = my_row;
-          a.local_row[t * a.k + lane] = my_rank == h.rank ? my_row : -1;
+          a.row_of[t * a.k + slot] = my_row;
+          a.local_row[t * a.k + slot] = my_rank == h.rank ? my_row : -1;
         }
         if (my_row >= 0) {
-          MoeMeta m{t, lane, my_w, h.rank};
+          MoeMeta m{t, slot, my_w, h.rank};
           *reinterpret_cast<int4*>(h.window[my_rank] + a.meta_off + static_cast<size_t>(my_row) * sizeof(MoeMeta)) =
               *reinterpret_cast<const int4*>(&m);
         }
       } else if (!a.use_saved_rows) {
-        a.row_of[t * a.k + lane] = -1;
-        a.local_row[t * a.k + lane] = -1;
+        a.row_of[t * a.k + slot] = -1;
+        a.local_row[t * a.k + slot] = -1;
       }
+      slot_rank[slot] = my_rank;
+      slot_row[slot] = my_row;
+      slot_w[slot] = my_w;
     }
-    // ---- the row itself, 256 elements (two scale groups) per pass; an unweighted row is
-    // quantised once and stored k times, a weighted one is scaled and quantised per slot
-    const uint4* src = reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(t) * a.H);
-    const bool weighted = a.scale_by_weight != 0;
-    // first byte of the row of slot s, for every lane
-    auto row_base = [&](int drank, int drow) {
-      return a.local_out && drank == h.rank ? reinterpret_cast<uint8_t*>(a.local_out) + static_cast<size_t>(drow) * row_bytes
-                                            : h.window[drank] + a.recv_off + static_cast<size_t>(drow) * row_bytes;
-    };
-    for (int c = 0; c < chunks; ++c) {
-      const uint4 raw = src[c * 32 + lane];
+    __syncthreads();
+    // ---- the row itself; an unweighted row is quantised once and stored k times, a weighted one is
+    // scaled and quantised per slot
+#pragma unroll
+    for (int i = 0; i < MAX_PASSES; ++i) {
+      const int c = team.warp + i * team.warps;
+      if (!live || c >= chunks) break;
+      const uint4 raw = raws[i];
       const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
       float v[8];
 #pragma unroll
@@ -232,14 +272,15 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
       float scale = 1.f;
       if (a.fp8 && !weighted) {
         q = quantize8(v, 1.f, scale);
-        if ((lane & 15) == 0) scale_buf[warp][2 * c + (lane >> 4)] = scale;
+        if ((lane & 15) == 0) scale_buf[2 * c + (lane >> 4)] = scale;
       }
       for (int s = 0; s < a.k; ++s) {
-        const int drank = __shfl_sync(0xffffffffu, my_rank, s);
-        const int drow = __shfl_sync(0xffffffffu, my_row, s);
-        const float w = __shfl_sync(0xffffffffu, my_w, s);
-        if (drow < 0) continue;  // uniform over the warp
-        uint8_t* dst = row_base(drank, drow);
+        const int drank = slot_rank[s], drow = slot_row[s];
+        const float w = slot_w[s];
+        if (drow < 0) continue;  // uniform over the team
+        uint8_t* dst = a.local_out && drank == h.rank
+                           ? reinterpret_cast<uint8_t*>(a.local_out) + static_cast<size_t>(drow) * row_bytes
+                           : h.window[drank] + a.recv_off + static_cast<size_t>(drow) * row_bytes;
         if (a.fp8) {
           if (weighted) {
             q = quantize8(v, w, scale);
@@ -258,15 +299,12 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
       }
     }
     if (a.fp8 && !weighted) {
-      __syncwarp();
-      for (int s = 0; s < a.k; ++s) {
-        const int drank = __shfl_sync(0xffffffffu, my_rank, s);
-        const int drow = __shfl_sync(0xffffffffu, my_row, s);
-        if (drow < 0) continue;
-        float* sd = reinterpret_cast<float*>(h.window[drank] + a.scale_off) + static_cast<size_t>(drow) * groups;
-        for (int g = lane; g < groups; g += 32) sd[g] = scale_buf[warp][g];
+      __syncthreads();
+      for (int i = team.thread(); live && i < a.k * groups; i += team.warps * 32) {
+        const int s = i / groups, g = i - s * groups;
+        if (slot_row[s] >= 0)
+          reinterpret_cast<float*>(h.window[slot_rank[s]] + a.scale_off)[static_cast<size_t>(slot_row[s]) * groups + g] = scale_buf[g];
       }
-      __syncwarp();
     }
   }
   if (!last_cta_done(a.done)) return;
@@ -364,30 +402,35 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
   }
   // ---- ... and every CTA waits for all ranks' rows before it reduces its share of the tokens
   if (!moe_wait_all(h, 2, a.epoch)) return;
-  // One CTA per token: its threads read 4 KiB of each of the token's rows at a time. With a warp per
+  // A team per token: from 2048 elements on it reads 4 KiB of each of the token's rows at a time. With a warp per
   // token every row is visited 512 bytes at a time by thousands of warps at once: 4096 tokens x 7168,
   // top-8, one rank took 194 us that way (314 with eight loads in flight per warp instead of four)
-  // and take 138 now, on average over the forward call, which copies the cells, and the backward call,
+  // and take 140 now, on average over the forward call, which copies the cells, and the backward call,
   // which does not; 299 when every row went through its cell in the window. Four cells' loads are issued
   // together and added in the order of the slots.
   uint4* comb = reinterpret_cast<uint4*>(h.window[h.rank] + a.comb_off);
-  __shared__ float slot_w[MOE_MAX_TOPK];
-  __shared__ int slot_row[MOE_MAX_TOPK];   // row of y, -1: the cell in the window, -2: never sent
-  for (int t = blockIdx.x; t < a.T; t += gridDim.x) {
-    __syncthreads();   // the slots of the token before have been read
-    if (static_cast<int>(threadIdx.x) < a.k) {
-      const int i = t * a.k + threadIdx.x;
+  const TokenTeam team(a.H);
+  __shared__ float team_w[TokenTeam::WARPS][MOE_MAX_TOPK];
+  __shared__ int team_row[TokenTeam::WARPS][MOE_MAX_TOPK];   // row of y, -1: the cell in the window, -2: never sent
+  float* slot_w = team_w[team.team];
+  int* slot_row = team_row[team.team];
+  for (int t0 = blockIdx.x * team.teams; t0 < a.T; t0 += gridDim.x * team.teams) {
+    const int t = t0 + team.team;
+    const bool on = t < a.T;
+    __syncthreads();   // the slots of the tokens before have been read
+    if (on && team.thread() < a.k) {
+      const int i = t * a.k + team.thread();
       int row = a.row_of[i] < 0 ? -2 : a.local_row[i];
       if (row >= rows) {
         gin_record_error(h, DEV_ERR_BOUNDS);
         row = -2;
       }
-      slot_row[threadIdx.x] = row;
-      slot_w[threadIdx.x] = a.topk_w ? a.topk_w[i] : 1.f;
+      slot_row[team.thread()] = row;
+      slot_w[team.thread()] = a.topk_w ? a.topk_w[i] : 1.f;
     }
     __syncthreads();
     constexpr int U = 4;
-    for (int v = threadIdx.x; v < vec; v += MOE_THREADS) {
+    for (int v = team.thread(); on && v < vec; v += team.warps * 32) {
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       for (int s0 = 0; s0 < a.k; s0 += U) {
         uint4 q[U];
@@ -561,7 +604,9 @@ int b200_moe_dispatch(int comm, const void* x, const void* topk_idx, const void*
                  static_cast<const float*>(topk_w), T, k, H, E, fp8, use_saved_rows, scale_by_weight,
                  static_cast<const int32_t*>(dest_base), static_cast<int32_t*>(cursor), static_cast<int32_t*>(row_of),
                  static_cast<int32_t*>(local_row), static_cast<__nv_bfloat16*>(local_out), recv_off, scale_off, meta_off, capacity_rows, static_cast<unsigned int*>(done), ++g_moe_epoch[comm][1]};
-  moe_dispatch_kernel<<<moe_grid(T), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  const int per_cta = TokenTeam::WARPS / TokenTeam::warps_for(H);
+  const int cap = sm_count() * 4, grid = (T + per_cta - 1) / per_cta;
+  moe_dispatch_kernel<<<grid < cap ? grid : cap, MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
