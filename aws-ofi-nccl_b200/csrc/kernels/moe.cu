@@ -13,9 +13,10 @@
 //  moe_combine  : every expert-output row travels back to its source token's (token, slot) cell;
 //                 when all ranks have delivered, the source sums its k cells, gate-weighted.
 //
-// Rows that stay on their rank need no mailbox: dispatch can store them straight into the tensor that
-// the experts read (moe_collect_rows adds what came through the window), and combine sums them from
-// the expert outputs.
+// Rows that stay on their rank need not be read back from the window: dispatch can store them into the
+// tensor that the experts read as well (moe_collect_rows adds what other ranks sent), and combine sums
+// them from the expert outputs. The window holds every row and every cell after each call all the same,
+// since its views are part of the interface.
 //
 // The reference moves such traffic as host-proxied RDMA writes with immediate data and signal
 // atomics (reference: src/rdma/gin/nccl_ofi_gin.cpp, nccl_ofi_gin_resources.cpp); here the GPU
@@ -141,7 +142,7 @@ struct DispatchArgs {
   int32_t* cursor;           // [E]
   int32_t* row_of;           // [T][k] receive-buffer row of every (token, slot); -1 = dropped
   int32_t* local_row;        // [T][k] the same row where this rank owns the expert, else -1 (written with row_of)
-  __nv_bfloat16* local_out;  // bf16 payload: rows of this rank's own tokens go here instead of the window, or null
+  __nv_bfloat16* local_out;  // bf16 payload: rows of this rank's own tokens go here as well, or null
   size_t recv_off, scale_off, meta_off;  // window offsets on the receiving side
   int capacity_rows;
   unsigned int* done;
@@ -195,7 +196,8 @@ __device__ __forceinline__ uint2 quantize8(const float (&v)[8], float w, float& 
 
 // A team per token: from 2048 elements on it writes one destination row 2 KiB (fp8) or 4 KiB (bf16) at a time,
 // where a warp per token left every row 256 or 512 bytes at a time among thousands of others (4096 tokens x
-// 7168, top-8: 92 us on average over the fp8 and the weighted bf16 call, 86 now).
+// 7168, top-8: 92 us on average over the fp8 and the weighted bf16 call, 86 so; 141 with local_out, which
+// doubles the stores of the bf16 call and saves reading the window back).
 __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs a) {
   const GinDevHandle& h = a.h;
   const TokenTeam team(a.H);
@@ -278,9 +280,10 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
         const int drank = slot_rank[s], drow = slot_row[s];
         const float w = slot_w[s];
         if (drow < 0) continue;  // uniform over the team
-        uint8_t* dst = a.local_out && drank == h.rank
-                           ? reinterpret_cast<uint8_t*>(a.local_out) + static_cast<size_t>(drow) * row_bytes
-                           : h.window[drank] + a.recv_off + static_cast<size_t>(drow) * row_bytes;
+        uint8_t* dst = h.window[drank] + a.recv_off + static_cast<size_t>(drow) * row_bytes;
+        uint4* own = a.local_out && drank == h.rank   // bf16 only (the launcher checks)
+                         ? reinterpret_cast<uint4*>(a.local_out) + static_cast<size_t>(drow) * (a.H / 8)
+                         : nullptr;
         if (a.fp8) {
           if (weighted) {
             q = quantize8(v, w, scale);
@@ -288,13 +291,15 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
               reinterpret_cast<float*>(h.window[drank] + a.scale_off)[static_cast<size_t>(drow) * groups + 2 * c + (lane >> 4)] = scale;
           }
           reinterpret_cast<uint2*>(dst)[c * 32 + lane] = q;
-        } else if (!weighted) {
-          reinterpret_cast<uint4*>(dst)[c * 32 + lane] = raw;
         } else {
-          __nv_bfloat162 r[4];
+          uint4 r = raw;
+          if (weighted) {
+            __nv_bfloat162* rp = reinterpret_cast<__nv_bfloat162*>(&r);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) r[j] = __floats2bfloat162_rn(v[2 * j] * w, v[2 * j + 1] * w);
-          reinterpret_cast<uint4*>(dst)[c * 32 + lane] = *reinterpret_cast<const uint4*>(r);
+            for (int j = 0; j < 4; ++j) rp[j] = __floats2bfloat162_rn(v[2 * j] * w, v[2 * j + 1] * w);
+          }
+          reinterpret_cast<uint4*>(dst)[c * 32 + lane] = r;
+          if (own) own[c * 32 + lane] = r;
         }
       }
     }
@@ -358,7 +363,6 @@ struct CombineArgs {
   const float* topk_w;             // [T][k] on the source, or null for an unweighted sum
   const int32_t* row_of;           // [T][k] on the source: cells whose row is < 0 were never sent
   const int32_t* local_row;        // [T][k] row of y for the cells whose expert is on the source itself, else -1
-  int keep_cells;                  // 1: the window's cells of those rows are filled too
   __nv_bfloat16* cells_out;        // [T][k][H] a copy of every sent cell, or null
   int T, k, H;
   __nv_bfloat16* out;              // [T][H]
@@ -405,9 +409,10 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
   // A team per token: from 2048 elements on it reads 4 KiB of each of the token's rows at a time. With a warp per
   // token every row is visited 512 bytes at a time by thousands of warps at once: 4096 tokens x 7168,
   // top-8, one rank took 194 us that way (314 with eight loads in flight per warp instead of four)
-  // and take 140 now, on average over the forward call, which copies the cells, and the backward call,
-  // which does not; 299 when every row went through its cell in the window. Four cells' loads are issued
-  // together and added in the order of the slots.
+  // and 140 so, before the stores to the window's cells: 215 with them, on average over the forward call,
+  // which copies the cells out as well, and the backward call, which does not; 299 (and 150 for the copy)
+  // when every row was read back from its cell. Four cells' loads are issued together and added in the
+  // order of the slots.
   uint4* comb = reinterpret_cast<uint4*>(h.window[h.rank] + a.comb_off);
   const TokenTeam team(a.H);
   __shared__ float team_w[TokenTeam::WARPS][MOE_MAX_TOPK];
@@ -446,7 +451,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
         for (int u = 0; u < U; ++u) {
           if (row[u] == -2) continue;
           const size_t cell = (static_cast<size_t>(t) * a.k + s0 + u) * vec + v;
-          if (row[u] >= 0 && a.keep_cells) comb[cell] = q[u];
+          if (row[u] >= 0) comb[cell] = q[u];   // what another rank sent is there already
           if (a.cells_out) reinterpret_cast<uint4*>(a.cells_out)[cell] = q[u];
           const float ws = slot_w[s0 + u];
           const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q[u]);
@@ -629,8 +634,8 @@ int b200_moe_collect_rows(int comm, const void* rows_ptr, size_t recv_off, size_
 // Collective. Every CTA of this kernel waits for the other ranks, so the grid is limited to what
 // is resident at once.
 int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int experts_local, size_t meta_off, size_t comb_off,
-                     const void* topk_w, const void* row_of, const void* local_row, int keep_cells, void* cells_out, int T, int k,
-                     int H, void* out, void* done, void* stream) {
+                     const void* topk_w, const void* row_of, const void* local_row, void* cells_out, int T, int k, int H,
+                     void* out, void* done, void* stream) {
   ensure_context();
   const GinDevHandle* hp = comm_handle(comm);
   if (!hp || comm < 0 || comm >= 64) return B200_ERR_BAD_ARG;
@@ -639,7 +644,7 @@ int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int ex
   if (comb_off % 16 || comb_off + static_cast<size_t>(T) * k * H * 2 > h.window_bytes) return B200_ERR_BAD_ARG;
   CombineArgs a{h, static_cast<const __nv_bfloat16*>(y), static_cast<const int32_t*>(expert_offsets), experts_local, meta_off,
                 comb_off, static_cast<const float*>(topk_w), static_cast<const int32_t*>(row_of),
-                static_cast<const int32_t*>(local_row), keep_cells, static_cast<__nv_bfloat16*>(cells_out), T, k, H,
+                static_cast<const int32_t*>(local_row), static_cast<__nv_bfloat16*>(cells_out), T, k, H,
                 static_cast<__nv_bfloat16*>(out), static_cast<unsigned int*>(done), ++g_moe_epoch[comm][2]};
   int per_sm = 0;
   B200_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_combine_kernel, MOE_THREADS, 0));

@@ -28,7 +28,7 @@ _lib.register("b200_moe_route", [_i, _vp, _i, _i, _i, _sz, _vp, _vp, _vp, _vp, _
 _lib.register("b200_moe_dispatch", [_i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _sz, _sz, _sz,
                                     _i, _vp, _vp], _i)
 _lib.register("b200_moe_collect_rows", [_i, _vp, _sz, _sz, _i, _i, _i, _vp, _vp], _i)
-_lib.register("b200_moe_combine", [_i, _vp, _vp, _i, _sz, _sz, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _vp, _vp, _vp], _i)
+_lib.register("b200_moe_combine", [_i, _vp, _vp, _i, _sz, _sz, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp], _i)
 _lib.register("b200_moe_combine_wgrad", [_vp, _vp, _vp, _vp, _i, _i, _i, _vp], _i)
 _lib.register("b200_fp8_dequant_rows", [_vp, _vp, _vp, _vp, _i, _i, _i, _vp], _i)
 
@@ -71,7 +71,8 @@ class ExpertParallel:
         return (_align(2 * world * experts * 4) + _align(cap * hidden * 2) + _align(cap * (hidden // 128) * 4) +
                 _align(cap * 16) + _align(tokens * topk * hidden * 2) + 8192)
 
-    # ---- views of the receive side
+    # ---- views of the receive side: what the last dispatch (the last combine, for the cells) left there,
+    # be it a raw call, a differentiable one or the backward pass of one
     def recv_rows(self, fp8: bool) -> torch.Tensor:
         if fp8:
             return self.comm.local[self.recv_off:self.recv_off + self.capacity * self.H].view(self.capacity, self.H)
@@ -102,7 +103,7 @@ class ExpertParallel:
                      use_saved_rows: bool = False, scale_by_weight: bool = False,
                      local_out: torch.Tensor | None = None) -> None:
         """With ``local_out`` (bf16 payload, [capacity, H]) the rows of this rank's own tokens are stored
-        there instead of in the window; ``collect`` adds the others."""
+        there as well as in the window; ``collect`` adds the others."""
         assert x.shape == (self.T, self.H) and x.dtype == torch.bfloat16 and x.is_contiguous()
         rc = _lib.load().b200_moe_dispatch(
             self.comm.id, x.data_ptr(), topk_idx.data_ptr(), topk_w.data_ptr() if topk_w is not None else None,
@@ -121,21 +122,20 @@ class ExpertParallel:
         return out
 
     def _dispatch_rows(self, x, topk_idx, topk_w, **kw) -> torch.Tensor:
-        """bf16 dispatch into a tensor of its own: no row is copied that need not cross to another rank."""
+        """bf16 dispatch into a tensor of its own: this rank's rows are not read back from the window."""
         rows = torch.empty(self.capacity, self.H, device=x.device, dtype=torch.bfloat16)
         self.dispatch_raw(x, topk_idx, topk_w, fp8=False, local_out=rows, **kw)
         return self.collect(rows, True)
 
     def combine_raw(self, y_rows: torch.Tensor, topk_w: torch.Tensor | None, out: torch.Tensor,
-                    cells_out: torch.Tensor | None = None, keep_cells: bool = True) -> None:
-        """``cells_out`` [T, k, H] receives a copy of every sent cell; without ``keep_cells`` the window's
-        combine cells are filled only where the expert is on another rank."""
+                    cells_out: torch.Tensor | None = None) -> None:
+        """``cells_out`` [T, k, H] receives a copy of every sent cell."""
         assert y_rows.dtype == torch.bfloat16 and y_rows.is_contiguous() and y_rows.shape[1] == self.H
         assert out.shape == (self.T, self.H) and out.dtype == torch.bfloat16 and out.is_contiguous()
         rc = _lib.load().b200_moe_combine(
             self.comm.id, y_rows.data_ptr(), self.expert_offsets.data_ptr(), self.experts_local, self.meta_off,
             self.comb_off, topk_w.data_ptr() if topk_w is not None else None, self.row_of.data_ptr(),
-            self.local_row.data_ptr(), int(keep_cells), cells_out.data_ptr() if cells_out is not None else None, self.T, self.k,
+            self.local_row.data_ptr(), cells_out.data_ptr() if cells_out is not None else None, self.T, self.k,
             self.H, out.data_ptr(), self._done[2:].data_ptr(), _lib.stream_ptr())
         _lib.check(rc, "b200_moe_combine")
 
@@ -175,7 +175,7 @@ class _Dispatch(torch.autograd.Function):
     def backward(ctx, d_rows):
         ep = ctx.ep
         dx = torch.empty(ep.T, ep.H, device=d_rows.device, dtype=torch.bfloat16)
-        ep.combine_raw(d_rows.contiguous(), None, dx, keep_cells=False)   # unweighted sum of the k row gradients of each token
+        ep.combine_raw(d_rows.contiguous(), None, dx)   # unweighted sum of the k row gradients of each token
         return dx, None, None, None, None
 
 
@@ -185,7 +185,7 @@ class _Combine(torch.autograd.Function):
         out = torch.empty(ep.T, ep.H, device=y_rows.device, dtype=torch.bfloat16)
         w = topk_w.detach().float().contiguous()
         cells = torch.empty(ep.T, ep.k, ep.H, device=y_rows.device, dtype=torch.bfloat16)
-        ep.combine_raw(y_rows.contiguous(), w, out, cells_out=cells, keep_cells=False)
+        ep.combine_raw(y_rows.contiguous(), w, out, cells_out=cells)
         ctx.ep = ep
         ctx.n_rows = y_rows.shape[0]
         ctx.save_for_backward(w, cells)

@@ -76,3 +76,29 @@ def test_raw_calls_leave_rows_and_cells_in_the_window(comm):
     ep.combine_raw(ep.recv_rows(False)[: T * k].clone(), None, out)
     assert torch.equal(ep.combine_cells(), x[:, None].expand(T, k, H))
     assert torch.equal(out, (2 * x.float()).bfloat16())
+
+
+@pytest.mark.parametrize("T,H,E,k", [(1, 256, 8, 1), (50, 512, 8, 2), (70, 2304, 16, 3)])
+def test_views_of_the_window_hold_what_the_differentiable_calls_moved(comm, T, H, E, k):
+    from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
+
+    ep = ExpertParallel(comm, T, H, E, k)
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    x, dy = (torch.randn(T, H, device="cuda", generator=g).bfloat16() for _ in range(2))
+    x.requires_grad_(True)
+    w, idx = torch.topk(torch.softmax(torch.randn(T, E, device="cuda", generator=g), -1), k, dim=-1)
+    idx, w = idx.to(torch.int32).contiguous(), w.contiguous().requires_grad_(True)
+    ep.recv_rows(False).fill_(7.0)
+    ep.combine_cells().fill_(7.0)
+    rows = ep.dispatch(x, idx, w)
+    meta = ep.recv_meta()[: T * k].long()
+    token, slot = meta[:, 0], meta[:, 1]
+    assert torch.equal(ep.recv_rows(False)[: T * k], x.detach()[token])
+    assert torch.equal(rows.detach()[: T * k], x.detach()[token])
+    out = ep.combine(rows, w)
+    assert torch.equal(ep.combine_cells(), x.detach()[:, None].expand(T, k, H))
+    out.backward(dy)
+    # the backward pass sends w * dy along the same rows and gathers what came back into the same cells
+    sent = (w.detach()[token, slot][:, None] * dy[token].float()).bfloat16()
+    assert torch.equal(ep.recv_rows(False)[: T * k], sent)
+    assert torch.equal(ep.combine_cells()[token, slot], sent)
