@@ -141,7 +141,7 @@ struct DispatchArgs {
   const int32_t* dest_base;  // [E]
   int32_t* cursor;           // [E]
   int32_t* row_of;           // [T][k] receive-buffer row of every (token, slot); -1 = dropped
-  int32_t* local_row;        // [T][k] the same row where this rank owns the expert, else -1 (written with row_of)
+  int32_t* local_row;        // [T][k] out: the same row where this rank owns the expert, else -1
   __nv_bfloat16* local_out;  // bf16 payload: rows of this rank's own tokens go here as well, or null
   size_t recv_off, scale_off, meta_off;  // window offsets on the receiving side
   int capacity_rows;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
     __syncthreads();   // the slots and scales of the token before have been read
     if (live && team.thread() < a.k) {
       const int slot = team.thread();
-      int my_rank = 0, my_row = -1;
+      int my_rank = -1, my_row = -1;
       const int e = a.topk_idx[t * a.k + slot];
       const float my_w = a.topk_w ? a.topk_w[t * a.k + slot] : 1.f;
       if (e >= 0 && e < a.E) {
@@ -240,7 +240,6 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
             my_row = -1;
           }
           a.row_of[t * a.k + slot] = my_row;
-          a.local_row[t * a.k + slot] = my_rank == h.rank ? my_row : -1;
         }
         if (my_row >= 0) {
           MoeMeta m{t, slot, my_w, h.rank};
@@ -249,8 +248,9 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
         }
       } else if (!a.use_saved_rows) {
         a.row_of[t * a.k + slot] = -1;
-        a.local_row[t * a.k + slot] = -1;
       }
+      // saved rows too: a program that keeps row_of of several routings puts back the one it continues with
+      a.local_row[t * a.k + slot] = my_rank == h.rank ? my_row : -1;
       slot_rank[slot] = my_rank;
       slot_row[slot] = my_row;
       slot_w[slot] = my_w;

@@ -61,7 +61,7 @@ class ExpertParallel:
         self.cursor = torch.zeros(experts, device=dev, dtype=torch.int32)
         self.expert_offsets = torch.zeros(self.experts_local + 1, device=dev, dtype=torch.int32)
         self.row_of = torch.full((tokens, topk), -1, device=dev, dtype=torch.int32)
-        self.local_row = torch.full((tokens, topk), -1, device=dev, dtype=torch.int32)   # row_of where this rank owns the expert
+        self.local_row = torch.full((tokens, topk), -1, device=dev, dtype=torch.int32)   # row_of where this rank owns the expert, as of the last dispatch
         self._done = torch.zeros(4, device=dev, dtype=torch.int32)
         self._last_topk_idx = None
 

@@ -102,3 +102,25 @@ def test_views_of_the_window_hold_what_the_differentiable_calls_moved(comm, T, H
     sent = (w.detach()[token, slot][:, None] * dy[token].float()).bfloat16()
     assert torch.equal(ep.recv_rows(False)[: T * k], sent)
     assert torch.equal(ep.combine_cells()[token, slot], sent)
+
+
+def test_an_earlier_routing_is_continued_from_its_saved_rows(comm):
+    from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
+
+    T, H, E, k = 60, 256, 16, 2
+    ep = ExpertParallel(comm, T, H, E, k)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    batches = []
+    for _ in range(2):
+        x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+        idx = torch.rand(T, E, device="cuda", generator=g).topk(k, dim=-1).indices.to(torch.int32).contiguous()
+        ep.route(idx)
+        ep.dispatch_raw(x, idx, None, fp8=False)
+        batches.append((x, idx, ep.row_of.clone(), ep.expert_offsets.clone()))
+    x, idx, row_of, offsets = batches[0]
+    ep.row_of.copy_(row_of)
+    ep.expert_offsets.copy_(offsets)
+    ep.dispatch_raw(x, idx, None, fp8=False, use_saved_rows=True)
+    out = torch.empty_like(x)
+    ep.combine_raw(ep.recv_rows(False)[: T * k].clone(), None, out)
+    assert torch.equal(out, (2 * x.float()).bfloat16())
