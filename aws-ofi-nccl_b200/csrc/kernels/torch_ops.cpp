@@ -13,6 +13,8 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+#include <torch/library.h>
 
 #include <atomic>
 
@@ -280,15 +282,41 @@ struct RopeQKV : public Function<RopeQKV> {
   }
 };
 
+Tensor linear(const Tensor& x, const Tensor& w) { return Linear::apply(x, w); }
+variable_list rmsnorm(const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
+  return RMSNorm::apply(x, res, w, eps);
+}
+Tensor swiglu(const Tensor& gu) { return SwiGLU::apply(gu); }
+variable_list rope_qkv(const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S, int64_t nq, int64_t nkv,
+                       int64_t hd) {
+  return RopeQKV::apply(qkv, cos, sin, B, S, nq, nkv, hd);
+}
+
+// The call itself, or under torch.jit.trace the operator of the same name: the tracer records operators,
+// and of the bodies above it would see nothing but the allocation of their outputs.
+template <class R, class... A, class... Args>
+R traced_or_direct(const char* name, R (*fn)(A...), const Args&... args) {
+  if (!torch::jit::tracer::isTracing()) return fn(args...);
+  return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<R(A...)>().call(args...);
+}
+
 }  // namespace
 
+TORCH_LIBRARY(b200ops, m) {
+  m.def("linear(Tensor x, Tensor weight) -> Tensor", linear);
+  m.def("rmsnorm(Tensor x, Tensor? res, Tensor weight, float eps) -> Tensor[]", rmsnorm);
+  m.def("swiglu(Tensor gate_up) -> Tensor", swiglu);
+  m.def("rope_qkv(Tensor qkv, Tensor cos, Tensor sin, int batch, int seq, int heads, int kv_heads, int head_dim) -> Tensor[]",
+        rope_qkv);
+}
+
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  m.def("linear", [](const Tensor& x, const Tensor& w) { return Linear::apply(x, w); });
+  m.def("linear", [](const Tensor& x, const Tensor& w) { return traced_or_direct("b200ops::linear", linear, x, w); });
   m.def("rmsnorm", [](const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
-    return RMSNorm::apply(x, res, w, eps);
+    return traced_or_direct("b200ops::rmsnorm", rmsnorm, x, res, w, eps);
   });
-  m.def("swiglu", [](const Tensor& gu) { return SwiGLU::apply(gu); });
+  m.def("swiglu", [](const Tensor& gu) { return traced_or_direct("b200ops::swiglu", swiglu, gu); });
   m.def("rope_qkv", [](const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S, int64_t nq, int64_t nkv,
-                       int64_t hd) { return RopeQKV::apply(qkv, cos, sin, B, S, nq, nkv, hd); });
+                       int64_t hd) { return traced_or_direct("b200ops::rope_qkv", rope_qkv, qkv, cos, sin, B, S, nq, nkv, hd); });
   m.def("launches", [] { return g_launches.load(std::memory_order_relaxed); });
 }
