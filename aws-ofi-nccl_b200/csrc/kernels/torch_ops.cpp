@@ -58,6 +58,11 @@ std::atomic<int64_t> g_launches{0};
 void require(bool ok, const char* what) {
   if (!ok) raise(PyExc_AssertionError, what);
 }
+// Rows of `width` elements; an empty row is the error that the division is in Python, not a signal.
+int64_t rows_of(const Tensor& t, int64_t width) {
+  if (width == 0) raise(PyExc_ZeroDivisionError, "the last dimension holds no element of a row");
+  return t.numel() / width;
+}
 void check(int rc, const char* what) {
   if (rc == 0) return;
   PyObject* type = PyExc_RuntimeError;
@@ -174,8 +179,8 @@ struct Linear : public Function<Linear> {
 struct RMSNorm : public Function<RMSNorm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const c10::optional<Tensor>& res, const Tensor& weight,
                                double eps) {
+    const int64_t H = x.size(-1), T = rows_of(x, H);
     require(x.is_contiguous() && (!res || res->is_contiguous()), "x and the residual are contiguous");
-    const int64_t H = x.size(-1), T = x.numel() / H;
     Tensor y = at::empty_like(x), h = res ? at::empty_like(x) : x;
     Tensor rstd = at::empty({T}, x.options().dtype(at::kFloat));
     g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -193,7 +198,7 @@ struct RMSNorm : public Function<RMSNorm> {
       const auto saved = ctx->get_saved_variables();
       const Tensor &x = saved[0], &weight = saved[1], &rstd = saved[2];
       const bool has_res = ctx->saved_data["res"].toBool();
-      const int64_t H = x.size(-1), T = x.numel() / H;
+      const int64_t H = x.size(-1), T = rows_of(x, H);
       const Tensor dy = grads[0].contiguous();
       const Tensor dres = has_res ? grads[1].contiguous() : Tensor();
       Tensor dx = at::empty_like(x);
@@ -213,7 +218,7 @@ struct RMSNorm : public Function<RMSNorm> {
 // silu(gate) * up of a [..., 2F] tensor laid out as gate | up
 struct SwiGLU : public Function<SwiGLU> {
   static Tensor forward(AutogradContext* ctx, const Tensor& gu) {
-    const int64_t F = gu.size(-1) / 2, T = gu.numel() / (2 * F);
+    const int64_t F = gu.size(-1) / 2, T = rows_of(gu, 2 * F);
     require(gu.is_contiguous(), "gate_up is contiguous");
     auto shape = gu.sizes().vec();
     shape.back() = F;
@@ -227,7 +232,7 @@ struct SwiGLU : public Function<SwiGLU> {
     return on_engine_thread([&]() -> variable_list {
       const auto saved = ctx->get_saved_variables();
       const Tensor& gu = saved[0];
-      const int64_t F = gu.size(-1) / 2, T = gu.numel() / (2 * F);
+      const int64_t F = gu.size(-1) / 2, T = rows_of(gu, 2 * F);
       const Tensor dout = grads[0].contiguous();
       Tensor dgu = at::empty_like(gu);
       g_launches.fetch_add(1, std::memory_order_relaxed);

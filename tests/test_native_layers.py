@@ -39,3 +39,15 @@ def test_a_traced_layer_computes(name):
         grads.append(torch.autograd.grad([o.float().sum() for o in out], args))
     assert all(torch.equal(a, b) for a, b in zip(*outs))
     assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+@pytest.mark.parametrize("call", [
+    lambda llm: llm.swiglu(torch.empty(4, 0, dtype=torch.bfloat16)),
+    lambda llm: llm.swiglu(torch.empty(4, 1, dtype=torch.bfloat16)),
+    lambda llm: llm.rmsnorm(torch.empty(4, 0, dtype=torch.bfloat16), torch.empty(0, dtype=torch.bfloat16)),
+])
+def test_an_empty_row_is_an_exception(call):
+    from aws_ofi_nccl_b200.ops import llm
+
+    with pytest.raises(ZeroDivisionError):
+        call(llm)
