@@ -613,6 +613,12 @@ __global__ void sumsq_kernel(const bf16* __restrict__ x, int64_t n, float* __res
   if (threadIdx.x == 0) atomicAdd(out, s);
 }
 
+// Rows move as 16-byte vectors: null (an argument left out) or on a 16-byte boundary.
+template <class... P>
+static bool aligned16(const P*... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) == 0;
+}
+
 static inline int grid_for(int64_t work_items, int threads) {
   int64_t b = (work_items + threads - 1) / threads;
   const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
@@ -647,6 +653,7 @@ int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w,
   b200::ensure_context();
   if (H % 8 || H > NORM_THREADS * 8 * 4) return B200_ERR_BAD_ARG;
   if (res && !h_out) return B200_ERR_BAD_ARG;
+  if (!aligned16(x, res, h_out, w, y)) return B200_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto X = static_cast<const bf16*>(x);
   auto R = static_cast<const bf16*>(res);
@@ -669,7 +676,7 @@ int b200_rmsnorm_bwd_partial_rows() {
 int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                      float* dw_partial, void* dw, int accumulate_dw, int T, int H, void* stream) {
   b200::ensure_context();
-  if (H % 8 || H > NORM_THREADS * 8 * 4) return B200_ERR_BAD_ARG;
+  if (H % 8 || H > NORM_THREADS * 8 * 4 || !aligned16(dy, x, w, dres, dx, dw_partial)) return B200_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int grid = sm_count() * 2;
   auto DY = static_cast<const bf16*>(dy);
@@ -692,7 +699,7 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
 
 int b200_swiglu_fwd(const void* gu, void* out, long long T, int F, void* stream) {
   b200::ensure_context();
-  if (F % 8) return B200_ERR_BAD_ARG;
+  if (F % 8 || !aligned16(gu, out)) return B200_ERR_BAD_ARG;
   const int grid = grid_for((T * F / 8 + SWIGLU_U - 1) / SWIGLU_U, 256);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto GU = static_cast<const bf16*>(gu);
@@ -705,7 +712,7 @@ int b200_swiglu_fwd(const void* gu, void* out, long long T, int F, void* stream)
 
 int b200_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, int F, void* stream) {
   b200::ensure_context();
-  if (F % 8) return B200_ERR_BAD_ARG;
+  if (F % 8 || !aligned16(dout, gu, dgu)) return B200_ERR_BAD_ARG;
   auto kern = swiglu_small(T, F) ? swiglu_bwd_kernel<false, unsigned> : swiglu_bwd_kernel<false, int64_t>;
   kern<<<grid_for(T * F / 8, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(dout), static_cast<const bf16*>(gu), static_cast<bf16*>(dgu), T, F);
@@ -714,7 +721,7 @@ int b200_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, in
 }
 int b200_swiglu_bwd_interleaved(const void* dout, const void* gu, void* dgu, long long T, int F, void* stream) {
   b200::ensure_context();
-  if (F % 32) return B200_ERR_BAD_ARG;
+  if (F % 32 || !aligned16(dout, gu, dgu)) return B200_ERR_BAD_ARG;
   auto kern = swiglu_small(T, F) ? swiglu_bwd_kernel<true, unsigned> : swiglu_bwd_kernel<true, int64_t>;
   kern<<<grid_for(T * F / 8, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(dout), static_cast<const bf16*>(gu), static_cast<bf16*>(dgu), T, F);

@@ -74,12 +74,17 @@ void check(int rc, const char* what) {
   }
   raise(type, std::string(what) + " failed with code " + std::to_string(rc));
 }
+bool bf16_cuda(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16; }
+// An incoming gradient as the kernels read it: contiguous and on a 16-byte boundary, whatever view it is.
+Tensor rows16(const Tensor& g) {
+  const Tensor c = g.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+}
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
 // C[M,N] (+)= op(A) op(B); the checks of ops.gemm.gemm
 void gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const Tensor& out, bool accumulate) {
-  require(a.is_cuda() && b.is_cuda() && a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16,
-          "operands are bfloat16 CUDA tensors");
+  require(bf16_cuda(a) && bf16_cuda(b), "operands are bfloat16 CUDA tensors");
   require(a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1, "operands are matrices with contiguous rows");
   const int64_t M = a.size(a_mn ? 1 : 0), K = a.size(a_mn ? 0 : 1), N = b.size(b_mn ? 1 : 0);
   require(b.size(b_mn ? 0 : 1) == K, "reduction dims differ");
@@ -181,6 +186,9 @@ struct RMSNorm : public Function<RMSNorm> {
                                double eps) {
     const int64_t H = x.size(-1), T = rows_of(x, H);
     require(x.is_contiguous() && (!res || res->is_contiguous()), "x and the residual are contiguous");
+    require(bf16_cuda(x) && (!res || (bf16_cuda(*res) && res->numel() == x.numel())),
+            "x and the residual are bfloat16 CUDA tensors of one size");
+    require(bf16_cuda(weight) && weight.is_contiguous() && weight.numel() == H, "the weight is a bfloat16 CUDA tensor of one row");
     Tensor y = at::empty_like(x), h = res ? at::empty_like(x) : x;
     Tensor rstd = at::empty({T}, x.options().dtype(at::kFloat));
     g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -199,11 +207,12 @@ struct RMSNorm : public Function<RMSNorm> {
       const Tensor &x = saved[0], &weight = saved[1], &rstd = saved[2];
       const bool has_res = ctx->saved_data["res"].toBool();
       const int64_t H = x.size(-1), T = rows_of(x, H);
-      const Tensor dy = grads[0].contiguous();
-      const Tensor dres = has_res ? grads[1].contiguous() : Tensor();
+      const Tensor dy = rows16(grads[0]);
+      const Tensor dres = has_res ? rows16(grads[1]) : Tensor();
       Tensor dx = at::empty_like(x);
       const Tensor partial = at::empty({b200_rmsnorm_bwd_partial_rows(), H}, rstd.options());
       const Tensor dw = write_param_grad(weight, [&](const Tensor& out, bool accumulate) {
+        require(bf16_cuda(out) && out.is_contiguous() && out.numel() == H, "the gradient buffer is a bfloat16 CUDA tensor of one row");
         g_launches.fetch_add(2, std::memory_order_relaxed);
         check(b200_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), weight.data_ptr(), rstd.data_ptr<float>(),
                                has_res ? dres.data_ptr() : nullptr, dx.data_ptr(), partial.data_ptr<float>(), out.data_ptr(),
@@ -220,6 +229,7 @@ struct SwiGLU : public Function<SwiGLU> {
   static Tensor forward(AutogradContext* ctx, const Tensor& gu) {
     const int64_t F = gu.size(-1) / 2, T = rows_of(gu, 2 * F);
     require(gu.is_contiguous(), "gate_up is contiguous");
+    require(bf16_cuda(gu) && gu.size(-1) == 2 * F, "gate_up is a bfloat16 CUDA tensor with two halves");
     auto shape = gu.sizes().vec();
     shape.back() = F;
     Tensor out = at::empty(shape, gu.options());
@@ -233,7 +243,7 @@ struct SwiGLU : public Function<SwiGLU> {
       const auto saved = ctx->get_saved_variables();
       const Tensor& gu = saved[0];
       const int64_t F = gu.size(-1) / 2, T = rows_of(gu, 2 * F);
-      const Tensor dout = grads[0].contiguous();
+      const Tensor dout = rows16(grads[0]);
       Tensor dgu = at::empty_like(gu);
       g_launches.fetch_add(1, std::memory_order_relaxed);
       check(b200_swiglu_bwd(dout.data_ptr(), gu.data_ptr(), dgu.data_ptr(), T, static_cast<int>(F), stream()), "swiglu_bwd");

@@ -51,3 +51,75 @@ def test_an_empty_row_is_an_exception(call):
 
     with pytest.raises(ZeroDivisionError):
         call(llm)
+
+
+def test_layers_refuse_what_their_kernels_cannot_read():
+    from aws_ofi_nccl_b200.ops import llm
+
+    def bf(*shape):
+        return torch.zeros(*shape, dtype=torch.bfloat16)
+
+    for call in (lambda: llm.rmsnorm(bf(4, 16), bf(16)),                      # not on a GPU
+                 lambda: llm.rmsnorm(torch.zeros(4, 16), torch.zeros(16)),    # not bfloat16
+                 lambda: llm.swiglu(bf(4, 16)),
+                 lambda: llm.swiglu(torch.zeros(4, 16))):
+        with pytest.raises(AssertionError):
+            call()
+
+
+@pytest.mark.parametrize("name,args", [
+    ("b200_rmsnorm_fwd", lambda p: (p[0], p[1], p[2], p[3], p[4], 64, 4, 64, 1e-5, None)),
+    ("b200_rmsnorm_bwd", lambda p: (p[0], p[1], p[2], 64, p[3], p[4], p[5], 64, 0, 4, 64, None)),
+    ("b200_swiglu_fwd", lambda p: (p[0], p[1], 4, 64, None)),
+    ("b200_swiglu_bwd", lambda p: (p[0], p[1], p[2], 4, 64, None)),
+    ("b200_swiglu_bwd_interleaved", lambda p: (p[0], p[1], p[2], 4, 64, None)),
+])
+def test_entry_points_refuse_a_misaligned_pointer(name, args):
+    """Refused before anything is launched: the addresses are made up."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    if torch.cuda.is_available():
+        pytest.skip("made-up addresses stay off the GPU")
+    fn = getattr(_lib.load(), name)
+    used = []
+    args(type("P", (), {"__getitem__": lambda self, i: used.append(i)})())
+    for bad in set(used):
+        ptrs = [4096 * (i + 1) + (2 if i == bad else 0) for i in range(8)]
+        assert fn(*args(ptrs)) == 10001
+
+
+@pytest.mark.gpu
+def test_gradients_of_any_view_are_taken():
+    """Contiguous gradients that start at an odd element."""
+    from aws_ofi_nccl_b200.ops import llm
+
+    def odd(*shape):
+        n = torch.Size(shape).numel()
+        return torch.randn(n + 1, device="cuda").bfloat16()[1:].view(*shape)
+
+    x, r, w = (torch.randn(*s, device="cuda").bfloat16().requires_grad_(True) for s in ((5, 64), (5, 64), (64,)))
+    gu = torch.randn(5, 64, device="cuda").bfloat16().requires_grad_(True)
+    cases = [(lambda: llm.rmsnorm(x, w, residual=r), (x, r, w), [odd(5, 64), odd(5, 64)]),
+             (lambda: (llm.swiglu(gu),), (gu,), [odd(5, 32)])]
+    for fn, inputs, grads in cases:
+        got = torch.autograd.grad(fn(), inputs, grads)
+        want = torch.autograd.grad(fn(), inputs, [g.clone(memory_format=torch.contiguous_format) for g in grads])
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+def test_layers_refuse_misaligned_and_misshapen_inputs():
+    from aws_ofi_nccl_b200.ops import _lib, llm
+
+    def odd(*shape):
+        n = torch.Size(shape).numel()
+        return torch.zeros(n + 1, device="cuda", dtype=torch.bfloat16)[1:].view(*shape)
+
+    x, w = (torch.zeros(*s, device="cuda", dtype=torch.bfloat16) for s in ((5, 64), (64,)))
+    for call in (lambda: llm.rmsnorm(odd(5, 64), w), lambda: llm.rmsnorm(x, odd(64)), lambda: llm.swiglu(odd(5, 64))):
+        with pytest.raises(_lib.B200OpsError):
+            call()
+    for call in (lambda: llm.rmsnorm(x, w[:56]), lambda: llm.rmsnorm(x, w.float()), lambda: llm.rmsnorm(x, w, residual=x[:4]),
+                 lambda: llm.swiglu(torch.zeros(16, 17, device="cuda", dtype=torch.bfloat16))):
+        with pytest.raises(AssertionError):
+            call()
