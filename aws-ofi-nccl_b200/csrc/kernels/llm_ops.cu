@@ -732,7 +732,9 @@ int b200_swiglu_bwd_interleaved(const void* dout, const void* gu, void* dgu, lon
 int b200_rope(void* x, const float* cs, const float* sn, long long T, int nheads, int hd, long long pitch, int seq,
               int backward, void* stream) {
   b200::ensure_context();
-  if (hd % 4) return B200_ERR_BAD_ARG;
+  if (hd % 4 || reinterpret_cast<uintptr_t>(x) % 4 || (T > 1 && pitch % 2) ||
+      (reinterpret_cast<uintptr_t>(cs) | reinterpret_cast<uintptr_t>(sn)) % 8)
+    return B200_ERR_BAD_ARG;
   rope_kernel<<<grid_for(T * nheads * (hd / 4), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<bf16*>(x), cs, sn, T, nheads, hd, pitch, seq, backward ? -1.f : 1.f);
   B200_CUDA_OK(cudaGetLastError());
@@ -753,7 +755,7 @@ int b200_rope_qkv(void* qkv, long long pitch, void* q, void* k, void* v, const l
     ptrs |= reinterpret_cast<uint64_t>(base[i]);
     steps |= static_cast<uint64_t>(w[i].batch) | static_cast<uint64_t>(w[i].tok) | static_cast<uint64_t>(w[i].head);
   }
-  if (ptrs % 4 || steps % 2) return B200_ERR_BAD_ARG;
+  if (ptrs % 4 || steps % 2 || (reinterpret_cast<uintptr_t>(cs) | reinterpret_cast<uintptr_t>(sn)) % 8) return B200_ERR_BAD_ARG;
   const bool wide = hd % 16 == 0 && ptrs % 16 == 0 && steps % 8 == 0;
   const int grid = grid_for(T * (nq + 2 * nkv) * (hd / 2 / (wide ? 8 : 2)), 256);
   cudaStream_t s = static_cast<cudaStream_t>(stream);

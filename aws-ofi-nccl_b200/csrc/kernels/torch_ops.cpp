@@ -257,9 +257,9 @@ struct RopeQKV : public Function<RopeQKV> {
   static void launch(const Tensor& qkv, const Tensor (&part)[3], const Tensor& cos, const Tensor& sin, int64_t S, bool backward) {
     long long strides[9];
     for (int i = 0; i < 3; ++i)
-      for (int d = 0; d < 3; ++d) strides[3 * i + d] = part[i].stride(d);
+      for (int d = 0; d < 3; ++d) strides[3 * i + d] = part[i].size(d) == 1 ? 0 : part[i].stride(d);   // no step, no alignment
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    check(b200_rope_qkv(qkv.data_ptr(), qkv.stride(0), part[0].data_ptr(), part[1].data_ptr(), part[2].data_ptr(), strides,
+    check(b200_rope_qkv(qkv.data_ptr(), qkv.size(0) == 1 ? 0 : qkv.stride(0), part[0].data_ptr(), part[1].data_ptr(), part[2].data_ptr(), strides,
                         cos.data_ptr<float>(), sin.data_ptr<float>(), qkv.size(0), static_cast<int>(part[0].size(2)),
                         static_cast<int>(part[1].size(2)), static_cast<int>(part[0].size(3)), static_cast<int>(S), backward,
                         stream()),
@@ -286,7 +286,7 @@ struct RopeQKV : public Function<RopeQKV> {
       auto rows = [](const Tensor& g) {
         const bool fits = g.stride(3) == 1 && g.stride(0) % 8 == 0 && g.stride(1) % 8 == 0 && g.stride(2) % 8 == 0 &&
                           reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
-        return fits ? g : g.contiguous();
+        return fits ? g : g.clone(at::MemoryFormat::Contiguous);
       };
       const Tensor part[3] = {rows(grads[0]), rows(grads[1]), rows(grads[2])};
       const int64_t B = part[0].size(0), S = part[0].size(1), hd = part[0].size(3);

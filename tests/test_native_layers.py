@@ -1,5 +1,7 @@
 """The native layers (linear, RMSNorm, SwiGLU, rotary split) as callables: what they refuse, and that
 they can be traced."""
+import ctypes
+
 import pytest
 import torch
 
@@ -90,7 +92,7 @@ def test_entry_points_refuse_a_misaligned_pointer(name, args):
 
 @pytest.mark.gpu
 def test_gradients_of_any_view_are_taken():
-    """Contiguous gradients that start at an odd element."""
+    """Contiguous gradients that start at an odd element, and a batch of one whose stride is odd."""
     from aws_ofi_nccl_b200.ops import llm
 
     def odd(*shape):
@@ -99,8 +101,12 @@ def test_gradients_of_any_view_are_taken():
 
     x, r, w = (torch.randn(*s, device="cuda").bfloat16().requires_grad_(True) for s in ((5, 64), (5, 64), (64,)))
     gu = torch.randn(5, 64, device="cuda").bfloat16().requires_grad_(True)
+    qkv = torch.randn(8, 128, device="cuda").bfloat16().requires_grad_(True)
+    ang = torch.rand(8, 16, device="cuda")
     cases = [(lambda: llm.rmsnorm(x, w, residual=r), (x, r, w), [odd(5, 64), odd(5, 64)]),
-             (lambda: (llm.swiglu(gu),), (gu,), [odd(5, 32)])]
+             (lambda: (llm.swiglu(gu),), (gu,), [odd(5, 32)]),
+             (lambda: llm.rope_qkv(qkv, ang.cos(), ang.sin(), 1, 8, 2, 1, 32), (qkv,),
+              [odd(1, 8, 2, 32), odd(1, 8, 1, 32), torch.randn(300, device="cuda").bfloat16().as_strided((1, 8, 1, 32), (257, 32, 32, 1))])]
     for fn, inputs, grads in cases:
         got = torch.autograd.grad(fn(), inputs, grads)
         want = torch.autograd.grad(fn(), inputs, [g.clone(memory_format=torch.contiguous_format) for g in grads])
@@ -123,3 +129,17 @@ def test_layers_refuse_misaligned_and_misshapen_inputs():
                  lambda: llm.swiglu(torch.zeros(16, 17, device="cuda", dtype=torch.bfloat16))):
         with pytest.raises(AssertionError):
             call()
+
+
+def test_the_rotary_split_refuses_misaligned_tables():
+    from aws_ofi_nccl_b200.ops import _lib
+
+    if torch.cuda.is_available():
+        pytest.skip("made-up addresses stay off the GPU")
+    lib = _lib.load()
+    strides = (ctypes.c_longlong * 9)(64, 32, 32, 64, 32, 32, 64, 32, 32)
+    for cos, sin in ((4096 + 4, 8192), (4096, 8192 + 4)):
+        args = [ctypes.c_void_p(64), ctypes.c_longlong(128), *(ctypes.c_void_p(64 * i) for i in (2, 3, 4)), strides,
+                ctypes.c_void_p(cos), ctypes.c_void_p(sin), ctypes.c_longlong(2)]
+        assert lib.b200_rope_qkv(*args, 1, 1, 32, 2, 0, None) == 10001
+        assert lib.b200_rope(64, cos, sin, 2, 1, 32, 32, 2, 0, None) == 10001
