@@ -41,6 +41,7 @@ using torch::autograd::Function;
 using torch::autograd::variable_list;
 
 std::atomic<int64_t> g_launches{0};
+PyObject* g_error = nullptr;   // the package's B200OpsError (a RuntimeError), looked up when the module is loaded
 
 // Raises a Python exception from either side: in a call from Python (the GIL is held) it travels as
 // error_already_set; on an autograd thread torch's own carrier takes it to the caller of backward().
@@ -64,15 +65,7 @@ int64_t rows_of(const Tensor& t, int64_t width) {
   return t.numel() / width;
 }
 void check(int rc, const char* what) {
-  if (rc == 0) return;
-  PyObject* type = PyExc_RuntimeError;
-  {
-    py::gil_scoped_acquire gil;
-    // the package's own class (a RuntimeError); it lives as long as the module
-    static PyObject* own = py::object(py::module_::import("aws_ofi_nccl_b200.ops._lib").attr("B200OpsError")).release().ptr();
-    type = own;
-  }
-  raise(type, std::string(what) + " failed with code " + std::to_string(rc));
+  if (rc != 0) raise(g_error, std::string(what) + " failed with code " + std::to_string(rc));
 }
 bool bf16_cuda(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16; }
 // An incoming gradient as the kernels read it: contiguous and on a 16-byte boundary, whatever view it is.
@@ -326,6 +319,7 @@ TORCH_LIBRARY(b200ops, m) {
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  g_error = py::object(py::module_::import("aws_ofi_nccl_b200.ops._lib").attr("B200OpsError")).release().ptr();
   m.def("linear", [](const Tensor& x, const Tensor& w) { return traced_or_direct("b200ops::linear", linear, x, w); });
   m.def("rmsnorm", [](const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
     return traced_or_direct("b200ops::rmsnorm", rmsnorm, x, res, w, eps);
