@@ -14,10 +14,12 @@ Targets
 from __future__ import annotations
 
 import concurrent.futures as cf
+import importlib.metadata
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent
@@ -91,13 +93,17 @@ def build_kernels(force: bool = False, extra_flags: list[str] | None = None) -> 
     return out
 
 
+def torch_ops_tag() -> str:
+    """The torch and the Python that _b200torch.so is built for."""
+    return f"torch {importlib.metadata.version('torch')} {sysconfig.get_config_var('SOABI')}"
+
+
 def build_torch_ops(force: bool = False) -> Path:
     """csrc/kernels/torch_ops.cpp -> lib/_b200torch.so: the differentiable layers, linked against torch
-    and against libb200ops.so next to it."""
+    and against libb200ops.so next to it. Built for one torch and one Python, which the stamp beside it names."""
     src, out = CSRC / "kernels" / "torch_ops.cpp", LIB / "_b200torch.so"
-    if force or _stale(out, [src]):
-        import sysconfig
-
+    stamp, tag = LIB / "_b200torch.stamp", torch_ops_tag()
+    if force or _stale(out, [src, src.parent / "b200ops.h"]) or not stamp.exists() or stamp.read_text() != tag:
         import torch
 
         root = Path(torch.__file__).resolve().parent
@@ -106,6 +112,7 @@ def build_torch_ops(force: bool = False) -> Path:
               "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-I", sysconfig.get_paths()["include"],
               "-I", f"{CUDA_HOME}/include", str(src), "-o", str(out), "-L", str(root / "lib"), "-ltorch", "-ltorch_cpu", "-lc10",
               "-lc10_cuda", "-ltorch_python", "-L", str(LIB), "-lb200ops", "-Wl,-rpath,$ORIGIN"])
+        stamp.write_text(tag)
     return out
 
 

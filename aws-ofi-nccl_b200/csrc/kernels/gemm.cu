@@ -9,6 +9,7 @@
 // on the same kernel without materialising a transpose.
 #include <cuda_fp8.h>
 
+#include "b200ops.h"
 #include "gemm_epilogues.cuh"
 #include "gemm_splitk.h"
 #include "gemm_tcgen05.cuh"

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "b200ops.h"
 #include "host_util.h"
 
 namespace b200 {

@@ -18,19 +18,7 @@
 
 #include <atomic>
 
-extern "C" {
-int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
-                   int a_mn, int b_mn, int out_fp32, int accumulate, int bn, int max_ctas, void* stream);
-int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w, void* y, float* rstd, int T, int H, float eps,
-                     void* stream);
-int b200_rmsnorm_bwd_partial_rows();
-int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                     float* dw_partial, void* dw, int accumulate_dw, int T, int H, void* stream);
-int b200_swiglu_fwd(const void* gu, void* out, long long T, int F, void* stream);
-int b200_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, int F, void* stream);
-int b200_rope_qkv(void* qkv, long long pitch, void* q, void* k, void* v, const long long* strides, const float* cs,
-                  const float* sn, long long T, int nq, int nkv, int hd, int seq, int backward, void* stream);
-}
+#include "b200ops.h"
 
 namespace {
 

@@ -41,3 +41,27 @@ def test_bench_reference_arm_reports_unavailable():
                          text=True, check=True).stdout.strip().splitlines()[-1]
     d = json.loads(out)
     assert d["impl"] == "reference" and "unavailable" in d
+
+
+def test_native_layers_are_rebuilt_for_another_torch_or_header(tmp_path, monkeypatch):
+    """What the module was built against decides, not the age of its own source alone."""
+    import os
+
+    from aws_ofi_nccl_b200 import build
+
+    runs = []
+    monkeypatch.setattr(build, "LIB", tmp_path)
+    monkeypatch.setattr(build, "_run", runs.append)
+    out, header = tmp_path / "_b200torch.so", build.CSRC / "kernels" / "b200ops.h"
+    out.write_bytes(b"")
+    (tmp_path / "_b200torch.stamp").write_text(build.torch_ops_tag())
+    build.build_torch_ops()
+    assert not runs                                    # up to date
+    (tmp_path / "_b200torch.stamp").write_text("torch 1.0 another-python")
+    build.build_torch_ops()
+    assert len(runs) == 1                              # another torch
+    build.build_torch_ops()
+    assert len(runs) == 1                              # and the stamp says so
+    os.utime(out, (0, header.stat().st_mtime - 1))
+    build.build_torch_ops()
+    assert len(runs) == 2                              # a signature may have changed
