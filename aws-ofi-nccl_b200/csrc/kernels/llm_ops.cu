@@ -303,52 +303,29 @@ __global__ void __launch_bounds__(256)
 }
 
 // ------------------------------------------------------------------ SwiGLU on a fused [T, 2F] gate|up tensor
-// 1 / (1 + exp(-g)) with the reciprocal unit (relative error 2^-23, subnormal results kept) instead of
-// an IEEE division, whose ten instructions per element outweigh everything else these kernels do.
-__device__ __forceinline__ float sigmoid(float g) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-g)));
-  return r;
-}
 // Element vectors are spread over the grid as (row, vector in the row); the row comes from a 32-bit
-// division where the number of vectors allows it (the launcher checks). Two vectors per thread and pass,
-// so that four 16-byte loads are in flight: 64 us at 4096 x 14336 (5.5 TB/s), from 73 with one vector
-// and IEEE divisions.
-constexpr int SWIGLU_U = 2;
+// division where the number of vectors allows it (the launcher checks): 73 us at 4096 x 14336 (CUDA events
+// around the launch, L2 flushed), 80 with a 64-bit one. One vector per thread and pass: with two, 90 us,
+// since an IEEE division is a sequence that does not interleave with another. The reciprocal unit takes
+// 71 but has twice the division's rounding error.
 template <typename Index>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, int64_t T, int F) {
   const Index nvec = static_cast<Index>(T * F / 8), fv = F / 8;
-  const Index step = static_cast<Index>(gridDim.x) * blockDim.x;
-  for (Index i = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; i < nvec; i += SWIGLU_U * step) {
-    Bf16x8 gv[SWIGLU_U], uv[SWIGLU_U];
+  for (Index k = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; k < nvec; k += static_cast<Index>(gridDim.x) * blockDim.x) {
+    const Index t = k / fv, c = k - t * fv;
+    const Bf16x8* row = reinterpret_cast<const Bf16x8*>(gu) + static_cast<int64_t>(t) * 2 * fv;
+    float g[8], u[8], o[8];
+    unpack8(row[c], g);
+    unpack8(row[fv + c], u);
 #pragma unroll
-    for (int q = 0; q < SWIGLU_U; ++q) {
-      const Index k = i + q * step;
-      if (k < nvec) {
-        const Index t = k / fv, c = k - t * fv;
-        const Bf16x8* row = reinterpret_cast<const Bf16x8*>(gu) + static_cast<int64_t>(t) * 2 * fv;
-        gv[q] = row[c];
-        uv[q] = row[fv + c];
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < SWIGLU_U; ++q) {
-      const Index k = i + q * step;
-      if (k < nvec) {
-        float g[8], u[8], o[8];
-        unpack8(gv[q], g);
-        unpack8(uv[q], u);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoid(g[j]) * u[j];
-        reinterpret_cast<Bf16x8*>(out)[k] = pack8(o);
-      }
-    }
+    for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
+    reinterpret_cast<Bf16x8*>(out)[k] = pack8(o);
   }
 }
 // dgu[T,2F] from dout[T,F] and the saved gate|up. INTERLEAVED: gate and up alternate in blocks of
 // 32 columns (the layout the fused GEMM+SwiGLU epilogue produces) instead of two halves. One vector per
-// thread and pass: three loads and two stores already, and more registers cost resident warps. 95 us at
-// 4096 x 14336 (6.2 TB/s), 105 with IEEE divisions, 112 with two vectors.
+// thread and pass: three loads and two stores already, and more registers cost resident warps (105 -> 112 us
+// with two vectors). 101 us at 4096 x 14336, timed as above; 111 with a 64-bit division for the row.
 template <bool INTERLEAVED, typename Index>
 __global__ void __launch_bounds__(256)
     swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu, int64_t T, int F) {
@@ -371,7 +348,7 @@ __global__ void __launch_bounds__(256)
     unpack8(dv, d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float s = sigmoid(g[j]);
+      const float s = 1.f / (1.f + __expf(-g[j]));
       const float silu = g[j] * s;
       du[j] = d[j] * silu;
       dg[j] = d[j] * u[j] * (s + silu * (1.f - s));
@@ -701,7 +678,7 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
 int b200_swiglu_fwd(const void* gu, void* out, long long T, int F, void* stream) {
   b200::ensure_context();
   if (F % 8 || !aligned16(gu, out)) return B200_ERR_BAD_ARG;
-  const int grid = grid_for((T * F / 8 + SWIGLU_U - 1) / SWIGLU_U, 256);
+  const int grid = grid_for(T * F / 8, 256);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto GU = static_cast<const bf16*>(gu);
   auto O = static_cast<bf16*>(out);
