@@ -246,6 +246,49 @@ static int dispatch_major(const void* A, const void* B, void* C, int M, int N, i
   return launch_gemm<BN, true, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, max_ctas, stream);
 }
 
+static bool gemm_args_ok(const void* A, const void* B, const void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
+                         int out_fp32) {
+  if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return false;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return false;
+  return lda % 8 == 0 && ldb % 8 == 0 && ldc % (out_fp32 ? 4 : 8) == 0;
+}
+
+static bool use_pairs(int M, int N, int max_ctas) {
+  return gemm_pair_mode() != 0 && M >= 256 && N >= 128 && (max_ctas == 0 || max_ctas >= 2);
+}
+
+// What a product with bn = 0 runs on: the tile width of the persistent kernel, or a split along K.
+// `base_offset`: how far the operands' addresses are from a 128-byte line.
+struct GemmChoice {
+  int bn;
+  SplitkPlan split;
+};
+static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, uintptr_t base_offset, int max_ctas) {
+  const bool pairs = use_pairs(M, N, max_ctas);
+  int bn;
+  // Wider tiles re-read A less; fall back to the narrower tile when that fills the SMs better.
+  const int units = pairs ? sm_count() / 2 : sm_count();
+  const long rows = pairs ? (M + 255) / 256 : (M + 127) / 128;
+  const long t256 = rows * ((N + 255) / 256);
+  const long t128 = rows * ((N + 127) / 128);
+  const long w256 = (t256 + units - 1) / units, w128 = (t128 + units - 1) / units;
+  if (pairs) {
+    // With CTA pairs the tile is 256 rows tall and a wave is one tile per pair of SMs. A wave of narrow
+    // tiles costs about 0.56 of one of wide tiles (4096 x 4096 x 14336: seven waves 408 us, four wide ones
+    // 444), but nearly as much where the 128-byte rows of the operand boxes straddle cache lines and L2
+    // delivers the operands late (1000 x 5160 x 2568: three waves 46 us, two wide ones 41;
+    // 4096 x 4096 x 16040: seven 660 us, four wide ones 436).
+    const bool aligned = lda % 64 == 0 && ldb % 64 == 0 && base_offset == 0;
+    bn = (N >= 256 && w256 <= (aligned ? 0.56 : 0.85) * w128) ? 256 : 128;
+  } else {
+    const double eff256 = static_cast<double>(t256) / (w256 * units);
+    const double eff128 = static_cast<double>(t128) / (w128 * units);
+    bn = (N >= 256 && eff256 + 0.08 >= eff128) ? 256 : 128;
+  }
+  // Few tiles and a long K: the chip is filled by splitting K over clusters.
+  return {bn, max_ctas == 0 ? plan_splitk(M, N, K, pairs, bn) : SplitkPlan{1}};
+}
+
 }  // namespace b200
 
 extern "C" {
@@ -257,39 +300,14 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
                    void* stream) {
   b200::ensure_context();
   using namespace b200;
-  if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return B200_ERR_BAD_ARG;
-  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15)
-    return B200_ERR_BAD_ARG;
-  if ((lda % 8) || (ldb % 8) || (ldc % (out_fp32 ? 4 : 8))) return B200_ERR_BAD_ARG;
+  if (!gemm_args_ok(A, B, C, M, N, K, lda, ldb, ldc, out_fp32)) return B200_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool pairs = gemm_pair_mode() != 0 && M >= 256 && N >= 128 && (max_ctas == 0 || max_ctas >= 2);
+  const bool pairs = use_pairs(M, N, max_ctas);
   if (bn == 0) {
-    // Wider tiles re-read A less; fall back to the narrower tile when that fills the SMs better.
-    const int units = pairs ? sm_count() / 2 : sm_count();
-    const long rows = pairs ? (M + 255) / 256 : (M + 127) / 128;
-    const long t256 = rows * ((N + 255) / 256);
-    const long t128 = rows * ((N + 127) / 128);
-    const long w256 = (t256 + units - 1) / units, w128 = (t128 + units - 1) / units;
-    if (pairs) {
-      // With CTA pairs the tile is 256 rows tall and a wave is one tile per pair of SMs. A wave of narrow
-      // tiles costs about 0.56 of one of wide tiles (4096 x 4096 x 14336: seven waves 408 us, four wide ones
-      // 444), but nearly as much where the 128-byte rows of the operand boxes straddle cache lines and L2
-      // delivers the operands late (1000 x 5160 x 2568: three waves 46 us, two wide ones 41;
-      // 4096 x 4096 x 16040: seven 660 us, four wide ones 436).
-      const bool aligned = lda % 64 == 0 && ldb % 64 == 0 &&
-                           ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 127) == 0;
-      bn = (N >= 256 && w256 <= (aligned ? 0.56 : 0.85) * w128) ? 256 : 128;
-    } else {
-      const double eff256 = static_cast<double>(t256) / (w256 * units);
-      const double eff128 = static_cast<double>(t128) / (w128 * units);
-      bn = (N >= 256 && eff256 + 0.08 >= eff128) ? 256 : 128;
-    }
-    // Few tiles and a long K: the chip is filled by splitting K over clusters.
-    if (max_ctas == 0) {
-      const SplitkPlan plan = plan_splitk(M, N, K, pairs, bn);
-      if (plan.slices > 1)
-        return launch_splitk({A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate}, pairs, plan, s);
-    }
+    const GemmChoice g = choose_gemm(M, N, K, lda, ldb, (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 127, max_ctas);
+    if (g.split.slices > 1)
+      return launch_splitk({A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate}, pairs, g.split, s);
+    bn = g.bn;
   }
   if (pairs) {
     if (bn == 256)
@@ -307,6 +325,32 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
   return out_fp32 ? dispatch_major<128, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, max_ctas, s)
                   : dispatch_major<128, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate,
                                                        max_ctas, s);
+}
+
+// What b200_gemm_bf16 with bn = 0 and max_ctas = 0 runs on for operands on cache-line boundaries: CTA pairs
+// or single CTAs, slices of K (1: the persistent kernel) and its tile width.
+int b200_gemm_plan(int M, int N, int K, long long lda, long long ldb, int* pair, int* bn, int* slices) {
+  b200::ensure_context();
+  using namespace b200;
+  if (M <= 0 || N <= 0 || K <= 0 || !pair || !bn || !slices) return B200_ERR_BAD_ARG;
+  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, 0, 0);
+  *pair = use_pairs(M, N, 0);
+  *slices = g.split.slices;
+  *bn = g.split.slices > 1 ? 128 : g.bn;
+  return 0;
+}
+
+// b200_gemm_bf16 on the split kernel whatever the plan says: slices 2, 4 or 8 (with pair at most 4) and no
+// more than K has 64-deep blocks.
+int b200_gemm_bf16_split(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                         long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate, int pair, int slices, void* stream) {
+  b200::ensure_context();
+  using namespace b200;
+  if (!gemm_args_ok(A, B, C, M, N, K, lda, ldb, ldc, out_fp32)) return B200_ERR_BAD_ARG;
+  if ((slices != 2 && slices != 4 && slices != 8) || slices * (pair ? 2 : 1) > 8 || (K + GEMM_BK - 1) / GEMM_BK < slices)
+    return B200_ERR_BAD_ARG;
+  return launch_splitk({A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate}, pair != 0, SplitkPlan{slices},
+                       static_cast<cudaStream_t>(stream));
 }
 
 // C[M,N] (bf16) = (A8[M,K] * B8[N,K]^T) * a_scale[M] x b_scale[N]; A8, B8 e4m3, K-major, K % 16 == 0.

@@ -33,10 +33,14 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
 }
 
 constexpr int SPLITK_MAX_CLUSTER = 8;   // portable cluster size
+// Tile width. Wider tiles have half the CTAs and twice the partial sums to join: at no size of 16 to 1024
+// rows, 64 to 4096 columns and K from 256 to 14336 were they the faster split.
+constexpr int SPLITK_BN = 128;
 
 // Operand stages of a member CTA: the same as the persistent kernels' (Gemm2Smem / GemmSmem).
-template <bool PAIR, int BN>
+template <bool PAIR>
 struct SplitkSmem {
+  static constexpr int BN = SPLITK_BN;
   static constexpr int STAGE_BYTES = PAIR ? Gemm2Smem<BN>::STAGE_BYTES : GemmSmem<BN>::STAGE_BYTES;
   static constexpr int STAGES = PAIR ? Gemm2Smem<BN>::STAGES : GemmSmem<BN>::STAGES;
   static constexpr int A_BYTES = 128 * GEMM_BK * 2;
@@ -48,11 +52,12 @@ struct SplitkSmem {
 
 // grid = tiles x cluster size, cluster size = slices x (PAIR ? 2 : 1); shape.tiles_m counts 128-row
 // tiles (256-row tiles with PAIR). 1 <= slices <= number of 64-deep k-blocks.
-template <bool PAIR, int BN, bool A_MN, bool B_MN, typename OutT>
+template <bool PAIR, bool A_MN, bool B_MN, typename OutT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OutT* C, int64_t ldc,
                        GemmShape shape, int slices, int accumulate, int* err_word) {
-  using S = SplitkSmem<PAIR, BN>;
+  using S = SplitkSmem<PAIR>;
+  constexpr int BN = SPLITK_BN;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t crank = cluster_ctarank();

@@ -14,7 +14,6 @@ struct SplitkCall {
 };
 
 struct SplitkPlan {
-  int bn;       // tile width, 128 or 256
   int slices;   // 1: do not split
 };
 

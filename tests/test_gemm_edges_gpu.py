@@ -1,14 +1,16 @@
 """Products with few output tiles and a long reduction (cluster split-K) and the edges of the stored
 tiles, against a product in 64 bits."""
+import ctypes
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-# one 128-row tile / ragged rows and columns; both tile widths; 256-row tiles on CTA pairs; K with a tail
-SPLIT = [(1, 8, 4096), (16, 72, 2056), (128, 4096, 14336), (130, 264, 8200), (256, 128, 4096), (300, 520, 8248), (512, 768, 16384)]
+# one 128-row tile / ragged rows and columns; single CTAs and 256-row tiles on CTA pairs; K with a tail
+SPLIT = [(1, 8, 4096), (128, 4096, 14336), (130, 264, 8200), (256, 128, 4096), (300, 520, 8248), (512, 768, 16384), (1000, 1000, 8200)]
 # no split: edges of the 64-column and 32-row slabs that the epilogue stores
-WHOLE = [(33, 72, 64), (129, 200, 136), (257, 328, 72), (2000, 1032, 128)]
+WHOLE = [(16, 72, 2056), (33, 72, 64), (129, 200, 136), (257, 328, 72), (2000, 1032, 128)]
 
 
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
@@ -37,6 +39,59 @@ def test_product_and_accumulation(M, N, K, out_dtype, a_mn, b_mn):
     want = first + ref
     assert ((out.double() - want).abs() <= bound + step * want.abs() + 2.0 ** -24 * (first.abs() + mag)).all()
     assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
+
+
+def _plan(M, N, K, a_mn=False, b_mn=False):
+    """(pair, tile width, slices) of the automatic choice."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    out = [ctypes.c_int() for _ in range(3)]
+    lda, ldb = ctypes.c_longlong(M if a_mn else K), ctypes.c_longlong(N if b_mn else K)
+    assert _lib.load().b200_gemm_plan(M, N, K, lda, ldb, *(ctypes.byref(o) for o in out)) == 0
+    return tuple(o.value for o in out)
+
+
+def test_the_listed_sizes_take_the_path_that_they_are_listed_for():
+    assert all(_plan(*s)[2] > 1 for s in SPLIT) and all(_plan(*s)[2] == 1 for s in WHOLE)
+    assert {_plan(*s)[::2] for s in SPLIT} == {(0, 4), (0, 8), (1, 2), (1, 4)}
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 1024), (512, 1024, 2048), (128, 4096, 1024), (768, 1536, 2048)])
+def test_a_short_reduction_is_not_split(M, N, K):
+    """Products that a split made up to 1.4 times slower."""
+    assert _plan(M, N, K)[2] == 1
+
+
+@pytest.mark.parametrize("pair,slices", [(0, 2), (0, 4), (0, 8), (1, 2), (1, 4)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_every_split_kernel(pair, slices, a_mn, b_mn, out_dtype):
+    """Each member, major and output, asked for by name: ragged rows, columns and K, fewer blocks of K than
+    a slice's pipeline has stages, one block per slice."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    ll = ctypes.c_longlong
+    step = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -24
+    for M, N, K in ((8, 16, 64 * slices), (264, 200, 1096), (520, 136, 2056)):
+        g = torch.Generator(device="cuda").manual_seed(M + slices)
+        a = torch.randn((K, M) if a_mn else (M, K), device="cuda", generator=g).bfloat16()
+        b = torch.randn((K, N) if b_mn else (N, K), device="cuda", generator=g).bfloat16()
+        A, B = (a.T if a_mn else a).double(), (b if b_mn else b.T).double()
+        ref, mag = A @ B, A.abs() @ B.abs()
+        pad = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=out_dtype)
+        want = torch.zeros_like(ref)
+        for accumulate in (0, 1):
+            rc = _lib.load().b200_gemm_bf16_split(
+                ctypes.c_void_p(a.data_ptr()), ctypes.c_void_p(b.data_ptr()), ctypes.c_void_p(pad.data_ptr()), M, N, K,
+                ll(a.stride(0)), ll(b.stride(0)), ll(pad.stride(0)), int(a_mn), int(b_mn), int(out_dtype == torch.float32), accumulate,
+                pair, slices, ctypes.c_void_p(_lib.stream_ptr()))
+            assert rc == 0
+            want = want + ref
+            # fp32 sums of K exact products in any order, one rounding of the output
+            bound = K * 2.0 ** -24 * mag + 2 * step * want.abs()
+            assert ((pad[:M, :N].double() - want).abs() <= bound).all()
+            want = pad[:M, :N].double()
+        assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
 
 
 def test_split_sums_are_the_same_every_time_and_on_two_streams():
