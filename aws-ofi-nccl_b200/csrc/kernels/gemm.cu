@@ -258,12 +258,12 @@ static bool use_pairs(int M, int N, int max_ctas) {
 }
 
 // What a product with bn = 0 runs on: the tile width of the persistent kernel, or a split along K.
-// `base_offset`: how far the operands' addresses are from a 128-byte line.
+// `a_at`, `b_at`: the operands' addresses (their alignment counts).
 struct GemmChoice {
   int bn;
   SplitkPlan split;
 };
-static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, uintptr_t base_offset, int max_ctas) {
+static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, uintptr_t a_at, uintptr_t b_at, int max_ctas) {
   const bool pairs = use_pairs(M, N, max_ctas);
   int bn;
   // Wider tiles re-read A less; fall back to the narrower tile when that fills the SMs better.
@@ -277,9 +277,15 @@ static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, uin
     // tiles costs about 0.56 of one of wide tiles (4096 x 4096 x 14336: seven waves 408 us, four wide ones
     // 444), but nearly as much where the 128-byte rows of the operand boxes straddle cache lines and L2
     // delivers the operands late (1000 x 5160 x 2568: three waves 46 us, two wide ones 41;
-    // 4096 x 4096 x 16040: seven 660 us, four wide ones 436).
-    const bool aligned = lda % 64 == 0 && ldb % 64 == 0 && base_offset == 0;
-    bn = (N >= 256 && w256 <= (aligned ? 0.56 : 0.85) * w128) ? 256 : 128;
+    // 4096 x 4096 x 16040: seven 660 us, four wide ones 436). Where one operand straddles none, or every
+    // second row of both straddles none (rows on 64 bytes), it lies between: two wide waves for three
+    // narrow ones are slower (1068 x 3832 x 6432: 70 us, 60), three for five faster (by 3 to 18 %). With a
+    // short K what a tile costs besides its products weighs more, and there are half as many: four wide waves for seven narrow
+    // ones gain 2 to 20 % up to K = 2048 (6286 x 2368 x 640: 21 us, 25).
+    const uintptr_t a_low = a_at | (static_cast<uintptr_t>(lda) * 2), b_low = b_at | (static_cast<uintptr_t>(ldb) * 2);
+    const bool a_lines = a_low % 128 == 0, b_lines = b_low % 128 == 0, halves = (a_low | b_low) % 64 == 0;
+    const double narrow_wave = a_lines && b_lines ? (K <= 2048 ? 0.58 : 0.56) : a_lines || b_lines || halves ? 0.62 : 0.85;
+    bn = (N >= 256 && w256 <= narrow_wave * w128) ? 256 : 128;
   } else {
     const double eff256 = static_cast<double>(t256) / (w256 * units);
     const double eff128 = static_cast<double>(t128) / (w128 * units);
@@ -304,7 +310,7 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool pairs = use_pairs(M, N, max_ctas);
   if (bn == 0) {
-    const GemmChoice g = choose_gemm(M, N, K, lda, ldb, (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 127, max_ctas);
+    const GemmChoice g = choose_gemm(M, N, K, lda, ldb, reinterpret_cast<uintptr_t>(A), reinterpret_cast<uintptr_t>(B), max_ctas);
     if (g.split.slices > 1)
       return launch_splitk({A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate}, pairs, g.split, s);
     bn = g.bn;
@@ -333,7 +339,7 @@ int b200_gemm_plan(int M, int N, int K, long long lda, long long ldb, int* pair,
   b200::ensure_context();
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || !pair || !bn || !slices) return B200_ERR_BAD_ARG;
-  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, 0, 0);
+  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, 0, 0, 0);
   *pair = use_pairs(M, N, 0);
   *slices = g.split.slices;
   *bn = g.split.slices > 1 ? 128 : g.bn;

@@ -62,6 +62,13 @@ def test_a_short_reduction_is_not_split(M, N, K):
     assert _plan(M, N, K)[2] == 1
 
 
+@pytest.mark.parametrize("M,N,K,wide", [(1068, 3832, 6432, False), (744, 8592, 2336, False),   # rows on 64 bytes
+                                        (1000, 5160, 2568, True), (4096, 4096, 16040, True),     # rows anywhere
+                                        (4096, 4096, 14336, False), (6286, 2368, 640, True)])    # rows on cache lines
+def test_tile_width_follows_how_the_rows_lie(M, N, K, wide):
+    assert _plan(M, N, K) == (1, 256 if wide else 128, 1)
+
+
 @pytest.mark.parametrize("pair,slices", [(0, 2), (0, 4), (0, 8), (1, 2), (1, 4)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
