@@ -86,13 +86,15 @@ class _CrossEntropy(torch.autograd.Function):
         return loss.mean(), logits
 
     @staticmethod
-    def backward(ctx, dloss, _unused):
+    def backward(ctx, dloss, dlogits_out):
         (dlogits,) = ctx.saved_tensors
-        unit = getattr(_CrossEntropy, "assume_unit_grad", True)
-        if dloss is None:   # only the logits output was differentiated
-            return (dlogits if unit else torch.zeros_like(dlogits)), None
+        if dlogits_out is not None:
+            raise RuntimeError("cross_entropy overwrites its logits with their gradient: nothing can be differentiated "
+                               "through them afterwards")
+        if dloss is None:   # the loss was not differentiated
+            return None, None
         # dloss is 1.0 in the training loop; avoid a 1 GB multiply in that case
-        if dloss.numel() == 1 and unit:
+        if dloss.numel() == 1 and getattr(_CrossEntropy, "assume_unit_grad", True):
             return dlogits, None
         return dlogits * dloss, None
 

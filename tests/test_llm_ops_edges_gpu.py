@@ -84,3 +84,19 @@ def test_rope_qkv(hd, nq, nkv, layout):
     (d,) = torch.autograd.grad(outs, (qkv,), grads)
     want = torch.cat((turn(grads[0], -1), turn(grads[1], -1), grads[2].double()), 2).view(B * S, -1)
     _within(d, want, BF, 2.0 ** -7)   # the two products of a rotation cancel: an error of one bf16 step of them
+
+
+def test_nothing_is_differentiated_through_overwritten_logits():
+    """Afterwards they hold the loss's gradient: what else is derived from them has no gradient of its own."""
+    from aws_ofi_nccl_b200.ops import llm
+
+    leaf = torch.randn(6, 64, device="cuda").bfloat16().requires_grad_(True)
+    targets = torch.arange(6, device="cuda")
+    logits = leaf * 1.0
+    loss = llm.cross_entropy(logits, targets)
+    with pytest.raises(RuntimeError, match="overwrites"):
+        torch.autograd.grad(logits.float().sum(), leaf, retain_graph=True)
+    with pytest.raises(RuntimeError, match="overwrites"):
+        torch.autograd.grad(loss + logits.float().square().sum(), leaf, retain_graph=True)
+    (d,) = torch.autograd.grad(loss, leaf)
+    assert torch.equal(d, logits.detach())
