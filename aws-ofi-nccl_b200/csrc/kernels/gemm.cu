@@ -30,17 +30,19 @@ int* device_status_word() {
   return words[dev];
 }
 
-// C as the epilogues store it: boxes of 32 rows x 128 bytes.
+// C as the epilogues store it: boxes of 32 rows x 128 bytes. A store clips a row at 16 bytes, not at an
+// element, so the map ends at the last whole vector (a C narrower than one has no use for its map).
 template <typename OutT>
 static int make_tmap_out(CUtensorMap* tm, const void* C, int M, int N, int64_t ldc) {
   if (M == 1) ldc = (static_cast<int64_t>(N) + 7) / 8 * 8;   // a single row may come with any pitch
-  return make_tmap_2d(tm, C, M, N, ldc, 32, 128 / sizeof(OutT), sizeof(OutT), true);
+  const int cols = whole_vectors<OutT>(N);
+  return make_tmap_2d(tm, C, M, cols ? cols : 16 / sizeof(OutT), ldc, 32, 128 / sizeof(OutT), sizeof(OutT), true);
 }
 
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const __grid_constant__ CUtensorMap tmC, const OutT* C, int64_t ldc, GemmShape shape, int accumulate,
+                     const __grid_constant__ CUtensorMap tmC, OutT* C, int64_t ldc, GemmShape shape, int accumulate,
                      int* err_word) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   StoreEpilogue<OutT> epi{&tmC, C, ldc, accumulate, {}};
@@ -91,7 +93,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
   if (grid > cap) grid = cap;
   int* err = device_status_word();
-  kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<const OutT*>(C), ldc, shape, accumulate, err);
+  kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -100,7 +102,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                          const __grid_constant__ CUtensorMap tmC, const OutT* C, int64_t ldc, GemmShape shape, int accumulate,
+                          const __grid_constant__ CUtensorMap tmC, OutT* C, int64_t ldc, GemmShape shape, int accumulate,
                           int* err_word) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   StoreEpilogue<OutT> epi{&tmC, C, ldc, accumulate, {}};
@@ -139,7 +141,7 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
   int grid = 2 * shape.tiles_m * shape.tiles_n;
   if (grid > cap) grid = cap & ~1;
   int* err = device_status_word();
-  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<const OutT*>(C), ldc, shape, accumulate, err);
+  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -157,10 +159,10 @@ static int dispatch_major_2cta(const void* A, const void* B, void* C, int M, int
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                         const __grid_constant__ CUtensorMap tmC, const float* row_scale, const float* col_scale, GemmShape shape,
-                         int* err_word) {
+                         const __grid_constant__ CUtensorMap tmC, __nv_bfloat16* C, int64_t ldc, const float* row_scale,
+                         const float* col_scale, GemmShape shape, int* err_word) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  ScaledStoreEpilogue epi{&tmC, row_scale, col_scale, {}};
+  ScaledStoreEpilogue epi{&tmC, C, ldc, row_scale, col_scale, {}};
   epi.slab.init(smem_raw, Gemm2Smem<BN>::EPI_OFF);
   NoGate gate;
   gemm_mainloop_2cta<BN, false, false, ScaledStoreEpilogue, NoGate, true>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
@@ -186,7 +188,8 @@ static int launch_gemm_fp8(const void* A, const void* B, const float* a_scale, c
   int grid = 2 * shape.tiles_m * shape.tiles_n;
   const int cap = sm_count() & ~1;
   if (grid > cap) grid = cap;
-  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, a_scale, b_scale, shape, device_status_word());
+  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<__nv_bfloat16*>(C), ldc, a_scale, b_scale,
+                                                                     shape, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -6,7 +6,8 @@
 // K loop costs more than its products. All functors therefore turn their 32 rows x 64 columns through
 // shared memory (16-byte chunks XOR-swizzled by row: no bank conflict) and hand the slab to a TMA
 // store, which writes whole 128-byte row segments, clips the edges of C and leaves the warp free for
-// the next slab while it drains. Kernel times from register stores to TMA stores: the weight gradient
+// the next slab while it drains. It clips a row at 16 bytes: a width that is no multiple of that has
+// its last elements stored from registers (store_row). Kernel times from register stores to TMA stores: the weight gradient
 // 4096 x 14336 of 128 tokens 95 -> 38 us (117 MB stored), the fp8 product 4096 x 14336 x 4096
 // 192 -> 158 us, one 256 x 768 x 256 product 12 -> 7 us.
 #pragma once
@@ -30,8 +31,9 @@ struct SlabStore {
   __device__ __forceinline__ void drain() {
     if ((threadIdx.x & 31) == 0) tma_store_wait<0>();
   }
-  // 32 rows x 128 bytes; lane i passes its row as 32 words.
-  __device__ __forceinline__ void put128(const CUtensorMap* tm, int x, int y, const uint32_t (&w)[32]) {
+  // 32 rows x 128 bytes; lane i passes its row as 32 words. Returns where its row lies in shared memory
+  // (16-byte chunk j at j ^ (lane & 7)); without `store` it only goes there.
+  __device__ __forceinline__ uint32_t put128(const CUtensorMap* tm, int x, int y, const uint32_t (&w)[32], bool store) {
     const int lane = threadIdx.x & 31;
     if (lane == 0) tma_store_wait_read<1>();
     __syncwarp();
@@ -42,12 +44,49 @@ struct SlabStore {
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
-      tma_store_2d(tm, slab, x, y);
+      if (store) tma_store_2d(tm, slab, x, y);
       tma_store_commit();
     }
     which ^= 1u;
+    return slab + lane * 128;
   }
 };
+
+// The columns that TMA stores: whole 16-byte vectors.
+template <typename OutT>
+__host__ __device__ __forceinline__ int whole_vectors(int N) {
+  return N & ~static_cast<int>(16 / sizeof(OutT) - 1);
+}
+
+// The elements of one row from column nv on, less than 16 bytes; `chunk` is where they lie in shared memory.
+// A call of its own, out of the loop that every other width runs.
+template <typename OutT>
+__device__ __noinline__ void store_tail(uint32_t chunk, OutT* dst, int n) {
+  uint32_t v[4];
+  ld_shared_v4(chunk, v);
+#pragma unroll
+  for (int e = 0; e < static_cast<int>(16 / sizeof(OutT)) - 1; ++e) {
+    if (e >= n) break;
+    if constexpr (sizeof(OutT) == 2)
+      reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>(v[e / 2] >> (16 * (e % 2)));
+    else
+      reinterpret_cast<uint32_t*>(dst)[e] = v[e];
+  }
+}
+
+// A warp's 32 rows from `row0` on, 128 bytes of each from column col0 on (w: this lane's row). The map of C
+// ends at whole_vectors(N); what is left of a row beyond it each lane stores itself.
+template <typename OutT>
+__device__ __forceinline__ void store_row(SlabStore& slab, const CUtensorMap* tmC, OutT* C, int64_t ldc, int row0, int col0,
+                                          const uint32_t (&w)[32], const GemmShape& s) {
+  const int nv = whole_vectors<OutT>(s.N);
+  const uint32_t mine = slab.put128(tmC, col0, row0, w, col0 < nv);
+  if (nv == s.N) return;
+  const int lane = threadIdx.x & 31;
+  const int chunk = (nv - col0) * static_cast<int>(sizeof(OutT)) / 16;
+  if (nv < col0 || chunk >= 8 || row0 + lane >= s.M) return;
+  store_tail(mine + ((chunk ^ (lane & 7)) << 4), C + static_cast<int64_t>(row0 + lane) * ldc + nv, s.N - nv);
+}
 
 __device__ __forceinline__ void pack_row64(uint32_t (&w)[32], const uint32_t (&a0)[32], const uint32_t (&a1)[32]) {
 #pragma unroll
@@ -62,7 +101,7 @@ template <typename OutT>
 struct StoreEpilogue {
   static constexpr bool kPair = true;
   const CUtensorMap* tmC;
-  const OutT* C;   // read when accumulating
+  OutT* C;   // read when accumulating
   int64_t ldc;
   int accumulate;
   SlabStore slab;
@@ -107,10 +146,10 @@ struct StoreEpilogue {
     if constexpr (sizeof(OutT) == 2) {
       uint32_t w[32];
       pack_row64(w, a0, a1);
-      slab.put128(tmC, col0, row0, w);
+      store_row(slab, tmC, C, ldc, row0, col0, w, s);
     } else {
-      slab.put128(tmC, col0, row0, a0);
-      if (col0 + 32 < s.N) slab.put128(tmC, col0 + 32, row0, a1);
+      store_row(slab, tmC, C, ldc, row0, col0, a0, s);
+      if (col0 + 32 < s.N) store_row(slab, tmC, C, ldc, row0, col0 + 32, a1, s);
     }
   }
 };
@@ -121,6 +160,8 @@ struct StoreEpilogue {
 struct ScaledStoreEpilogue {
   static constexpr bool kPair = true;
   const CUtensorMap* tmC;
+  __nv_bfloat16* C;
+  int64_t ldc;
   const float* row_scale;   // [M]
   const float* col_scale;   // [N]
   SlabStore slab;
@@ -143,7 +184,7 @@ struct ScaledStoreEpilogue {
     uint32_t w[32];
     scale32(w, a0, rs, col0, s.N);
     scale32(w + 16, a1, rs, col0 + 32, s.N);
-    slab.put128(tmC, col0, row0, w);
+    store_row(slab, tmC, C, ldc, row0, col0, w, s);
   }
 };
 

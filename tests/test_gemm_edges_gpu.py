@@ -116,11 +116,10 @@ def test_split_sums_are_the_same_every_time_and_on_two_streams():
     assert all(torch.equal(o, want) for o in outs)
 
 
-@pytest.mark.parametrize("M,N,K", [(256, 132, 128), (300, 200, 144), (257, 1000, 272)])
+@pytest.mark.parametrize("M,N,K", [(256, 128, 128), (300, 200, 144), (257, 1000, 272)])
 def test_fp8_product_at_ragged_edges(M, N, K):
     from aws_ofi_nccl_b200.ops.gemm import gemm_fp8, quantize_rows_fp8
 
-    N = N // 8 * 8
     xq, xs = quantize_rows_fp8(torch.randn(M, K, device="cuda").bfloat16())
     wq, ws = quantize_rows_fp8(torch.randn(N, K, device="cuda").bfloat16())
     X, W = xq.double() * xs.double()[:, None], wq.double() * ws.double()[:, None]
@@ -128,3 +127,57 @@ def test_fp8_product_at_ragged_edges(M, N, K):
     out = gemm_fp8(xq, wq, xs, ws)
     # bf16 rounding of the result, two fp32 roundings of the scales, fp32 sums
     assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (K + 4) * 2.0 ** -24 * mag).all()
+
+
+def _padded(rows, cols, g):
+    """A [rows, cols] matrix whose pitch is a multiple of 16 bytes."""
+    return torch.randn(rows, (cols + 7) // 8 * 8, device="cuda", generator=g).bfloat16()[:, :cols]
+
+
+@pytest.mark.parametrize("split", [0, 2, 4])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K", [(5, 3, 264), (129, 130, 517), (258, 133, 263), (300, 257, 520), (1030, 389, 261)])
+def test_widths_that_are_no_multiple_of_a_vector(M, N, K, out_dtype, a_mn, b_mn, split):
+    """The stores end in the middle of a 16-byte vector, and nothing beyond is touched."""
+    from aws_ofi_nccl_b200.ops import _lib
+    from aws_ofi_nccl_b200.ops.gemm import gemm
+
+    ll, vp = ctypes.c_longlong, ctypes.c_void_p
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = _padded(*((K, M) if a_mn else (M, K)), g), _padded(*((K, N) if b_mn else (N, K)), g)
+    A, B = (a.T if a_mn else a).double(), (b if b_mn else b.T).double()
+    ref, mag = A @ B, A.abs() @ B.abs()
+    pad = torch.full((M + 1, (N + 15) // 8 * 8), 7.0, device="cuda", dtype=out_dtype)
+    out = pad[:M, :N]
+    step = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -24
+    want = torch.zeros_like(ref)
+    for accumulate in (False, True):
+        if split:
+            rc = _lib.load().b200_gemm_bf16_split(
+                vp(a.data_ptr()), vp(b.data_ptr()), vp(out.data_ptr()), M, N, K, ll(a.stride(0)), ll(b.stride(0)),
+                ll(out.stride(0)), int(a_mn), int(b_mn), int(out_dtype == torch.float32), int(accumulate), int(M >= 256 and N >= 128),
+                split, vp(_lib.stream_ptr()))
+            assert rc == 0
+        else:
+            gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, accumulate=accumulate)
+        want = want + ref
+        # fp32 sums of K exact products in any order, one rounding of the output
+        assert ((out.double() - want).abs() <= K * 2.0 ** -24 * mag + 2 * step * want.abs()).all()
+        want = out.double()
+    assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 132, 128), (257, 300, 272), (515, 260, 144)])
+def test_fp8_widths_that_are_no_multiple_of_a_vector(M, N, K):
+    from aws_ofi_nccl_b200.ops.gemm import gemm_fp8, quantize_rows_fp8
+
+    xq, xs = quantize_rows_fp8(torch.randn(M, K, device="cuda").bfloat16())
+    wq, ws = quantize_rows_fp8(torch.randn(N, K, device="cuda").bfloat16())
+    X, W = xq.double() * xs.double()[:, None], wq.double() * ws.double()[:, None]
+    ref, mag = X @ W.T, X.abs() @ W.T.abs()
+    pad = torch.full((M + 1, (N + 15) // 8 * 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm_fp8(xq, wq, xs, ws, out=pad[:M, :N])
+    # bf16 rounding of the result, two fp32 roundings of the scales, fp32 sums
+    assert ((pad[:M, :N].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (K + 4) * 2.0 ** -24 * mag).all()
+    assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
