@@ -21,7 +21,10 @@ def comm():
         dist.destroy_process_group()
 
 
-@pytest.mark.parametrize("T,H,E,k", [(1, 256, 8, 1), (37, 512, 16, 3), (130, 1280, 64, 5), (64, 2048, 8, 8)])
+# a team of one warp, of several, of the whole CTA with one column step; then rows of several steps (ragged, full,
+# the largest), several tokens per team, several teams of one warp with a ragged last group
+@pytest.mark.parametrize("T,H,E,k", [(1, 256, 8, 1), (37, 512, 16, 3), (130, 1280, 64, 5), (64, 2048, 8, 8),
+                                     (37, 2304, 16, 3), (21, 7168, 64, 8), (9, 8192, 8, 2), (2500, 1280, 16, 2), (10003, 256, 8, 1)])
 @pytest.mark.parametrize("fp8", [False, True])
 def test_roundtrip_and_gradients(comm, T, H, E, k, fp8):
     from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
@@ -124,3 +127,51 @@ def test_an_earlier_routing_is_continued_from_its_saved_rows(comm):
     out = torch.empty_like(x)
     ep.combine_raw(ep.recv_rows(False)[: T * k].clone(), None, out)
     assert torch.equal(out, (2 * x.float()).bfloat16())
+
+
+def test_collect_copies_what_other_ranks_sent(comm):
+    """Records name another rank for half of the rows, as after a dispatch of two ranks."""
+    from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
+
+    T, H, E, k = 700, 768, 8, 2
+    ep = ExpertParallel(comm, T, H, E, k, capacity_factor=1.5)
+    idx = torch.randint(0, E, (T, k), device="cuda", dtype=torch.int32)
+    idx[5:30, 0] = -1   # fewer rows than capacity
+    ep.route(idx)
+    ep.dispatch_raw(torch.randn(T, H, device="cuda").bfloat16(), idx, None, fp8=False)
+    n = int(ep.expert_offsets[-1].item())
+    assert n == T * k - 25 < ep.capacity
+    remote = torch.rand(n, device="cuda") < 0.5
+    ep.recv_meta()[:n, 3] = remote.int()
+    window = ep.recv_rows(False)[:n].clone()
+    own = torch.full((ep.capacity, H), 3.0, device="cuda", dtype=torch.bfloat16)
+    got = ep.collect(own.clone(), True)
+    assert torch.equal(got[:n], torch.where(remote[:, None], window, own[:n])) and (got[n:] == 0).all()
+    got = ep.collect(own.clone(), False)
+    assert torch.equal(got[:n], window) and (got[n:] == 0).all()
+
+
+@pytest.mark.parametrize("T,H,k", [(40, 256, 2), (600, 768, 5), (21, 7168, 8)])
+def test_combine_sums_own_rows_and_delivered_cells(comm, T, H, k):
+    """Half of the cells are planted in the window, as another rank delivers them; the others come from y."""
+    from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
+
+    E = 16
+    ep = ExpertParallel(comm, T, H, E, k)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    idx = torch.rand(T, E, device="cuda", generator=g).topk(k, dim=-1).indices.to(torch.int32).contiguous()
+    ep.route(idx)
+    ep.dispatch_raw(torch.randn(T, H, device="cuda", generator=g).bfloat16(), idx, None, fp8=False)
+    y = torch.randn(T * k, H, device="cuda", generator=g).bfloat16()
+    w = torch.rand(T, k, device="cuda", generator=g)
+    remote = torch.rand(T, k, device="cuda", generator=g) < 0.5
+    delivered = torch.randn(T, k, H, device="cuda", generator=g).bfloat16()
+    cells = torch.where(remote[..., None], delivered, y[ep.row_of.long()])
+    ep.combine_cells().copy_(torch.where(remote[..., None], delivered, torch.full_like(delivered, 9.0)))
+    ep.local_row[remote] = -1
+    out, kept = torch.empty(T, H, device="cuda", dtype=torch.bfloat16), torch.empty_like(cells)
+    ep.combine_raw(y, w, out, cells_out=kept)
+    assert torch.equal(kept, cells) and torch.equal(ep.combine_cells(), cells)
+    terms = w.double()[..., None] * cells.double()
+    # fp32 sums of k products, one rounding to bf16
+    assert ((out.double() - terms.sum(1)).abs() <= 2.0 ** -8 * terms.sum(1).abs() + (k + 1) * 2.0 ** -24 * terms.abs().sum(1)).all()
