@@ -508,59 +508,66 @@ __global__ void __launch_bounds__(MOE_THREADS)
   }
 }
 
-// fp8 (e4m3) rows with one fp32 scale per 128 elements -> bf16. One warp per row; a lane takes 8 values
+// 8-element vectors of a row that a warp takes at a time: four per lane.
+constexpr int DEQUANT_PIECE = 128;
+__host__ __device__ inline int dequant_pieces(int H) { return (H / 8 + DEQUANT_PIECE - 1) / DEQUANT_PIECE; }
+
+// fp8 (e4m3) rows with one fp32 scale per 128 elements -> bf16. One warp per 1024 elements of a row; a lane takes 8 values
 // at a time, so that the warp's stores are 512 consecutive bytes, and four such loads are in flight: 32768 x
-// 7168 in 125 us (5.6 TB/s), 175 with a grid-stride loop over single vectors. With zero_tail the rows past
+// 7168 in 125 us (5.6 TB/s), 175 with a grid-stride loop over single vectors; 128 rows 8 us, 16 with a warp
+// for a whole row. With zero_tail the rows past
 // the last received one are written as zeros, in place of a fill of the whole output before (120 us).
 __global__ void __launch_bounds__(MOE_THREADS)
     fp8_dequant_rows_kernel(const uint8_t* q, const float* scales, __nv_bfloat16* out, const int32_t* rows_ptr, int rows_max,
                             int H, int zero_tail) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int rows = rows_ptr ? min(*rows_ptr, rows_max) : rows_max;
-  const int vec = H / 8, groups = H / 128;
-  for (int r = blockIdx.x * warps + warp; r < (zero_tail ? rows_max : rows); r += gridDim.x * warps) {
+  const int vec = H / 8, groups = H / 128, pieces = dequant_pieces(H);
+  const int64_t items = static_cast<int64_t>(zero_tail ? rows_max : rows) * pieces;
+  for (int64_t i = blockIdx.x * warps + warp; i < items; i += gridDim.x * warps) {
+    const int r = static_cast<int>(i / pieces);
+    const int v0 = static_cast<int>(i - static_cast<int64_t>(r) * pieces) * DEQUANT_PIECE + lane;
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(r) * H);
+    constexpr int U = DEQUANT_PIECE / 32;
     if (r >= rows) {
-      for (int v = lane; v < vec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (v0 + 32 * u < vec) dst[v0 + 32 * u] = make_uint4(0, 0, 0, 0);
       continue;
     }
     const uint2* src = reinterpret_cast<const uint2*>(q + static_cast<size_t>(r) * H);
     const float* sc = scales + static_cast<size_t>(r) * groups;
-    constexpr int U = 4;
-    for (int v0 = lane; v0 < vec; v0 += 32 * U) {
-      uint2 raw[U];
-      float s[U];
+    uint2 raw[U];
+    float s[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (v0 + 32 * u < vec) {
-          raw[u] = src[v0 + 32 * u];
-          s[u] = sc[(v0 + 32 * u) / 16];
-        }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (v0 + 32 * u >= vec) break;
-        const __nv_fp8x2_storage_t* p = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw[u]);
-        __nv_bfloat162 o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[j], __NV_E4M3);
-          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
-          o[j] = __floats2bfloat162_rn(f.x * s[u], f.y * s[u]);
-        }
-        dst[v0 + 32 * u] = *reinterpret_cast<const uint4*>(o);
+    for (int u = 0; u < U; ++u)
+      if (v0 + 32 * u < vec) {
+        raw[u] = src[v0 + 32 * u];
+        s[u] = sc[(v0 + 32 * u) / 16];
       }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (v0 + 32 * u >= vec) break;
+      const __nv_fp8x2_storage_t* p = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw[u]);
+      __nv_bfloat162 o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[j], __NV_E4M3);
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+        o[j] = __floats2bfloat162_rn(f.x * s[u], f.y * s[u]);
+      }
+      dst[v0 + 32 * u] = *reinterpret_cast<const uint4*>(o);
     }
   }
 }
 
 static uint64_t g_moe_epoch[64][3] = {};
 
-static int moe_grid(int work_warps) {
+static int moe_grid(int64_t work_warps) {
   const int per_cta = MOE_THREADS / 32;
-  int grid = (work_warps + per_cta - 1) / per_cta;
+  const int64_t grid = (work_warps + per_cta - 1) / per_cta;
   const int cap = sm_count() * 4;
-  if (grid > cap) grid = cap;
-  return grid < 1 ? 1 : grid;
+  return grid > cap ? cap : grid < 1 ? 1 : static_cast<int>(grid);
 }
 
 }  // namespace b200
@@ -671,7 +678,7 @@ int b200_fp8_dequant_rows(const void* q, const void* scales, void* out, const vo
                           void* stream) {
   ensure_context();
   if (H % 128) return B200_ERR_BAD_ARG;
-  fp8_dequant_rows_kernel<<<moe_grid(rows_max), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+  fp8_dequant_rows_kernel<<<moe_grid(static_cast<int64_t>(rows_max) * dequant_pieces(H)), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint8_t*>(q), static_cast<const float*>(scales), static_cast<__nv_bfloat16*>(out),
       static_cast<const int32_t*>(rows_ptr), rows_max, H, zero_tail);
   B200_CUDA_OK(cudaGetLastError());
