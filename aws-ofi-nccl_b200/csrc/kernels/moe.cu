@@ -135,6 +135,7 @@ struct DispatchArgs {
   const int32_t* topk_idx;   // [T][k]
   const float* topk_w;       // [T][k]
   int T, k, H, E;
+  int team_warps;            // TokenTeam
   int fp8;                   // 1: payload e4m3 + fp32 scale per 128 elements; 0: payload bf16
   int use_saved_rows;        // 1: rows come from row_of (backward pass); 0: assigned here and saved there
   int scale_by_weight;       // 1: the row is multiplied by its gate weight before it is sent
@@ -157,23 +158,33 @@ __device__ __forceinline__ float warp_half_max(float v) {  // max over each grou
 
 constexpr int MOE_MAX_TOPK = 16;
 
-// How the warps of a CTA share tokens in dispatch and in combine's sum: the smallest power of two of
-// warps that covers a row of H elements, 256 per warp, works on one token (a whole CTA from 2048
-// elements on), so that a wide row moves in pieces of several KiB and a narrow one leaves no warp idle.
+// How the warps of a CTA share tokens in dispatch and in combine's sum: a team of them, the smallest power
+// of two that covers a row, works on one token and synchronises on a barrier of its own, so that a wide row
+// moves in pieces of several KiB and a narrow one leaves no warp idle. A warp takes 1024 elements of the
+// row where that gives every SM 16 warps, and 256 where there are too few tokens for it: 4096 x 3072, top-2,
+// sum 43 -> 38 us and dispatch 46 -> 40 against 256 elements a warp; 64 x 1024 sum 15 us, 17 with 1024.
 struct TokenTeam {
   static constexpr int WARPS = MOE_THREADS / 32;
   int warps, teams;   // warps of a team, teams of the CTA
   int team, warp;     // this thread's team and its warp in the team
-  __host__ __device__ static int warps_for(int H) {
+  static int warps_for(int T, int H) {
+    const int64_t wide = static_cast<int64_t>(T) * ((H + 1023) / 1024);
+    const int per_warp = wide >= 16ll * sm_count() ? 1024 : 256;
     int w = 1;
-    while (w < WARPS && w * 256 < H) w *= 2;
+    while (w < WARPS && w * per_warp < H) w *= 2;
     return w;
   }
-  __device__ __forceinline__ explicit TokenTeam(int H) {
-    warps = warps_for(H);
+  __device__ __forceinline__ explicit TokenTeam(int team_warps) {
+    warps = team_warps;
     teams = WARPS / warps;
     team = static_cast<int>(threadIdx.x >> 5) / warps;
     warp = static_cast<int>(threadIdx.x >> 5) % warps;
+  }
+  __device__ __forceinline__ void sync() const {
+    if (warps == 1)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(warps * 32) : "memory");
   }
   __device__ __forceinline__ int thread() const { return warp * 32 + static_cast<int>(threadIdx.x & 31); }
 };
@@ -194,13 +205,13 @@ __device__ __forceinline__ uint2 quantize8(const float (&v)[8], float w, float& 
   return q;
 }
 
-// A team per token: from 2048 elements on it writes one destination row 2 KiB (fp8) or 4 KiB (bf16) at a time,
-// where a warp per token left every row 256 or 512 bytes at a time among thousands of others (4096 tokens x
-// 7168, top-8: 92 us on average over the fp8 and the weighted bf16 call, 86 so; 141 with local_out, which
-// doubles the stores of the bf16 call and saves reading the window back).
-__global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs a) {
+// A team per token: a wide one writes a destination row 2 KiB (fp8) or 4 KiB (bf16) at a time, where a warp
+// per token left every row 256 or 512 bytes at a time among thousands of others (4096 tokens x 7168, top-8,
+// routing included: fp8 95 -> 79 us, bf16 140 -> 120). Four CTAs per SM: with the registers of three the
+// fp8 call took 101 us. local_out doubles the stores of a bf16 call and saves reading the window back.
+__global__ void __launch_bounds__(MOE_THREADS, 4) moe_dispatch_kernel(DispatchArgs a) {
   const GinDevHandle& h = a.h;
-  const TokenTeam team(a.H);
+  const TokenTeam team(a.team_warps);
   const int lane = threadIdx.x & 31;
   const int el = a.E / h.nranks;
   const int chunks = a.H / 256;      // 256 elements (two scale groups) per warp pass
@@ -223,7 +234,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
 #pragma unroll
     for (int i = 0; i < MAX_PASSES; ++i)
       if (live && team.warp + i * team.warps < chunks) raws[i] = src[(team.warp + i * team.warps) * 32 + lane];
-    __syncthreads();   // the slots and scales of the token before have been read
+    team.sync();   // the slots and scales of the token before have been read
     if (live && team.thread() < a.k) {
       const int slot = team.thread();
       int my_rank = -1, my_row = -1;
@@ -255,7 +266,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
       slot_row[slot] = my_row;
       slot_w[slot] = my_w;
     }
-    __syncthreads();
+    team.sync();
     // ---- the row itself; an unweighted row is quantised once and stored k times, a weighted one is
     // scaled and quantised per slot
 #pragma unroll
@@ -304,7 +315,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(DispatchArgs 
       }
     }
     if (a.fp8 && !weighted) {
-      __syncthreads();
+      team.sync();
       for (int i = team.thread(); live && i < a.k * groups; i += team.warps * 32) {
         const int s = i / groups, g = i - s * groups;
         if (slot_row[s] >= 0)
@@ -365,6 +376,7 @@ struct CombineArgs {
   const int32_t* local_row;        // [T][k] row of y for the cells whose expert is on the source itself, else -1
   __nv_bfloat16* cells_out;        // [T][k][H] a copy of every sent cell, or null
   int T, k, H;
+  int team_warps;                  // TokenTeam
   __nv_bfloat16* out;              // [T][H]
   unsigned int* done;
   uint64_t epoch;
@@ -406,7 +418,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
   }
   // ---- ... and every CTA waits for all ranks' rows before it reduces its share of the tokens
   if (!moe_wait_all(h, 2, a.epoch)) return;
-  // A team per token: from 2048 elements on it reads 4 KiB of each of the token's rows at a time. With a warp per
+  // A team per token: a wide one reads 4 KiB of each of the token's rows at a time. With a warp per
   // token every row is visited 512 bytes at a time by thousands of warps at once: 4096 tokens x 7168,
   // top-8, one rank took 194 us that way (314 with eight loads in flight per warp instead of four)
   // and 140 so, before the stores to the window's cells: 215 with them, on average over the forward call,
@@ -414,7 +426,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
   // when every row was read back from its cell. Four cells' loads are issued together and added in the
   // order of the slots.
   uint4* comb = reinterpret_cast<uint4*>(h.window[h.rank] + a.comb_off);
-  const TokenTeam team(a.H);
+  const TokenTeam team(a.team_warps);
   __shared__ float team_w[TokenTeam::WARPS][MOE_MAX_TOPK];
   __shared__ int team_row[TokenTeam::WARPS][MOE_MAX_TOPK];   // row of y, -1: the cell in the window, -2: never sent
   float* slot_w = team_w[team.team];
@@ -422,10 +434,11 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
   for (int t0 = blockIdx.x * team.teams; t0 < a.T; t0 += gridDim.x * team.teams) {
     const int t = t0 + team.team;
     const bool on = t < a.T;
-    __syncthreads();   // the slots of the tokens before have been read
+    team.sync();   // the slots of the token before have been read
     if (on && team.thread() < a.k) {
       const int i = t * a.k + team.thread();
-      int row = a.row_of[i] < 0 ? -2 : a.local_row[i];
+      const int sent = a.row_of[i], own = a.local_row[i];
+      int row = sent < 0 ? -2 : own;
       if (row >= rows) {
         gin_record_error(h, DEV_ERR_BOUNDS);
         row = -2;
@@ -433,7 +446,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
       slot_row[team.thread()] = row;
       slot_w[team.thread()] = a.topk_w ? a.topk_w[i] : 1.f;
     }
-    __syncthreads();
+    team.sync();
     constexpr int U = 4;
     for (int v = team.thread(); on && v < vec; v += team.warps * 32) {
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -613,10 +626,10 @@ int b200_moe_dispatch(int comm, const void* x, const void* topk_idx, const void*
       (fp8 && scale_off + 4ull * (H / 128) * capacity_rows > h.window_bytes))
     return B200_ERR_BAD_ARG;
   DispatchArgs a{h, static_cast<const __nv_bfloat16*>(x), static_cast<const int32_t*>(topk_idx),
-                 static_cast<const float*>(topk_w), T, k, H, E, fp8, use_saved_rows, scale_by_weight,
+                 static_cast<const float*>(topk_w), T, k, H, E, TokenTeam::warps_for(T, H), fp8, use_saved_rows, scale_by_weight,
                  static_cast<const int32_t*>(dest_base), static_cast<int32_t*>(cursor), static_cast<int32_t*>(row_of),
                  static_cast<int32_t*>(local_row), static_cast<__nv_bfloat16*>(local_out), recv_off, scale_off, meta_off, capacity_rows, static_cast<unsigned int*>(done), ++g_moe_epoch[comm][1]};
-  const int per_cta = TokenTeam::WARPS / TokenTeam::warps_for(H);
+  const int per_cta = TokenTeam::WARPS / a.team_warps;
   const int cap = sm_count() * 4, grid = (T + per_cta - 1) / per_cta;
   moe_dispatch_kernel<<<grid < cap ? grid : cap, MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
   B200_CUDA_OK(cudaGetLastError());
@@ -651,7 +664,7 @@ int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int ex
   if (comb_off % 16 || comb_off + static_cast<size_t>(T) * k * H * 2 > h.window_bytes) return B200_ERR_BAD_ARG;
   CombineArgs a{h, static_cast<const __nv_bfloat16*>(y), static_cast<const int32_t*>(expert_offsets), experts_local, meta_off,
                 comb_off, static_cast<const float*>(topk_w), static_cast<const int32_t*>(row_of),
-                static_cast<const int32_t*>(local_row), static_cast<__nv_bfloat16*>(cells_out), T, k, H,
+                static_cast<const int32_t*>(local_row), static_cast<__nv_bfloat16*>(cells_out), T, k, H, TokenTeam::warps_for(T, H),
                 static_cast<__nv_bfloat16*>(out), static_cast<unsigned int*>(done), ++g_moe_epoch[comm][2]};
   int per_sm = 0;
   B200_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_combine_kernel, MOE_THREADS, 0));
