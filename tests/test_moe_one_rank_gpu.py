@@ -24,7 +24,8 @@ def comm():
 # a team of one warp, of several, of the whole CTA with one column step; then rows of several steps (ragged, full,
 # the largest), several tokens per team, several teams of one warp with a ragged last group
 @pytest.mark.parametrize("T,H,E,k", [(1, 256, 8, 1), (37, 512, 16, 3), (130, 1280, 64, 5), (64, 2048, 8, 8),
-                                     (37, 2304, 16, 3), (21, 7168, 64, 8), (9, 8192, 8, 2), (2500, 1280, 16, 2), (10003, 256, 8, 1)])
+                                     (37, 2304, 16, 3), (21, 7168, 64, 8), (9, 8192, 8, 2), (2500, 1280, 16, 2), (1300, 4096, 8, 1),
+                                     (10003, 256, 8, 1)])
 @pytest.mark.parametrize("fp8", [False, True])
 def test_roundtrip_and_gradients(comm, T, H, E, k, fp8):
     from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
