@@ -65,6 +65,8 @@ class _RoPE(torch.autograd.Function):
 
 
 def rope_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, seq: int) -> torch.Tensor:
+    """Rotary embedding in place, for programs that hold q or k as [T, heads, head_dim] tensors; the model
+    rotates while it splits its fused projection (``rope_qkv``)."""
     return _RoPE.apply(x, cos, sin, seq)
 
 

@@ -109,7 +109,8 @@ class ExpertParallel:
             self.comm.id, x.data_ptr(), topk_idx.data_ptr(), topk_w.data_ptr() if topk_w is not None else None,
             self.T, self.k, self.H, self.E, int(fp8), int(use_saved_rows), int(scale_by_weight),
             self.dest_base.data_ptr(), self.cursor.data_ptr(), self.row_of.data_ptr(), self.local_row.data_ptr(),
-            local_out.data_ptr() if local_out is not None else None, self.recv_off, self.scale_off, self.meta_off, self.capacity, self._done[1:].data_ptr(), _lib.stream_ptr())
+            local_out.data_ptr() if local_out is not None else None, self.recv_off, self.scale_off, self.meta_off,
+            self.capacity, self._done[1:].data_ptr(), _lib.stream_ptr())
         _lib.check(rc, "b200_moe_dispatch")
 
     def collect(self, out: torch.Tensor, local_in_place: bool) -> torch.Tensor:
@@ -140,7 +141,8 @@ class ExpertParallel:
         _lib.check(rc, "b200_moe_combine")
 
     def dequant(self, out: torch.Tensor | None = None) -> torch.Tensor:
-        """fp8 receive rows + scales -> bf16 [capacity, H] (only the rows actually received are written)."""
+        """fp8 receive rows + scales -> bf16 [capacity, H].  Rows past the last received one are zeros in a new
+        tensor and are left alone in ``out``."""
         fresh = out is None
         if fresh:   # the kernel writes the zeros of the rows that nobody sent
             out = torch.empty(self.capacity, self.H, device=self.comm.device, dtype=torch.bfloat16)
@@ -153,7 +155,7 @@ class ExpertParallel:
     # ---- differentiable forms
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.Tensor, fp8: bool = False) -> torch.Tensor:
         """Route + dispatch.  Returns bf16 rows [capacity, H]; rows [expert_offsets[e], expert_offsets[e+1])
-        belong to local expert e, rows past expert_offsets[-1] are unspecified."""
+        belong to local expert e, rows past expert_offsets[-1] are zeros."""
         return _Dispatch.apply(x, self, topk_idx, topk_w, fp8)
 
     def combine(self, y_rows: torch.Tensor, topk_w: torch.Tensor) -> torch.Tensor:
