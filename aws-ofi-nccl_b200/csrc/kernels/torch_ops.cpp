@@ -31,8 +31,8 @@ using torch::autograd::variable_list;
 std::atomic<int64_t> g_launches{0};
 PyObject* g_error = nullptr;   // the package's B200OpsError (a RuntimeError), looked up when the module is loaded
 
-// Raises a Python exception from either side: in a call from Python (the GIL is held) it travels as
-// error_already_set; on an autograd thread torch's own carrier takes it to the caller of backward().
+// Raises a Python exception with or without the interpreter lock: with it as error_already_set, without (in a
+// layer's body, forward or on an autograd thread) in torch's own carrier.
 [[noreturn]] void raise(PyObject* type, const std::string& what) {
   if (PyGILState_Check()) {
     PyErr_SetString(type, what.c_str());
@@ -80,39 +80,49 @@ void gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const Tensor& 
 }
 
 PyObject* interned(const char* name) { return PyUnicode_InternFromString(name); }
+PyObject* name_written() {
+  static PyObject* const name = interned("grad_written");
+  return name;
+}
 
 // Runs produce(out, accumulate) into weight.main_grad when the parameter has one (and returns an
 // undefined tensor), else into a new tensor of the weight's shape.
 template <class Produce>
 Tensor write_param_grad(const Tensor& weight, Produce produce) {
+  Tensor main;
+  bool accumulate = false;
+  auto attribute = [](const py::object& of, PyObject* name) {
+    PyObject* v = PyObject_GetAttr(of.ptr(), name);
+    if (!v) {
+      if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw py::error_already_set();
+      PyErr_Clear();
+    }
+    return py::reinterpret_steal<py::object>(v);
+  };
   {
     py::gil_scoped_acquire gil;
     static PyObject* const kMain = interned("main_grad");
-    static PyObject* const kWritten = interned("grad_written");
-    static PyObject* const kReady = interned("grad_ready");
     const py::object w = py::reinterpret_steal<py::object>(THPVariable_Wrap(weight));
-    auto attribute = [&](PyObject* name) {
-      PyObject* v = PyObject_GetAttr(w.ptr(), name);
-      if (!v) {
-        if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw py::error_already_set();
-        PyErr_Clear();
-      }
-      return py::reinterpret_steal<py::object>(v);
-    };
-    const py::object main = attribute(kMain);
-    if (main && !main.is_none()) {
-      const py::object written = attribute(kWritten);
-      const bool accumulate = written && PyObject_IsTrue(written.ptr()) == 1;
-      produce(main.cast<Tensor>(), accumulate);
-      if (PyObject_SetAttr(w.ptr(), kWritten, Py_True) != 0) throw py::error_already_set();
-      const py::object ready = attribute(kReady);
-      if (ready && !ready.is_none()) ready(w);
-      return {};
+    const py::object buffer = attribute(w, kMain);
+    if (buffer && !buffer.is_none()) {
+      const py::object written = attribute(w, name_written());
+      accumulate = written && PyObject_IsTrue(written.ptr()) == 1;
+      main = buffer.cast<Tensor>();
     }
   }
-  Tensor dw = at::empty_like(weight);
-  produce(dw, false);
-  return dw;
+  if (!main.defined()) {
+    const Tensor dw = at::empty_like(weight);
+    produce(dw, false);
+    return dw;
+  }
+  produce(main, accumulate);   // without the interpreter lock: a launch may wait for the GPU
+  py::gil_scoped_acquire gil;
+  static PyObject* const kReady = interned("grad_ready");
+  const py::object w = py::reinterpret_steal<py::object>(THPVariable_Wrap(weight));
+  if (PyObject_SetAttr(w.ptr(), name_written(), Py_True) != 0) throw py::error_already_set();
+  const py::object ready = attribute(w, kReady);
+  if (ready && !ready.is_none()) ready(w);
+  return {};
 }
 
 // pybind's exception cannot cross the autograd engine's threads; torch's carrier can.
@@ -308,12 +318,19 @@ TORCH_LIBRARY(b200ops, m) {
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   g_error = py::object(py::module_::import("aws_ofi_nccl_b200.ops._lib").attr("B200OpsError")).release().ptr();
-  m.def("linear", [](const Tensor& x, const Tensor& w) { return traced_or_direct("b200ops::linear", linear, x, w); });
-  m.def("rmsnorm", [](const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
-    return traced_or_direct("b200ops::rmsnorm", rmsnorm, x, res, w, eps);
-  });
-  m.def("swiglu", [](const Tensor& gu) { return traced_or_direct("b200ops::swiglu", swiglu, gu); });
-  m.def("rope_qkv", [](const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S, int64_t nq, int64_t nkv,
-                       int64_t hd) { return traced_or_direct("b200ops::rope_qkv", rope_qkv, qkv, cos, sin, B, S, nq, nkv, hd); });
+  // Like torch's own operators these run without the interpreter lock, which a launch into a full queue would
+  // otherwise hold for as long as it waits; the wrapper takes exceptions back to Python.
+  m.def("linear", torch::wrap_pybind_function_no_gil(
+                      [](const Tensor& x, const Tensor& w) { return traced_or_direct("b200ops::linear", linear, x, w); }));
+  m.def("rmsnorm", torch::wrap_pybind_function_no_gil(
+                       [](const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
+                         return traced_or_direct("b200ops::rmsnorm", rmsnorm, x, res, w, eps);
+                       }));
+  m.def("swiglu", torch::wrap_pybind_function_no_gil(
+                      [](const Tensor& gu) { return traced_or_direct("b200ops::swiglu", swiglu, gu); }));
+  m.def("rope_qkv", torch::wrap_pybind_function_no_gil([](const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S,
+                                                          int64_t nq, int64_t nkv, int64_t hd) {
+          return traced_or_direct("b200ops::rope_qkv", rope_qkv, qkv, cos, sin, B, S, nq, nkv, hd);
+        }));
   m.def("launches", [] { return g_launches.load(std::memory_order_relaxed); });
 }

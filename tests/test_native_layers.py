@@ -143,3 +143,62 @@ def test_the_rotary_split_refuses_misaligned_tables():
                 ctypes.c_void_p(cos), ctypes.c_void_p(sin), ctypes.c_longlong(2)]
         assert lib.b200_rope_qkv(*args, 1, 1, 32, 2, 0, None) == 10001
         assert lib.b200_rope(64, cos, sin, 2, 1, 32, 32, 2, 0, None) == 10001
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("backward", [False, True])
+def test_other_threads_run_while_a_launch_waits(backward):
+    """A launch into a full queue waits for the GPU; the interpreter must not wait with it."""
+    import threading
+    import time
+
+    from aws_ofi_nccl_b200.ops import gemm
+
+    x = torch.randn(8, 64, device="cuda").bfloat16()
+    w = torch.randn(64, 64, device="cuda").bfloat16()
+    w.main_grad = torch.zeros_like(w)
+    if backward:
+        w.requires_grad_(True)
+    scratch = torch.zeros(8, device="cuda").add_(1)   # every kernel is loaded before the queue is filled
+    y = gemm.linear(x, w)
+    if backward:
+        y.backward(torch.randn_like(y))
+    torch.cuda.synchronize()
+    gaps, stop = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    outs = [gemm.linear(x, w) for _ in range(200)] if backward else None
+    dy = torch.randn_like(outs[0]) if backward else None
+    torch.cuda.synchronize()
+    pause = 1_000_000_000   # clocks: about half a second
+    torch.cuda._sleep(pause)
+    depth, waited = 0, 0.0
+    while waited < 0.05 and depth < 20000:    # launches until one waits
+        t0 = time.perf_counter()
+        scratch.add_(1)
+        depth, waited = depth + 1, time.perf_counter() - t0
+    torch.cuda.synchronize()
+    thread = threading.Thread(target=tick)
+    thread.start()
+    torch.cuda._sleep(pause)
+    for _ in range(depth - 20):
+        scratch.add_(1)
+    t0 = time.perf_counter()
+    if backward:
+        torch.autograd.backward(outs, [dy] * len(outs))   # one weight-gradient product each
+    else:
+        for _ in range(200):
+            gemm.linear(x, w)
+    issued = time.perf_counter() - t0
+    stop.set()
+    thread.join()
+    torch.cuda.synchronize()
+    assert issued > 0.2, "the queue did not fill: nothing was tested"
+    assert max(gaps) < 0.1, (issued, max(gaps))
