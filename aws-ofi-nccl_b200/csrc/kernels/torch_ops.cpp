@@ -106,7 +106,9 @@ Tensor write_param_grad(const Tensor& weight, Produce produce) {
     const py::object buffer = attribute(w, kMain);
     if (buffer && !buffer.is_none()) {
       const py::object written = attribute(w, name_written());
-      accumulate = written && PyObject_IsTrue(written.ptr()) == 1;
+      const int truth = written ? PyObject_IsTrue(written.ptr()) : 0;
+      if (truth < 0) throw py::error_already_set();
+      accumulate = truth == 1;
       main = buffer.cast<Tensor>();
     }
   }

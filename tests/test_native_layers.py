@@ -203,3 +203,25 @@ def test_other_threads_run_while_a_launch_waits(backward):
     if issued < 0.2:
         pytest.skip("no launch waited for the queue")
     assert max(gaps) < issued / 2, (issued, max(gaps))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", ["grad_written", "grad_ready"])
+def test_an_exception_of_a_parameters_attribute_reaches_the_caller(where):
+    from aws_ofi_nccl_b200.ops import gemm
+
+    class Odd(Exception):
+        pass
+
+    class Raises:
+        def __bool__(self):
+            raise Odd
+
+        def __call__(self, weight):
+            raise Odd
+
+    w = torch.randn(16, 16, device="cuda").bfloat16().requires_grad_(True)
+    w.main_grad = torch.zeros_like(w)
+    setattr(w, where, Raises())
+    with pytest.raises(Odd):
+        gemm.linear(torch.randn(8, 16, device="cuda").bfloat16(), w).float().sum().backward()
