@@ -289,7 +289,7 @@ struct RingEpilogue {
     }
   }
 
-  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape& s) {
+  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape& s, int) {
     if (col0 >= s.N) return;  // uniform over the warp
     const int lane = threadIdx.x & 31;
     uint8_t* buf = stage + ((threadIdx.x >> 5) - 2) * 4096;

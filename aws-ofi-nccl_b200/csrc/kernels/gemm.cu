@@ -111,35 +111,58 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   gemm_mainloop_2cta<BN, A_MN, B_MN>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
 }
 
+// Tiles of a product on CTA pairs: their width (a multiple of 32, 128 to 256) and whether those of the last
+// wave are halved.
+struct PairTiles {
+  int width;
+  bool halves;
+};
+
+// Fills in the tiles of `shape` (M, N and K are set). bn: the kernel's BN; ctas: how many may run. Returns how
+// many are launched.
+static int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas) {
+  const int pairs = ctas / 2;
+  shape.tiles_m = (shape.M + GEMM2_BM - 1) / GEMM2_BM;
+  shape.tiles_n = (shape.N + tiles.width - 1) / tiles.width;
+  shape.group_m = (gemm_group_m(bn) + 1) / 2;
+  shape.bn = tiles.width;
+  const int all = shape.tiles_m * shape.tiles_n;
+  int items = all;
+  if (tiles.halves) {
+    shape.halve_from = all / pairs * pairs;
+    items = 2 * all - shape.halve_from;
+  }
+  shape.b_box = tiles.width / (tiles.halves ? 4 : 2);
+  return 2 * (items < pairs ? items : pairs);
+}
+
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
-                            int64_t ldc, int accumulate, int max_ctas, cudaStream_t stream) {
+                            int64_t ldc, int accumulate, PairTiles tiles, int max_ctas, cudaStream_t stream) {
   CUtensorMap tmA, tmB, tmC;
   int rc;
-  // every CTA loads 128 rows of A and BN/2 rows (its half) of B per k-block
+  GemmShape shape{M, N, K, 0, 0};
+  int cap = sm_count();
+  if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
+  const int grid = pair_grid(shape, tiles, BN, cap);
+  // every CTA loads 128 rows of A and its half of the tile's rows of B per k-block
   if (!A_MN)
     rc = make_tmap_2d(&tmA, A, M, K, lda, 128, GEMM_BK, 2, true);
   else
     rc = make_tmap_2d(&tmA, A, K, M, lda, GEMM_BK, 64, 2, true);
   if (rc) return rc;
   if (!B_MN)
-    rc = make_tmap_2d(&tmB, B, N, K, ldb, BN / 2, GEMM_BK, 2, true);
+    rc = make_tmap_2d(&tmB, B, N, K, ldb, shape.b_box, GEMM_BK, 2, true);
   else
     rc = make_tmap_2d(&tmB, B, K, N, ldb, GEMM_BK, 64, 2, true);
   if (rc) return rc;
   if ((rc = make_tmap_out<OutT>(&tmC, C, M, N, ldc))) return rc;
-  GemmShape shape{M, N, K, (M + GEMM2_BM - 1) / GEMM2_BM, (N + BN - 1) / BN};
-  shape.group_m = (gemm_group_m(BN) + 1) / 2;
   auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, OutT>;
   static bool attr_set = false;
   if (!attr_set) {
     B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
     attr_set = true;
   }
-  int cap = sm_count();
-  if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
-  int grid = 2 * shape.tiles_m * shape.tiles_n;
-  if (grid > cap) grid = cap & ~1;
   int* err = device_status_word();
   kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
@@ -148,11 +171,21 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
 
 template <int BN, typename OutT>
 static int dispatch_major_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
-                               int64_t ldc, int a_mn, int b_mn, int accumulate, int max_ctas, cudaStream_t stream) {
-  if (!a_mn && !b_mn) return launch_gemm_2cta<BN, false, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, max_ctas, stream);
-  if (!a_mn && b_mn) return launch_gemm_2cta<BN, false, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, max_ctas, stream);
-  if (a_mn && !b_mn) return launch_gemm_2cta<BN, true, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, max_ctas, stream);
-  return launch_gemm_2cta<BN, true, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, max_ctas, stream);
+                               int64_t ldc, int a_mn, int b_mn, int accumulate, PairTiles tiles, int max_ctas, cudaStream_t stream) {
+  if (!a_mn && !b_mn) return launch_gemm_2cta<BN, false, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
+  if (!a_mn && b_mn) return launch_gemm_2cta<BN, false, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
+  if (a_mn && !b_mn) return launch_gemm_2cta<BN, true, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
+  return launch_gemm_2cta<BN, true, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
+}
+
+// The narrow kernel has more stages; tiles of any other width run on the wide one.
+static int gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_mn,
+                     int b_mn, int out_fp32, int accumulate, PairTiles tiles, int max_ctas, cudaStream_t s) {
+  if (tiles.width == 128)
+    return out_fp32 ? dispatch_major_2cta<128, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
+                    : dispatch_major_2cta<128, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
+  return out_fp32 ? dispatch_major_2cta<256, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
+                  : dispatch_major_2cta<256, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
 }
 
 // ---------------------------------------------------------------- fp8 (e4m3) x fp8 -> bf16 with row / column scales
@@ -170,24 +203,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 
 template <int BN>
 static int launch_gemm_fp8(const void* A, const void* B, const float* a_scale, const float* b_scale, void* C, int M, int N,
-                           int K, int64_t lda, int64_t ldb, int64_t ldc, cudaStream_t stream) {
+                           int K, int64_t lda, int64_t ldb, int64_t ldc, PairTiles tiles, cudaStream_t stream) {
   CUtensorMap tmA, tmB, tmC;
+  GemmShape shape{M, N, K, 0, 0};
+  const int grid = pair_grid(shape, tiles, BN, sm_count());
   int rc = make_tmap_2d(&tmA, A, M, K, lda, 128, 2 * GEMM_BK, 1, true);   // 128 one-byte elements = 128 B per row
   if (rc) return rc;
-  rc = make_tmap_2d(&tmB, B, N, K, ldb, BN / 2, 2 * GEMM_BK, 1, true);
+  rc = make_tmap_2d(&tmB, B, N, K, ldb, shape.b_box, 2 * GEMM_BK, 1, true);
   if (rc) return rc;
   if ((rc = make_tmap_out<__nv_bfloat16>(&tmC, C, M, N, ldc))) return rc;
-  GemmShape shape{M, N, K, (M + GEMM2_BM - 1) / GEMM2_BM, (N + BN - 1) / BN};
-  shape.group_m = (gemm_group_m(BN) + 1) / 2;
   auto kern = gemm_fp8_2cta_kernel<BN>;
   static bool attr_set = false;
   if (!attr_set) {
     B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
     attr_set = true;
   }
-  int grid = 2 * shape.tiles_m * shape.tiles_n;
-  const int cap = sm_count() & ~1;
-  if (grid > cap) grid = cap;
   kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<__nv_bfloat16*>(C), ldc, a_scale, b_scale,
                                                                      shape, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
@@ -263,12 +293,53 @@ static bool use_pairs(int M, int N, int max_ctas) {
 // What a product with bn = 0 runs on: the tile width of the persistent kernel, or a split along K.
 // `a_at`, `b_at`: the operands' addresses (their alignment counts).
 struct GemmChoice {
-  int bn;
+  int bn;            // the plain width that fits better, 128 or 256
+  PairTiles tiles;   // on CTA pairs: what the product runs on
   SplitkPlan split;
 };
-static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, uintptr_t a_at, uintptr_t b_at, int max_ctas) {
+
+// Tiles of a product on CTA pairs whose better plain width is `bn`; a_low, b_low: what decides how the operands' rows
+// lie on cache lines. A wave of narrower tiles costs more than their share of a wide one: their loads bring the
+// same rows of A for fewer columns, and an SM takes in 64 bytes a clock. Rows off cache lines take three clocks
+// each instead of two, and the boxes of an N-major B are 64 columns, so that 160 and 224 columns (80 and 112
+// for a CTA) load as much as 256. The costs are medians over 110 products of 256 to 8192 rows, 128 to 28672
+// columns and K from 64 to 16040 in three majors; the rule's choice took 0.971 of the plain width's time on average
+// there, the best choice 0.962, and none more than 1.025. What it gains is the last wave: 4096 x 4096 x
+// 14336, 256 tiles for 74 pairs, takes 333 us in four wide waves, 363 in seven narrow ones, 308 with the last of
+// four halved; 4096 x 14336 x 4096 343 us, 325 with 14 waves of 224 columns for 13 of 256.
+static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint64_t b_low, int units, int bn) {
+  struct Costs {
+    double at[5];   // 128, 160, 192, 224, 256 columns
+  };
+  static constexpr double NO = 9;
+  static constexpr Costs ON_LINES[2] = {{{.635, .72, .79, .88, 1}}, {{.635, .79, .81, .89, 1}}};
+  static constexpr Costs BETWEEN[2] = {{{.635, .76, .83, .90, 1}}, {{.64, NO, .90, .95, 1}}};
+  static constexpr Costs OFF_LINES[2] = {{{.72, .82, .88, .95, 1}}, {{.72, NO, NO, NO, 1}}};
+  const bool a_lines = a_low % 128 == 0, b_lines = b_low % 128 == 0;
+  const Costs& c = a_lines && b_lines ? ON_LINES[b_mn] : a_lines || b_lines || (a_low | b_low) % 64 == 0 ? BETWEEN[b_mn] : OFF_LINES[b_mn];
+  const int64_t rows = (M + GEMM2_BM - 1) / GEMM2_BM;
+  constexpr double GAIN = 1.03;   // a width that is not the plain one has to promise 3 %, halves of the last wave 1 %
+  PairTiles best{bn, false};
+  double best_cost = 1e30;
+  for (int i = 0; i < 5; ++i) {
+    const int width = 128 + 32 * i;
+    if (width > 128 && N <= width - 32) break;   // a narrower one covers the row as well
+    if (width % 64 && K < 1024) continue;        // the last 32 columns of a tile leave as vectors, not by TMA: with few k-blocks that counts
+    const int64_t tiles = rows * ((N + width - 1) / width);
+    const double cost = static_cast<double>((tiles + units - 1) / units) * c.at[i] * (width == bn ? 1 : GAIN);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = {width, false};
+    }
+  }
+  const int64_t wide = rows * ((N + 255) / 256), last = wide % units;
+  if (wide > units && last > 0 && 2 * last <= units && (static_cast<double>(wide / units) + c.at[0]) * 1.01 <= best_cost) best = {256, true};
+  return best;
+}
+static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, uintptr_t a_at, uintptr_t b_at, int max_ctas) {
   const bool pairs = use_pairs(M, N, max_ctas);
   int bn;
+  PairTiles tiles{};
   // Wider tiles re-read A less; fall back to the narrower tile when that fills the SMs better.
   const int units = pairs ? sm_count() / 2 : sm_count();
   const long rows = pairs ? (M + 255) / 256 : (M + 127) / 128;
@@ -289,13 +360,14 @@ static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, uin
     const bool a_lines = a_low % 128 == 0, b_lines = b_low % 128 == 0, halves = (a_low | b_low) % 64 == 0;
     const double narrow_wave = a_lines && b_lines ? (K <= 2048 ? 0.58 : 0.56) : a_lines || b_lines || halves ? 0.62 : 0.85;
     bn = (N >= 256 && w256 <= narrow_wave * w128) ? 256 : 128;
+    tiles = max_ctas == 0 ? fit_tiles(M, N, K, b_mn, a_low, b_low, units, bn) : PairTiles{bn, false};
   } else {
     const double eff256 = static_cast<double>(t256) / (w256 * units);
     const double eff128 = static_cast<double>(t128) / (w128 * units);
     bn = (N >= 256 && eff256 + 0.08 >= eff128) ? 256 : 128;
   }
   // Few tiles and a long K: the chip is filled by splitting K over clusters.
-  return {bn, max_ctas == 0 ? plan_splitk(M, N, K, pairs, bn) : SplitkPlan{1}};
+  return {bn, tiles, max_ctas == 0 ? plan_splitk(M, N, K, pairs, bn) : SplitkPlan{1}};
 }
 
 }  // namespace b200
@@ -312,20 +384,17 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
   if (!gemm_args_ok(A, B, C, M, N, K, lda, ldb, ldc, out_fp32)) return B200_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool pairs = use_pairs(M, N, max_ctas);
+  PairTiles tiles{bn, false};
   if (bn == 0) {
-    const GemmChoice g = choose_gemm(M, N, K, lda, ldb, reinterpret_cast<uintptr_t>(A), reinterpret_cast<uintptr_t>(B), max_ctas);
+    const GemmChoice g =
+        choose_gemm(M, N, K, lda, ldb, b_mn != 0, reinterpret_cast<uintptr_t>(A), reinterpret_cast<uintptr_t>(B), max_ctas);
     if (g.split.slices > 1)
       return launch_splitk({A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate}, pairs, g.split, s);
     bn = g.bn;
+    tiles = g.tiles;
   }
-  if (pairs) {
-    if (bn == 256)
-      return out_fp32 ? dispatch_major_2cta<256, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, max_ctas, s)
-                      : dispatch_major_2cta<256, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, max_ctas, s);
-    if (bn == 128)
-      return out_fp32 ? dispatch_major_2cta<128, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, max_ctas, s)
-                      : dispatch_major_2cta<128, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, max_ctas, s);
-  }
+  if (pairs && (bn == 256 || bn == 128))
+    return gemm_2cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, tiles, max_ctas, s);
   if (bn == 256) {
     return out_fp32 ? dispatch_major<256, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, max_ctas, s)
                     : dispatch_major<256, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate,
@@ -336,17 +405,42 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
                                                        max_ctas, s);
 }
 
-// What b200_gemm_bf16 with bn = 0 and max_ctas = 0 runs on for operands on cache-line boundaries: CTA pairs
-// or single CTAs, slices of K (1: the persistent kernel) and its tile width.
+// What b200_gemm_bf16 with bn = 0 and max_ctas = 0 starts from for operands on cache-line boundaries: CTA pairs
+// or single CTAs, slices of K (1: the persistent kernel) and the better one of its plain tile widths
+// (b200_gemm_tiles has the tiles that CTA pairs then run on).
 int b200_gemm_plan(int M, int N, int K, long long lda, long long ldb, int* pair, int* bn, int* slices) {
   b200::ensure_context();
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || !pair || !bn || !slices) return B200_ERR_BAD_ARG;
-  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, 0, 0, 0);
+  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, false, 0, 0, 0);
   *pair = use_pairs(M, N, 0);
   *slices = g.split.slices;
   *bn = g.split.slices > 1 ? 128 : g.bn;
   return 0;
+}
+
+// The tiles of the same call where it runs on the persistent kernel of CTA pairs: their width and whether those
+// of the last wave are halved.
+int b200_gemm_tiles(int M, int N, int K, long long lda, long long ldb, int b_mn, int* width, int* halves) {
+  b200::ensure_context();
+  using namespace b200;
+  if (M <= 0 || N <= 0 || K <= 0 || !width || !halves || !use_pairs(M, N, 0)) return B200_ERR_BAD_ARG;
+  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, b_mn != 0, 0, 0, 0);
+  *width = g.tiles.width;
+  *halves = g.tiles.halves;
+  return 0;
+}
+
+// b200_gemm_bf16 on CTA pairs with tiles of `width` columns (128 to 256 in steps of 32), those of the last wave
+// halved or not (width 256 only), whatever the plan says.
+int b200_gemm_bf16_tiles(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
+                         int a_mn, int b_mn, int out_fp32, int accumulate, int width, int halves, void* stream) {
+  b200::ensure_context();
+  using namespace b200;
+  if (!gemm_args_ok(A, B, C, M, N, K, lda, ldb, ldc, out_fp32)) return B200_ERR_BAD_ARG;
+  if (width < 128 || width > 256 || width % 32 || (halves && width != 256)) return B200_ERR_BAD_ARG;
+  return gemm_2cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, PairTiles{width, halves != 0}, 0,
+                   static_cast<cudaStream_t>(stream));
 }
 
 // b200_gemm_bf16 on the split kernel whatever the plan says: slices 2, 4 or 8 (with pair at most 4) and no
@@ -379,8 +473,12 @@ int b200_gemm_fp8(const void* A, const void* B, const float* a_scale, const floa
   const long t256 = rows * ((N + 255) / 256), t128 = rows * ((N + 127) / 128);
   const double eff256 = static_cast<double>(t256) / (((t256 + units - 1) / units) * units);
   const double eff128 = static_cast<double>(t128) / (((t128 + units - 1) / units) * units);
-  if (N >= 256 && eff256 + 0.08 >= eff128) return launch_gemm_fp8<256>(A, B, a_scale, b_scale, C, M, N, K, lda, ldb, ldc, s);
-  return launch_gemm_fp8<128>(A, B, a_scale, b_scale, C, M, N, K, lda, ldb, ldc, s);
+  const int bn = N >= 256 && eff256 + 0.08 >= eff128 ? 256 : 128;
+  // a k-block is 128 elements here, the same bytes
+  const PairTiles tiles = fit_tiles(M, N, K / 2, false, reinterpret_cast<uintptr_t>(A) | static_cast<uint64_t>(lda),
+                                    reinterpret_cast<uintptr_t>(B) | static_cast<uint64_t>(ldb), units, bn);
+  if (tiles.width == 128) return launch_gemm_fp8<128>(A, B, a_scale, b_scale, C, M, N, K, lda, ldb, ldc, tiles, s);
+  return launch_gemm_fp8<256>(A, B, a_scale, b_scale, C, M, N, K, lda, ldb, ldc, tiles, s);
 }
 
 // q[rows,K] (e4m3) and scale[rows] (fp32) from x[rows,K] (bf16); K % 8 == 0, 16-byte aligned rows.

@@ -78,12 +78,36 @@ __device__ __noinline__ void store_tail(uint32_t chunk, OutT* dst, int n) {
   }
 }
 
-// A warp's 32 rows from `row0` on, 128 bytes of each from column col0 on (w: this lane's row). The map of C
-// ends at whole_vectors(N); what is left of a row beyond it each lane stores itself.
+// The first 32 columns of a slab of 16-bit elements that lies in shared memory at `slab` -> C: what a tile holds of
+// its last 64 columns where its width ends inside them (a TMA store would write the next tile's columns too).
+template <typename OutT>
+__device__ __noinline__ void store_half_slab(uint32_t slab, OutT* C, int64_t ldc, int row0, int M) {
+  const int lane = threadIdx.x & 31, v = lane & 3;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = i * 8 + (lane >> 2);
+    uint32_t x[4];
+    ld_shared_v4(slab + r * 128 + ((v ^ (r & 7)) << 4), x);
+    if (row0 + r < M) *reinterpret_cast<uint4*>(C + static_cast<int64_t>(row0 + r) * ldc + v * 8) = make_uint4(x[0], x[1], x[2], x[3]);
+  }
+  __syncwarp();
+}
+
+// A warp's 32 rows from `row0` on, 128 bytes of each from column col0 on (w: this lane's row), of which a bf16
+// tile may hold the first 32 columns only (left < 64). The map of C ends at whole_vectors(N); what is left of
+// a row beyond it each lane stores itself.
 template <typename OutT>
 __device__ __forceinline__ void store_row(SlabStore& slab, const CUtensorMap* tmC, OutT* C, int64_t ldc, int row0, int col0,
-                                          const uint32_t (&w)[32], const GemmShape& s) {
+                                          const uint32_t (&w)[32], const GemmShape& s, int left) {
   const int nv = whole_vectors<OutT>(s.N);
+  if constexpr (sizeof(OutT) == 2) {
+    if (left < 64 && col0 + left < s.N) {   // 32 whole columns, others to their right
+      const uint32_t mine = slab.put128(tmC, col0, row0, w, false);
+      store_half_slab(mine - (threadIdx.x & 31) * 128, C + col0, ldc, row0, s.M);
+      return;
+    }
+  }
   const uint32_t mine = slab.put128(tmC, col0, row0, w, col0 < nv);
   if (nv == s.N) return;
   const int lane = threadIdx.x & 31;
@@ -141,7 +165,7 @@ struct StoreEpilogue {
 #pragma unroll
       for (int j = 0; j < 32; ++j) acc[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(acc[j]));
     }
-    store_row(slab, tmC, C, ldc, row0, col0, acc, s);
+    store_row(slab, tmC, C, ldc, row0, col0, acc, s, 64);
   }
   // v = 128 bytes of old C from column col0 on, of this lane's row. They come in as they are stored, whole
   // row segments by eight lanes each, and turn through the buffer that put128 fills next. Loads of a lane's own
@@ -178,7 +202,7 @@ struct StoreEpilogue {
       for (int e = 0; e < 4; ++e) v[4 * c + e] = w[e];
     }
   }
-  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape& s) {
+  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape& s, int left) {
     const int row0 = row - static_cast<int>(threadIdx.x & 31);
     if (row0 >= s.M || col0 >= s.N) return;   // uniform over the warp
     if constexpr (sizeof(OutT) == 2) {
@@ -192,10 +216,10 @@ struct StoreEpilogue {
         }
       }
       pack_row64(w, a0, a1);
-      store_row(slab, tmC, C, ldc, row0, col0, w, s);
+      store_row(slab, tmC, C, ldc, row0, col0, w, s, left);
     } else {
       store_fp32(a0, row0, col0, s);
-      if (col0 + 32 < s.N) store_fp32(a1, row0, col0 + 32, s);
+      if (left > 32 && col0 + 32 < s.N) store_fp32(a1, row0, col0 + 32, s);
     }
   }
 };
@@ -223,14 +247,14 @@ struct ScaledStoreEpilogue {
       w[2 * v + 1] = pack_bf16x2(__uint_as_float(acc[4 * v + 2]) * rs * cs.z, __uint_as_float(acc[4 * v + 3]) * rs * cs.w);
     }
   }
-  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape& s) {
+  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape& s, int left) {
     const int row0 = row - static_cast<int>(threadIdx.x & 31);
     if (row0 >= s.M || col0 >= s.N) return;
     const float rs = row < s.M ? row_scale[row] : 0.f;
     uint32_t w[32];
     scale32(w, a0, rs, col0, s.N);
     scale32(w + 16, a1, rs, col0 + 32, s.N);
-    store_row(slab, tmC, C, ldc, row0, col0, w, s);
+    store_row(slab, tmC, C, ldc, row0, col0, w, s, left);
   }
 };
 
@@ -249,7 +273,7 @@ struct SwiGluEpilogue {
   __device__ __forceinline__ void tile_end(int, int) {}
   __device__ __forceinline__ void drain() { slab.drain(); }
   // col0 is the first column of the 64-wide (gate|up) block
-  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&g)[32], uint32_t (&u)[32], const GemmShape& s) {
+  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&g)[32], uint32_t (&u)[32], const GemmShape& s, int) {
     const int lane = threadIdx.x & 31;
     const int row0 = row - lane;
     if (row0 >= s.M || col0 >= s.N) return;

@@ -40,6 +40,10 @@ struct GemmShape {
   int m_major = 0;     // 1: walk all N tiles of an M tile before the next M tile
   int n_rot = 0;       // tile_n = (raw + n_rot) % tiles_n
   int group_m = 0;     // default order only: M tiles are walked in groups of this many (0 = all)
+  // CTA pairs only, see TileSpan:
+  int bn = 0;               // columns of a tile (0 = the kernel's BN)
+  int halve_from = 1 << 30; // tiles from this number on are computed as two halves
+  int b_box = 0;            // K-major B: rows of a load's box (0 = a CTA's share of a tile, BN / 2)
 };
 
 // The tile id -> (tile_m, tile_n) map. Default: M fastest inside a group of group_m M tiles, so
@@ -70,7 +74,9 @@ __device__ __forceinline__ void tile_coords(const GemmShape& s, int tile, int& t
 
 // Epilogue functor contract:
 //   __device__ void operator()(int row, int col0, const uint32_t (&acc)[32], const GemmShape&)
-// called by one thread per accumulator row for 32 consecutive columns starting at col0 (fp32 bits).
+// called by one thread per accumulator row for 32 consecutive columns starting at col0 (fp32 bits), or with kPair
+//   __device__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape&, int left)
+// for 64, of which the first `left` (32 or at least 64) belong to the tile.
 // Hooks: tile_begin(tm, tn) / tile_end(tm, tn) and, after the last tile, drain(), called by every
 // epilogue thread.
 
@@ -226,7 +232,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
           tmem_ld_32x32(taddr + c * 64, acc0);
           tmem_ld_32x32(taddr + c * 64 + 32, acc1);
           tmem_ld_wait();
-          epi(row, tn * BN + c * 64, acc0, acc1, shape);
+          epi(row, tn * BN + c * 64, acc0, acc1, shape, BN - c * 64);
         }
       } else {
 #pragma unroll 1

@@ -32,6 +32,28 @@ struct Gemm2Smem {
 };
 constexpr int GEMM2_BM = 256;  // rows per cluster tile
 
+// What a pair works on at a time: columns [col0, col0 + width) of tile row tm. The last, partly filled wave
+// of tiles leaves pairs idle; where halving its tiles fills them (GemmShape::halve_from is then the number of
+// tiles in whole waves) it takes the time of a narrow wave instead of a wide one.
+struct TileSpan {
+  int tm, tn, col0, width;
+};
+__device__ __forceinline__ int tile_items(const GemmShape& s) {
+  const int tiles = s.tiles_m * s.tiles_n;
+  return tiles <= s.halve_from ? tiles : 2 * tiles - s.halve_from;
+}
+template <int BN>
+__device__ __forceinline__ TileSpan tile_span(const GemmShape& s, int item) {
+  TileSpan t;
+  const int bn = s.bn ? s.bn : BN;
+  const bool half = item >= s.halve_from;
+  const int beyond = item - s.halve_from;
+  tile_coords(s, half ? s.halve_from + (beyond >> 1) : item, t.tm, t.tn);
+  t.col0 = t.tn * bn + (half && (beyond & 1) ? bn / 2 : 0);
+  t.width = half ? bn / 2 : bn;
+  return t;
+}
+
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -105,6 +127,8 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
 // 128-row tile (2 * pair tile + rank in the pair), so gates and epilogues written for the one-CTA
 // mainloop work unchanged. shape.cta_first / num_ctas (both even) restrict the GEMM to a part of
 // the grid.
+// A tile is 256 rows and BN columns, or shape.bn of them (a multiple of 32, at most BN); its columns and
+// those of the halves of the last wave come from tile_span.
 // FP8: both operands are 1-byte e4m3, K-major only; a k-block is then 128 elements (the same 128
 // bytes per row, so stages, swizzle and descriptors do not change) and one MMA covers K = 32.
 template <int BN, bool A_MN, bool B_MN, class Epilogue, class LoadGate, bool FP8 = false>
@@ -114,7 +138,6 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
   static_assert(BN == 128 || BN == 256, "cluster tile is 256 x 128 or 256 x 256");
   static_assert(!FP8 || (!A_MN && !B_MN), "fp8 operands are K-major");
   constexpr int BK_ELEMS = FP8 ? 2 * GEMM_BK : GEMM_BK;   // elements per 128-byte row of a stage
-  constexpr int HALF_N = BN / 2;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();   // 0 = leader
@@ -155,7 +178,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int num_tiles = shape.tiles_m * shape.tiles_n;
+  const int num_items = tile_items(shape);
   const int num_kb = (shape.K + BK_ELEMS - 1) / BK_ELEMS;
   const int pair_id = (static_cast<int>(blockIdx.x) - shape.cta_first) >> 1;
   const int pair_stride = (shape.num_ctas > 0 ? shape.num_ctas : static_cast<int>(gridDim.x)) >> 1;
@@ -166,12 +189,15 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = pair_id; tile < num_tiles && ok; tile += pair_stride) {
-        int tm, tn;
-        tile_coords(shape, tile, tm, tn);
-        const int row0 = tm * GEMM2_BM + static_cast<int>(rank) * 128;   // this CTA's rows of A
-        const int col0 = tn * BN + static_cast<int>(rank) * HALF_N;   // this CTA's half of B
-        if (!gate.wait_tile(2 * tm + static_cast<int>(rank), tn, abort_flag, err_word)) break;
+      const int box = shape.b_box ? shape.b_box : BN / 2;
+      for (int item = pair_id; item < num_items && ok; item += pair_stride) {
+        const TileSpan t = tile_span<BN>(shape, item);
+        const int half = t.width >> 1;
+        const int row0 = t.tm * GEMM2_BM + static_cast<int>(rank) * 128;   // this CTA's rows of A
+        const int col0 = t.col0 + static_cast<int>(rank) * half;   // this CTA's half of B
+        const int b_boxes = B_MN ? (half + 63) / 64 : half / box;
+        const uint32_t pair_bytes = 2 * (S::A_BYTES + b_boxes * (B_MN ? 64 : box) * 128);
+        if (!gate.wait_tile(2 * t.tm + static_cast<int>(rank), t.tn, abort_flag, err_word)) break;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1, abort_flag, err_word, DEV_ERR_EMPTY_BAR_TIMEOUT,
                                  GEMM_WAIT_LIMIT_NS)) {
@@ -181,7 +207,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
           const uint32_t a_dst = smem_base + stage * S::STAGE_BYTES;
           const uint32_t b_dst = a_dst + S::A_BYTES;
           const uint32_t bar = map_to_cta(full_bar(stage), 0);
-          if (leader) mbar_expect_tx(full_bar(stage), 2 * S::STAGE_BYTES);  // both CTAs' bytes
+          if (leader) mbar_expect_tx(full_bar(stage), pair_bytes);  // both CTAs' bytes
           if constexpr (!A_MN) {
             tma_load_2d_pair(a_dst, tmA, kb * BK_ELEMS, row0, bar);
           } else {
@@ -189,10 +215,9 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
             for (int j = 0; j < 2; ++j) tma_load_2d_pair(a_dst + j * 8192, tmA, row0 + j * 64, kb * GEMM_BK, bar);
           }
           if constexpr (!B_MN) {
-            tma_load_2d_pair(b_dst, tmB, kb * BK_ELEMS, col0, bar);
+            for (int j = 0; j < b_boxes; ++j) tma_load_2d_pair(b_dst + j * box * 128, tmB, kb * BK_ELEMS, col0 + j * box, bar);
           } else {
-#pragma unroll
-            for (int j = 0; j < HALF_N / 64; ++j) tma_load_2d_pair(b_dst + j * 8192, tmB, col0 + j * 64, kb * GEMM_BK, bar);
+            for (int j = 0; j < b_boxes; ++j) tma_load_2d_pair(b_dst + j * 8192, tmB, col0 + j * 64, kb * GEMM_BK, bar);
           }
           if (++stage == S::STAGES) {
             stage = 0;
@@ -205,13 +230,13 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     if (leader && elect_one_sync()) {
       // operand format field: 1 = bf16 for kind::f16, 0 = e4m3 for kind::f8f6f4
-      constexpr uint32_t idesc = make_instr_desc(FP8 ? 0 : 1, FP8 ? 0 : 1, GEMM2_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
       int acc_buf = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int tile = pair_id; tile < num_tiles && ok; tile += pair_stride) {
+      for (int item = pair_id; item < num_items && ok; item += pair_stride) {
+        const uint32_t idesc = make_instr_desc(FP8 ? 0 : 1, FP8 ? 0 : 1, GEMM2_BM, tile_span<BN>(shape, item).width, A_MN ? 1 : 0, B_MN ? 1 : 0);
         if (!mbar_wait_bounded(tempty_bar(acc_buf), acc_phase ^ 1, abort_flag, err_word, DEV_ERR_TMEM_EMPTY_TIMEOUT,
                                GEMM_WAIT_LIMIT_NS))
           break;
@@ -253,38 +278,37 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
     const int quarter = warp & 3;
     int acc_buf = 0;
     uint32_t acc_phase = 0;
-    for (int tile = pair_id; tile < num_tiles; tile += pair_stride) {
-      int tm, tn;
-      tile_coords(shape, tile, tm, tn);
+    for (int item = pair_id; item < num_items; item += pair_stride) {
+      const TileSpan t = tile_span<BN>(shape, item);
       if (!mbar_wait_bounded(tfull_bar(acc_buf), acc_phase, abort_flag, err_word, DEV_ERR_TMEM_FULL_TIMEOUT,
                              GEMM_WAIT_LIMIT_NS))
         break;
       tc_fence_after();
-      epi.tile_begin(2 * tm + static_cast<int>(rank), tn);
-      const int row = tm * GEMM2_BM + static_cast<int>(rank) * 128 + quarter * 32 + lane;
+      epi.tile_begin(2 * t.tm + static_cast<int>(rank), t.tn);
+      const int row = t.tm * GEMM2_BM + static_cast<int>(rank) * 128 + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc_buf * BN;
       if constexpr (Epilogue::kPair) {
 #pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
+        for (int c = 0; c < t.width; c += 64) {
           uint32_t acc0[32], acc1[32];
-          tmem_ld_32x32(taddr + c * 64, acc0);
-          tmem_ld_32x32(taddr + c * 64 + 32, acc1);
+          tmem_ld_32x32(taddr + c, acc0);
+          tmem_ld_32x32(taddr + c + 32, acc1);
           tmem_ld_wait();
-          epi(row, tn * BN + c * 64, acc0, acc1, shape);
+          epi(row, t.col0 + c, acc0, acc1, shape, t.width - c);
         }
       } else {
 #pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
+        for (int c = 0; c < t.width; c += 32) {
           uint32_t acc[32];
-          tmem_ld_32x32(taddr + c * 32, acc);
+          tmem_ld_32x32(taddr + c, acc);
           tmem_ld_wait();
-          epi(row, tn * BN + c * 32, acc, shape);
+          epi(row, t.col0 + c, acc, shape);
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(map_to_cta(tempty_bar(acc_buf), 0));
-      epi.tile_end(2 * tm + static_cast<int>(rank), tn);
+      epi.tile_end(2 * t.tm + static_cast<int>(rank), t.tn);
       acc_buf ^= 1;
       if (acc_buf == 0) acc_phase ^= 1;
     }

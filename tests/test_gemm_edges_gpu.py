@@ -181,3 +181,69 @@ def test_fp8_widths_that_are_no_multiple_of_a_vector(M, N, K):
     # bf16 rounding of the result, two fp32 roundings of the scales, fp32 sums
     assert ((pad[:M, :N].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (K + 4) * 2.0 ** -24 * mag).all()
     assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("width,halves", [(128, 0), (160, 0), (192, 0), (224, 0), (256, 0), (256, 1)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_every_tile_width_and_the_halved_last_wave(width, halves, out_dtype, a_mn, b_mn):
+    """Tiles that end inside a 64-column slab, beside others and at the last column; rows, columns and K that fill
+    no tile; one tile and 126 of them (74 whole ones and a last wave whose halves may lie beyond the last column)."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    ll, vp = ctypes.c_longlong, ctypes.c_void_p
+    step = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -24
+    for M, N, K in ((256, 128, 64), (296, 333, 200), (512, 1027, 72), (2304, 3330, 136)):
+        g = torch.Generator(device="cuda").manual_seed(M + width)
+        a, b = _padded(*((K, M) if a_mn else (M, K)), g), _padded(*((K, N) if b_mn else (N, K)), g)
+        A, B = (a.T if a_mn else a).double(), (b if b_mn else b.T).double()
+        ref, mag = A @ B, A.abs() @ B.abs()
+        pad = torch.full((M + 1, (N + 15) // 8 * 8), 7.0, device="cuda", dtype=out_dtype)
+        want = torch.zeros_like(ref)
+        for accumulate in (0, 1):
+            rc = _lib.load().b200_gemm_bf16_tiles(
+                vp(a.data_ptr()), vp(b.data_ptr()), vp(pad.data_ptr()), M, N, K, ll(a.stride(0)), ll(b.stride(0)),
+                ll(pad.stride(0)), int(a_mn), int(b_mn), int(out_dtype == torch.float32), accumulate, width, halves,
+                vp(_lib.stream_ptr()))
+            assert rc == 0
+            want = want + ref
+            # fp32 sums of K exact products in any order, one rounding of the output
+            assert ((pad[:M, :N].double() - want).abs() <= K * 2.0 ** -24 * mag + 2 * step * want.abs()).all()
+            want = pad[:M, :N].double()
+        assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
+
+
+def _tiles(M, N, K, b_mn=False):
+    """(width, halves) that the automatic choice runs on, for operands with contiguous rows."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    w, h = ctypes.c_int(), ctypes.c_int()
+    ll = ctypes.c_longlong
+    assert _lib.load().b200_gemm_tiles(M, N, K, ll(K), ll(N if b_mn else K), int(b_mn), ctypes.byref(w), ctypes.byref(h)) == 0
+    return w.value, h.value
+
+
+@pytest.mark.parametrize("M,N,K,b_mn,want", [
+    (4096, 4096, 4096, False, (256, 1)), (4096, 14336, 4096, False, (224, 0)), (4096, 28672, 4096, True, (256, 1)),
+    (384, 10736, 3712, False, (160, 0)), (1280, 7744, 328, False, (192, 0)),
+    (1000, 2568, 5160, False, (160, 0)), (1000, 2568, 5160, True, (256, 0)),   # rows off cache lines
+    (768, 256, 768, False, (128, 0)), (1920, 4280, 824, False, (256, 0))])
+def test_tiles_follow_the_waves_that_they_fill(M, N, K, b_mn, want):
+    """Choices that were measured to be the faster ones."""
+    assert _tiles(M, N, K, b_mn) == want
+
+
+@pytest.mark.parametrize("M,N,K", [(4096, 2072, 256), (2304, 3332, 144), (513, 300, 272)])
+def test_fp8_product_on_every_kind_of_tile(M, N, K):
+    """A last wave of halves, a ragged width, single tiles."""
+    from aws_ofi_nccl_b200.ops.gemm import gemm_fp8, quantize_rows_fp8
+
+    xq, xs = quantize_rows_fp8(torch.randn(M, K, device="cuda").bfloat16())
+    wq, ws = quantize_rows_fp8(torch.randn(N, K, device="cuda").bfloat16())
+    X, W = xq.double() * xs.double()[:, None], wq.double() * ws.double()[:, None]
+    ref, mag = X @ W.T, X.abs() @ W.T.abs()
+    pad = torch.full((M + 1, (N + 15) // 8 * 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm_fp8(xq, wq, xs, ws, out=pad[:M, :N])
+    # bf16 rounding of the result, two fp32 roundings of the scales, fp32 sums
+    assert ((pad[:M, :N].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (K + 4) * 2.0 ** -24 * mag).all()
+    assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
