@@ -300,21 +300,20 @@ struct GemmChoice {
 
 // Tiles of a product on CTA pairs whose better plain width is `bn`; a_low, b_low: what decides how the operands' rows
 // lie on cache lines. A wave of narrower tiles costs more than their share of a wide one: their loads bring the
-// same rows of A for fewer columns, and an SM takes in 64 bytes a clock. Rows off cache lines take three clocks
-// each instead of two, and the boxes of an N-major B are 64 columns, so that 160 and 224 columns (80 and 112
-// for a CTA) load as much as 256. The costs are medians over 110 products of 256 to 8192 rows, 128 to 28672
-// columns and K from 64 to 16040 in three majors; the rule's choice took 0.971 of the plain width's time on average
-// there, the best choice 0.962, and none more than 1.025. What it gains is the last wave: 4096 x 4096 x
-// 14336, 256 tiles for 74 pairs, takes 333 us in four wide waves, 363 in seven narrow ones, 308 with the last of
-// four halved; 4096 x 14336 x 4096 343 us, 325 with 14 waves of 224 columns for 13 of 256.
+// same rows of A for fewer columns. Rows off cache lines take the loads half as long again, and the boxes of an N-major B
+// are 64 columns, so that 160 and 224 columns (80 and 112 for a CTA) load as much as 256. The costs are medians over
+// 140 products of 256 to 8192 rows, 128 to 28672 columns and K from 64 to 16040 in three majors; the rule's choice
+// took 0.977 of the plain width's time on average there, the best choice 0.969, and none more than 1.03. What it
+// gains is the last wave: 4096 x 4096 x 14336, 256 tiles for 74 pairs, takes 333 us in four wide waves and 308 with
+// the last of them halved; 4096 x 6144 x 4096 132 us, 123 in five waves of 192 columns for six of 256.
 static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint64_t b_low, int units, int bn) {
   struct Costs {
     double at[5];   // 128, 160, 192, 224, 256 columns
   };
   static constexpr double NO = 9;
-  static constexpr Costs ON_LINES[2] = {{{.635, .72, .79, .88, 1}}, {{.635, .79, .81, .89, 1}}};
-  static constexpr Costs BETWEEN[2] = {{{.635, .76, .83, .90, 1}}, {{.64, NO, .90, .95, 1}}};
-  static constexpr Costs OFF_LINES[2] = {{{.72, .82, .88, .95, 1}}, {{.72, NO, NO, NO, 1}}};
+  static constexpr Costs ON_LINES[2] = {{{.58, .70, .785, .90, 1}}, {{.58, .79, .81, .90, 1}}};
+  static constexpr Costs BETWEEN[2] = {{{.60, .72, .80, .90, 1}}, {{.605, NO, .90, .95, 1}}};
+  static constexpr Costs OFF_LINES[2] = {{{.72, .79, .86, .925, 1}}, {{.72, NO, NO, NO, 1}}};
   const bool a_lines = a_low % 128 == 0, b_lines = b_low % 128 == 0;
   const Costs& c = a_lines && b_lines ? ON_LINES[b_mn] : a_lines || b_lines || (a_low | b_low) % 64 == 0 ? BETWEEN[b_mn] : OFF_LINES[b_mn];
   const int64_t rows = (M + GEMM2_BM - 1) / GEMM2_BM;

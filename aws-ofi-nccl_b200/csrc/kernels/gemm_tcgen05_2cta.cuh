@@ -69,8 +69,12 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
+// Hands tensor memory back: what it orders are tcgen05 operations, by the tcgen05 fences on both sides, and no other
+// memory. As a release at cluster scope it waited for everything that the warp had stored, 1600 clocks a tile: the
+// weight gradient 4096 x 14336 of 128 tokens (two k-blocks per tile) takes 37 us, 47 with it (39
+// and 60 in narrow tiles).
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Tiled load into this CTA's shared memory whose byte count is reported to a barrier of the pair's
 // leader (`bar_cluster` is a shared::cluster address).
