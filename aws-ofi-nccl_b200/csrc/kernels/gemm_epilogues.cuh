@@ -12,6 +12,7 @@
 // 192 -> 158 us, one 256 x 768 x 256 product 12 -> 7 us.
 #pragma once
 #include "gemm_tcgen05.cuh"
+#include "swiglu_math.cuh"
 
 namespace b200 {
 
@@ -258,6 +259,24 @@ struct ScaledStoreEpilogue {
   }
 };
 
+// silu(g) * u of 32 columns, two to a word
+__device__ __forceinline__ void swiglu32(uint32_t* act, const uint32_t (&g)[32], const uint32_t (&u)[32]) {
+  bool ordinary = true;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) ordinary &= fabsf(__uint_as_float(g[j])) < ORDINARY_GATE;
+  if (ordinary) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      act[j] = pack_bf16x2(silu_ordinary(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
+                           silu_ordinary(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      act[j] = pack_bf16x2(silu_rare(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
+                           silu_rare(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]));
+  }
+}
+
 // SwiGLU fused into the up/gate GEMM. The weight rows are interleaved in blocks of 64 output
 // columns: 32 gate columns followed by their 32 up columns, so one call sees a gate chunk and the
 // matching up chunk and writes act = silu(gate) * up (and, optionally, the raw gate|up pair that
@@ -278,13 +297,7 @@ struct SwiGluEpilogue {
     const int row0 = row - lane;
     if (row0 >= s.M || col0 >= s.N) return;
     uint32_t act[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float g0 = __uint_as_float(g[2 * j]), g1 = __uint_as_float(g[2 * j + 1]);
-      const float a0 = g0 / (1.f + __expf(-g0)) * __uint_as_float(u[2 * j]);
-      const float a1 = g1 / (1.f + __expf(-g1)) * __uint_as_float(u[2 * j + 1]);
-      act[j] = pack_bf16x2(a0, a1);
-    }
+    swiglu32(act, g, u);
     if (lane == 0) tma_store_wait_read<0>();
     __syncwarp();
     if (keep_gu) {

@@ -7,6 +7,7 @@
 
 #include "b200ops.h"
 #include "host_util.h"
+#include "swiglu_math.cuh"
 
 namespace b200 {
 
@@ -304,10 +305,17 @@ __global__ void __launch_bounds__(256)
 
 // ------------------------------------------------------------------ SwiGLU on a fused [T, 2F] gate|up tensor
 // Element vectors are spread over the grid as (row, vector in the row); the row comes from a 32-bit
-// division where the number of vectors allows it (the launcher checks): 73 us at 4096 x 14336 (CUDA events
-// around the launch, L2 flushed), 80 with a 64-bit one. One vector per thread and pass: with two, 90 us,
-// since an IEEE division is a sequence that does not interleave with another. The reciprocal unit takes
-// 71 but has twice the division's rounding error.
+// division where the number of vectors allows it (the launcher checks). One vector per thread and pass; carrying row and
+// vector along instead of dividing takes as long. 4096 x 14336, L2 flushed: 60 us;
+// 72 with IEEE divisions, cached accesses and a quarter of the CTAs.
+// Read once, written once: neither is worth a place in the caches.
+__device__ __forceinline__ Bf16x8 load_stream(const Bf16x8* p) {
+  const uint4 r = __ldcs(reinterpret_cast<const uint4*>(p));
+  return *reinterpret_cast<const Bf16x8*>(&r);
+}
+__device__ __forceinline__ void store_stream(Bf16x8* p, const Bf16x8& v) {
+  __stcs(reinterpret_cast<uint4*>(p), *reinterpret_cast<const uint4*>(&v));
+}
 template <typename Index>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, int64_t T, int F) {
   const Index nvec = static_cast<Index>(T * F / 8), fv = F / 8;
@@ -315,17 +323,16 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict_
     const Index t = k / fv, c = k - t * fv;
     const Bf16x8* row = reinterpret_cast<const Bf16x8*>(gu) + static_cast<int64_t>(t) * 2 * fv;
     float g[8], u[8], o[8];
-    unpack8(row[c], g);
-    unpack8(row[fv + c], u);
+    unpack8(load_stream(row + c), g);
+    unpack8(load_stream(row + fv + c), u);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
-    reinterpret_cast<Bf16x8*>(out)[k] = pack8(o);
+    for (int j = 0; j < 8; ++j) o[j] = silu(g[j]) * u[j];
+    store_stream(reinterpret_cast<Bf16x8*>(out) + k, pack8(o));
   }
 }
 // dgu[T,2F] from dout[T,F] and the saved gate|up. INTERLEAVED: gate and up alternate in blocks of
 // 32 columns (the layout the fused GEMM+SwiGLU epilogue produces) instead of two halves. One vector per
-// thread and pass: three loads and two stores already, and more registers cost resident warps (105 -> 112 us
-// with two vectors). 101 us at 4096 x 14336, timed as above; 111 with a 64-bit division for the row.
+// thread and pass: three loads and two stores already. 4096 x 14336, timed as above: 96 us; 101.
 template <bool INTERLEAVED, typename Index>
 __global__ void __launch_bounds__(256)
     swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu, int64_t T, int F) {
@@ -340,21 +347,21 @@ __global__ void __launch_bounds__(256)
       gi = static_cast<int64_t>(t) * 2 * fv + (k - t * fv);
       ui = gi + fv;
     }
-    const Bf16x8 gv = reinterpret_cast<const Bf16x8*>(gu)[gi], uv = reinterpret_cast<const Bf16x8*>(gu)[ui];
-    const Bf16x8 dv = reinterpret_cast<const Bf16x8*>(dout)[k];
+    const Bf16x8 gv = load_stream(reinterpret_cast<const Bf16x8*>(gu) + gi), uv = load_stream(reinterpret_cast<const Bf16x8*>(gu) + ui);
+    const Bf16x8 dv = load_stream(reinterpret_cast<const Bf16x8*>(dout) + k);
     float g[8], u[8], d[8], dg[8], du[8];
     unpack8(gv, g);
     unpack8(uv, u);
     unpack8(dv, d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float s = 1.f / (1.f + __expf(-g[j]));
+      const float s = logistic(g[j]);
       const float silu = g[j] * s;
       du[j] = d[j] * silu;
       dg[j] = d[j] * u[j] * (s + silu * (1.f - s));
     }
-    reinterpret_cast<Bf16x8*>(dgu)[gi] = pack8(dg);
-    reinterpret_cast<Bf16x8*>(dgu)[ui] = pack8(du);
+    store_stream(reinterpret_cast<Bf16x8*>(dgu) + gi, pack8(dg));
+    store_stream(reinterpret_cast<Bf16x8*>(dgu) + ui, pack8(du));
   }
 }
 
@@ -597,9 +604,13 @@ static bool aligned16(const P*... p) {
   return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) == 0;
 }
 
-static inline int grid_for(int64_t work_items, int threads) {
+// CTAs for a grid-stride loop over `work_items`, at most per_sm for every SM. With no more than run at once (8 of 256
+// threads) the SMs that memory serves last finish last; several times as many even that out, until a thread
+// has a single pass left: AdamW over 218 M parameters takes 1032 us with 16
+// CTAs per SM, 1004 with 64, 975 with 256 and 1060 with one pass per thread (CUDA events, L2 flushed before).
+static inline int grid_for(int64_t work_items, int threads, int per_sm = 16) {
   int64_t b = (work_items + threads - 1) / threads;
-  const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
+  const int64_t cap = static_cast<int64_t>(sm_count()) * per_sm;
   if (b > cap) b = cap;
   if (b < 1) b = 1;
   return static_cast<int>(b);
@@ -678,7 +689,7 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
 int b200_swiglu_fwd(const void* gu, void* out, long long T, int F, void* stream) {
   b200::ensure_context();
   if (F % 8 || !aligned16(gu, out)) return B200_ERR_BAD_ARG;
-  const int grid = grid_for(T * F / 8, 256);
+  const int grid = grid_for(T * F / 8, 256, 64);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto GU = static_cast<const bf16*>(gu);
   auto O = static_cast<bf16*>(out);
@@ -692,7 +703,7 @@ int b200_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, in
   b200::ensure_context();
   if (F % 8 || !aligned16(dout, gu, dgu)) return B200_ERR_BAD_ARG;
   auto kern = swiglu_small(T, F) ? swiglu_bwd_kernel<false, unsigned> : swiglu_bwd_kernel<false, int64_t>;
-  kern<<<grid_for(T * F / 8, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  kern<<<grid_for(T * F / 8, 256, 64), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(dout), static_cast<const bf16*>(gu), static_cast<bf16*>(dgu), T, F);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -701,7 +712,7 @@ int b200_swiglu_bwd_interleaved(const void* dout, const void* gu, void* dgu, lon
   b200::ensure_context();
   if (F % 32 || !aligned16(dout, gu, dgu)) return B200_ERR_BAD_ARG;
   auto kern = swiglu_small(T, F) ? swiglu_bwd_kernel<true, unsigned> : swiglu_bwd_kernel<true, int64_t>;
-  kern<<<grid_for(T * F / 8, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  kern<<<grid_for(T * F / 8, 256, 64), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(dout), static_cast<const bf16*>(gu), static_cast<bf16*>(dgu), T, F);
   B200_CUDA_OK(cudaGetLastError());
   return 0;

@@ -1,0 +1,38 @@
+// silu and the logistic function as the SwiGLU kernels and the epilogues of the MLP's products use them.
+//
+// IEEE division is a sequence with a branch for rare operands, and elements on either side of such a branch do not
+// overlap: a warp that is alone on its scheduler, as in an epilogue, took 125 clocks for each. The quotients are
+// written out instead, for denominators that need no such branch: the reciprocal unit's value and one residual
+// correction of the quotient (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990), which rounds like IEEE division. What errs is the exponential. Against 64
+// bits, over bf16's gates within 20, silu is off by 0.16 ulp on average and the logistic function by 0.13, with IEEE
+// division by 0.17 and 0.15; over normally distributed gates of 32 bits silu_ordinary by 0.82 like the division.
+#pragma once
+
+namespace b200 {
+
+// n / d for 1 <= d < 2^126 and finite n
+__device__ __forceinline__ float quotient(float n, float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = n * r;
+  return fmaf(r, fmaf(-d, q, n), q);
+}
+
+// With t = exp(-|g|) the denominator lies in [1, 2] whatever the gate.
+__device__ __forceinline__ float silu(float g) {
+  const float t = __expf(-fabsf(g));
+  const float q = quotient(g < 0.f ? g * t : g, 1.f + t);
+  return g == INFINITY ? g : q;
+}
+__device__ __forceinline__ float logistic(float g) {
+  const float t = __expf(-fabsf(g));
+  return quotient(g < 0.f ? t : 1.f, 1.f + t);
+}
+
+// For gates of 32 bits, where the rounding of g * t would show: 1 + exp(-g) itself, while it is in range.
+constexpr float ORDINARY_GATE = 80.f;
+__device__ __forceinline__ float silu_ordinary(float g) { return quotient(g, 1.f + __expf(-g)); }
+__device__ __noinline__ inline float silu_rare(float g) { return g / (1.f + __expf(-g)); }
+
+}  // namespace b200

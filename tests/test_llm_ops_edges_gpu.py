@@ -100,3 +100,27 @@ def test_nothing_is_differentiated_through_overwritten_logits():
         torch.autograd.grad(loss + logits.float().square().sum(), leaf, retain_graph=True)
     (d,) = torch.autograd.grad(loss, leaf)
     assert torch.equal(d, logits.detach())
+
+
+@pytest.mark.parametrize("F", [8, 72])
+def test_swiglu_of_rare_gates(F):
+    """Infinities, NaN and gates at both ends of the range whose division is written out."""
+    from aws_ofi_nccl_b200.ops import llm
+
+    gate = torch.tensor([80.0, -80.0, 79.5, -79.5, 88.5, -88.0, 120.0, -120.0, math.inf, -math.inf, math.nan, 0.0, -0.0, 1e-38, 3e38, -3e38],
+                        device="cuda")
+    g = torch.zeros(gate.numel(), F, device="cuda")
+    g[:, F // 2] = gate
+    gu = torch.cat((g, torch.full_like(g, 0.75)), -1).bfloat16().requires_grad_(True)
+    out = llm.swiglu(gu)
+    d = torch.full_like(out, 0.5)
+    (dgu,) = torch.autograd.grad(out, (gu,), d)
+    gf = gu.detach()[:, :F].float()
+    s = 1 / (1 + torch.exp(-gf))
+    want = gf / (1 + torch.exp(-gf)) * 0.75
+    silu = gf * s
+    want_d = torch.cat((0.5 * 0.75 * (s + silu * (1 - s)), 0.5 * silu), -1)
+    for a, b in ((out, want), (dgu, want_d)):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.bfloat16().isinf())
+        ok = b.isfinite()
+        _within(a.detach()[ok], b[ok].double(), 2 * BF, 1e-30)
