@@ -788,7 +788,7 @@ int b200_adamw(void* p, void* g, float* m, float* v, float* master, long long n,
   if (n % 8) return B200_ERR_BAD_ARG;
   const float bc1 = 1.f - powf(beta1, static_cast<float>(step));
   const float bc2 = 1.f - powf(beta2, static_cast<float>(step));
-  adamw_kernel<<<grid_for(n / 8, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  adamw_kernel<<<grid_for(n / 8, 256, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<bf16*>(p), static_cast<bf16*>(g), m, v, master, n, lr, beta1, beta2, eps, wd, bc1, bc2, grad_scale,
       zero_grad);
   B200_CUDA_OK(cudaGetLastError());

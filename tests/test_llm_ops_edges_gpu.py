@@ -124,3 +124,21 @@ def test_swiglu_of_rare_gates(F):
         assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.bfloat16().isinf())
         ok = b.isfinite()
         _within(a.detach()[ok], b[ok].double(), 2 * BF, 1e-30)
+
+
+@pytest.mark.parametrize("n", [8, 1024, 8 * 256 * 148 * 256 + 8])   # one vector; less than a CTA; one pass more than a full grid
+def test_adamw_over_the_whole_grid(n):
+    from aws_ofi_nccl_b200.ops import llm
+
+    p, g = torch.randn(n, device="cuda").bfloat16(), torch.randn(n, device="cuda").bfloat16()
+    m, v = torch.randn(n, device="cuda") * 0.1, torch.rand(n, device="cuda") * 0.01
+    w = p.float()
+    w0, terms = w.double(), 0.9 * m.double().abs() + 0.1 * g.double().abs()
+    em, ev = 0.9 * m.double() + 0.1 * g.double(), 0.95 * v.double() + 0.05 * g.double() ** 2
+    per_m = 1e-2 / (1 - 0.9 ** 3) / ((ev / (1 - 0.95 ** 3)).sqrt() + 1e-8)
+    llm.adamw_step(p, g, m, v, w, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3)
+    # fp32 holds 1 - beta to 4 ulp, 1 - beta^3 to 16; a handful of roundings besides
+    ulp = 2.0 ** -24
+    assert ((m - em).abs() <= 16 * ulp * terms).all() and ((v - ev).abs() <= 16 * ulp * ev).all()
+    assert ((w - (w0 * (1 - 1e-2 * 0.1) - per_m * em)).abs() <= 4 * ulp * w0.abs() + 64 * ulp * per_m * terms).all()
+    assert torch.equal(p, w.bfloat16()) and not g.any()
