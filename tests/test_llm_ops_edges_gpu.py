@@ -142,3 +142,46 @@ def test_adamw_over_the_whole_grid(n):
     assert ((m - em).abs() <= 16 * ulp * terms).all() and ((v - ev).abs() <= 16 * ulp * ev).all()
     assert ((w - (w0 * (1 - 1e-2 * 0.1) - per_m * em)).abs() <= 4 * ulp * w0.abs() + 64 * ulp * per_m * terms).all()
     assert torch.equal(p, w.bfloat16()) and not g.any()
+
+# a vector, a thread's vectors (one to eight), a cluster of two to eight CTAs and the widest row that it holds, each with
+# one element or vector more; the last is a row for two passes
+@pytest.mark.parametrize("T,V", [(1, 1), (5, 7), (3, 2048), (300, 2049), (4, 4104), (7, 8200), (5, 16384), (40, 16392), (3, 32771),
+                                 (6, 65544), (20, 128256), (2, 131072), (2, 131073)])
+def test_cross_entropy(T, V):
+    from aws_ofi_nccl_b200.ops import llm
+
+    g = torch.Generator(device="cuda").manual_seed(T + V)
+    pad = torch.full((T, (V + 7) // 8 * 8 + 8), 5.0, device="cuda").bfloat16()
+    logits = pad[:, :V]
+    logits.copy_(torch.randn(T, V, device="cuda", generator=g) * 3)
+    if V > 64:
+        logits[0, :48] = -math.inf   # whole vectors that are masked out
+        logits[-1, V // 2:V // 2 + 3] = 60.0
+    targets = torch.randint(0, V, (T,), device="cuda", generator=g)
+    targets[0] = V - 1
+    if T > 2:
+        targets[1], targets[2] = -1, 0   # an ignored row
+    x = logits.double()
+    lse = torch.logsumexp(x, -1)
+    counts = targets >= 0
+    want_loss = torch.where(counts, lse - x.gather(1, targets.clamp_min(0)[:, None])[:, 0], torch.zeros_like(lse)).mean()
+    want = torch.exp(x - lse[:, None])
+    want.scatter_add_(1, targets.clamp_min(0)[:, None], -torch.ones_like(lse)[:, None])
+    want = torch.where(counts[:, None], want / T, torch.zeros_like(want))
+    loss = llm.cross_entropy(logits, targets)
+    finite = lse.isfinite() & (x.gather(1, targets.clamp_min(0)[:, None])[:, 0].isfinite() | ~counts)
+    assert finite.all()
+    # exponentials of arguments up to 90 whose product with log2(e) is rounded to 24 bits, and sums of them
+    err = 128 * 2.0 ** -24
+    assert abs(loss.double() - want_loss) <= err * (1 + lse.abs().max())
+    _within(logits, want, BF + err, err / T)
+    assert (pad[:, V:] == 5).all()
+
+
+def test_cross_entropy_of_a_row_with_nan_is_nan():
+    from aws_ofi_nccl_b200.ops import llm
+
+    logits = torch.randn(2, 128256, device="cuda").bfloat16()
+    logits[0, 16384:32768] = math.nan   # all that one CTA holds
+    targets = torch.zeros(2, device="cuda", dtype=torch.int64)
+    assert llm.cross_entropy(logits, targets).isnan()
