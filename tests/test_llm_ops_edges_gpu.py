@@ -185,3 +185,20 @@ def test_cross_entropy_of_a_row_with_nan_is_nan():
     logits[0, 16384:32768] = math.nan   # all that one CTA holds
     targets = torch.zeros(2, device="cuda", dtype=torch.int64)
     assert llm.cross_entropy(logits, targets).isnan()
+
+
+@pytest.mark.parametrize("T,K", [(1, 8), (9, 256), (17, 264), (5, 512), (9, 520), (3, 1032), (7, 2056), (300, 4096), (5, 4104), (3, 8200),
+                                 (2, 16384), (3, 16392), (1200, 16400)])
+def test_quantize_rows_fp8(T, K):
+    """Bit for bit: the scale is amax / 448, the values are rounded once."""
+    from aws_ofi_nccl_b200.ops.gemm import quantize_rows_fp8
+
+    x = torch.randn(T, K + 8, device="cuda").bfloat16()[:, :K]
+    x[0] *= 1e-3
+    if T > 2:
+        x[2] = 0
+    q, s = quantize_rows_fp8(x)
+    scale = x.float().abs().amax(-1).clamp_min(1e-12) * (1.0 / 448.0)
+    assert torch.equal(s, scale)
+    want = (x.float() * (1.0 / scale)[:, None]).clamp(-448, 448).to(torch.float8_e4m3fn)
+    assert torch.equal(q.view(torch.uint8), want.view(torch.uint8))
