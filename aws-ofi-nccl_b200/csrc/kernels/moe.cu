@@ -143,7 +143,7 @@ struct DispatchArgs {
   int32_t* cursor;           // [E]
   int32_t* row_of;           // [T][k] receive-buffer row of every (token, slot); -1 = dropped
   int32_t* local_row;        // [T][k] out: the same row where this rank owns the expert, else -1
-  __nv_bfloat16* local_out;  // bf16 payload: rows of this rank's own tokens go here as well, or null
+  __nv_bfloat16* local_out;  // rows of this rank's own tokens go here as well (as the dequantised values), or null
   size_t recv_off, scale_off, meta_off;  // window offsets on the receiving side
   int capacity_rows;
   unsigned int* done;
@@ -205,10 +205,23 @@ __device__ __forceinline__ uint2 quantize8(const float (&v)[8], float w, float& 
   return q;
 }
 
+// Eight e4m3 bytes times their scale, as bf16.
+__device__ __forceinline__ uint4 dequantize8(uint2 q, float scale) {
+  const __nv_fp8x2_storage_t* p = reinterpret_cast<const __nv_fp8x2_storage_t*>(&q);
+  __nv_bfloat162 o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[j], __NV_E4M3);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+    o[j] = __floats2bfloat162_rn(f.x * scale, f.y * scale);
+  }
+  return *reinterpret_cast<const uint4*>(o);
+}
+
 // A team per token: a wide one writes a destination row 2 KiB (fp8) or 4 KiB (bf16) at a time, where a warp
 // per token left every row 256 or 512 bytes at a time among thousands of others (4096 tokens x 7168, top-8,
 // routing included: fp8 95 -> 79 us, bf16 140 -> 120). Four CTAs per SM: with the registers of three the
-// fp8 call took 101 us. local_out doubles the stores of a bf16 call and saves reading the window back.
+// fp8 call took 101 us. local_out adds stores to the call and saves reading the window back.
 __global__ void __launch_bounds__(MOE_THREADS, 4) moe_dispatch_kernel(DispatchArgs a) {
   const GinDevHandle& h = a.h;
   const TokenTeam team(a.team_warps);
@@ -287,12 +300,14 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_dispatch_kernel(DispatchAr
         q = quantize8(v, 1.f, scale);
         if ((lane & 15) == 0) scale_buf[2 * c + (lane >> 4)] = scale;
       }
+      uint4 plain = make_uint4(0, 0, 0, 0);
+      if (a.fp8 && !weighted && a.local_out) plain = dequantize8(q, scale);
       for (int s = 0; s < a.k; ++s) {
         const int drank = slot_rank[s], drow = slot_row[s];
         const float w = slot_w[s];
         if (drow < 0) continue;  // uniform over the team
         uint8_t* dst = h.window[drank] + a.recv_off + static_cast<size_t>(drow) * row_bytes;
-        uint4* own = a.local_out && drank == h.rank   // bf16 only (the launcher checks)
+        uint4* own = a.local_out && drank == h.rank
                          ? reinterpret_cast<uint4*>(a.local_out) + static_cast<size_t>(drow) * (a.H / 8)
                          : nullptr;
         if (a.fp8) {
@@ -302,6 +317,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_dispatch_kernel(DispatchAr
               reinterpret_cast<float*>(h.window[drank] + a.scale_off)[static_cast<size_t>(drow) * groups + 2 * c + (lane >> 4)] = scale;
           }
           reinterpret_cast<uint2*>(dst)[c * 32 + lane] = q;
+          if (own) own[c * 32 + lane] = weighted ? dequantize8(q, scale) : plain;
         } else {
           uint4 r = raw;
           if (weighted) {
@@ -525,51 +541,58 @@ __global__ void __launch_bounds__(MOE_THREADS)
 constexpr int DEQUANT_PIECE = 128;
 __host__ __device__ inline int dequant_pieces(int H) { return (H / 8 + DEQUANT_PIECE - 1) / DEQUANT_PIECE; }
 
-// fp8 (e4m3) rows with one fp32 scale per 128 elements -> bf16. One warp per 1024 elements of a row; a lane takes 8 values
-// at a time, so that the warp's stores are 512 consecutive bytes, and four such loads are in flight: 32768 x
+// fp8 (e4m3) rows with one fp32 scale per 128 elements -> bf16. A warp takes 1024 elements of a row at a time, a lane 8
+// values, so that the warp's stores are 512 consecutive bytes, and four such loads are in flight: 32768 x
 // 7168 in 125 us (5.6 TB/s), 175 with a grid-stride loop over single vectors; 128 rows 8 us, 16 with a warp
 // for a whole row. With zero_tail the rows past
-// the last received one are written as zeros, in place of a fill of the whole output before (120 us).
+// the last received one are written as zeros, in place of a fill of the whole output before (120 us). With `meta`
+// the rows of rank `here` are in `out` already. Dispatch and combine of 4096 x 7168, top-8, with their gradients on one
+// rank: 889 us, 922 when every row was read back here.
 __global__ void __launch_bounds__(MOE_THREADS)
     fp8_dequant_rows_kernel(const uint8_t* q, const float* scales, __nv_bfloat16* out, const int32_t* rows_ptr, int rows_max,
-                            int H, int zero_tail) {
+                            int H, int zero_tail, const MoeMeta* meta, int here) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int rows = rows_ptr ? min(*rows_ptr, rows_max) : rows_max;
   const int vec = H / 8, groups = H / 128, pieces = dequant_pieces(H);
   const int64_t items = static_cast<int64_t>(zero_tail ? rows_max : rows) * pieces;
-  for (int64_t i = blockIdx.x * warps + warp; i < items; i += gridDim.x * warps) {
-    const int r = static_cast<int>(i / pieces);
-    const int v0 = static_cast<int>(i - static_cast<int64_t>(r) * pieces) * DEQUANT_PIECE + lane;
-    uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(r) * H);
-    constexpr int U = DEQUANT_PIECE / 32;
-    if (r >= rows) {
+  const int64_t all_warps = static_cast<int64_t>(gridDim.x) * warps;
+  // Pieces of one warp at a time: its lanes look their rows up together, and the warp goes on to those it has to do.
+  const int64_t share = (items + all_warps - 1) / all_warps;
+  const int batch = !meta ? 1 : share < 32 ? static_cast<int>(share) : 32;
+  for (int64_t i0 = (static_cast<int64_t>(blockIdx.x) * warps + warp) * batch; i0 < items; i0 += all_warps * batch) {
+    const int64_t mine = i0 + lane;
+    bool todo = lane < batch && mine < items;
+    if (meta && todo) {
+      const int64_t r = mine / pieces;
+      todo = r >= rows || meta[r].src_rank != here;
+    }
+    for (unsigned left = __ballot_sync(0xffffffffu, todo); left; left &= left - 1) {
+      const int64_t i = i0 + __ffs(left) - 1;
+      const int r = static_cast<int>(i / pieces);
+      const int v0 = static_cast<int>(i - static_cast<int64_t>(r) * pieces) * DEQUANT_PIECE + lane;
+      uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(r) * H);
+      constexpr int U = DEQUANT_PIECE / 32;
+      if (r >= rows) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (v0 + 32 * u < vec) dst[v0 + 32 * u] = make_uint4(0, 0, 0, 0);
+        continue;
+      }
+      const uint2* src = reinterpret_cast<const uint2*>(q + static_cast<size_t>(r) * H);
+      const float* sc = scales + static_cast<size_t>(r) * groups;
+      uint2 raw[U];
+      float s[U];
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (v0 + 32 * u < vec) dst[v0 + 32 * u] = make_uint4(0, 0, 0, 0);
-      continue;
-    }
-    const uint2* src = reinterpret_cast<const uint2*>(q + static_cast<size_t>(r) * H);
-    const float* sc = scales + static_cast<size_t>(r) * groups;
-    uint2 raw[U];
-    float s[U];
+        if (v0 + 32 * u < vec) {
+          raw[u] = src[v0 + 32 * u];
+          s[u] = sc[(v0 + 32 * u) / 16];
+        }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (v0 + 32 * u < vec) {
-        raw[u] = src[v0 + 32 * u];
-        s[u] = sc[(v0 + 32 * u) / 16];
+      for (int u = 0; u < U; ++u) {
+        if (v0 + 32 * u >= vec) break;
+        dst[v0 + 32 * u] = dequantize8(raw[u], s[u]);
       }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (v0 + 32 * u >= vec) break;
-      const __nv_fp8x2_storage_t* p = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw[u]);
-      __nv_bfloat162 o[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[j], __NV_E4M3);
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
-        o[j] = __floats2bfloat162_rn(f.x * s[u], f.y * s[u]);
-      }
-      dst[v0 + 32 * u] = *reinterpret_cast<const uint4*>(o);
     }
   }
 }
@@ -621,7 +644,7 @@ int b200_moe_dispatch(int comm, const void* x, const void* topk_idx, const void*
   if (H / 128 > 64) return B200_ERR_TOO_LARGE;
   const size_t row_bytes = fp8 ? static_cast<size_t>(H) : static_cast<size_t>(H) * 2;
   if (recv_off % 16 || meta_off % 16 || scale_off % 16) return B200_ERR_BAD_ARG;
-  if (!local_row || (local_out && (fp8 || reinterpret_cast<uintptr_t>(local_out) % 16))) return B200_ERR_BAD_ARG;
+  if (!local_row || reinterpret_cast<uintptr_t>(local_out) % 16) return B200_ERR_BAD_ARG;
   if (recv_off + row_bytes * capacity_rows > h.window_bytes || meta_off + 16ull * capacity_rows > h.window_bytes ||
       (fp8 && scale_off + 4ull * (H / 128) * capacity_rows > h.window_bytes))
     return B200_ERR_BAD_ARG;
@@ -693,7 +716,26 @@ int b200_fp8_dequant_rows(const void* q, const void* scales, void* out, const vo
   if (H % 128) return B200_ERR_BAD_ARG;
   fp8_dequant_rows_kernel<<<moe_grid(static_cast<int64_t>(rows_max) * dequant_pieces(H)), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint8_t*>(q), static_cast<const float*>(scales), static_cast<__nv_bfloat16*>(out),
-      static_cast<const int32_t*>(rows_ptr), rows_max, H, zero_tail);
+      static_cast<const int32_t*>(rows_ptr), rows_max, H, zero_tail, nullptr, 0);
+  B200_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// The fp8 rows of the last dispatch that other ranks sent -> out[capacity_rows][H]; this rank's own are there already
+// (dispatch's local_out). Rows past the last received one become zeros.
+int b200_moe_collect_rows_fp8(int comm, const void* rows_ptr, size_t recv_off, size_t scale_off, size_t meta_off, int capacity_rows,
+                              int H, void* out, void* stream) {
+  ensure_context();
+  const GinDevHandle* hp = comm_handle(comm);
+  if (!hp || !rows_ptr || !out || H % 128 || capacity_rows <= 0 || (recv_off | scale_off | meta_off) % 16) return B200_ERR_BAD_ARG;
+  const size_t rows = capacity_rows;
+  if (recv_off + H * rows > hp->window_bytes || scale_off + 4ull * (H / 128) * rows > hp->window_bytes ||
+      meta_off + 16ull * rows > hp->window_bytes)
+    return B200_ERR_BAD_ARG;
+  const uint8_t* window = static_cast<const uint8_t*>(hp->window[hp->rank]);
+  fp8_dequant_rows_kernel<<<moe_grid(static_cast<int64_t>(rows) * dequant_pieces(H)), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      window + recv_off, reinterpret_cast<const float*>(window + scale_off), static_cast<__nv_bfloat16*>(out),
+      static_cast<const int32_t*>(rows_ptr), capacity_rows, H, 1, reinterpret_cast<const MoeMeta*>(window + meta_off), hp->rank);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -28,6 +28,7 @@ _lib.register("b200_moe_route", [_i, _vp, _i, _i, _i, _sz, _vp, _vp, _vp, _vp, _
 _lib.register("b200_moe_dispatch", [_i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _sz, _sz, _sz,
                                     _i, _vp, _vp], _i)
 _lib.register("b200_moe_collect_rows", [_i, _vp, _sz, _sz, _i, _i, _i, _vp, _vp], _i)
+_lib.register("b200_moe_collect_rows_fp8", [_i, _vp, _sz, _sz, _sz, _i, _i, _vp, _vp], _i)
 _lib.register("b200_moe_combine", [_i, _vp, _vp, _i, _sz, _sz, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp], _i)
 _lib.register("b200_moe_combine_wgrad", [_vp, _vp, _vp, _vp, _i, _i, _i, _vp], _i)
 _lib.register("b200_fp8_dequant_rows", [_vp, _vp, _vp, _vp, _i, _i, _i, _vp], _i)
@@ -102,8 +103,8 @@ class ExpertParallel:
     def dispatch_raw(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.Tensor | None, *, fp8: bool,
                      use_saved_rows: bool = False, scale_by_weight: bool = False,
                      local_out: torch.Tensor | None = None) -> None:
-        """With ``local_out`` (bf16 payload, [capacity, H]) the rows of this rank's own tokens are stored
-        there as well as in the window; ``collect`` adds the others."""
+        """With ``local_out`` (bf16 [capacity, H]) the rows of this rank's own tokens are stored there as well as in
+        the window, those of an fp8 payload as the values that it stands for; ``collect`` adds the others."""
         assert x.shape == (self.T, self.H) and x.dtype == torch.bfloat16 and x.is_contiguous()
         rc = _lib.load().b200_moe_dispatch(
             self.comm.id, x.data_ptr(), topk_idx.data_ptr(), topk_w.data_ptr() if topk_w is not None else None,
@@ -112,6 +113,14 @@ class ExpertParallel:
             local_out.data_ptr() if local_out is not None else None, self.recv_off, self.scale_off, self.meta_off,
             self.capacity, self._done[1:].data_ptr(), _lib.stream_ptr())
         _lib.check(rc, "b200_moe_dispatch")
+
+    def collect_fp8(self, out: torch.Tensor) -> torch.Tensor:
+        """``collect`` with the local rows in place for an fp8 payload: the rows that other ranks sent, dequantised."""
+        rc = _lib.load().b200_moe_collect_rows_fp8(self.comm.id, self.expert_offsets[self.experts_local:].data_ptr(), self.recv_off,
+                                                   self.scale_off, self.meta_off, self.capacity, self.H, out.data_ptr(),
+                                                   _lib.stream_ptr())
+        _lib.check(rc, "b200_moe_collect_rows_fp8")
+        return out
 
     def collect(self, out: torch.Tensor, local_in_place: bool) -> torch.Tensor:
         """The bf16 rows of the last dispatch -> ``out`` [capacity, H]: all of them, or (``local_in_place``)
@@ -122,11 +131,11 @@ class ExpertParallel:
         _lib.check(rc, "b200_moe_collect_rows")
         return out
 
-    def _dispatch_rows(self, x, topk_idx, topk_w, **kw) -> torch.Tensor:
-        """bf16 dispatch into a tensor of its own: this rank's rows are not read back from the window."""
+    def _dispatch_rows(self, x, topk_idx, topk_w, fp8: bool = False, **kw) -> torch.Tensor:
+        """Dispatch into a bf16 tensor of its own: this rank's rows are not read back from the window."""
         rows = torch.empty(self.capacity, self.H, device=x.device, dtype=torch.bfloat16)
-        self.dispatch_raw(x, topk_idx, topk_w, fp8=False, local_out=rows, **kw)
-        return self.collect(rows, True)
+        self.dispatch_raw(x, topk_idx, topk_w, fp8=fp8, local_out=rows, **kw)
+        return self.collect_fp8(rows) if fp8 else self.collect(rows, True)
 
     def combine_raw(self, y_rows: torch.Tensor, topk_w: torch.Tensor | None, out: torch.Tensor,
                     cells_out: torch.Tensor | None = None) -> None:
@@ -168,10 +177,7 @@ class _Dispatch(torch.autograd.Function):
         ep.route(topk_idx)
         ep._last_topk_idx = topk_idx
         ctx.ep = ep
-        if fp8:
-            ep.dispatch_raw(x.contiguous(), topk_idx, topk_w, fp8=True)
-            return ep.dequant()
-        return ep._dispatch_rows(x.contiguous(), topk_idx, topk_w)
+        return ep._dispatch_rows(x.contiguous(), topk_idx, topk_w, fp8)
 
     @staticmethod
     def backward(ctx, d_rows):

@@ -176,3 +176,28 @@ def test_combine_sums_own_rows_and_delivered_cells(comm, T, H, k):
     terms = w.double()[..., None] * cells.double()
     # fp32 sums of k products, one rounding to bf16
     assert ((out.double() - terms.sum(1)).abs() <= 2.0 ** -8 * terms.sum(1).abs() + (k + 1) * 2.0 ** -24 * terms.abs().sum(1)).all()
+
+
+@pytest.mark.parametrize("T,H,k", [(1, 256, 1), (40, 1280, 3), (700, 768, 2), (3000, 768, 4)])
+def test_fp8_rows_are_those_of_the_window(comm, T, H, k):
+    """Dispatch stores this rank's rows as the values that their fp8 payload stands for; rows whose records name another
+    rank come from the window, rows that nobody sent are zeros."""
+    from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
+
+    E = 8
+    ep = ExpertParallel(comm, T, H, E, k, capacity_factor=1.5)
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    idx = torch.rand(T, E, device="cuda", generator=g).topk(k, dim=-1).indices.to(torch.int32).contiguous()
+    idx[T // 2:T // 2 + 30, 0] = -1   # fewer rows than capacity
+    x, w = torch.randn(T, H, device="cuda", generator=g).bfloat16(), torch.rand(T, k, device="cuda", generator=g)
+    rows = ep.dispatch(x, idx, w, True)
+    assert torch.equal(rows, ep.dequant())
+    n = int(ep.expert_offsets[-1].item())
+    remote = torch.rand(n, device="cuda", generator=g) < 0.5
+    ep.recv_meta()[:n, 3] = remote.int()
+    own = torch.full_like(rows, 3.0)
+    got = ep.collect_fp8(own.clone())
+    assert torch.equal(got[:n], torch.where(remote[:, None], rows[:n], own[:n])) and (got[n:] == 0).all()
+    # weighted rows are scaled and quantised one by one
+    ep.dispatch_raw(x, idx, w, fp8=True, use_saved_rows=True, scale_by_weight=True, local_out=own)
+    assert torch.equal(own[:n], ep.dequant()[:n])
