@@ -99,16 +99,16 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
 }
 
 // ---------------------------------------------------------------- CTA-pair variant (256 x 256 tile per cluster)
-template <int BN, bool A_MN, bool B_MN, typename OutT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+template <int BN, bool A_MN, bool B_MN, typename OutT, int EW>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Gemm2Smem<BN, EW>::THREADS, 1)
     gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                           const __grid_constant__ CUtensorMap tmC, OutT* C, int64_t ldc, GemmShape shape, int accumulate,
                           int* err_word) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   StoreEpilogue<OutT> epi{&tmC, C, ldc, accumulate, {}};
-  epi.slab.init(smem_raw, Gemm2Smem<BN>::EPI_OFF);
+  epi.slab.init(smem_raw, Gemm2Smem<BN, EW>::EPI_OFF);
   NoGate gate;
-  gemm_mainloop_2cta<BN, A_MN, B_MN>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
+  gemm_mainloop_2cta<BN, A_MN, B_MN, StoreEpilogue<OutT>, NoGate, false, EW>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
 }
 
 // Tiles of a product on CTA pairs: their width (a multiple of 32, 128 to 256) and whether those of the last
@@ -136,9 +136,10 @@ static int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas) {
   return 2 * (items < pairs ? items : pairs);
 }
 
-template <int BN, bool A_MN, bool B_MN, typename OutT>
+template <int BN, bool A_MN, bool B_MN, typename OutT, int EW>
 static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                             int64_t ldc, int accumulate, PairTiles tiles, int max_ctas, cudaStream_t stream) {
+  using S = Gemm2Smem<BN, EW>;
   CUtensorMap tmA, tmB, tmC;
   int rc;
   GemmShape shape{M, N, K, 0, 0};
@@ -157,26 +158,31 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
     rc = make_tmap_2d(&tmB, B, K, N, ldb, GEMM_BK, 64, 2, true);
   if (rc) return rc;
   if ((rc = make_tmap_out<OutT>(&tmC, C, M, N, ldc))) return rc;
-  auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, OutT>;
+  auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, OutT, EW>;
   static bool attr_set = false;
   if (!attr_set) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
+    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL_EPI));
     attr_set = true;
   }
   int* err = device_status_word();
-  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
+  kern<<<grid, S::THREADS, S::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
-template <int BN, typename OutT>
+template <int BN, typename OutT, int EW = 4>
 static int dispatch_major_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                                int64_t ldc, int a_mn, int b_mn, int accumulate, PairTiles tiles, int max_ctas, cudaStream_t stream) {
-  if (!a_mn && !b_mn) return launch_gemm_2cta<BN, false, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
-  if (!a_mn && b_mn) return launch_gemm_2cta<BN, false, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
-  if (a_mn && !b_mn) return launch_gemm_2cta<BN, true, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
-  return launch_gemm_2cta<BN, true, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
+  if (!a_mn && !b_mn) return launch_gemm_2cta<BN, false, false, OutT, EW>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
+  if (!a_mn && b_mn) return launch_gemm_2cta<BN, false, true, OutT, EW>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
+  if (a_mn && !b_mn) return launch_gemm_2cta<BN, true, false, OutT, EW>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
+  return launch_gemm_2cta<BN, true, true, OutT, EW>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
 }
+
+// Up to this K a tile's stores take longer than its products, and eight epilogue warps are worth the stage that their
+// staging area costs: 4096 x 14336 of K = 128 takes 31 us in wide tiles, 35 with four warps; at K = 256 both take 37 to
+// 39, at 320 four warps are ahead (39 and 47).
+constexpr int SHORT_K = 192;
 
 // The narrow kernel has more stages; tiles of any other width run on the wide one.
 static int gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_mn,
@@ -184,6 +190,8 @@ static int gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K,
   if (tiles.width == 128)
     return out_fp32 ? dispatch_major_2cta<128, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
                     : dispatch_major_2cta<128, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
+  if (K <= SHORT_K && !out_fp32)
+    return dispatch_major_2cta<256, __nv_bfloat16, 8>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
   return out_fp32 ? dispatch_major_2cta<256, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
                   : dispatch_major_2cta<256, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
 }

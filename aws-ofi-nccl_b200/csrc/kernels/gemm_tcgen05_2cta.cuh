@@ -12,23 +12,27 @@
 //   full[s]   leader only : both CTAs' TMA loads report their bytes here
 //   empty[s]  both CTAs   : the leader's tcgen05.commit arrives on both (multicast commit)
 //   tfull[b]  both CTAs   : accumulator b complete (multicast commit)
-//   tempty[b] leader only : all eight epilogue warps of the pair have drained accumulator b
+//   tempty[b] leader only : all epilogue warps of the pair have drained accumulator b
 // None of the loads uses cluster multicast; only tcgen05.commit does.
 #pragma once
 #include "gemm_tcgen05.cuh"
 
 namespace b200 {
 
-template <int BN>   // 256 or 128 output columns per cluster tile
+// BN: 256 or 128 output columns per cluster tile; EW: epilogue warps of a CTA, 4 or 8
+template <int BN, int EW = 4>
 struct Gemm2Smem {
   static constexpr int A_BYTES = 128 * GEMM_BK * 2;
   static constexpr int B_BYTES = (BN / 2) * GEMM_BK * 2;   // this CTA's half of the B tile
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 6 : 8;
+  static constexpr int STAGES = (BN == 256) ? (EW == 8 ? 5 : 6) : (EW == 8 ? 6 : 8);
+  static constexpr int THREADS = 64 + 32 * EW;
   static constexpr int BAR_BYTES = 256;
   static constexpr int TOTAL = 1024 + STAGES * STAGE_BYTES + BAR_BYTES;
   static constexpr int EPI_OFF = STAGES * STAGE_BYTES + 1024;
-  static constexpr int TOTAL_EPI = 1024 + EPI_OFF + GEMM_EPI_BYTES;
+  static constexpr int TOTAL_EPI = 1024 + EPI_OFF + EW * GEMM_EPI_WARP_BYTES;
+  static_assert(EW == 4 || EW == 8, "one or two epilogue warps per quarter of the accumulator's rows");
+  static_assert(TOTAL_EPI <= 232448, "more than a CTA's shared memory");
 };
 constexpr int GEMM2_BM = 256;  // rows per cluster tile
 
@@ -125,7 +129,7 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                : "memory");
 }
 
-// Launch with cluster dimension (2,1,1), 192 threads, Gemm2Smem<BN>::TOTAL (+ epilogue extras)
+// Launch with cluster dimension (2,1,1), Gemm2Smem<BN, EW>::THREADS threads, its TOTAL (+ epilogue extras)
 // bytes of dynamic shared memory and an even grid. shape.tiles_m counts 256-row tiles here.
 // The gate and the epilogue hooks (tile_begin / tile_end) are called with the index of this CTA's
 // 128-row tile (2 * pair tile + rank in the pair), so gates and epilogues written for the one-CTA
@@ -135,10 +139,10 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
 // those of the halves of the last wave come from tile_span.
 // FP8: both operands are 1-byte e4m3, K-major only; a k-block is then 128 elements (the same 128
 // bytes per row, so stages, swizzle and descriptors do not change) and one MMA covers K = 32.
-template <int BN, bool A_MN, bool B_MN, class Epilogue, class LoadGate, bool FP8 = false>
+template <int BN, bool A_MN, bool B_MN, class Epilogue, class LoadGate, bool FP8 = false, int EW = 4>
 __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const CUtensorMap* tmB, GemmShape shape,
                                                    Epilogue& epi, LoadGate& gate, int* err_word, uint8_t* smem_raw) {
-  using S = Gemm2Smem<BN>;
+  using S = Gemm2Smem<BN, EW>;
   static_assert(BN == 128 || BN == 256, "cluster tile is 256 x 128 or 256 x 256");
   static_assert(!FP8 || (!A_MN && !B_MN), "fp8 operands are K-major");
   constexpr int BK_ELEMS = FP8 ? 2 * GEMM_BK : GEMM_BK;   // elements per 128-byte row of a stage
@@ -164,7 +168,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 8);
+      mbar_init(tempty_bar(b), 2 * EW);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -278,8 +282,11 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
+    // ------------------------------------------------------------ epilogue (warps from 2 on, both CTAs)
     const int quarter = warp & 3;
+    // with eight warps the two of a quarter take every second 64 columns each
+    constexpr int STEP = 64 * (EW / 4);
+    const int first = EW == 4 ? 0 : 64 * ((warp - 2) >> 2);
     int acc_buf = 0;
     uint32_t acc_phase = 0;
     for (int item = pair_id; item < num_items; item += pair_stride) {
@@ -293,7 +300,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc_buf * BN;
       if constexpr (Epilogue::kPair) {
 #pragma unroll 1
-        for (int c = 0; c < t.width; c += 64) {
+        for (int c = first; c < t.width; c += STEP) {
           uint32_t acc0[32], acc1[32];
           tmem_ld_32x32(taddr + c, acc0);
           tmem_ld_32x32(taddr + c + 32, acc1);
@@ -301,6 +308,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
           epi(row, t.col0 + c, acc0, acc1, shape, t.width - c);
         }
       } else {
+        static_assert(EW == 4 || Epilogue::kPair, "two warps share a quarter 64 columns at a time");
 #pragma unroll 1
         for (int c = 0; c < t.width; c += 32) {
           uint32_t acc[32];
