@@ -16,6 +16,14 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
 int b200_swiglu_fwd(const void* gu, void* out, long long T, int F, void* stream);
 int b200_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, int F, void* stream);
 
+// gate|up = x w^T with act = silu(gate) * up, and the gradient at gate|up from dy and the down projection w; see
+// gemm_swiglu.cu. The bwd call wants `scratch` [M][F] bf16 where b200_gemm_swiglu_bwd_launches says 2.
+int b200_gemm_swiglu(const void* x, const void* w, void* gu, void* act, int M, int F, int K, long long ldx, void* stream);
+int b200_gemm_swiglu_bwd(const void* dy, const void* w, const void* gu, void* dgu, void* scratch, int M, int F, int K, long long lddy,
+                         void* stream);
+int b200_gemm_swiglu_launches(const void* x, const void* w, int M, int F, int K, long long ldx);
+int b200_gemm_swiglu_bwd_launches(const void* dy, const void* w, int M, int F, int K, long long lddy);
+
 int b200_rope_qkv(void* qkv, long long pitch, void* q, void* k, void* v, const long long* strides, const float* cs,
                   const float* sn, long long T, int nq, int nkv, int hd, int seq, int backward, void* stream);
 

@@ -174,16 +174,27 @@ __device__ __forceinline__ void ag_mover(const AgGemmArgs& a, uint8_t* smem_raw)
   gin_barrier(h, a.channel, blockIdx.x);  // nobody overwrites a shard that a peer is still reading
 }
 
-// The epilogue of an ag_gemm kernel: SwiGLU (activation and, if wanted, the raw pair) or a plain store.
-template <bool SWIGLU>
-__device__ __forceinline__ auto ag_epilogue(const CUtensorMap* tmC, const CUtensorMap* tmAct, int keep_c) {
-  if constexpr (SWIGLU)
-    return SwiGluEpilogue{tmAct, tmC, keep_c, {}};
-  else
-    return StoreEpilogue<__nv_bfloat16>{tmC, nullptr, 0, 0, {}};
+// The epilogue of an ag_gemm kernel: a plain store, SwiGLU (activation and, if wanted, the raw pair) or the
+// gradient of SwiGLU (tmAct is the saved pair then, tmC its gradient).
+enum AgEpilogue { AG_STORE = 0, AG_SWIGLU = 1, AG_SWIGLU_BWD = 2 };
+template <int EPI, int EW>
+__device__ __forceinline__ auto ag_epilogue(const CUtensorMap* tmC, const CUtensorMap* tmAct, int keep_c, uint8_t* smem_raw, uint32_t epi_off) {
+  if constexpr (EPI == AG_SWIGLU_BWD) {
+    SwiGluBwdEpilogue<EW> epi{tmAct, tmAct, tmC, tmC, 1, 0, 0, 0, nullptr, nullptr};
+    epi.init(smem_raw, epi_off);
+    return epi;
+  } else if constexpr (EPI == AG_SWIGLU) {
+    SwiGluEpilogue epi{tmAct, tmC, keep_c, {}};
+    epi.slab.init(smem_raw, epi_off);
+    return epi;
+  } else {
+    StoreEpilogue<__nv_bfloat16> epi{tmC, nullptr, 0, 0, {}};
+    epi.slab.init(smem_raw, epi_off);
+    return epi;
+  }
 }
 
-template <int BN, bool B_MN, bool SWIGLU>
+template <int BN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     ag_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAct, GemmShape shape,
@@ -195,15 +206,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   }
   ChunkGate gate{reinterpret_cast<const uint32_t*>(args.h.pad[args.h.rank] + TP_READY_OFF), args.epoch,
                  args.chunks_per_shard, args.h.rank, gate_on_b, args.h.wait_limit_ns};
-  auto epi = ag_epilogue<SWIGLU>(&tmC, &tmAct, keep_c);
-  epi.slab.init(smem_raw, GemmSmem<BN>::EPI_OFF);
+  auto epi = ag_epilogue<EPI, 4>(&tmC, &tmAct, keep_c, smem_raw, GemmSmem<BN>::EPI_OFF);
   gemm_mainloop<BN, false, B_MN>(&tmA, &tmB, shape, epi, gate, args.h.status, smem_raw);
 }
 
+// The gradient waits for its loads: eight warps, at the price of a stage.
+__host__ __device__ constexpr int ag_epi_warps(int epi) { return epi == AG_SWIGLU_BWD ? 8 : 4; }
+template <int EPI>
+using AgPairSmem = Gemm2Smem<256, ag_epi_warps(EPI)>;
+
 // The same kernel on CTA pairs (256-row cluster tiles, tcgen05.mma.cta_group::2). Movers come in
 // pairs too (n_movers is even), so every cluster is either two movers or two GEMM CTAs.
-template <bool B_MN, bool SWIGLU>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+template <bool B_MN, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(AgPairSmem<EPI>::THREADS, 1)
     ag_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAct, GemmShape shape,
                         AgGemmArgs args, int keep_c, int gate_on_b) {
@@ -214,9 +229,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   }
   ChunkGate gate{reinterpret_cast<const uint32_t*>(args.h.pad[args.h.rank] + TP_READY_OFF), args.epoch,
                  args.chunks_per_shard, args.h.rank, gate_on_b, args.h.wait_limit_ns};
-  auto epi = ag_epilogue<SWIGLU>(&tmC, &tmAct, keep_c);
-  epi.slab.init(smem_raw, Gemm2Smem<256>::EPI_OFF);
-  gemm_mainloop_2cta<256, false, B_MN>(&tmA, &tmB, shape, epi, gate, args.h.status, smem_raw);
+  auto epi = ag_epilogue<EPI, ag_epi_warps(EPI)>(&tmC, &tmAct, keep_c, smem_raw, AgPairSmem<EPI>::EPI_OFF);
+  gemm_mainloop_2cta<256, false, B_MN, decltype(epi), ChunkGate, false, ag_epi_warps(EPI)>(&tmA, &tmB, shape, epi, gate, args.h.status, smem_raw);
 }
 
 // B200_TP_2CTA=0 keeps the fused kernels on single CTAs.
@@ -251,7 +265,7 @@ struct RsArgs {
 
 template <int BN>
 struct RingEpilogue {
-  static constexpr bool kPair = true;   // called with 64 consecutive columns per row
+  static constexpr bool kPair = true, kSplit = false, kAhead = false;   // called with 64 consecutive columns per row
   RsArgs a;
   int N, tiles_n;
   // Shared-memory counters of epilogue warps that finished a tile, indexed by (tile sequence & 3):
@@ -414,7 +428,8 @@ using namespace b200;
 // operand B is passed in `other`.
 //   b_mn     : B stored [K][N] instead of [N][K]
 //   epilogue : 0 = store C (bf16, ldc), 1 = SwiGLU on interleaved gate|up columns -> act [M][N/2]
-//              (ld_act), also storing the raw gate|up into C when C is non-null
+//              (ld_act), also storing the raw gate|up into C when C is non-null, 2 = the gradient of SwiGLU: the
+//              product is d(act), act the saved gate|up [M][2N] (ld_act) and C its gradient, laid out the same
 // M must be a multiple of 128 * nranks.
 // gather_b = 1 gathers B instead (FSDP: the weight [N][K] is sharded over ranks along N, the
 // activation A [M][K] is local and passed in `other`); then N must be a multiple of 256 * nranks
@@ -427,7 +442,7 @@ int b200_ag_gemm(int comm, size_t gathered_off, int gather_b, int M, int N, int 
   if (!hp || comm < 0 || comm >= 64 || !other) return B200_ERR_BAD_ARG;
   GinDevHandle h = *hp;
   constexpr int BN = 256;
-  if (K % 8 || N % 64 || (epilogue == 1 && !act) || (epilogue == 0 && !C)) return B200_ERR_BAD_ARG;
+  if (K % 8 || N % 64 || (epilogue >= AG_SWIGLU && !act) || (epilogue != AG_SWIGLU && !C)) return B200_ERR_BAD_ARG;
   if (!gather_b && M % (GEMM_BM * h.nranks)) return B200_ERR_BAD_ARG;
   if (gather_b && (N % (BN * h.nranks) || b_mn)) return B200_ERR_BAD_ARG;
   const size_t shard_bytes = static_cast<size_t>((gather_b ? N : M) / h.nranks) * K * 2;
@@ -496,39 +511,37 @@ int b200_ag_gemm(int comm, size_t gathered_off, int gather_b, int M, int N, int 
   if (rc) return rc;
   // what the epilogue stores: boxes of 32 rows x 128 bytes, the activation 32 rows x 64 bytes; a map
   // that is not used stays a copy of the other
-  if (C && (rc = make_tmap_2d(&tmC, C, M, N, ldc, 32, 64, 2, true))) return rc;
-  if (epilogue == 1 && (rc = make_tmap_2d(&tmAct, act, M, N / 2, ld_act, 32, 32, 2, true, true))) return rc;
+  const int c_cols = epilogue == AG_SWIGLU_BWD ? 2 * N : N;
+  if (C && (rc = make_tmap_2d(&tmC, C, M, c_cols, ldc, 32, 64, 2, true))) return rc;
+  if (epilogue == AG_SWIGLU && (rc = make_tmap_2d(&tmAct, act, M, N / 2, ld_act, 32, 32, 2, true, true))) return rc;
+  if (epilogue == AG_SWIGLU_BWD && (rc = make_tmap_2d(&tmAct, act, M, c_cols, ld_act, 32, 64, 2, true))) return rc;
   if (!C) tmC = tmAct;
-  if (epilogue != 1) tmAct = tmC;
+  if (epilogue != AG_SWIGLU && epilogue != AG_SWIGLU_BWD) tmAct = tmC;
   AgGemmArgs args{h, gathered_off, shard_bytes, static_cast<size_t>(gather_b ? BN : GEMM_BM) * K * 2, chunks_per_shard,
                   n_movers, channel, ++g_ag_epoch[comm]};
   const int grid = n_movers + shape.num_ctas;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int smem = pairs ? Gemm2Smem<BN>::TOTAL_EPI : GemmSmem<BN>::TOTAL_EPI;
   const int keep_c = C != nullptr;
-#define B200_AG_LAUNCH(KERNEL)                                                                        \
+#define B200_AG_LAUNCH(KERNEL, THREADS, SMEM)                                                         \
   do {                                                                                                \
     auto k = KERNEL;                                                                                  \
-    if (set_smem(k, smem)) return B200_ERR_BAD_ARG;                                                   \
-    k<<<grid, GEMM_THREADS, smem, s>>>(tmA, tmB, tmC, tmAct, shape, args, keep_c, gather_b);          \
+    if (set_smem(k, SMEM)) return B200_ERR_BAD_ARG;                                                   \
+    k<<<grid, THREADS, SMEM, s>>>(tmA, tmB, tmC, tmAct, shape, args, keep_c, gather_b);               \
   } while (0)
-  if (epilogue == 1) {
-    if (pairs) {
-      if (b_mn) B200_AG_LAUNCH((ag_gemm_pair_kernel<true, true>));
-      else B200_AG_LAUNCH((ag_gemm_pair_kernel<false, true>));
-    } else {
-      if (b_mn) B200_AG_LAUNCH((ag_gemm_kernel<BN, true, true>));
-      else B200_AG_LAUNCH((ag_gemm_kernel<BN, false, true>));
-    }
-  } else {
-    if (pairs) {
-      if (b_mn) B200_AG_LAUNCH((ag_gemm_pair_kernel<true, false>));
-      else B200_AG_LAUNCH((ag_gemm_pair_kernel<false, false>));
-    } else {
-      if (b_mn) B200_AG_LAUNCH((ag_gemm_kernel<BN, true, false>));
-      else B200_AG_LAUNCH((ag_gemm_kernel<BN, false, false>));
-    }
-  }
+#define B200_AG_MAJOR(EPI)                                                                                              \
+  do {                                                                                                                  \
+    if (pairs) {                                                                                                        \
+      if (b_mn) B200_AG_LAUNCH((ag_gemm_pair_kernel<true, EPI>), AgPairSmem<EPI>::THREADS, AgPairSmem<EPI>::TOTAL_EPI); \
+      else B200_AG_LAUNCH((ag_gemm_pair_kernel<false, EPI>), AgPairSmem<EPI>::THREADS, AgPairSmem<EPI>::TOTAL_EPI);     \
+    } else {                                                                                                            \
+      if (b_mn) B200_AG_LAUNCH((ag_gemm_kernel<BN, true, EPI>), GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI);                 \
+      else B200_AG_LAUNCH((ag_gemm_kernel<BN, false, EPI>), GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI);                     \
+    }                                                                                                                   \
+  } while (0)
+  if (epilogue == AG_SWIGLU_BWD) B200_AG_MAJOR(AG_SWIGLU_BWD);
+  else if (epilogue == AG_SWIGLU) B200_AG_MAJOR(AG_SWIGLU);
+  else B200_AG_MAJOR(AG_STORE);
+#undef B200_AG_MAJOR
 #undef B200_AG_LAUNCH
   B200_CUDA_OK(cudaGetLastError());
   return 0;

@@ -11,6 +11,7 @@
 
 #include "b200ops.h"
 #include "gemm_epilogues.cuh"
+#include "gemm_plan.h"
 #include "gemm_splitk.h"
 #include "gemm_tcgen05.cuh"
 #include "gemm_tcgen05_2cta.cuh"
@@ -111,16 +112,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Gemm2Smem<BN, EW>::T
   gemm_mainloop_2cta<BN, A_MN, B_MN, StoreEpilogue<OutT>, NoGate, false, EW>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
 }
 
-// Tiles of a product on CTA pairs: their width (a multiple of 32, 128 to 256) and whether those of the last
-// wave are halved.
-struct PairTiles {
-  int width;
-  bool halves;
-};
-
-// Fills in the tiles of `shape` (M, N and K are set). bn: the kernel's BN; ctas: how many may run. Returns how
-// many are launched.
-static int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas) {
+int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas) {
   const int pairs = ctas / 2;
   shape.tiles_m = (shape.M + GEMM2_BM - 1) / GEMM2_BM;
   shape.tiles_n = (shape.N + tiles.width - 1) / tiles.width;
@@ -350,7 +342,7 @@ struct GemmChoice {
   SplitkPlan split;
 };
 
-// Tiles of a product on CTA pairs whose better plain width is `bn`; a_low, b_low: what decides how the operands' rows
+// Tiles of a product on CTA pairs, in steps of `step` columns, whose better plain width is `bn`; a_low, b_low: what decides how the operands' rows
 // lie on cache lines. A wave of narrower tiles costs more than their share of a wide one: their loads bring the
 // same rows of A for fewer columns. Rows off cache lines take the loads half as long again, and the boxes of an N-major B
 // are 64 columns, so that 160 and 224 columns (80 and 112 for a CTA) load as much as 256. The costs are medians over
@@ -358,7 +350,8 @@ struct GemmChoice {
 // took 0.977 of the plain width's time on average there, the best choice 0.969, and none more than 1.03. What it
 // gains is the last wave: 4096 x 4096 x 14336, 256 tiles for 74 pairs, takes 333 us in four wide waves and 308 with
 // the last of them halved; 4096 x 6144 x 4096 132 us, 123 in five waves of 192 columns for six of 256.
-static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint64_t b_low, int units, int bn) {
+static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint64_t b_low, int units, int bn,
+                           int step = 32) {
   struct Costs {
     double at[5];   // 128, 160, 192, 224, 256 columns
   };
@@ -372,9 +365,9 @@ static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint6
   constexpr double GAIN = 1.03;   // a width that is not the plain one has to promise 3 %, halves of the last wave 1 %
   PairTiles best{bn, false};
   double best_cost = 1e30;
-  for (int i = 0; i < 5; ++i) {
+  for (int i = 0; i < 5; i += step / 32) {
     const int width = 128 + 32 * i;
-    if (width > 128 && N <= width - 32) break;   // a narrower one covers the row as well
+    if (width > 128 && N <= width - step) break;   // a narrower one covers the row as well
     if (width % 64 && K < 1024) continue;        // the last 32 columns of a tile leave as vectors, not by TMA: with few k-blocks that counts
     const int64_t tiles = rows * ((N + width - 1) / width);
     const double cost = static_cast<double>((tiles + units - 1) / units) * c.at[i] * (width == bn ? 1 : GAIN);
@@ -419,6 +412,16 @@ static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, boo
   }
   // Few tiles and a long K: the chip is filled by splitting K over clusters.
   return {bn, tiles, max_ctas == 0 ? plan_splitk(M, N, K, pairs, bn) : SplitkPlan{1}};
+}
+
+bool runs_on_pairs(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, const void* A, const void* B, PairTiles* tiles) {
+  if (!use_pairs(M, N, 0)) return false;
+  const uintptr_t a_at = reinterpret_cast<uintptr_t>(A), b_at = reinterpret_cast<uintptr_t>(B);
+  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, b_mn, a_at, b_at, 0);
+  if (g.split.slices > 1) return false;
+  *tiles = fit_tiles(M, N, K, b_mn, a_at | (static_cast<uint64_t>(lda) * 2), b_at | (static_cast<uint64_t>(ldb) * 2), sm_count() / 2,
+                     g.bn, 128);
+  return true;
 }
 
 }  // namespace b200

@@ -1,5 +1,5 @@
 // Epilogue functors for the tcgen05 GEMM mainloops: plain store (bf16 / fp32, optional accumulate),
-// the scaled store of the fp8 product and the fused SwiGLU store of the tensor-parallel MLP.
+// the scaled store of the fp8 product, and SwiGLU and its gradient in the products of an MLP.
 //
 // A thread holds one accumulator row, so storing from registers writes 16 bytes to each of 32 rows
 // per instruction: half a sector at a time, 32 lines in flight per warp, and the epilogue of a short
@@ -150,7 +150,7 @@ __device__ __noinline__ uint4 part_vector(const OutT* src, int n) {
 // C (+)= acc. The tensor map of C has boxes of 32 rows x 128 bytes (64 bf16 or 32 fp32 columns).
 template <typename OutT>
 struct StoreEpilogue {
-  static constexpr bool kPair = true;
+  static constexpr bool kPair = true, kSplit = false, kAhead = false;
   const CUtensorMap* tmC;
   OutT* C;   // read when accumulating
   int64_t ldc;
@@ -229,7 +229,7 @@ struct StoreEpilogue {
 // operands were quantised per row (activations: one scale per token, weights: one per output
 // channel). N is a multiple of 4.
 struct ScaledStoreEpilogue {
-  static constexpr bool kPair = true;
+  static constexpr bool kPair = true, kSplit = false, kAhead = false;
   const CUtensorMap* tmC;
   __nv_bfloat16* C;
   int64_t ldc;
@@ -283,7 +283,7 @@ __device__ __forceinline__ void swiglu32(uint32_t* act, const uint32_t (&g)[32],
 // the backward pass needs). The warp's staging area holds the pair (4 KiB, boxes of 64 columns) and
 // behind it the activation (2 KiB, boxes of 32 columns, 64-byte swizzle).
 struct SwiGluEpilogue {
-  static constexpr bool kPair = true;
+  static constexpr bool kPair = true, kSplit = false, kAhead = false;
   const CUtensorMap* tmAct;   // [M][N/2]
   const CUtensorMap* tmGu;    // [M][N] interleaved as computed
   int keep_gu;
@@ -318,6 +318,134 @@ struct SwiGluEpilogue {
       tma_store_2d(tmAct, slab.buf + 4096, col0 / 2, row0);
       tma_store_commit();
     }
+  }
+};
+
+// SwiGLU in the gate|up product of weights that are stored as two halves, [gate; up]: a tile's first half of
+// columns are gates and its second the matching ups (GemmShape::b_second). Stores both, which the backward pass
+// reads, and act = silu(gate) * up.
+struct SwiGluSplitEpilogue {
+  static constexpr bool kPair = false, kSplit = true, kAhead = false;
+  const CUtensorMap *tmGate, *tmUp, *tmAct;   // [M][F] each, boxes of 32 rows x 64 columns
+  int F;
+  SlabStore slab;
+  uint32_t gate[32], up[32], act[32];   // this lane's 64 columns of each, two to a word
+  __device__ __forceinline__ void tile_begin(int, int) {}
+  __device__ __forceinline__ void tile_end(int, int) {}
+  __device__ __forceinline__ void drain() { slab.drain(); }
+  template <int J>
+  __device__ __forceinline__ void part(const uint32_t (&g)[32], const uint32_t (&u)[32]) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      gate[16 * J + j] = pack_bf16x2(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]));
+      up[16 * J + j] = pack_bf16x2(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1]));
+    }
+    swiglu32(act + 16 * J, g, u);
+  }
+  __device__ __forceinline__ void store(int row, int col, const GemmShape& s) {
+    const int row0 = row - static_cast<int>(threadIdx.x & 31);
+    if (row0 >= s.M || col >= F) return;   // uniform over the warp
+    slab.put128(tmGate, col, row0, gate, true);
+    slab.put128(tmUp, col, row0, up, true);
+    slab.put128(tmAct, col, row0, act, true);
+  }
+};
+
+// The gradient of SwiGLU in the product that makes d(act): stores d(gate) and d(up) from the sums and the saved
+// gate and up, so that d(act) is neither rounded nor written and read back. Gate and up come through TMA into the
+// warp's staging area, the gradients replace them there and leave the same way; the loads of a tile's first columns
+// are under way while its products are computed. interleaved: gate and up alternate in blocks of 32 columns
+// (one map, 64 columns of d(act) are 128 there, N is a multiple of 64); otherwise they are two halves with a map each.
+template <int EW>   // epilogue warps of a CTA
+struct SwiGluBwdEpilogue {
+  static constexpr bool kPair = true, kSplit = false, kAhead = true;
+  static constexpr int STEP = 64 * (EW / 4);   // from one of this warp's slabs of columns to the next
+  const CUtensorMap *in0, *in1, *out0, *out1;   // boxes of 32 rows x 64 columns
+  int interleaved;
+  uint32_t buf, bar;   // this warp's 8 KiB and its barrier for the loads
+  uint32_t phase;
+  volatile int* abort_flag;
+  int* err_word;
+  __device__ __forceinline__ void init(uint8_t* smem_raw, uint32_t epi_off) {
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t warp = threadIdx.x >> 5, mine = warp >= 2 ? warp - 2 : 0;
+    buf = base + epi_off + mine * GEMM_EPI_WARP_BYTES;
+    bar = base + epi_off - 64 + 8 * mine;   // behind the mainloop's barriers
+    phase = 0;
+    if (warp >= 2 && (threadIdx.x & 31) == 0) {
+      mbar_init(bar, 1);
+      fence_barrier_init();
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ void load(int row0, int col0, const GemmShape& s) {
+    if (row0 >= s.M || col0 >= s.N || (threadIdx.x & 31) != 0) return;
+    tma_store_wait_read<0>();
+    mbar_expect_tx(bar, 8192);
+    tma_load_2d(buf, in0, interleaved ? 2 * col0 : col0, row0, bar);
+    tma_load_2d(buf + 4096, in1, interleaved ? 2 * col0 + 64 : col0, row0, bar);
+  }
+  __device__ __forceinline__ void tile_ahead(int row0, int col0, const GemmShape& s, volatile int* abort, int* err) {
+    abort_flag = abort;
+    err_word = err;
+    load(row0, col0, s);
+  }
+  __device__ __forceinline__ void tile_begin(int, int) {}
+  __device__ __forceinline__ void tile_end(int, int) {}
+  __device__ __forceinline__ void drain() {
+    if ((threadIdx.x & 31) == 0) tma_store_wait<0>();
+  }
+  // d: eight sums; g_at, u_at: the chunks of gate and up, replaced by their gradients
+  __device__ __forceinline__ void chunk(const uint32_t* d, uint32_t g_at, uint32_t u_at) const {
+    uint32_t g[4], u[4];
+    ld_shared_v4(g_at, g);
+    ld_shared_v4(u_at, u);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const __nv_bfloat162 gp = *reinterpret_cast<const __nv_bfloat162*>(&g[p]), up = *reinterpret_cast<const __nv_bfloat162*>(&u[p]);
+      float dg[2], du[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float gf = e ? __high2float(gp) : __low2float(gp), uf = e ? __high2float(up) : __low2float(up);
+        const float df = __uint_as_float(d[2 * p + e]), s = logistic(gf), si = gf * s;
+        du[e] = df * si;
+        dg[e] = df * uf * (s + si * (1.f - s));
+      }
+      g[p] = pack_bf16x2(dg[0], dg[1]);
+      u[p] = pack_bf16x2(du[0], du[1]);
+    }
+    st_shared_v4(g_at, g[0], g[1], g[2], g[3]);
+    st_shared_v4(u_at, u[0], u[1], u[2], u[3]);
+  }
+  __device__ __forceinline__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape& s, int left) {
+    const int lane = threadIdx.x & 31, row0 = row - lane;
+    if (row0 >= s.M || col0 >= s.N) return;   // uniform over the warp
+    const bool here = mbar_wait_bounded(bar, phase, abort_flag, err_word, DEV_ERR_FULL_BAR_TIMEOUT, GEMM_WAIT_LIMIT_NS);
+    if (!__all_sync(0xffffffffu, here)) return;
+    phase ^= 1;
+    const uint32_t first = buf + lane * 128, second = first + 4096;
+    auto at = [&](uint32_t slab, int j) { return slab + ((j ^ (lane & 7)) << 4); };
+    if (interleaved) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        chunk(a0 + 8 * j, at(first, j), at(first, 4 + j));
+        chunk(a1 + 8 * j, at(second, j), at(second, 4 + j));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        chunk(a0 + 8 * j, at(first, j), at(second, j));
+        chunk(a1 + 8 * j, at(first, 4 + j), at(second, 4 + j));
+      }
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(out0, buf, interleaved ? 2 * col0 : col0, row0);
+      tma_store_2d(out1, buf + 4096, interleaved ? 2 * col0 + 64 : col0, row0);
+      tma_store_commit();
+    }
+    if (left > STEP) load(row0, col0 + STEP, s);
   }
 };
 

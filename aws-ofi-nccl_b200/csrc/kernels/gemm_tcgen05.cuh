@@ -44,6 +44,7 @@ struct GemmShape {
   int bn = 0;               // columns of a tile (0 = the kernel's BN)
   int halve_from = 1 << 30; // tiles from this number on are computed as two halves
   int b_box = 0;            // K-major B: rows of a load's box (0 = a CTA's share of a tile, BN / 2)
+  int b_second = 0;         // > 0: the second half of a tile's columns comes from the rows of B this much further down
 };
 
 // The tile id -> (tile_m, tile_n) map. Default: M fastest inside a group of group_m M tiles, so
@@ -76,7 +77,11 @@ __device__ __forceinline__ void tile_coords(const GemmShape& s, int tile, int& t
 //   __device__ void operator()(int row, int col0, const uint32_t (&acc)[32], const GemmShape&)
 // called by one thread per accumulator row for 32 consecutive columns starting at col0 (fp32 bits), or with kPair
 //   __device__ void operator()(int row, int col0, uint32_t (&a0)[32], uint32_t (&a1)[32], const GemmShape&, int left)
-// for 64, of which the first `left` (32 or at least 64) belong to the tile.
+// for 64, of which the first `left` (32 or at least 64) belong to the tile. With kAhead the warp announces
+// a tile's rows and columns with tile_ahead(row0, col0, shape, abort_flag, err_word) before it waits for its sums.
+// With kSplit (CTA pairs) the first half of a tile's columns and the second half come together, 64 of each in two parts:
+//   template <int J> __device__ void part(const uint32_t (&a)[32], const uint32_t (&b)[32])
+//   __device__ void store(int row, int col, const GemmShape&)
 // Hooks: tile_begin(tm, tn) / tile_end(tm, tn) and, after the last tile, drain(), called by every
 // epilogue thread.
 
@@ -218,6 +223,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
     for (int tile = cta_id; tile < num_tiles; tile += cta_stride) {
       int tm, tn;
       tile_coords(shape, tile, tm, tn);
+      if constexpr (Epilogue::kAhead) epi.tile_ahead(tm * GEMM_BM + quarter * 32, tn * BN, shape, abort_flag, err_word);
       if (!mbar_wait_bounded(tfull_bar(acc_buf), acc_phase, abort_flag, err_word, DEV_ERR_TMEM_FULL_TIMEOUT,
                              GEMM_WAIT_LIMIT_NS))
         break;

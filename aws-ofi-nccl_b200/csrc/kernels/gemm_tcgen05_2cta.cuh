@@ -202,7 +202,8 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
         const TileSpan t = tile_span<BN>(shape, item);
         const int half = t.width >> 1;
         const int row0 = t.tm * GEMM2_BM + static_cast<int>(rank) * 128;   // this CTA's rows of A
-        const int col0 = t.col0 + static_cast<int>(rank) * half;   // this CTA's half of B
+        const int col0 = shape.b_second ? (t.col0 >> 1) + static_cast<int>(rank) * shape.b_second   // this CTA's half of B
+                                        : t.col0 + static_cast<int>(rank) * half;
         const int b_boxes = B_MN ? (half + 63) / 64 : half / box;
         const uint32_t pair_bytes = 2 * (S::A_BYTES + b_boxes * (B_MN ? 64 : box) * 128);
         if (!gate.wait_tile(2 * t.tm + static_cast<int>(rank), t.tn, abort_flag, err_word)) break;
@@ -291,6 +292,8 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
     uint32_t acc_phase = 0;
     for (int item = pair_id; item < num_items; item += pair_stride) {
       const TileSpan t = tile_span<BN>(shape, item);
+      if constexpr (Epilogue::kAhead)
+        epi.tile_ahead(t.tm * GEMM2_BM + static_cast<int>(rank) * 128 + quarter * 32, t.col0 + first, shape, abort_flag, err_word);
       if (!mbar_wait_bounded(tfull_bar(acc_buf), acc_phase, abort_flag, err_word, DEV_ERR_TMEM_FULL_TIMEOUT,
                              GEMM_WAIT_LIMIT_NS))
         break;
@@ -298,7 +301,22 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
       epi.tile_begin(2 * t.tm + static_cast<int>(rank), t.tn);
       const int row = t.tm * GEMM2_BM + static_cast<int>(rank) * 128 + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc_buf * BN;
-      if constexpr (Epilogue::kPair) {
+      if constexpr (Epilogue::kSplit) {
+        const int half = t.width >> 1;
+#pragma unroll 1
+        for (int c = first; c < half; c += STEP) {
+          uint32_t a[32], b[32];
+          tmem_ld_32x32(taddr + c, a);
+          tmem_ld_32x32(taddr + half + c, b);
+          tmem_ld_wait();
+          epi.template part<0>(a, b);
+          tmem_ld_32x32(taddr + c + 32, a);
+          tmem_ld_32x32(taddr + half + c + 32, b);
+          tmem_ld_wait();
+          epi.template part<1>(a, b);
+          epi.store(row, (t.col0 >> 1) + c, shape);
+        }
+      } else if constexpr (Epilogue::kPair) {
 #pragma unroll 1
         for (int c = first; c < t.width; c += STEP) {
           uint32_t acc0[32], acc1[32];
@@ -308,7 +326,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
           epi(row, t.col0 + c, acc0, acc1, shape, t.width - c);
         }
       } else {
-        static_assert(EW == 4 || Epilogue::kPair, "two warps share a quarter 64 columns at a time");
+        static_assert(EW == 4 || Epilogue::kPair || Epilogue::kSplit, "two warps share a quarter 64 columns at a time");
 #pragma unroll 1
         for (int c = 0; c < t.width; c += 32) {
           uint32_t acc[32];

@@ -1,4 +1,4 @@
-// The differentiable layers of the training path (linear, RMSNorm, SwiGLU, rotary split of the fused
+// The differentiable layers of the training path (linear, RMSNorm, SwiGLU, SwiGLU MLP, rotary split of the fused
 // projection) as autograd functions in native code: shape checks, output allocation, the calls into
 // libb200ops.so and the weight-gradient hand-over run without the interpreter. A layer's launches are
 // a few microseconds of device time each at small sizes, and the interpreter's share of a forward and
@@ -245,6 +245,62 @@ struct SwiGLU : public Function<SwiGLU> {
   }
 };
 
+// The SwiGLU MLP of a decoder layer, gate over up in w_gu. One layer instead of three, so that the activation and its
+// gradient ride in the products beside them.
+struct SwiGLUMLP : public Function<SwiGLUMLP> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w_gu, const Tensor& w_down) {
+    require(bf16_cuda(x) && bf16_cuda(w_gu) && bf16_cuda(w_down), "x and the weights are bfloat16 CUDA tensors");
+    require(x.dim() >= 1 && w_gu.dim() == 2 && w_down.dim() == 2 && w_gu.is_contiguous() && w_down.is_contiguous(),
+            "x has a last dimension and the weights are contiguous matrices");
+    const int64_t F = w_down.size(1), K = w_gu.size(1);
+    require(w_gu.size(0) == 2 * F && x.size(-1) == K, "the weights are [2F, hidden] and [out, F]");
+    const Tensor x2 = x.reshape({-1, K});
+    require(x2.stride(1) == 1, "x has contiguous rows");
+    const int T = static_cast<int>(x2.size(0));
+    const Tensor gu = at::empty({T, 2 * F}, x.options()), act = at::empty({T, F}, x.options());
+    g_launches.fetch_add(b200_gemm_swiglu_launches(x2.data_ptr(), w_gu.data_ptr(), T, static_cast<int>(F), static_cast<int>(K), x2.stride(0)),
+                         std::memory_order_relaxed);
+    check(b200_gemm_swiglu(x2.data_ptr(), w_gu.data_ptr(), gu.data_ptr(), act.data_ptr(), T, static_cast<int>(F), static_cast<int>(K),
+                           x2.stride(0), stream()),
+          "b200_gemm_swiglu");
+    auto shape = x.sizes().vec();
+    shape.back() = w_down.size(0);
+    Tensor y = at::empty(shape, x.options());
+    gemm(act, w_down, false, false, y.view({-1, w_down.size(0)}), false);
+    ctx->save_for_backward({x, w_gu, w_down, gu, act});
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return on_engine_thread([&]() -> variable_list {
+      const auto saved = ctx->get_saved_variables();
+      const Tensor &x = saved[0], &w_gu = saved[1], &w_down = saved[2], &gu = saved[3], &act = saved[4];
+      const Tensor dy = rows16(grads[0].reshape({-1, grads[0].size(-1)}));
+      const int T = static_cast<int>(dy.size(0)), F = static_cast<int>(act.size(1)), H = static_cast<int>(dy.size(1));
+      Tensor dgu, dx, dw_gu, dw_down;
+      if (ctx->needs_input_grad(0) || ctx->needs_input_grad(1)) {
+        const int launches = b200_gemm_swiglu_bwd_launches(dy.data_ptr(), w_down.data_ptr(), T, F, H, dy.stride(0));
+        const Tensor scratch = launches == 1 ? Tensor() : at::empty_like(act);
+        dgu = at::empty_like(gu);
+        g_launches.fetch_add(launches, std::memory_order_relaxed);
+        check(b200_gemm_swiglu_bwd(dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), dgu.data_ptr(),
+                                   scratch.defined() ? scratch.data_ptr() : nullptr, T, F, H, dy.stride(0), stream()),
+              "b200_gemm_swiglu_bwd");
+      }
+      if (ctx->needs_input_grad(2))
+        dw_down = write_param_grad(w_down, [&](const Tensor& out, bool accumulate) { gemm(dy, act, true, true, out, accumulate); });
+      const Tensor x2 = x.reshape({-1, x.size(-1)});
+      if (ctx->needs_input_grad(0)) {
+        dx = at::empty_like(x2, x2.options(), at::MemoryFormat::Contiguous);
+        gemm(dgu, w_gu, false, true, dx, false);
+        dx = dx.view(x.sizes());
+      }
+      if (ctx->needs_input_grad(1))
+        dw_gu = write_param_grad(w_gu, [&](const Tensor& out, bool accumulate) { gemm(dgu, x2, true, true, out, accumulate); });
+      return {dx, dw_gu, dw_down};
+    });
+  }
+};
+
 // q, k (rotated) and v as [B, S, heads, hd] tensors of their own from the fused projection [B*S, (nq+2nkv)*hd]
 struct RopeQKV : public Function<RopeQKV> {
   static void launch(const Tensor& qkv, const Tensor (&part)[3], const Tensor& cos, const Tensor& sin, int64_t S, bool backward) {
@@ -295,6 +351,7 @@ variable_list rmsnorm(const Tensor& x, const c10::optional<Tensor>& res, const T
   return RMSNorm::apply(x, res, w, eps);
 }
 Tensor swiglu(const Tensor& gu) { return SwiGLU::apply(gu); }
+Tensor swiglu_mlp(const Tensor& x, const Tensor& w_gu, const Tensor& w_down) { return SwiGLUMLP::apply(x, w_gu, w_down); }
 variable_list rope_qkv(const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S, int64_t nq, int64_t nkv,
                        int64_t hd) {
   return RopeQKV::apply(qkv, cos, sin, B, S, nq, nkv, hd);
@@ -314,6 +371,7 @@ TORCH_LIBRARY(b200ops, m) {
   m.def("linear(Tensor x, Tensor weight) -> Tensor", linear);
   m.def("rmsnorm(Tensor x, Tensor? res, Tensor weight, float eps) -> Tensor[]", rmsnorm);
   m.def("swiglu(Tensor gate_up) -> Tensor", swiglu);
+  m.def("swiglu_mlp(Tensor x, Tensor w_gate_up, Tensor w_down) -> Tensor", swiglu_mlp);
   m.def("rope_qkv(Tensor qkv, Tensor cos, Tensor sin, int batch, int seq, int heads, int kv_heads, int head_dim) -> Tensor[]",
         rope_qkv);
 }
@@ -330,6 +388,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                        }));
   m.def("swiglu", torch::wrap_pybind_function_no_gil(
                       [](const Tensor& gu) { return traced_or_direct("b200ops::swiglu", swiglu, gu); }));
+  m.def("swiglu_mlp", torch::wrap_pybind_function_no_gil([](const Tensor& x, const Tensor& w_gu, const Tensor& w_down) {
+          return traced_or_direct("b200ops::swiglu_mlp", swiglu_mlp, x, w_gu, w_down);
+        }));
   m.def("rope_qkv", torch::wrap_pybind_function_no_gil([](const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S,
                                                           int64_t nq, int64_t nkv, int64_t hd) {
           return traced_or_direct("b200ops::rope_qkv", rope_qkv, qkv, cos, sin, B, S, nq, nkv, hd);

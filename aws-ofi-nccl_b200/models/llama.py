@@ -129,9 +129,7 @@ class Llama:
             attn = self._attention(qkv, B, S)
             o = gemm_ops.linear(attn, P[f"l{i}.wo"])
             n2, h = llm_ops.rmsnorm(o, P[f"l{i}.norm2"], cfg.rms_eps, residual=h)
-            gu = gemm_ops.linear(n2, P[f"l{i}.wgu"])
-            act = llm_ops.swiglu(gu)
-            delta = gemm_ops.linear(act, P[f"l{i}.wdown"])
+            delta = llm_ops.swiglu_mlp(n2, P[f"l{i}.wgu"], P[f"l{i}.wdown"])
         nf, _ = llm_ops.rmsnorm(delta, P["normf"], cfg.rms_eps, residual=h)
         logits = gemm_ops.linear(nf, P["lm_head"])
         return llm_ops.cross_entropy(logits, labels.reshape(-1))

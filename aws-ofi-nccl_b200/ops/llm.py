@@ -33,6 +33,13 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     return _lib.native().swiglu(gate_up)
 
 
+def swiglu_mlp(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> torch.Tensor:
+    """``linear(swiglu(linear(x, w_gate_up)), w_down)`` as one layer: the activation and its gradient are part of
+    the products beside them.  w_gate_up [2F, hidden] (gate over up) and w_down [out, F] are contiguous; their
+    gradients go where those of ``linear`` go."""
+    return _lib.native().swiglu_mlp(x, w_gate_up, w_down)
+
+
 def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, seq: int, n_heads: int, n_kv_heads: int,
              head_dim: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """Rotated q and k, and v, as [batch, seq, heads, head_dim] tensors of their own from the fused

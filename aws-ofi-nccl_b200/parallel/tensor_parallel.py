@@ -46,13 +46,14 @@ def deinterleave_gate_up(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
 
 def ag_gemm(comm: Communicator, gathered_off: int, rows: int, k: int, other: torch.Tensor, *, b_mn: bool = False,
             gather_b: bool = False, out: torch.Tensor | None = None, act: torch.Tensor | None = None,
-            swiglu: bool = False, n_movers: int = 0, channel: int = TP_CHANNEL) -> None:
+            swiglu: bool = False, n_movers: int = 0, channel: int = TP_CHANNEL, swiglu_grad: torch.Tensor | None = None) -> None:
     """One kernel: all-gather the operand whose shards sit at ``gathered_off`` in every rank's
     window (``rows`` x ``k`` bf16 in total, this rank's shard already written in place), and
     multiply.  gather_b=False: C = gathered[rows,k] @ op(other), ``other`` is [N,k] (or [k,N] with
     b_mn).  gather_b=True: C = other[M,k] @ gathered[rows=N,k]^T.  With ``swiglu`` the product's
     interleaved gate|up columns are reduced to ``act`` [M,N/2]; ``out`` (optional then) keeps the
-    raw product for the backward pass."""
+    raw product for the backward pass.  With ``swiglu_grad`` (that raw product, [M,2N]) C is the gradient of the
+    activation, and ``out`` [M,2N] becomes the gradient of the raw product."""
     assert other.dtype == torch.bfloat16 and other.stride(1) == 1
     if gather_b:
         M, N = other.shape[0], rows
@@ -62,14 +63,18 @@ def ag_gemm(comm: Communicator, gathered_off: int, rows: int, k: int, other: tor
         N = other.shape[1] if b_mn else other.shape[0]
         assert (other.shape[0] if b_mn else other.shape[1]) == k
     if out is not None:
-        assert out.shape == (M, N) and out.dtype == torch.bfloat16 and out.stride(1) == 1
-    if swiglu:
+        assert out.shape == (M, N if swiglu_grad is None else 2 * N) and out.dtype == torch.bfloat16 and out.stride(1) == 1
+    if swiglu_grad is not None:
+        assert not swiglu and act is None and out is not None
+        assert swiglu_grad.shape == (M, 2 * N) and swiglu_grad.dtype == torch.bfloat16 and swiglu_grad.stride(1) == 1
+        act = swiglu_grad
+    elif swiglu:
         assert act is not None and act.shape == (M, N // 2) and act.stride(1) == 1
     rc = _lib.load().b200_ag_gemm(
         comm.id, gathered_off, int(gather_b), M, N, k, other.data_ptr(), other.stride(0), int(b_mn),
         out.data_ptr() if out is not None else None, out.stride(0) if out is not None else 0,
         act.data_ptr() if act is not None else None, act.stride(0) if act is not None else 0,
-        int(swiglu), n_movers, channel, _lib.stream_ptr())
+        2 if swiglu_grad is not None else int(swiglu), n_movers, channel, _lib.stream_ptr())
     _lib.check(rc, "b200_ag_gemm")
 
 
@@ -121,14 +126,11 @@ class _TPMlpFn(torch.autograd.Function):
         comm, T, H, Fl = mlp.comm, mlp.tokens, mlp.hidden, mlp.ffn_local
         Ts = T // comm.world
         mlp.dy_full[comm.rank * Ts:(comm.rank + 1) * Ts].copy_(dy_shard)
-        # dact[T,Fl] = gather(dy)[T,H] @ w_down[H,Fl]   (w_down is stored [K=H][N=Fl])
-        dact = torch.empty((T, Fl), device=dy_shard.device, dtype=torch.bfloat16)
-        ag_gemm(comm, mlp.dy_off, T, H, w_down, b_mn=True, out=dact, n_movers=mlp.n_helpers)
+        # dact[T,Fl] = gather(dy)[T,H] @ w_down[H,Fl]   (w_down is stored [K=H][N=Fl]); its epilogue goes on to dgu
+        dgu = torch.empty_like(gu)
+        ag_gemm(comm, mlp.dy_off, T, H, w_down, b_mn=True, out=dgu, n_movers=mlp.n_helpers, swiglu_grad=gu)
         # dW_down[H,Fl] = dy_full^T @ act
         _accumulate_wgrad(w_down, mlp.dy_full, act)
-        dgu = torch.empty_like(gu)
-        _lib.check(_lib.load().b200_swiglu_bwd_interleaved(dact.data_ptr(), gu.data_ptr(), dgu.data_ptr(), T, Fl,
-                                                           _lib.stream_ptr()), "swiglu_bwd_interleaved")
         # dx[T/n,H] = reduce_scatter(dgu[T,2Fl] @ w_gu[2Fl,H])   (w_gu is stored [K=2Fl][N=H])
         dx_shard = torch.empty((Ts, H), device=dy_shard.device, dtype=torch.bfloat16)
         gemm_rs(comm, dgu, w_gu, mlp.stage_off, dx_shard, b_mn=True)
