@@ -7,6 +7,10 @@ extern "C" {
 int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                    int a_mn, int b_mn, int out_fp32, int accumulate, int bn, int max_ctas, void* stream);
 
+// Both gradients of a linear layer; see gemm_grads.cu. *launches: kernels launched, 1 or 2.
+int b200_linear_grads(const void* dy, const void* x, const void* w, void* dx, void* dw, int M, int N, int K, long long lddy,
+                      long long ldx, long long ldw, long long lddx, long long lddw, int accumulate, int* launches, void* stream);
+
 int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w, void* y, float* rstd, int T, int H, float eps,
                      void* stream);
 int b200_rmsnorm_bwd_partial_rows();

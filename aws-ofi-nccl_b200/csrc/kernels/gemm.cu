@@ -9,6 +9,8 @@
 // on the same kernel without materialising a transpose.
 #include <cuda_fp8.h>
 
+#include <algorithm>
+
 #include "b200ops.h"
 #include "gemm_epilogues.cuh"
 #include "gemm_plan.h"
@@ -170,11 +172,6 @@ static int dispatch_major_2cta(const void* A, const void* B, void* C, int M, int
   if (a_mn && !b_mn) return launch_gemm_2cta<BN, true, false, OutT, EW>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
   return launch_gemm_2cta<BN, true, true, OutT, EW>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
 }
-
-// Up to this K a tile's stores take longer than its products, and eight epilogue warps are worth the stage that their
-// staging area costs: 4096 x 14336 of K = 128 takes 31 us in wide tiles, 35 with four warps; at K = 256 both take 37 to
-// 39, at 320 four warps are ahead (39 and 47).
-constexpr int SHORT_K = 192;
 
 // The narrow kernel has more stages; tiles of any other width run on the wide one.
 static int gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_mn,
@@ -408,10 +405,28 @@ static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, boo
   } else {
     const double eff256 = static_cast<double>(t256) / (w256 * units);
     const double eff128 = static_cast<double>(t128) / (w128 * units);
-    bn = (N >= 256 && eff256 + 0.08 >= eff128) ? 256 : 128;
+    // Where the narrow tiles need no more waves they are done sooner: 16 x 624 x 256 8 us, 10 in wide ones.
+    bn = (N >= 256 && w256 < w128 && eff256 + 0.08 >= eff128) ? 256 : 128;
   }
   // Few tiles and a long K: the chip is filled by splitting K over clusters.
   return {bn, tiles, max_ctas == 0 ? plan_splitk(M, N, K, pairs, bn) : SplitkPlan{1}};
+}
+
+double product_clocks(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, const void* A, const void* B) {
+  const uintptr_t a_at = reinterpret_cast<uintptr_t>(A), b_at = reinterpret_cast<uintptr_t>(B);
+  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, b_mn, a_at, b_at, 0);
+  const double floor = memory_clocks(M, N, K);
+  // what the split model was fitted to had slower waits
+  if (g.split.slices > 1) return std::max((g.split.clocks - LAUNCH_CLOCKS) * 0.7, floor) + LAUNCH_CLOCKS;
+  if (!use_pairs(M, N, 0)) return std::max((g.split.clocks - LAUNCH_CLOCKS) * 0.8, floor) + LAUNCH_CLOCKS;
+  const bool lines = (a_at | b_at | static_cast<uint64_t>(lda | ldb) * 2) % 128 == 0;
+  const int64_t rows = (M + GEMM2_BM - 1) / GEMM2_BM, units = sm_count() / 2;
+  double best = 1e30;
+  for (int width = 128; width <= 256; width += 64) {
+    const int64_t tiles = rows * ((N + width - 1) / width);
+    best = std::min(best, static_cast<double>((tiles + units - 1) / units) * pair_tile_clocks(K, width, lines, K <= SHORT_K ? 8 : 4));
+  }
+  return std::max(best, floor) + LAUNCH_CLOCKS;
 }
 
 bool runs_on_pairs(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, const void* A, const void* B, PairTiles* tiles) {

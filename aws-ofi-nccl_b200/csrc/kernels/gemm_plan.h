@@ -13,6 +13,11 @@ struct PairTiles {
   bool halves;
 };
 
+// Up to this K a tile's stores take longer than its products, and eight epilogue warps are worth the stage that their
+// staging area costs: 4096 x 14336 of K = 128 takes 31 us in wide tiles, 35 with four warps; at K = 256 both take 37 to
+// 39, at 320 four warps are ahead (39 and 47).
+constexpr int SHORT_K = 192;
+
 // Fills in the tiles of `shape` (M, N and K are set). bn: the kernel's BN; ctas: how many may run. Returns how
 // many are launched.
 int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas);
@@ -20,5 +25,20 @@ int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas);
 // Whether a product runs whole on CTA pairs, neither on single CTAs nor split along K, and then its tiles among the
 // widths 128 and 256.
 bool runs_on_pairs(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, const void* A, const void* B, PairTiles* tiles);
+
+// Clocks of a tile on CTA pairs: its k-blocks, or the stores of the tile before it where those take longer. lines: the
+// operands' rows lie on cache lines; warps: epilogue warps.
+inline double pair_tile_clocks(int k, int width, bool lines, int warps) {
+  const double wide = lines ? 520 : 640;   // a k-block of 256 columns
+  const double part = width == 256 ? 1 : width == 192 ? (lines ? .81 : .95) : (lines ? .58 : .72);
+  const double blocks = (k + GEMM_BK - 1) / GEMM_BK * wide * part, stores = (width / 64) * 620.0 / (warps / 4) + 250;
+  return (blocks > stores ? blocks : stores) + 150;
+}
+constexpr double LAUNCH_CLOCKS = 10000;   // a launch besides its tiles: ramp, pipeline fill, last stores
+// Clocks that moving a product's operands and result takes at least.
+inline double memory_clocks(double m, double n, double k) { return 2 * (m * k + n * k + m * n) / 3500; }
+
+// Estimate for a product by itself, on what b200_gemm_bf16 would choose.
+double product_clocks(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, const void* A, const void* B);
 
 }  // namespace b200

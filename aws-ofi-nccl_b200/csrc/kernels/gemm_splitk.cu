@@ -112,7 +112,7 @@ SplitkPlan plan_splitk(int M, int N, int K, bool pair, int bn) {
       at_least_floor(static_cast<double>((whole_tiles + units - 1) / units) * kb * kblock_clocks(pair, bn, busy * per_tile)) + FIXED;
   const int64_t tiles = rows * ((N + SPLITK_BN - 1) / SPLITK_BN);
   int best = 1;
-  double best_t = 0.9 * whole;   // the model is rough: a split has to promise 10 %
+  double best_t = 0.9 * whole, clocks = whole;   // the model is rough: a split has to promise 10 %
   for (int l = 1; l <= 3; ++l) {
     const int slices = 1 << l;
     if (slices * per_tile > SPLITK_MAX_CLUSTER || kb < slices * MIN_KBLOCKS) break;
@@ -121,11 +121,11 @@ SplitkPlan plan_splitk(int M, int N, int K, bool pair, int bn) {
     const double est = at_least_floor(static_cast<double>((kb + slices - 1) / slices) * kblock_clocks(pair, SPLITK_BN, tiles * slices * per_tile)) +
                        FIXED + JOIN + JOIN_SLICE * slices;
     if (est < best_t) {
-      best_t = est;
+      best_t = clocks = est;
       best = slices;
     }
   }
-  return SplitkPlan{best};
+  return SplitkPlan{best, clocks};
 }
 
 int launch_splitk(const SplitkCall& c, bool pair, SplitkPlan plan, cudaStream_t s) {

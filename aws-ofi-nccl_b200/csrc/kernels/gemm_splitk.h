@@ -15,6 +15,7 @@ struct SplitkCall {
 
 struct SplitkPlan {
   int slices;   // 1: do not split
+  double clocks = 0;   // estimate of the chosen way, a launch included
 };
 
 // Whether the product is better split along K than run on the persistent kernel of tile width `bn`

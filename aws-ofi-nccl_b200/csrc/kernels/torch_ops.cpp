@@ -79,6 +79,28 @@ void gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const Tensor& 
         "b200_gemm_bf16");
 }
 
+// dx = dy W and dw (+)= dy^T x, in one launch where that pays
+void linear_grads(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& dx, const Tensor& dw, bool accumulate) {
+  if (dw.scalar_type() != at::kBFloat16) {   // a gradient buffer of 32 bits
+    gemm(dy, w, false, true, dx, false);
+    gemm(dy, x, true, true, dw, accumulate);
+    return;
+  }
+  require(bf16_cuda(dy) && bf16_cuda(x) && bf16_cuda(w), "operands are bfloat16 CUDA tensors");
+  require(dy.dim() == 2 && x.dim() == 2 && w.dim() == 2 && dy.stride(1) == 1 && x.stride(1) == 1 && w.stride(1) == 1,
+          "operands are matrices with contiguous rows");
+  const int64_t M = dy.size(0), N = dy.size(1), K = w.size(1);
+  require(w.size(0) == N && x.size(0) == M && x.size(1) == K, "reduction dims differ");
+  require(dw.is_cuda() && dw.dim() == 2 && dw.size(0) == N && dw.size(1) == K && dw.stride(1) == 1,
+          "the output is an [M, N] bfloat16 or float32 matrix with contiguous rows");
+  int launches = 2;
+  const int rc = b200_linear_grads(dy.data_ptr(), x.data_ptr(), w.data_ptr(), dx.data_ptr(), dw.data_ptr(), static_cast<int>(M),
+                                   static_cast<int>(N), static_cast<int>(K), dy.stride(0), x.stride(0), w.stride(0), dx.stride(0),
+                                   dw.stride(0), accumulate, &launches, stream());
+  g_launches.fetch_add(launches, std::memory_order_relaxed);
+  check(rc, "b200_linear_grads");
+}
+
 PyObject* interned(const char* name) { return PyUnicode_InternFromString(name); }
 PyObject* name_written() {
   static PyObject* const name = interned("grad_written");
@@ -161,14 +183,18 @@ struct Linear : public Function<Linear> {
       const Tensor dy = grads[0].reshape({-1, grads[0].size(-1)}).contiguous();
       const Tensor x2 = x.reshape({-1, x.size(-1)});
       Tensor dx, dw;
-      if (ctx->needs_input_grad(0)) {
-        dx = at::empty_like(x2, x2.options(), at::MemoryFormat::Contiguous);
-        gemm(dy, weight, false, true, dx, false);
-        dx = dx.view(x.sizes());
-      }
+      const bool want_dx = ctx->needs_input_grad(0);
+      if (want_dx) dx = at::empty_like(x2, x2.options(), at::MemoryFormat::Contiguous);
       if (ctx->needs_input_grad(1))
-        dw = write_param_grad(weight, [&](const Tensor& out, bool accumulate) { gemm(dy, x2, true, true, out, accumulate); });
-      return {dx, dw};
+        dw = write_param_grad(weight, [&](const Tensor& out, bool accumulate) {
+          if (want_dx)
+            linear_grads(dy, x2, weight, dx, out, accumulate);
+          else
+            gemm(dy, x2, true, true, out, accumulate);
+        });
+      else if (want_dx)
+        gemm(dy, weight, false, true, dx, false);
+      return {want_dx ? dx.view(x.sizes()) : dx, dw};
     });
   }
 };
@@ -289,14 +315,18 @@ struct SwiGLUMLP : public Function<SwiGLUMLP> {
       if (ctx->needs_input_grad(2))
         dw_down = write_param_grad(w_down, [&](const Tensor& out, bool accumulate) { gemm(dy, act, true, true, out, accumulate); });
       const Tensor x2 = x.reshape({-1, x.size(-1)});
-      if (ctx->needs_input_grad(0)) {
-        dx = at::empty_like(x2, x2.options(), at::MemoryFormat::Contiguous);
-        gemm(dgu, w_gu, false, true, dx, false);
-        dx = dx.view(x.sizes());
-      }
+      const bool want_dx = ctx->needs_input_grad(0);
+      if (want_dx) dx = at::empty_like(x2, x2.options(), at::MemoryFormat::Contiguous);
       if (ctx->needs_input_grad(1))
-        dw_gu = write_param_grad(w_gu, [&](const Tensor& out, bool accumulate) { gemm(dgu, x2, true, true, out, accumulate); });
-      return {dx, dw_gu, dw_down};
+        dw_gu = write_param_grad(w_gu, [&](const Tensor& out, bool accumulate) {
+          if (want_dx)
+            linear_grads(dgu, x2, w_gu, dx, out, accumulate);
+          else
+            gemm(dgu, x2, true, true, out, accumulate);
+        });
+      else if (want_dx)
+        gemm(dgu, w_gu, false, true, dx, false);
+      return {want_dx ? dx.view(x.sizes()) : dx, dw_gu, dw_down};
     });
   }
 };
