@@ -63,7 +63,7 @@ bool one_wave(const GradsCall& c) {
 }
 
 GradsPlan plan_joint(const GradsCall& c) {
-  if (one_wave(c)) return {{128, 128}, c.M > c.N, 0, c.M <= SHORT_K ? 8 : 4, 0};
+  if (one_wave(c)) return {{128, 128}, c.M > c.N, 1, c.M <= SHORT_K ? 8 : 4, 0};   // one tile for every pair
   const bool lines = on_lines(c);
   const int pairs = sm_count() / 2;
   GradsPlan best{};
