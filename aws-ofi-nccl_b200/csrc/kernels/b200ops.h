@@ -13,6 +13,8 @@ int b200_linear_grads(const void* dy, const void* x, const void* w, void* dx, vo
 
 int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w, void* y, float* rstd, int T, int H, float eps,
                      void* stream);
+int b200_embedding_fwd(const long long* ids, const void* table, void* out, long long T, int H, void* stream);
+int b200_embedding_bwd(const long long* ids, const void* dout, void* dtable, long long T, int H, void* stream);
 int b200_rmsnorm_bwd_partial_rows();
 int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                      float* dw_partial, void* dw, int accumulate_dw, int T, int H, void* stream);

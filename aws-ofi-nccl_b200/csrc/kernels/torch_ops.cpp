@@ -1,5 +1,5 @@
-// The differentiable layers of the training path (linear, RMSNorm, SwiGLU, SwiGLU MLP, rotary split of the fused
-// projection) as autograd functions in native code: shape checks, output allocation, the calls into
+// The differentiable layers of the training path (linear, embedding, RMSNorm, SwiGLU, SwiGLU MLP, rotary split of
+// the fused projection) as autograd functions in native code: shape checks, output allocation, the calls into
 // libb200ops.so and the weight-gradient hand-over run without the interpreter. A layer's launches are
 // a few microseconds of device time each at small sizes, and the interpreter's share of a forward and
 // backward call was several times that: a linear layer of 256 x 768 x 256 took 148 us a pass through
@@ -199,6 +199,38 @@ struct Linear : public Function<Linear> {
   }
 };
 
+// Rows of the table by token id; the gradient is added up in the table's. What bounds a few hundred tokens is the host: a
+// forward and backward pass of the two-layer model of 256 channels on 256 tokens takes 923 us, and took 1011 with this layer in
+// Python (five processes of each in turn, within 2 %).
+struct Embedding : public Function<Embedding> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& ids, const Tensor& table) {
+    ctx->save_for_backward({ids, table});
+    const int64_t H = table.size(1);
+    auto shape = ids.sizes().vec();
+    shape.push_back(H);
+    Tensor out = at::empty(shape, table.options());
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    check(b200_embedding_fwd(static_cast<const long long*>(ids.data_ptr()), table.data_ptr(), out.data_ptr(), ids.numel(),
+                             static_cast<int>(H), stream()),
+          "embedding_fwd");
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return on_engine_thread([&]() -> variable_list {
+      const auto saved = ctx->get_saved_variables();
+      const Tensor &ids = saved[0], &table = saved[1];
+      const Tensor dout = rows16(grads[0]);
+      return {Tensor(), write_param_grad(table, [&](const Tensor& out, bool accumulate) {
+                if (!accumulate) out.zero_();
+                g_launches.fetch_add(1, std::memory_order_relaxed);
+                check(b200_embedding_bwd(static_cast<const long long*>(ids.data_ptr()), dout.data_ptr(), out.data_ptr(), ids.numel(),
+                                         static_cast<int>(table.size(1)), stream()),
+                      "embedding_bwd");
+              })};
+    });
+  }
+};
+
 // y = rmsnorm(h) * w with h = x (+ res), h a new tensor when there is a residual
 struct RMSNorm : public Function<RMSNorm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const c10::optional<Tensor>& res, const Tensor& weight,
@@ -381,6 +413,7 @@ variable_list rmsnorm(const Tensor& x, const c10::optional<Tensor>& res, const T
   return RMSNorm::apply(x, res, w, eps);
 }
 Tensor swiglu(const Tensor& gu) { return SwiGLU::apply(gu); }
+Tensor embedding(const Tensor& ids, const Tensor& table) { return Embedding::apply(ids, table); }
 Tensor swiglu_mlp(const Tensor& x, const Tensor& w_gu, const Tensor& w_down) { return SwiGLUMLP::apply(x, w_gu, w_down); }
 variable_list rope_qkv(const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S, int64_t nq, int64_t nkv,
                        int64_t hd) {
@@ -399,6 +432,7 @@ R traced_or_direct(const char* name, R (*fn)(A...), const Args&... args) {
 
 TORCH_LIBRARY(b200ops, m) {
   m.def("linear(Tensor x, Tensor weight) -> Tensor", linear);
+  m.def("embedding(Tensor ids, Tensor table) -> Tensor", embedding);
   m.def("rmsnorm(Tensor x, Tensor? res, Tensor weight, float eps) -> Tensor[]", rmsnorm);
   m.def("swiglu(Tensor gate_up) -> Tensor", swiglu);
   m.def("swiglu_mlp(Tensor x, Tensor w_gate_up, Tensor w_down) -> Tensor", swiglu_mlp);
@@ -412,6 +446,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   // otherwise hold for as long as it waits; the wrapper takes exceptions back to Python.
   m.def("linear", torch::wrap_pybind_function_no_gil(
                       [](const Tensor& x, const Tensor& w) { return traced_or_direct("b200ops::linear", linear, x, w); }));
+  m.def("embedding", torch::wrap_pybind_function_no_gil([](const Tensor& ids, const Tensor& table) {
+          return traced_or_direct("b200ops::embedding", embedding, ids, table);
+        }));
   m.def("rmsnorm", torch::wrap_pybind_function_no_gil(
                        [](const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
                          return traced_or_direct("b200ops::rmsnorm", rmsnorm, x, res, w, eps);

@@ -6,21 +6,6 @@ import torch
 from . import _lib
 
 
-def _write_param_grad(weight: torch.Tensor, producer) -> torch.Tensor | None:
-    """Run ``producer(out, accumulate)`` into weight.main_grad when present, else into a new tensor."""
-    main_grad = getattr(weight, "main_grad", None)
-    if main_grad is not None:
-        producer(main_grad, getattr(weight, "grad_written", False))
-        weight.grad_written = True
-        hook = getattr(weight, "grad_ready", None)
-        if hook is not None:
-            hook(weight)
-        return None
-    out = torch.empty_like(weight)
-    producer(out, False)
-    return out
-
-
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, residual: torch.Tensor | None = None):
     """Returns (normed, h) where h = x + residual (or x itself when residual is None); with a residual,
     h is a new tensor produced in the same pass as the normalisation."""
@@ -113,36 +98,8 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     return loss
 
 
-class _Embedding(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, ids, table):
-        T = ids.numel()
-        H = table.shape[1]
-        out = torch.empty((*ids.shape, H), device=table.device, dtype=table.dtype)
-        _lib.check(_lib.load().b200_embedding_fwd(ids.data_ptr(), table.data_ptr(), out.data_ptr(), T, H,
-                                                  _lib.stream_ptr()), "embedding_fwd")
-        ctx.save_for_backward(ids, table)
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        ids, table = ctx.saved_tensors
-        dout = dout.contiguous()
-        T = ids.numel()
-        H = table.shape[1]
-        lib = _lib.load()
-
-        def produce(out, acc):
-            if not acc:
-                out.zero_()
-            _lib.check(lib.b200_embedding_bwd(ids.data_ptr(), dout.data_ptr(), out.data_ptr(), T, H,
-                                              _lib.stream_ptr()), "embedding_bwd")
-
-        return None, _write_param_grad(table, produce)
-
-
 def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
-    return _Embedding.apply(ids, table)
+    return _lib.native().embedding(ids, table)
 
 
 def adamw_step(p: torch.Tensor, g: torch.Tensor, m: torch.Tensor, v: torch.Tensor, master: torch.Tensor | None,

@@ -225,3 +225,25 @@ def test_an_exception_of_a_parameters_attribute_reaches_the_caller(where):
     setattr(w, where, Raises())
     with pytest.raises(Odd):
         gemm.linear(torch.randn(8, 16, device="cuda").bfloat16(), w).float().sum().backward()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1,), (2, 65), (0, 4)])
+def test_the_embedding_adds_its_gradient_up_from_any_view(shape):
+    from aws_ofi_nccl_b200.ops import llm
+
+    table = torch.randn(33, 72, device="cuda").bfloat16().requires_grad_(True)
+    ids = torch.randint(0, 33, shape, device="cuda")
+    d = torch.randint(-2, 3, (ids.numel() * 72 + 1,), device="cuda").bfloat16()[1:].view(*shape, 72)   # at an odd element; sums exact
+    want = torch.zeros(33, 72, device="cuda").index_add_(0, ids.reshape(-1), d.reshape(-1, 72).float())
+    for written in (None, False, True):   # an ordinary gradient, the first into the flat buffer, one added to it
+        table.grad = None
+        if written is not None:
+            table.main_grad, table.grad_written = torch.ones(33, 72, device="cuda").bfloat16(), written
+        out = llm.embedding(ids, table)
+        assert torch.equal(out, table.detach()[ids])
+        out.backward(d)
+        got = table.grad if written is None else table.main_grad
+        assert torch.equal(got.float(), want + (1 if written else 0))
+    traced = torch.jit.trace(llm.embedding, (torch.zeros_like(ids), torch.zeros_like(table)), check_trace=False)
+    assert torch.equal(traced(ids, table), out)
