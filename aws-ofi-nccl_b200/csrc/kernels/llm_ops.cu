@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(CE_ROW_THREADS, CE_ROW_CTAS)
     }
   }
   const int64_t tgt = targets[row];
-  const bool counts = tgt >= 0 && tgt < V;   // other rows are ignored: no loss, zero gradient
+  const bool counts = tgt >= 0 && tgt < V;   // other rows are ignored: no loss, zeros for a gradient whatever the logits hold
   float lt = 0.f;
   if (rank == 0 && threadIdx.x == 0 && counts) lt = __bfloat162float(lr[tgt]);   // before anything is overwritten
   float m = -INFINITY;
@@ -570,13 +570,14 @@ __global__ void __launch_bounds__(CE_ROW_THREADS, CE_ROW_CTAS)
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // waited for below: `part` may be read until then
   }
   if (rank == 0 && threadIdx.x == 0) loss[row] = counts ? ce_loss(m, c, s, lt) : 0.f;
-  const float inv = counts ? grad_scale / s : 0.f;
+  const float inv = grad_scale / s, none[8] = {};
+  const Bf16x8 zero = pack8(none);
   const int own = counts ? static_cast<int>(tgt) - first : -1;   // the target's place from this thread's first element on
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int at = first + i * STEP;
     if (at >= V) break;
-    const Bf16x8 o = ce_gradient8(x[i], c, inv, own - i * STEP, grad_scale);
+    const Bf16x8 o = counts ? ce_gradient8(x[i], c, inv, own - i * STEP, grad_scale) : zero;
     if (at + 8 <= V) {
       *reinterpret_cast<Bf16x8*>(lr + at) = o;
     } else {
@@ -600,6 +601,15 @@ __global__ void __launch_bounds__(CE_THREADS)
   const int64_t row = blockIdx.x;
   bf16* lr = logits + row * ld;
   const int nvec = V / 8;
+  const int64_t tgt = targets[row];
+  if (tgt < 0 || tgt >= V) {   // an ignored row: no loss, zeros for a gradient whatever the logits hold
+    const float none[8] = {};
+    const Bf16x8 zero = pack8(none);
+    for (int i = threadIdx.x; i < nvec; i += CE_THREADS) reinterpret_cast<Bf16x8*>(lr)[i] = zero;
+    for (int i = nvec * 8 + threadIdx.x; i < V; i += CE_THREADS) lr[i] = __float2bfloat16(0.f);
+    if (threadIdx.x == 0) loss[row] = 0.f;
+    return;
+  }
   const Bf16x8* lv = reinterpret_cast<const Bf16x8*>(lr);
   float m = -FLT_MAX, s = 0.f;
   for (int i = threadIdx.x; i < nvec; i += CE_THREADS) {
@@ -625,14 +635,9 @@ __global__ void __launch_bounds__(CE_THREADS)
   }
   const float gm = block_max<CE_THREADS>(m, red);
   const float gs = block_sum<CE_THREADS>(s * __expf(m - gm), red);
-  const int64_t tgt = targets[row];
-  if (threadIdx.x == 0) {
-    const float lt = (tgt >= 0 && tgt < V) ? __bfloat162float(lr[tgt]) : 0.f;
-    loss[row] = (tgt >= 0 && tgt < V) ? (logf(gs) + gm - lt) : 0.f;
-  }
+  if (threadIdx.x == 0) loss[row] = logf(gs) + gm - __bfloat162float(lr[tgt]);
   __syncthreads();
-  const float inv = (tgt >= 0 && tgt < V) ? grad_scale / gs : 0.f;  // ignored rows get zero gradient
-  const float gsc = (tgt >= 0 && tgt < V) ? grad_scale : 0.f;
+  const float inv = grad_scale / gs;
   Bf16x8* ov = reinterpret_cast<Bf16x8*>(lr);
   for (int i = threadIdx.x; i < nvec; i += CE_THREADS) {
     float f[8];
@@ -640,13 +645,13 @@ __global__ void __launch_bounds__(CE_THREADS)
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       f[j] = __expf(f[j] - gm) * inv;
-      if (i * 8 + j == tgt) f[j] -= gsc;
+      if (i * 8 + j == tgt) f[j] -= grad_scale;
     }
     ov[i] = pack8(f);
   }
   for (int i = nvec * 8 + threadIdx.x; i < V; i += CE_THREADS) {
     float f = __expf(__bfloat162float(lr[i]) - gm) * inv;
-    if (i == tgt) f -= gsc;
+    if (i == tgt) f -= grad_scale;
     lr[i] = __float2bfloat16(f);
   }
 }

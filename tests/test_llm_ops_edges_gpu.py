@@ -187,6 +187,40 @@ def test_cross_entropy_of_a_row_with_nan_is_nan():
     assert llm.cross_entropy(logits, targets).isnan()
 
 
+def _loss_and_gradient(rows, targets):
+    """Loss of every row and gradient (scaled by 1) of rows that lie in a wider buffer, which stays as it is."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    T, V = rows.shape
+    pad = torch.full((T, (V + 7) // 8 * 8 + 8), 5.0, device="cuda").bfloat16()
+    pad[:, :V] = rows
+    loss = torch.full((T,), math.nan, device="cuda")
+    rc = _lib.load().b200_cross_entropy(pad.data_ptr(), targets.data_ptr(), loss.data_ptr(), T, V, pad.stride(0), 1.0, _lib.stream_ptr())
+    assert rc == 0 and (pad[:, V:] == 5).all()
+    return loss, pad[:, :V]
+
+
+LOWEST = torch.finfo(torch.bfloat16).min   # the usual value of a mask
+
+
+# rows of one CTA, of a cluster of two and of eight, more of them than run at once (two passes), and a wider row than a cluster holds
+CE_PATHS = [(6, 2045), (6, 16395), (6, 131069), (700, 16395), (6, 131075)]
+
+
+@pytest.mark.parametrize("T,V", CE_PATHS)
+@pytest.mark.parametrize("fill", [LOWEST, -math.inf, math.inf, math.nan, 3e38])
+def test_cross_entropy_of_an_ignored_row_is_zero(T, V, fill):
+    """Loss and gradient, whatever its logits hold."""
+    rows = torch.randn(T, V, device="cuda").bfloat16()
+    rows[::2] = fill
+    targets = torch.full((T,), 3, device="cuda")
+    targets[::2] = -1
+    targets[2] = V
+    loss, grad = _loss_and_gradient(rows, targets)
+    assert (loss[::2] == 0).all() and (grad[::2] == 0).all()
+    assert loss[1::2].isfinite().all() and (grad[1::2] != 0).any(-1).all()
+
+
 @pytest.mark.parametrize("T,K", [(1, 8), (9, 256), (17, 264), (5, 512), (9, 520), (3, 1032), (7, 2056), (300, 4096), (5, 4104), (3, 8200),
                                  (2, 16384), (3, 16392), (1200, 16400)])
 def test_quantize_rows_fp8(T, K):
