@@ -493,6 +493,14 @@ __device__ __forceinline__ Bf16x8 ce_gradient8(const Bf16x8& x, float c, float i
   return pack8(f);
 }
 
+// Eight elements of a row of V, or as many as are left of it
+__device__ __forceinline__ void zero8(bf16* row, int at, int V) {
+  if (at + 8 <= V)
+    *reinterpret_cast<uint4*>(row + at) = make_uint4(0, 0, 0, 0);
+  else
+    for (; at < V; ++at) row[at] = __float2bfloat16(0.f);
+}
+
 // A cluster of up to eight CTAs takes a row and keeps it in registers, 8 * VPT elements per thread: all loads of the
 // row are in flight at once, and maximum and sum of the CTAs' parts meet in shared memory. For rows of one CTA, and for
 // wider ones while all of them run at once: more rows than that are better off with two passes of a CTA each, whose
@@ -570,14 +578,18 @@ __global__ void __launch_bounds__(CE_ROW_THREADS, CE_ROW_CTAS)
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // waited for below: `part` may be read until then
   }
   if (rank == 0 && threadIdx.x == 0) loss[row] = counts ? ce_loss(m, c, s, lt) : 0.f;
-  const float inv = grad_scale / s, none[8] = {};
-  const Bf16x8 zero = pack8(none);
+  const float inv = counts ? grad_scale / s : 0.f;
+  if (!counts) {   // 0 * 2^0
+    c = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) *reinterpret_cast<uint4*>(&x[i]) = make_uint4(0, 0, 0, 0);
+  }
   const int own = counts ? static_cast<int>(tgt) - first : -1;   // the target's place from this thread's first element on
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int at = first + i * STEP;
     if (at >= V) break;
-    const Bf16x8 o = counts ? ce_gradient8(x[i], c, inv, own - i * STEP, grad_scale) : zero;
+    const Bf16x8 o = ce_gradient8(x[i], c, inv, own - i * STEP, grad_scale);
     if (at + 8 <= V) {
       *reinterpret_cast<Bf16x8*>(lr + at) = o;
     } else {
@@ -601,15 +613,6 @@ __global__ void __launch_bounds__(CE_THREADS)
   const int64_t row = blockIdx.x;
   bf16* lr = logits + row * ld;
   const int nvec = V / 8;
-  const int64_t tgt = targets[row];
-  if (tgt < 0 || tgt >= V) {   // an ignored row: no loss, zeros for a gradient whatever the logits hold
-    const float none[8] = {};
-    const Bf16x8 zero = pack8(none);
-    for (int i = threadIdx.x; i < nvec; i += CE_THREADS) reinterpret_cast<Bf16x8*>(lr)[i] = zero;
-    for (int i = nvec * 8 + threadIdx.x; i < V; i += CE_THREADS) lr[i] = __float2bfloat16(0.f);
-    if (threadIdx.x == 0) loss[row] = 0.f;
-    return;
-  }
   const Bf16x8* lv = reinterpret_cast<const Bf16x8*>(lr);
   float m = -FLT_MAX, s = 0.f;
   for (int i = threadIdx.x; i < nvec; i += CE_THREADS) {
@@ -635,8 +638,16 @@ __global__ void __launch_bounds__(CE_THREADS)
   }
   const float gm = block_max<CE_THREADS>(m, red);
   const float gs = block_sum<CE_THREADS>(s * __expf(m - gm), red);
-  if (threadIdx.x == 0) loss[row] = logf(gs) + gm - __bfloat162float(lr[tgt]);
+  const int64_t tgt = targets[row];
+  if (threadIdx.x == 0) {
+    const float lt = (tgt >= 0 && tgt < V) ? __bfloat162float(lr[tgt]) : 0.f;
+    loss[row] = (tgt >= 0 && tgt < V) ? (logf(gs) + gm - lt) : 0.f;
+  }
   __syncthreads();
+  if (tgt < 0 || tgt >= V) {   // an ignored row: zeros, whatever its logits hold
+    for (int at = 8 * threadIdx.x; at < V; at += 8 * CE_THREADS) zero8(lr, at, V);
+    return;
+  }
   const float inv = grad_scale / gs;
   Bf16x8* ov = reinterpret_cast<Bf16x8*>(lr);
   for (int i = threadIdx.x; i < nvec; i += CE_THREADS) {
