@@ -221,6 +221,29 @@ def test_cross_entropy_of_an_ignored_row_is_zero(T, V, fill):
     assert loss[1::2].isfinite().all() and (grad[1::2] != 0).any(-1).all()
 
 
+@pytest.mark.parametrize("T,V", CE_PATHS)
+def test_cross_entropy_at_both_ends_of_the_range(T, V):
+    """Masks of the lowest value, as a whole row, as all that some CTAs of a cluster hold and beside a huge maximum; equal logits far
+    from zero, whose distribution is uniform; every path against 64 bits."""
+    base = torch.randn(6, V, device="cuda").bfloat16()
+    targets = torch.tensor([3, V - 1, 5, 5, 1, V // 2], device="cuda")
+    base[0] = LOWEST
+    base[1, :V // 2] = LOWEST
+    base[2, 5:8] = 3e38
+    base[3], base[3, 5], base[3, 9] = LOWEST, -3e38, -3e38
+    base[4], base[5] = 5013504.0, -999424.0
+    rows, targets = base.repeat(T // 6 + 1, 1)[:T], targets.repeat(T // 6 + 1)[:T]
+    x = rows.double()
+    m = x.amax(-1, keepdim=True)
+    lse = (x - m).exp().sum(-1).log()   # less the maximum
+    want = (x - m - lse[:, None]).exp()
+    want.scatter_add_(1, targets[:, None], -torch.ones_like(m))
+    loss, grad = _loss_and_gradient(rows, targets)
+    err = 64 * 2.0 ** -24   # exponentials of arguments down to -20 whose product with log2(e) is rounded, and sums of them
+    _within(loss, lse + (m - x.gather(1, targets[:, None]))[:, 0], err, err)
+    _within(grad, want, BF + err, 1e-38)
+
+
 @pytest.mark.parametrize("T,K", [(1, 8), (9, 256), (17, 264), (5, 512), (9, 520), (3, 1032), (7, 2056), (300, 4096), (5, 4104), (3, 8200),
                                  (2, 16384), (3, 16392), (1200, 16400)])
 def test_quantize_rows_fp8(T, K):
