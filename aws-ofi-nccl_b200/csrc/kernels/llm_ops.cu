@@ -968,7 +968,7 @@ int b200_cross_entropy(void* logits, const long long* targets, float* loss, int 
 
 int b200_embedding_fwd(const long long* ids, const void* table, void* out, long long T, int H, void* stream) {
   b200::ensure_context();
-  if (H % 8) return B200_ERR_BAD_ARG;
+  if (H % 8 || !aligned16(table, out)) return B200_ERR_BAD_ARG;
   embedding_fwd_kernel<<<grid_for(T * H / 8, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const int64_t*>(ids), static_cast<const bf16*>(table), static_cast<bf16*>(out), T, H);
   B200_CUDA_OK(cudaGetLastError());
@@ -976,7 +976,8 @@ int b200_embedding_fwd(const long long* ids, const void* table, void* out, long 
 }
 int b200_embedding_bwd(const long long* ids, const void* dout, void* dtable, long long T, int H, void* stream) {
   b200::ensure_context();
-  if (H % 2) return B200_ERR_BAD_ARG;
+  // pairs of elements, and atomics on them
+  if (H % 2 || (reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dtable)) % 4) return B200_ERR_BAD_ARG;
   embedding_bwd_kernel<<<grid_for(T * H / 2, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const int64_t*>(ids), static_cast<const bf16*>(dout), static_cast<bf16*>(dtable), T, H);
   B200_CUDA_OK(cudaGetLastError());

@@ -204,6 +204,9 @@ struct Linear : public Function<Linear> {
 // Python (five processes of each in turn, within 2 %).
 struct Embedding : public Function<Embedding> {
   static Tensor forward(AutogradContext* ctx, const Tensor& ids, const Tensor& table) {
+    require(ids.scalar_type() == at::kLong && ids.is_contiguous() && (ids.is_cuda() || ids.is_pinned()),
+            "ids are contiguous 64-bit integers that the GPU can read");
+    require(bf16_cuda(table) && table.dim() == 2 && table.is_contiguous(), "the table is a contiguous bfloat16 CUDA matrix");
     ctx->save_for_backward({ids, table});
     const int64_t H = table.size(1);
     auto shape = ids.sizes().vec();
@@ -221,6 +224,8 @@ struct Embedding : public Function<Embedding> {
       const Tensor &ids = saved[0], &table = saved[1];
       const Tensor dout = rows16(grads[0]);
       return {Tensor(), write_param_grad(table, [&](const Tensor& out, bool accumulate) {
+                require(bf16_cuda(out) && out.sizes() == table.sizes() && out.is_contiguous(),
+                        "the table's gradient buffer is a contiguous bfloat16 CUDA matrix of its size");
                 if (!accumulate) out.zero_();
                 g_launches.fetch_add(1, std::memory_order_relaxed);
                 check(b200_embedding_bwd(static_cast<const long long*>(ids.data_ptr()), dout.data_ptr(), out.data_ptr(), ids.numel(),

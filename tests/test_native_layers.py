@@ -90,6 +90,50 @@ def test_entry_points_refuse_a_misaligned_pointer(name, args):
         assert fn(*args(ptrs)) == 10001
 
 
+@pytest.mark.parametrize("name,args", [
+    ("b200_embedding_fwd", lambda p: (4096, p, 8192, 4, 64, None)),
+    ("b200_embedding_fwd", lambda p: (4096, 8192, p, 4, 64, None)),
+    ("b200_embedding_bwd", lambda p: (4096, p, 8192, 4, 64, None)),
+    ("b200_embedding_bwd", lambda p: (4096, 8192, p, 4, 64, None)),
+])
+def test_the_embedding_refuses_a_misaligned_pointer(name, args):
+    """As above, refused before anything is launched: the addresses are made up."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    if torch.cuda.is_available():
+        pytest.skip("made-up addresses stay off the GPU")
+    assert getattr(_lib.load(), name)(*args(16386)) == 10001
+
+
+def test_the_embedding_refuses_what_its_kernel_cannot_read():
+    """Nothing here is on a GPU; what lies on one is tested below."""
+    from aws_ofi_nccl_b200.ops import llm
+
+    ids, table = torch.zeros(4, dtype=torch.int64), torch.zeros(3, 8, dtype=torch.bfloat16)
+    with pytest.raises(AssertionError, match="ids"):
+        llm.embedding(ids, table)
+
+
+@pytest.mark.gpu
+def test_the_embedding_refuses_other_types_and_layouts():
+    from aws_ofi_nccl_b200.ops import llm
+
+    ids, table = torch.arange(4, device="cuda"), torch.randn(6, 16, device="cuda").bfloat16()
+    for bad, what in ((ids.int(), "ids"), (ids.cpu(), "ids"), (torch.arange(8, device="cuda")[::2], "ids")):
+        with pytest.raises(AssertionError, match=what):
+            llm.embedding(bad, table)
+    for bad in (table.float(), table.cpu(), torch.randn(6, 24, device="cuda").bfloat16()[:, :16], table[0], table.T):
+        with pytest.raises(AssertionError, match="table"):
+            llm.embedding(ids, bad)
+    assert torch.equal(llm.embedding(ids.cpu().pin_memory(), table), table[:4])   # read in place
+    for buffer in (torch.zeros(6, 16, device="cuda"), torch.zeros(5, 16, device="cuda").bfloat16(), torch.zeros(6, 24, device="cuda").bfloat16()[:, :16]):
+        leaf = table.clone().requires_grad_(True)
+        leaf.main_grad = buffer
+        with pytest.raises(AssertionError, match="gradient buffer"):
+            llm.embedding(ids, leaf).sum().backward()
+        assert not buffer.any()
+
+
 @pytest.mark.gpu
 def test_gradients_of_any_view_are_taken():
     """Contiguous gradients that start at an odd element, and a batch of one whose stride is odd."""
