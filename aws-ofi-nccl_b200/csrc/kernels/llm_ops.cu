@@ -935,7 +935,7 @@ int b200_rope_qkv(void* qkv, long long pitch, void* q, void* k, void* v, const l
 int b200_cross_entropy(void* logits, const long long* targets, float* loss, int T, int V, long long ld,
                        float grad_scale, void* stream) {
   b200::ensure_context();
-  if (ld % 8) return B200_ERR_BAD_ARG;
+  if (ld % 8 || (V >= 8 && !aligned16(logits))) return B200_ERR_BAD_ARG;   // rows move as 16-byte vectors
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto L = static_cast<bf16*>(logits);
   auto TG = reinterpret_cast<const int64_t*>(targets);

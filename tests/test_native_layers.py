@@ -105,6 +105,16 @@ def test_the_embedding_refuses_a_misaligned_pointer(name, args):
     assert getattr(_lib.load(), name)(*args(16386)) == 10001
 
 
+@pytest.mark.parametrize("V", [8, 1000, 16392, 131080])
+def test_the_cross_entropy_refuses_misaligned_logits(V):
+    """On every path, before anything is launched."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    if torch.cuda.is_available():
+        pytest.skip("made-up addresses stay off the GPU")
+    assert _lib.load().b200_cross_entropy(16386, 4096, 8192, 4, V, (V + 7) // 8 * 8, 1.0, None) == 10001
+
+
 def test_the_embedding_refuses_what_its_kernel_cannot_read():
     """Nothing here is on a GPU; what lies on one is tested below."""
     from aws_ofi_nccl_b200.ops import llm
