@@ -300,8 +300,9 @@ __global__ void __launch_bounds__(QUANT_THREADS)
   }
 }
 
-// B200_GEMM_2CTA=0 keeps every GEMM on the one-CTA kernel; by default CTA pairs are used wherever
-// they apply (M >= 256, N >= 128).
+// B200_GEMM_2CTA=0 keeps every bf16 GEMM on the one-CTA kernel, and with it the joint gradients of a linear layer and the MLP's
+// products, which only exist on pairs, in two launches each. By default CTA pairs are used wherever they apply (M >= 256, N >= 128; joint
+// gradients from one row on). The fp8 product has no other kernel.
 static int gemm_pair_mode() {
   static int mode = -2;
   if (mode == -2) {
@@ -327,8 +328,9 @@ static bool gemm_args_ok(const void* A, const void* B, const void* C, int M, int
   return lda % 8 == 0 && ldb % 8 == 0 && ldc % (out_fp32 ? 4 : 8) == 0;
 }
 
+bool pairs_enabled() { return gemm_pair_mode() != 0; }
 static bool use_pairs(int M, int N, int max_ctas) {
-  return gemm_pair_mode() != 0 && M >= 256 && N >= 128 && (max_ctas == 0 || max_ctas >= 2);
+  return pairs_enabled() && M >= 256 && N >= 128 && (max_ctas == 0 || max_ctas >= 2);
 }
 
 // What a product with bn = 0 runs on: the tile width of the persistent kernel, or a split along K.

@@ -84,6 +84,7 @@ GradsPlan plan_joint(const GradsCall& c) {
 // rule takes one launch for 93; the mean of its times is 0.789 of two launches', the faster way's 0.785, and it is never
 // slower by more than 3 % than two. 256 x 768 x 256: 11 us for 20; 1000 x 2568 x 5160 58 for 75; 4096 x 4096 x 4096 158 for 169.
 bool pays(const GradsCall& c, const GradsPlan& p) {
+  if (!pairs_enabled()) return false;
   if (one_wave(c)) return true;
   const bool few_rows = c.M <= GEMM2_BM && 2.0 * c.N * c.K > 64e6;
   double alone = pair_tile_clocks(c.N, p.width[0], on_lines(c), p.warps);

@@ -18,6 +18,9 @@ struct PairTiles {
 // 39, at 320 four warps are ahead (39 and 47).
 constexpr int SHORT_K = 192;
 
+// Whether products may run on CTA pairs at all (B200_GEMM_2CTA).
+bool pairs_enabled();
+
 // Fills in the tiles of `shape` (M, N and K are set). bn: the kernel's BN; ctas: how many may run. Returns how
 // many are launched.
 int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas);
