@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 // M tiles per raster group: the CTAs of one wave (one per SM) then cover a patch of about
 // group_m x (SMs / group_m) tiles, which is close to square in elements for the default value.
 // B200_GEMM_GROUP_M overrides it (0 = plain column-major walk).
-static int gemm_group_m(int bn) {
+int gemm_group_m(int bn) {
   static int override_value = -2;
   if (override_value == -2) {
     const char* e = getenv("B200_GEMM_GROUP_M");
@@ -118,7 +118,7 @@ int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas) {
   const int pairs = ctas / 2;
   shape.tiles_m = (shape.M + GEMM2_BM - 1) / GEMM2_BM;
   shape.tiles_n = (shape.N + tiles.width - 1) / tiles.width;
-  shape.group_m = (gemm_group_m(bn) + 1) / 2;
+  shape.group_m = pair_group_m(bn);
   shape.bn = tiles.width;
   const int all = shape.tiles_m * shape.tiles_n;
   int items = all;

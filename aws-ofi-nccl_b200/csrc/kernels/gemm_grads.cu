@@ -94,6 +94,13 @@ bool pays(const GradsCall& c, const GradsPlan& p) {
   return joint < product_clocks(c.M, c.K, c.N, c.lddy, c.ldw, true, c.dy, c.w) + product_clocks(c.N, c.K, c.M, c.lddy, c.ldx, true, c.dy, c.x);
 }
 
+GemmShape product_shape(int rows, int cols, int k, int width) {
+  GemmShape s{rows, cols, k, (rows + GEMM2_BM - 1) / GEMM2_BM, (cols + width - 1) / width};
+  s.group_m = pair_group_m(GRADS_BN);
+  s.bn = width;
+  return s;
+}
+
 template <int EW>
 int launch(const GradsCall& c, const GradsPlan& p, cudaStream_t stream) {
   using S = Gemm2Smem<GRADS_BN, EW>;
@@ -110,14 +117,10 @@ int launch(const GradsCall& c, const GradsPlan& p, cudaStream_t stream) {
   if ((rc = make_tmap_2d(&dx, c.dx, c.M, out_cols, c.M == 1 ? one : c.lddx, 32, 64, 2, true))) return rc;
   if ((rc = make_tmap_2d(&dw, c.dw, c.N, out_cols, c.N == 1 ? one : c.lddw, 32, 64, 2, true))) return rc;
   GradsArgs a{};
-  const int m[2] = {c.M, c.N}, k[2] = {c.N, c.M};
   int64_t tiles = 0;
   for (int i = 0; i < 2; ++i) {
-    GemmShape s{m[i], c.K, k[i], (m[i] + GEMM2_BM - 1) / GEMM2_BM, (c.K + p.width[i] - 1) / p.width[i]};
-    s.group_m = 8;
-    s.bn = p.width[i];
-    a.shape[i] = s;
-    tiles += static_cast<int64_t>(s.tiles_m) * s.tiles_n;
+    a.shape[i] = i == 0 ? product_shape(c.M, c.K, c.N, p.width[0]) : product_shape(c.N, c.K, c.M, p.width[1]);
+    tiles += static_cast<int64_t>(a.shape[i].tiles_m) * a.shape[i].tiles_n;
   }
   a.out[0] = static_cast<__nv_bfloat16*>(c.dx);
   a.out[1] = static_cast<__nv_bfloat16*>(c.dw);
@@ -197,5 +200,8 @@ int b200_linear_grads_plan(int M, int N, int K, int* joint, int* w_dx, int* w_dw
   *w_dw = p.width[1];
   return 0;
 }
+
+// M tiles of 256 rows per raster group of the joint kernel.
+int b200_linear_grads_group(int M, int N, int K) { return product_shape(M, K, N, 128).group_m; }
 
 }  // extern "C"

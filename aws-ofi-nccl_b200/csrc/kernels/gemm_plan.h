@@ -21,6 +21,10 @@ constexpr int SHORT_K = 192;
 // Whether products may run on CTA pairs at all (B200_GEMM_2CTA).
 bool pairs_enabled();
 
+// M tiles of 128 rows per raster group of a kernel of BN `bn` (B200_GEMM_GROUP_M), and of 256 rows on CTA pairs.
+int gemm_group_m(int bn);
+inline int pair_group_m(int bn) { return (gemm_group_m(bn) + 1) / 2; }
+
 // Fills in the tiles of `shape` (M, N and K are set). bn: the kernel's BN; ctas: how many may run. Returns how
 // many are launched.
 int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas);

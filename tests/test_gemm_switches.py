@@ -19,6 +19,7 @@ for M, N, K in %r:
     assert lib.b200_linear_grads_plan(M, N, K, *(ctypes.byref(x) for x in r)) == 0
     out["joint"].append(r[0].value)
     out["mlp"].append([lib.b200_gemm_swiglu_launches(vp(4096), vp(4096), M, N, K, ll(K)), lib.b200_gemm_swiglu_bwd_launches(vp(4096), vp(4096), M, N, K, ll(K))])
+out["group"] = lib.b200_linear_grads_group(4096, 4096, 4096)
 print(json.dumps(out))
 """ % SIZES
 
@@ -32,4 +33,11 @@ def _plans(**env):
 
 @pytest.mark.parametrize("env,joint,mlp", [({}, 1, [1, 1]), ({"B200_GEMM_2CTA": "0"}, 0, [2, 2])])
 def test_without_pairs_no_product_runs_on_them(env, joint, mlp):
-    assert _plans(**env) == {"joint": [joint] * len(SIZES), "mlp": [mlp] * len(SIZES)}
+    plans = _plans(**env)
+    assert plans["joint"] == [joint] * len(SIZES) and plans["mlp"] == [mlp] * len(SIZES)
+
+
+@pytest.mark.parametrize("env,group", [({}, 8), ({"B200_GEMM_GROUP_M": "0"}, 0), ({"B200_GEMM_GROUP_M": "5"}, 3)])
+def test_the_raster_group_of_joint_gradients(env, group):
+    """In tiles of 256 rows, where the variable counts 128."""
+    assert _plans(**env)["group"] == group
