@@ -407,8 +407,13 @@ static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, boo
   } else {
     const double eff256 = static_cast<double>(t256) / (w256 * units);
     const double eff128 = static_cast<double>(t128) / (w128 * units);
-    // Where the narrow tiles need no more waves they are done sooner: 16 x 624 x 256 8 us, 10 in wide ones.
-    bn = (N >= 256 && w256 < w128 && eff256 + 0.08 >= eff128) ? 256 : 128;
+    bn = (N >= 256 && eff256 + 0.08 >= eff128) ? 256 : 128;
+    // Narrow tiles that need no more waves are done sooner: 16 x 624 x 256 8 us, 10 in wide ones. The split is weighed against the
+    // width above all the same, which its model was fitted to: against narrow tiles it would leave 24 x 560 x 2032 whole (12.8 us, 8.5 split).
+    if (w256 == w128) {
+      const SplitkPlan split = max_ctas == 0 ? plan_splitk(M, N, K, false, bn) : SplitkPlan{1};
+      return split.slices > 1 ? GemmChoice{bn, tiles, split} : GemmChoice{128, tiles, max_ctas == 0 ? plan_splitk(M, N, K, false, 128) : split};
+    }
   }
   // Few tiles and a long K: the chip is filled by splitting K over clusters.
   return {bn, tiles, max_ctas == 0 ? plan_splitk(M, N, K, pairs, bn) : SplitkPlan{1}};
