@@ -272,8 +272,8 @@ __device__ __forceinline__ void swiglu32(uint32_t* act, const uint32_t (&g)[32],
   } else {
 #pragma unroll
     for (int j = 0; j < 16; ++j)
-      act[j] = pack_bf16x2(silu_rare(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
-                           silu_rare(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]));
+      act[j] = pack_bf16x2(silu_any(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
+                           silu_any(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]));
   }
 }
 

