@@ -519,9 +519,9 @@ __device__ __forceinline__ void zero8(bf16* row, int at, int V) {
 
 // A cluster of up to eight CTAs takes a row and keeps it in registers, 8 * VPT elements per thread: all loads of the
 // row are in flight at once, and maximum and sum of the CTAs' parts meet in shared memory. For rows of one CTA, and for
-// wider ones while all of them run at once: more rows than that are better off with two passes of a CTA each, whose
-// many threads overlap one row's loads with another's stores (2048 x 128256: 294 us in clusters, 252 in two passes).
-// 4096 x 16040 takes 62 us, 103 in two passes; 2048 x 1024 13 and 24; 64 x 128256, in clusters, 20 and 28.
+// few wider ones (ce_row): many are better off with two passes of a CTA each, whose
+// many threads overlap one row's loads with another's stores (2048 x 128256: 294 us in clusters, 245 in two passes).
+// 4096 x 16040 takes 57 us, 97 in two passes; 2048 x 1024 8 and 18; 64 x 128256, in clusters, 13 and 22 (L2 flushed, launches in a graph).
 constexpr int CE_ROW_THREADS = 256;
 constexpr int CE_ROW_CTAS = 4;   // of an SM
 constexpr int CE_MAX_CLUSTER = 8;
@@ -775,6 +775,28 @@ __global__ void sumsq_kernel(const bf16* __restrict__ x, int64_t n, float* __res
   if (threadIdx.x == 0) atomicAdd(out, s);
 }
 
+// What holds a row of the cross-entropy in registers: CTAs of a cluster with `vpt` vectors per thread, the fewest that can; none where two
+// passes are better or a cluster is too small. One CTA always pays. Clusters use the SMs that two passes leave idle, so they pay for few rows, and for more
+// of them the fuller a row makes their registers. Of 240 pairs of 20 widths from 16392 to 131072 and 1 to 296 rows the rule takes clusters for 116, in
+// 0.29 to 1.10 of the time of two passes (1 x 65536 5.7 us, 12.1; 74 x 131072 16.4 and 22.3; 200 x 32768 10.6 and 12.4), and leaves out the slower
+// ones (148 x 65544 23.9 and 15.1, 74 x 32776 10.1 and 8.9, 1 x 16392 5.7 and 4.9); its times are 1.005 of the better ones'.
+struct CeRow {
+  int ctas, vpt;
+};
+static CeRow ce_row(int64_t T, int V) {
+  if (T <= 0 || V <= 0) return {0, 0};
+  const int64_t vecs = (static_cast<int64_t>(V) + 7) / 8, sms = sm_count();
+  int vpt = 1, ctas = 1;
+  while (vpt < CE_MAX_VPT && vpt * CE_ROW_THREADS < vecs) vpt *= 2;
+  while (ctas < CE_MAX_CLUSTER && ctas * vpt * CE_ROW_THREADS < vecs) ctas *= 2;
+  const int64_t held = ctas * vpt * CE_ROW_THREADS;
+  if (held < vecs) return {0, 0};
+  bool pays = true;
+  if (ctas == 2) pays = 6 * vecs >= 5 * held ? 2 * T <= 3 * sms : 3 * vecs >= 2 * held && 2 * T <= sms;
+  if (ctas > 2) pays = 10 * T * held <= 9 * sms * vecs && T * ctas <= CE_ROW_CTAS * sms;
+  return pays ? CeRow{ctas, vpt} : CeRow{0, 0};
+}
+
 // Rows move as 16-byte vectors: null (an argument left out) or on a 16-byte boundary.
 template <class... P>
 static bool aligned16(const P*... p) {
@@ -939,32 +961,30 @@ int b200_cross_entropy(void* logits, const long long* targets, float* loss, int 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto L = static_cast<bf16*>(logits);
   auto TG = reinterpret_cast<const int64_t*>(targets);
-  // the fewest vectors per thread with which a cluster of at most eight CTAs holds the row: one CTA where it can
-  const int vecs = (V + 7) / 8;
-  int vpt = 1, cluster = 1;
-  while (vpt < CE_MAX_VPT && vpt * CE_ROW_THREADS < vecs) vpt *= 2;
-  while (cluster < CE_MAX_CLUSTER && cluster * vpt * CE_ROW_THREADS < vecs) cluster *= 2;
-  const bool held = T > 0 && V > 0 && vecs <= cluster * vpt * CE_ROW_THREADS && aligned16(logits);
-  if (held && (cluster == 1 || T * static_cast<int64_t>(cluster) <= CE_ROW_CTAS * sm_count())) {
-    auto kern = vpt == 1 ? cross_entropy_row_kernel<1> : vpt == 2 ? cross_entropy_row_kernel<2>
-              : vpt == 4 ? cross_entropy_row_kernel<4> : cross_entropy_row_kernel<8>;
+  const CeRow r = ce_row(T, V);
+  if (r.ctas) {
+    auto kern = r.vpt == 1 ? cross_entropy_row_kernel<1> : r.vpt == 2 ? cross_entropy_row_kernel<2>
+              : r.vpt == 4 ? cross_entropy_row_kernel<4> : cross_entropy_row_kernel<8>;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = cluster;
+    attr.val.clusterDim.x = r.ctas;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(T * cluster);
+    cfg.gridDim = dim3(T * r.ctas);
     cfg.blockDim = dim3(CE_ROW_THREADS);
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, L, TG, loss, V, static_cast<int64_t>(ld), grad_scale, cluster));
+    B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, L, TG, loss, V, static_cast<int64_t>(ld), grad_scale, r.ctas));
     return 0;
   }
   cross_entropy_two_pass_kernel<<<T, CE_THREADS, 0, st>>>(L, TG, loss, V, ld, grad_scale);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
+
+// CTAs that share a row of that call, 0 for two passes.
+int b200_cross_entropy_ctas(int T, int V) { return ce_row(T, V).ctas; }
 
 int b200_embedding_fwd(const long long* ids, const void* table, void* out, long long T, int H, void* stream) {
   b200::ensure_context();

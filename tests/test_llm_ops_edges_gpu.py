@@ -203,8 +203,8 @@ def _loss_and_gradient(rows, targets):
 LOWEST = torch.finfo(torch.bfloat16).min   # the usual value of a mask
 
 
-# rows of one CTA, of a cluster of two and of eight, more of them than run at once (two passes), and a wider row than a cluster holds
-CE_PATHS = [(6, 2045), (6, 16395), (6, 131069), (700, 16395), (6, 131075)]
+# rows of one CTA, of a cluster of two, four and eight, too many of them (two passes), and a wider row than a cluster holds
+CE_PATHS = [(6, 2045), (6, 24587), (6, 40003), (6, 131069), (700, 24587), (6, 131075)]
 
 
 @pytest.mark.parametrize("T,V", CE_PATHS)

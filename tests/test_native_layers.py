@@ -115,6 +115,17 @@ def test_the_cross_entropy_refuses_misaligned_logits(V):
     assert _lib.load().b200_cross_entropy(16386, 4096, 8192, 4, V, (V + 7) // 8 * 8, 1.0, None) == 10001
 
 
+@pytest.mark.parametrize("T,V,ctas", [
+    (1, 8, 1), (100000, 16384, 1), (1, 131073, 0), (0, 8, 0),
+    (1, 24576, 2), (74, 24576, 2), (92, 24576, 0), (200, 32768, 2), (296, 32768, 0), (4, 40000, 4), (55, 40000, 4), (111, 40000, 0), (111, 65536, 4),
+    (148, 65536, 0), (37, 65544, 8), (74, 131072, 8), (1, 16392, 0), (148, 16392, 0), (148, 50264, 0), (148, 65544, 0), (92, 73000, 0)])
+def test_rows_of_the_cross_entropy_take_the_faster_way(T, V, ctas):
+    """CTAs that share a row as measured on 148 SMs, 0 for two passes."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    assert _lib.load().b200_cross_entropy_ctas(T, V) == ctas
+
+
 def test_the_embedding_refuses_what_its_kernel_cannot_read():
     """Nothing here is on a GPU; what lies on one is tested below."""
     from aws_ofi_nccl_b200.ops import llm
