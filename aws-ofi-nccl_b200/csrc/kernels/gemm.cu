@@ -347,8 +347,8 @@ struct GemmChoice {
 // are 64 columns, so that 160 and 224 columns (80 and 112 for a CTA) load as much as 256. The costs are medians over
 // 140 products of 256 to 8192 rows, 128 to 28672 columns and K from 64 to 16040 in three majors; the rule's choice
 // took 0.977 of the plain width's time on average there, the best choice 0.969, and none more than 1.03. What it
-// gains is the last wave: 4096 x 4096 x 14336, 256 tiles for 74 pairs, takes 333 us in four wide waves and 308 with
-// the last of them halved; 4096 x 6144 x 4096 132 us, 123 in five waves of 192 columns for six of 256.
+// gains is the last wave: 4096 x 4096 x 14336, 256 tiles for 74 pairs, takes 354 to 366 us in four wide waves and 329 with
+// the last of them halved; 2048 x 8192 x 4096 93 and 86; 1000 x 5160 x 2568 40 us in two wide waves, 34 in two of 160 columns.
 static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint64_t b_low, int units, int bn,
                            int step = 32) {
   struct Costs {
@@ -391,14 +391,15 @@ static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, boo
   const long w256 = (t256 + units - 1) / units, w128 = (t128 + units - 1) / units;
   if (pairs) {
     // With CTA pairs the tile is 256 rows tall and a wave is one tile per pair of SMs. A wave of narrow
-    // tiles costs about 0.56 of one of wide tiles (4096 x 4096 x 14336: seven waves 408 us, four wide ones
-    // 444), but nearly as much where the 128-byte rows of the operand boxes straddle cache lines and L2
-    // delivers the operands late (1000 x 5160 x 2568: three waves 46 us, two wide ones 41;
-    // 4096 x 4096 x 16040: seven 660 us, four wide ones 436). Where one operand straddles none, or every
+    // tiles costs about 0.58 of one of wide tiles (4096 x 4096 x 14336: seven waves 376 us, four wide ones
+    // 365), but nearly as much where the 128-byte rows of the operand boxes straddle cache lines and L2
+    // delivers the operands late (1000 x 5160 x 2568: three waves 43 us, two wide ones 40;
+    // 4096 x 4096 x 16040: seven 692 us, four wide ones 515). Where one operand straddles none, or every
     // second row of both straddles none (rows on 64 bytes), it lies between: two wide waves for three
-    // narrow ones are slower (1068 x 3832 x 6432: 70 us, 60), three for five faster (by 3 to 18 %). With a
+    // narrow ones are slower (1068 x 3832 x 6432: 68 us, 60), three for five faster (by 3 to 18 %). With a
     // short K what a tile costs besides its products weighs more, and there are half as many: four wide waves for seven narrow
-    // ones gain 2 to 20 % up to K = 2048 (6286 x 2368 x 640: 21 us, 25).
+    // ones gain up to K = 2048 (6286 x 2368 x 640: 20.4 us, 21.0). The lines below lie between the products of each kind that
+    // gained and those that lost, before waits suspended; the sizes here, timed since, are on the same side.
     const uintptr_t a_low = a_at | (static_cast<uintptr_t>(lda) * 2), b_low = b_at | (static_cast<uintptr_t>(ldb) * 2);
     const bool a_lines = a_low % 128 == 0, b_lines = b_low % 128 == 0, halves = (a_low | b_low) % 64 == 0;
     const double narrow_wave = a_lines && b_lines ? (K <= 2048 ? 0.58 : 0.56) : a_lines || b_lines || halves ? 0.62 : 0.85;

@@ -7,7 +7,11 @@
 // gate|up again (forward), or d(act), which was written for it, and gate|up (backward): 352 and 587 MB for 4096 tokens
 // of 14336, which memory bounds. Against two launches (CUDA events, L2 flushed), forward and backward: 4096 tokens x 14336 x
 // 4096 663 -> 587 us and 394 -> 337; 8192 x 8192 x 2048 413 -> 339 and 276 -> 216; 2048 x 8192 x 1024 87 -> 65 and
-// 73 -> 60; 8192 x 4096 x 256 99 -> 67 and 89 -> 81; 256 x 512 x 256 15 -> 13 and 15 -> 15.
+// 73 -> 60; 8192 x 4096 x 256 99 -> 67 and 89 -> 81; 256 x 512 x 256 15 -> 13 and 15 -> 15. Both times of launches alone, in
+// a graph: the gradient's product has tiles of two widths only and an epilogue that the last tile does not hide, and below about 8 M elements
+// of d(act) it is up to 14 % slower than a product and a pass (300 x 5632 x 2048 23.5 us, 20.6; 2048 x 1376 x 512 17.0 and 15.1; 256 x 512 x
+// 256 8.3 and 7.6), above 5 to 22 % faster. It keeps d(act) in 32 bits, which a pass would have to write and read; forward and backward
+// together are as fast as three launches and two or faster at 110 of 112 sizes (256 to 8192 tokens, 128 to 28672 x 64 to 8192).
 #include "b200ops.h"
 #include "gemm_epilogues.cuh"
 #include "gemm_plan.h"

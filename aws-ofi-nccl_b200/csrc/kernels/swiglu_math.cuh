@@ -4,14 +4,17 @@
 // overlap: a warp that is alone on its scheduler, as in an epilogue, took 125 clocks for each. The quotients are
 // written out instead, for denominators that need no such branch: the reciprocal unit's value and one residual
 // correction of the quotient (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
-// 1990), which rounds like IEEE division. What errs is the exponential. Against 64
+// 1990). His proof that this rounds correctly asks for a correctly rounded reciprocal, which the unit's is not: of 1.6
+// billion random quotients above 2^-99 three differed from IEEE division, by one ulp. Below, the residual
+// loses bits to underflow, and the quotient is within an ulp of IEEE division's (1 % differ between 2^-126 and 2^-100, 29 % of the subnormal ones). What
+// errs is the exponential. Against 64
 // bits, over bf16's gates within 20, silu is off by 0.16 ulp on average and the logistic function by 0.13, with IEEE
 // division by 0.17 and 0.15; over normally distributed gates of 32 bits silu_ordinary by 0.82 like the division.
 #pragma once
 
 namespace b200 {
 
-// n / d for 1 <= d < 2^126 and finite n
+// n / d for 1 <= d < 2^126 and finite n, within an ulp of IEEE division
 __device__ __forceinline__ float quotient(float n, float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));

@@ -126,6 +126,45 @@ def test_swiglu_of_rare_gates(F):
         _within(a.detach()[ok], b[ok].double(), 2 * BF, 1e-30)
 
 
+def _misses(got, exact):
+    """Elements that are not the exact value rounded to bf16. With a mean error of E ulp of 32 bits before that rounding a share of
+    E / 2^16 is to be expected: as often lies the middle between two bf16 values in between."""
+    return (got != exact.bfloat16()).sum().item() / got.numel() * 2.0 ** 16
+
+
+def test_swiglu_errs_by_ulps_of_32_bits():
+    """Its quotients and exponential are not correctly rounded; what is left of that in bf16 says by how much they err."""
+    from aws_ofi_nccl_b200.ops import llm
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    gu = (torch.randn(2048, 2 * 4096, device="cuda", generator=g) * 3).bfloat16().requires_grad_(True)
+    d = torch.randn(2048, 4096, device="cuda", generator=g).bfloat16()
+    out = llm.swiglu(gu)
+    (dgu,) = torch.autograd.grad(out, (gu,), d)
+    G, U = gu.detach().double().split(4096, -1)
+    s, D = torch.sigmoid(G), d.double()
+    # two roundings and the exponential's error each; d(gate) has six, and terms that cancel
+    assert _misses(out.detach(), G * s * U) < 2 and _misses(dgu[:, 4096:], D * G * s) < 2
+    assert _misses(dgu[:, :4096], D * U * s * (1 + G * (1 - s))) < 8
+
+
+@pytest.mark.parametrize("T,F", [(1, 32), (5, 96), (1000, 2080)])
+def test_interleaved_swiglu_gradient_is_that_of_halves(T, F):
+    """Gate and up alternate in blocks of 32 columns there: the same bits elsewhere."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    lib, d, gu = _lib.load(), torch.randn(T, F, device="cuda").bfloat16(), torch.randn(T, 2 * F, device="cuda").bfloat16()
+    half, mixed = torch.empty_like(gu), torch.full_like(gu, 7.0)
+    assert lib.b200_swiglu_bwd(d.data_ptr(), gu.data_ptr(), half.data_ptr(), T, F, _lib.stream_ptr()) == 0
+
+    def interleave(t):
+        return t.view(T, 2, F // 32, 32).transpose(1, 2).reshape(T, 2 * F).contiguous()
+
+    inter = interleave(gu)
+    assert lib.b200_swiglu_bwd_interleaved(d.data_ptr(), inter.data_ptr(), mixed.data_ptr(), T, F, _lib.stream_ptr()) == 0
+    assert torch.equal(mixed, interleave(half))
+
+
 @pytest.mark.parametrize("n", [8, 1024, 8 * 256 * 148 * 256 + 8])   # one vector; less than a CTA; one pass more than a full grid
 def test_adamw_over_the_whole_grid(n):
     from aws_ofi_nccl_b200.ops import llm

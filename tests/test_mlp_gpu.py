@@ -102,6 +102,21 @@ def test_gates_of_every_size_in_the_product():
     assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-38).all()
 
 
+def test_the_activation_of_the_product_errs_by_ulps_of_32_bits():
+    """Gates and ups that are exact in 32 bits. A share of E / 2^16 of the results is not the exact one rounded to bf16 where the error
+    before that rounding is E ulp of 32 bits on average."""
+    T = ffn = 2048
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x, w = torch.zeros(T, 8, device="cuda").bfloat16(), torch.zeros(2 * ffn, 8, device="cuda").bfloat16()
+    x[:, :2] = torch.randn(T, 2, device="cuda", generator=g) * 3
+    w[:ffn, 0], w[ffn:, 1] = torch.randn(ffn, device="cuda", generator=g), torch.randn(ffn, device="cuda", generator=g)
+    gu, act = torch.empty(T, 2 * ffn, device="cuda").bfloat16(), torch.empty(T, ffn, device="cuda").bfloat16()
+    _swiglu_product(x, w, gu, act)
+    G, U = x[:, :1].double() * w[:ffn, 0].double(), x[:, 1:2].double() * w[ffn:, 1].double()
+    misses = (act != (G * torch.sigmoid(G) * U).bfloat16()).sum().item()
+    assert misses / act.numel() * 2.0 ** 16 < 4
+
+
 def test_large_gates_take_no_longer():
     """Timed against ordinary ones in turn; a division as a call of its own took five times as long."""
     T, ffn, K = 4096, 4096, 512
