@@ -150,7 +150,8 @@ class ExpertParallel:
         _lib.check(rc, "b200_moe_combine")
 
     def dequant(self, out: torch.Tensor | None = None) -> torch.Tensor:
-        """fp8 receive rows + scales -> bf16 [capacity, H].  Rows past the last received one are zeros in a new
+        """fp8 receive rows + scales -> bf16 [capacity, H], for programs that dispatch with ``dispatch_raw`` and read the
+        window (``dispatch`` stores the rows that stay itself).  Rows past the last received one are zeros in a new
         tensor and are left alone in ``out``."""
         fresh = out is None
         if fresh:   # the kernel writes the zeros of the rows that nobody sent
