@@ -19,6 +19,7 @@
 #include <cstdlib>
 
 #include "gemm_epilogues.cuh"
+#include "gemm_plan.h"
 #include "gemm_tcgen05.cuh"
 #include "gemm_tcgen05_2cta.cuh"
 #include "gin_device.cuh"
@@ -494,6 +495,7 @@ int b200_ag_gemm(int comm, size_t gathered_off, int gather_b, int M, int N, int 
       shape.m_major = gm >= shape.tiles_m ? 1 : 0;
     }
   }
+  if (pairs && h.nranks == 1 && !gather_b) plan_walk(shape, 2);   // nothing arrives shard by shard
   CUtensorMap tmA, tmB, tmC, tmAct;
   int rc;
   const void* gathered = h.window[h.rank] + gathered_off;

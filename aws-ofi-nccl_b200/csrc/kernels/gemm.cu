@@ -54,17 +54,40 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   gemm_mainloop<BN, A_MN, B_MN>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
 }
 
+static int group_m_override() {
+  static const int value = [] {
+    const char* e = getenv("B200_GEMM_GROUP_M");
+    return e ? atoi(e) : -1;
+  }();
+  return value;
+}
+
 // M tiles per raster group: the CTAs of one wave (one per SM) then cover a patch of about
 // group_m x (SMs / group_m) tiles, which is close to square in elements for the default value.
 // B200_GEMM_GROUP_M overrides it (0 = plain column-major walk).
 int gemm_group_m(int bn) {
-  static int override_value = -2;
-  if (override_value == -2) {
-    const char* e = getenv("B200_GEMM_GROUP_M");
-    override_value = e ? atoi(e) : -1;
-  }
-  if (override_value >= 0) return override_value;
+  if (group_m_override() >= 0) return group_m_override();
   return bn == 256 ? 16 : 12;
+}
+
+// A group of M tiles reads its rows of A once and all of B, so several groups take B from memory as often. Where one operand
+// stays in L2 beside the streams, all of its tiles are walked before the next tile of the other operand, which is then read
+// once: 4096 x 28672 x 4096 takes 0.33 GB from memory where groups of eight took 0.52. What that gains is power, which these
+// products are bound by: looped over rotating buffers at the 1000 W limit it takes 711 us for 729, its weight gradient (N
+// tiles first) 4096 x 14336 x 4096 364 for 371, 8192 x 16384 x 2048 417 for 429, the fp8 product 4096 x 14336 x 4096 with its
+// quantiser 205 for 211. An operand of 34 MB stays; with 50 MB (6144 x 16384 x 4096, 5120 x 13824 x 5120) products took up to 2 %
+// longer so, with 67 MB 6 %: the two halves of L2 each hold what their own SMs read. Operands of no more tiles than a group are
+// walked whole by the groups (28672 x 2048 x 1024: N tiles first 105 us, 103 in groups).
+void plan_walk(GemmShape& s, int elem_bytes) {
+  constexpr int64_t ROOM = 40000000;
+  if (group_m_override() >= 0) return;
+  const int64_t a = static_cast<int64_t>(s.M) * s.K * elem_bytes, b = static_cast<int64_t>(s.N) * s.K * elem_bytes;
+  if (a <= b && a <= ROOM && s.tiles_m > s.group_m) {
+    s.one_group = 1;
+    s.m_major = 0;
+  } else if (b < a && b <= ROOM && s.tiles_n > s.group_m) {
+    s.m_major = 1;
+  }
 }
 
 template <int BN, bool A_MN, bool B_MN, typename OutT>
@@ -114,7 +137,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Gemm2Smem<BN, EW>::T
   gemm_mainloop_2cta<BN, A_MN, B_MN, StoreEpilogue<OutT>, NoGate, false, EW>(&tmA, &tmB, shape, epi, gate, err_word, smem_raw);
 }
 
-int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas) {
+int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas, int elem_bytes) {
   const int pairs = ctas / 2;
   shape.tiles_m = (shape.M + GEMM2_BM - 1) / GEMM2_BM;
   shape.tiles_n = (shape.N + tiles.width - 1) / tiles.width;
@@ -127,6 +150,7 @@ int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas) {
     items = 2 * all - shape.halve_from;
   }
   shape.b_box = tiles.width / (tiles.halves ? 4 : 2);
+  plan_walk(shape, elem_bytes);
   return 2 * (items < pairs ? items : pairs);
 }
 
@@ -203,7 +227,7 @@ static int launch_gemm_fp8(const void* A, const void* B, const float* a_scale, c
                            int K, int64_t lda, int64_t ldb, int64_t ldc, PairTiles tiles, cudaStream_t stream) {
   CUtensorMap tmA, tmB, tmC;
   GemmShape shape{M, N, K, 0, 0};
-  const int grid = pair_grid(shape, tiles, BN, sm_count());
+  const int grid = pair_grid(shape, tiles, BN, sm_count(), 1);
   int rc = make_tmap_2d(&tmA, A, M, K, lda, 128, 2 * GEMM_BK, 1, true);   // 128 one-byte elements = 128 B per row
   if (rc) return rc;
   rc = make_tmap_2d(&tmB, B, N, K, ldb, shape.b_box, 2 * GEMM_BK, 1, true);

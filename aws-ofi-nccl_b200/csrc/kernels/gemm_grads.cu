@@ -98,6 +98,7 @@ GemmShape product_shape(int rows, int cols, int k, int width) {
   GemmShape s{rows, cols, k, (rows + GEMM2_BM - 1) / GEMM2_BM, (cols + width - 1) / width};
   s.group_m = pair_group_m(GRADS_BN);
   s.bn = width;
+  plan_walk(s, 2);
   return s;
 }
 

@@ -25,9 +25,12 @@ bool pairs_enabled();
 int gemm_group_m(int bn);
 inline int pair_group_m(int bn) { return (gemm_group_m(bn) + 1) / 2; }
 
-// Fills in the tiles of `shape` (M, N and K are set). bn: the kernel's BN; ctas: how many may run. Returns how
+// Order of the tiles of a product on CTA pairs whose group_m, tiles_m and tiles_n are set; elem_bytes: an operand's element.
+void plan_walk(GemmShape& shape, int elem_bytes);
+
+// Fills in the tiles of `shape` (M, N and K are set) and their order. bn: the kernel's BN; ctas: how many may run; elem_bytes: an operand's element. Returns how
 // many are launched.
-int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas);
+int pair_grid(GemmShape& shape, PairTiles tiles, int bn, int ctas, int elem_bytes = 2);
 
 // Whether a product runs whole on CTA pairs, neither on single CTAs nor split along K, and then its tiles among the
 // widths 128 and 256.

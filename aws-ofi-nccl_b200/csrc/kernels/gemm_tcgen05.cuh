@@ -40,6 +40,7 @@ struct GemmShape {
   int m_major = 0;     // 1: walk all N tiles of an M tile before the next M tile
   int n_rot = 0;       // tile_n = (raw + n_rot) % tiles_n
   int group_m = 0;     // default order only: M tiles are walked in groups of this many (0 = all)
+  int one_group = 0;   // 1: all M tiles are one group, whatever group_m says (plan_walk)
   // CTA pairs only, see TileSpan:
   int bn = 0;               // columns of a tile (0 = the kernel's BN)
   int halve_from = 1 << 30; // tiles from this number on are computed as two halves
@@ -55,7 +56,7 @@ __device__ __forceinline__ void tile_coords(const GemmShape& s, int tile, int& t
   if (s.m_major) {
     raw_m = tile / s.tiles_n;
     tn = tile % s.tiles_n;
-  } else if (s.group_m > 0 && s.group_m < s.tiles_m) {
+  } else if (s.group_m > 0 && s.group_m < s.tiles_m && !s.one_group) {
     const int per_group = s.group_m * s.tiles_n;
     const int g = tile / per_group;
     const int first_m = g * s.group_m;

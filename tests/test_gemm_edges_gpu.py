@@ -41,6 +41,22 @@ def test_product_and_accumulation(M, N, K, out_dtype, a_mn, b_mn):
     assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
 
 
+# all M tiles of a column before the next column; all N tiles of a row before the next row; the last wave halved or not
+@pytest.mark.parametrize("M,N,K", [(2504, 2632, 72), (2632, 2504, 72), (2312, 4104, 200), (4104, 2312, 200)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_every_tile_is_computed_in_either_order_of_tiles(M, N, K, b_mn):
+    from aws_ofi_nccl_b200.ops.gemm import gemm
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    b = torch.randn(*((K, N) if b_mn else (N, K)), device="cuda", generator=g).bfloat16()
+    A, B = a.double(), (b if b_mn else b.T).double()
+    ref, out = A @ B, torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm(a, b, b_mn=b_mn, out=out)
+    # K products in fp32 in any order, rounded once to bf16
+    assert ((out.double() - ref).abs() <= K * 2.0 ** -24 * (A.abs() @ B.abs()) + 2.0 ** -8 * ref.abs()).all()
+
+
 def _plan(M, N, K, a_mn=False, b_mn=False):
     """(pair, tile width, slices) of the automatic choice."""
     from aws_ofi_nccl_b200.ops import _lib
