@@ -1,0 +1,53 @@
+// Kernels that start while the one before them in the stream ends (programmatic dependent launch).
+//
+// A kernel launched with launch_dependent may be scheduled once every CTA of the kernel before it has called grid_release (or
+// has exited), so that its launch, its barriers, its tensor memory and its first instructions are under way while the last
+// tiles of that kernel are stored. Every CTA of it calls grid_wait before it touches global memory: that returns when the
+// kernel before it, and by the same rule everything before that, has ended and its writes are visible. Behind a kernel that
+// never releases, or anything that is no kernel, such a launch is an ordinary one. What it gains is 2 to 2.5 us between two
+// kernels: forward and both gradients of 128 x 4096 x 14336, three of them, take 82.6 us for 89.6, 1000 x 2568 x 5160 85 for 90
+// (two), SwiGLU of 4096 x 14336 and its gradient 147.6 for 150.2. Kernels that wait for other ranks' tiles are launched ordinarily.
+//
+// Where a kernel takes const __restrict__ pointers (or restrict ones that it only reads from) the compiler may move loads through
+// them anywhere, before grid_wait too: such kernels use their pointers as after_wait returns them.
+//
+// grid_release stands near the end of a kernel's work, or at the start of kernels of several waves, where the last CTA to start
+// is what counts: from then on CTAs of the next kernel hold what room there is on an SM,
+// which kernels of other streams could use.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace b200 {
+
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename P>
+__device__ __forceinline__ void written_before(P& pointer) {
+  asm volatile("" : "+l"(pointer)::"memory");
+}
+template <typename... P>
+__device__ __forceinline__ void after_wait(P&... pointers) {
+  grid_wait();
+  (written_before(pointers), ...);
+}
+
+// The launch error, if any, is left for cudaGetLastError.
+template <typename... P, typename... A>
+void launch_dependent(void (*kern)(P...), int grid, int threads, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(std::forward<A>(args))...);
+}
+
+}  // namespace b200

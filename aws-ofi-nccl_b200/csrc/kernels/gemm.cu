@@ -119,7 +119,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
   if (grid > cap) grid = cap;
   int* err = device_status_word();
-  kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
+  launch_dependent(kern, grid, GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -183,7 +183,7 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
     attr_set = true;
   }
   int* err = device_status_word();
-  kern<<<grid, S::THREADS, S::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
+  launch_dependent(kern, grid, S::THREADS, S::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -239,7 +239,7 @@ static int launch_gemm_fp8(const void* A, const void* B, const float* a_scale, c
     B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
     attr_set = true;
   }
-  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmC, static_cast<__nv_bfloat16*>(C), ldc, a_scale, b_scale,
+  launch_dependent(kern, grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<__nv_bfloat16*>(C), ldc, a_scale, b_scale,
                                                                      shape, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -276,6 +276,8 @@ template <int TPR, int VPT>
 __global__ void __launch_bounds__(QUANT_THREADS)
     quant_rows_fp8_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, int rows, int K,
                           int64_t ldx, int64_t ldq) {
+  after_wait(x, q, scale);
+  grid_release();
   __shared__ float red[QUANT_THREADS / 32];
   const int t = threadIdx.x % TPR, warp = threadIdx.x >> 5;
   const int64_t r = static_cast<int64_t>(blockIdx.x) * (QUANT_THREADS / TPR) + threadIdx.x / TPR;
@@ -309,6 +311,8 @@ __global__ void __launch_bounds__(QUANT_THREADS)
 // Rows that a CTA's registers do not hold: a warp per row, twice over it.
 __global__ void __launch_bounds__(QUANT_THREADS)
     quant_wide_rows_fp8_kernel(const __nv_bfloat16* x, uint8_t* q, float* scale, int rows, int K, int64_t ldx, int64_t ldq) {
+  after_wait(x, q, scale);
+  grid_release();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   for (int64_t r = blockIdx.x * warps + warp; r < rows; r += gridDim.x * warps) {
     const uint4* src = reinterpret_cast<const uint4*>(x + r * ldx);
@@ -592,7 +596,7 @@ int b200_quant_rows_fp8(const void* x, void* q, float* scale, int rows, int K, l
   auto Q = static_cast<uint8_t*>(q);
   // up to four vectors per thread while a warp can hold the row, then eight and more threads
 #define B200_QUANT(TPR, VPT)                                                                                                   \
-  quant_rows_fp8_kernel<TPR, VPT><<<(rows + QUANT_THREADS / TPR - 1) / (QUANT_THREADS / TPR), QUANT_THREADS, 0, st>>>(X, Q, scale, rows, K, ldx, ldq)
+  launch_dependent(quant_rows_fp8_kernel<TPR, VPT>, (rows + QUANT_THREADS / TPR - 1) / (QUANT_THREADS / TPR), QUANT_THREADS, 0, st, X, Q, scale, rows, K, ldx, ldq)
   if (K <= 256) B200_QUANT(32, 1);
   else if (K <= 512) B200_QUANT(32, 2);
   else if (K <= 1024) B200_QUANT(32, 4);
@@ -604,7 +608,7 @@ int b200_quant_rows_fp8(const void* x, void* q, float* scale, int rows, int K, l
     int grid = (rows + 7) / 8;
     const int cap = sm_count() * 8;
     if (grid > cap) grid = cap;
-    quant_wide_rows_fp8_kernel<<<grid, QUANT_THREADS, 0, st>>>(X, Q, scale, rows, K, ldx, ldq);
+    launch_dependent(quant_wide_rows_fp8_kernel, grid, QUANT_THREADS, 0, st, X, Q, scale, rows, K, ldx, ldq);
   }
 #undef B200_QUANT
   B200_CUDA_OK(cudaGetLastError());

@@ -138,7 +138,7 @@ int launch(const GradsCall& c, const GradsPlan& p, cudaStream_t stream) {
   }
   const int pairs = sm_count() / 2;
   const int grid = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
-  kern<<<grid, S::THREADS, S::TOTAL_EPI, stream>>>(rows, cols, w, x, dx, dw, a, device_status_word());
+  launch_dependent(kern, grid, S::THREADS, S::TOTAL_EPI, stream, rows, cols, w, x, dx, dw, a, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -109,6 +109,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Gemm2Smem<GRADS_BN, 
   cluster_sync_all();   // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+  grid_wait();   // the operands may be the kernel before's
   GradsWalk walk(args);
 
   if (warp == 0) {
@@ -151,6 +152,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Gemm2Smem<GRADS_BN, 
           }
         }
       }
+      grid_release();   // what is left are the last stages' products and the last stores
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)

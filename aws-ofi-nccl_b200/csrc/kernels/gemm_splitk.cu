@@ -14,16 +14,18 @@ namespace {
 template <bool PAIR>
 cudaLaunchConfig_t config(cudaLaunchAttribute* attr, int tiles, int slices, cudaStream_t stream) {
   const int cluster = slices * (PAIR ? 2 : 1);
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = cluster;
-  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see dependent_launch.cuh
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(tiles * cluster);
   cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = SplitkSmem<PAIR>::TOTAL;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cfg;
 }
 
@@ -44,8 +46,8 @@ int launch(const SplitkCall& c, int slices, cudaStream_t stream) {
     B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitkSmem<PAIR>::TOTAL));
     attr_set.store(true, std::memory_order_release);
   }
-  cudaLaunchAttribute attr;
-  cudaLaunchConfig_t cfg = config<PAIR>(&attr, shape.tiles_m * shape.tiles_n, slices, stream);
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = config<PAIR>(attr, shape.tiles_m * shape.tiles_n, slices, stream);
   B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, static_cast<OutT*>(c.C), static_cast<int64_t>(c.ldc), shape, slices,
                                   c.accumulate, device_status_word()));
   return 0;
@@ -67,8 +69,8 @@ int resident_clusters(int log2_slices) {
   int n = known[log2_slices].load(std::memory_order_relaxed);
   if (n >= 0) return n;
   auto kern = gemm_splitk_kernel<PAIR, false, false, __nv_bfloat16>;
-  cudaLaunchAttribute attr;
-  cudaLaunchConfig_t cfg = config<PAIR>(&attr, 1, 1 << log2_slices, nullptr);
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = config<PAIR>(attr, 1, 1 << log2_slices, nullptr);
   n = 0;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitkSmem<PAIR>::TOTAL) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {

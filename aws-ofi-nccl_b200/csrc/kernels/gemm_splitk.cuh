@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+  grid_wait();   // the operands may be the kernel before's
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
           phase ^= 1;
         }
       }
+      grid_release();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer

@@ -66,7 +66,7 @@ static int launch_swiglu(const void* x, const void* w, void* gu, void* act, int 
   if ((rc = make_tmap_2d(&tmAct, act, M, F, F, 32, 64, 2, true))) return rc;
   auto kern = gemm_swiglu_kernel<BN>;
   B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
-  kern<<<grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream>>>(tmA, tmB, tmGate, tmUp, tmAct, shape, F, device_status_word());
+  launch_dependent(kern, grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream, tmA, tmB, tmGate, tmUp, tmAct, shape, F, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -87,7 +87,7 @@ static int launch_swiglu_bwd(const void* dy, const void* w, const void* gu, void
   }
   auto kern = gemm_swiglu_bwd_kernel<BN>;
   B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL_EPI));
-  kern<<<grid, S::THREADS, S::TOTAL_EPI, stream>>>(tmA, tmB, tm[0], tm[1], tm[2], tm[3], shape, device_status_word());
+  launch_dependent(kern, grid, S::THREADS, S::TOTAL_EPI, stream, tmA, tmB, tm[0], tm[1], tm[2], tm[3], shape, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

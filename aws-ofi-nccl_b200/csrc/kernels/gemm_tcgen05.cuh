@@ -127,6 +127,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+  grid_wait();   // the operands may be the kernel before's
 
   const int num_tiles = shape.tiles_m * shape.tiles_n;
   const int num_kb = (shape.K + GEMM_BK - 1) / GEMM_BK;
@@ -172,6 +173,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
           }
         }
       }
+      grid_release();   // what is left are the last stages' products and the last stores
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer

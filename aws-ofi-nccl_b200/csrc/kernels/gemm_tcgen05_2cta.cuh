@@ -185,6 +185,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
   cluster_sync_all();   // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+  grid_wait();   // the operands may be the kernel before's
 
   const int num_items = tile_items(shape);
   const int num_kb = (shape.K + BK_ELEMS - 1) / BK_ELEMS;
@@ -234,6 +235,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
           }
         }
       }
+      grid_release();   // what is left are the last stages' products and the last stores
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)

@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "b200ops.h"
+#include "dependent_launch.cuh"
 #include "host_util.h"
 #include "swiglu_math.cuh"
 
@@ -104,6 +105,8 @@ template <int TPR, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
     rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, bf16* __restrict__ h_out,
                        const bf16* __restrict__ w, bf16* __restrict__ y, float* __restrict__ rstd, int T, int H, float eps) {
+  after_wait(x, res, h_out, w, y, rstd);
+  grid_release();
   __shared__ float red[2][NORM_THREADS / 32];
   const int lane = threadIdx.x % TPR;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (NORM_THREADS / TPR) + threadIdx.x / TPR;
@@ -177,6 +180,7 @@ __global__ void __launch_bounds__(NORM_THREADS, 2)
     rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                        const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                        float* __restrict__ dw_partial, int T, int H) {
+  after_wait(dy, x, w, rstd, dres, dx, dw_partial);
   constexpr int R = NORM_THREADS / TPR;   // rows of a CTA at a time
   __shared__ float red[2][NORM_THREADS / 32];
   __shared__ float group_dw[R > 1 ? R - 1 : 1][R > 1 ? TPR * VPT * 8 : 1];
@@ -256,6 +260,7 @@ __global__ void __launch_bounds__(NORM_THREADS, 2)
     }
     if (AHEAD) cur = next;
   }
+  grid_release();
   if constexpr (R > 1) {
     if (group > 0) {
 #pragma unroll
@@ -286,6 +291,8 @@ __global__ void __launch_bounds__(NORM_THREADS, 2)
 // each, so that a column's rows are not one chain of dependent loads.
 __global__ void __launch_bounds__(256)
     colsum_partial_kernel(const float* __restrict__ partial, bf16* __restrict__ dw, int nrows, int H, int accumulate) {
+  after_wait(partial, dw);
+  grid_release();
   __shared__ float part[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int h = blockIdx.x * 32 + lane;
@@ -319,6 +326,8 @@ __device__ __forceinline__ void store_stream(Bf16x8* p, const Bf16x8& v) {
 }
 template <typename Index>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, int64_t T, int F) {
+  after_wait(gu, out);
+  grid_release();
   const Index nvec = static_cast<Index>(T * F / 8), fv = F / 8;
   for (Index k = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; k < nvec; k += static_cast<Index>(gridDim.x) * blockDim.x) {
     const Index t = k / fv, c = k - t * fv;
@@ -338,6 +347,8 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict_
 template <bool INTERLEAVED, typename Index>
 __global__ void __launch_bounds__(256)
     swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu, int64_t T, int F) {
+  after_wait(dout, gu, dgu);
+  grid_release();
   const Index nvec = static_cast<Index>(T * F / 8), fv = F / 8;
   for (Index k = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; k < nvec; k += static_cast<Index>(gridDim.x) * blockDim.x) {
     int64_t gi, ui;
@@ -372,6 +383,8 @@ __global__ void __launch_bounds__(256)
 // position of token t is t % seq. sign = +1 forward, -1 backward (the inverse rotation).
 __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn, int64_t T,
                             int nheads, int hd, int64_t pitch, int seq, float sign) {
+  after_wait(x, cs, sn);
+  grid_release();
   const int half = hd / 2;
   const int64_t total = T * nheads * (half / 2);  // each thread rotates two adjacent pairs (bf162 loads)
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -416,6 +429,8 @@ template <int V, bool BACKWARD>
 __global__ void __launch_bounds__(256)
     rope_qkv_kernel(bf16* __restrict__ qkv, int64_t pitch, HeadsView q, HeadsView k, HeadsView v, const float* __restrict__ cs,
                     const float* __restrict__ sn, int64_t T, int nq, int nkv, int hd, int seq) {
+  after_wait(qkv, cs, sn);
+  grid_release();
   using Vec = Bf16Vec<V>;
   const int half = hd / 2, per_head = half / V;
   const int heads = nq + 2 * nkv;
@@ -541,6 +556,8 @@ template <int VPT>
 __global__ void __launch_bounds__(CE_ROW_THREADS, CE_ROW_CTAS)
     cross_entropy_row_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ targets, float* __restrict__ loss, int V,
                              int64_t ld, float grad_scale, int cluster) {
+  after_wait(logits, targets, loss);
+  grid_release();
   __shared__ float red[32];
   __shared__ float2 part;   // maximum of this CTA's elements, sum of their exponentials relative to it
   const int rank = static_cast<int>(blockIdx.x) % cluster;
@@ -635,6 +652,8 @@ constexpr int CE_THREADS = 1024;
 __global__ void __launch_bounds__(CE_THREADS)
     cross_entropy_two_pass_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ targets,
                                   float* __restrict__ loss, int V, int64_t ld, float grad_scale) {
+  after_wait(logits, targets, loss);
+  grid_release();
   __shared__ float red[32];
   const int64_t row = blockIdx.x;
   bf16* lr = logits + row * ld;
@@ -696,6 +715,8 @@ __global__ void __launch_bounds__(CE_THREADS)
 // ------------------------------------------------------------------ embedding
 __global__ void embedding_fwd_kernel(const int64_t* __restrict__ ids, const bf16* __restrict__ table,
                                      bf16* __restrict__ out, int64_t T, int H) {
+  after_wait(ids, table, out);
+  grid_release();
   const int hv = H / 8;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < T * hv;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -707,6 +728,8 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ ids, const bf16
 // dtable[ids[t]] += dout[t]  (bf16x2 atomics: repeated tokens accumulate)
 __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids, const bf16* __restrict__ dout,
                                      bf16* __restrict__ dtable, int64_t T, int H) {
+  after_wait(ids, dout, dtable);
+  grid_release();
   const int hv = H / 2;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < T * hv;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -724,6 +747,8 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids, const bf16
 __global__ void adamw_kernel(bf16* __restrict__ p, bf16* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                              float* __restrict__ master, int64_t n, float lr, float beta1, float beta2, float eps,
                              float wd, float bc1, float bc2, float grad_scale, int zero_grad) {
+  after_wait(p, g, m, v, master);
+  grid_release();
   const int64_t nvec = n / 8;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < nvec;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -762,6 +787,8 @@ __global__ void adamw_kernel(bf16* __restrict__ p, bf16* __restrict__ g, float* 
 
 // sum of squares of a bf16 buffer -> out[0] (fp32 atomics; out must be zeroed by the caller)
 __global__ void sumsq_kernel(const bf16* __restrict__ x, int64_t n, float* __restrict__ out) {
+  after_wait(x, out);
+  grid_release();
   __shared__ float red[32];
   float s = 0.f;
   const int64_t nvec = n / 8;
@@ -850,7 +877,7 @@ int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w,
   auto W = static_cast<const bf16*>(w);
   auto Y = static_cast<bf16*>(y);
 #define B200_NORM_FWD(TPR, VPT)                                                              \
-  rmsnorm_fwd_kernel<TPR, VPT><<<(T + NORM_THREADS / TPR - 1) / (NORM_THREADS / TPR), NORM_THREADS, 0, s>>>(X, R, HO, W, Y, \
+  launch_dependent(rmsnorm_fwd_kernel<TPR, VPT>, (T + NORM_THREADS / TPR - 1) / (NORM_THREADS / TPR), NORM_THREADS, 0, s, X, R, HO, W, Y, \
                                                                                             rstd, T, H, eps)
   B200_NORM_DISPATCH(B200_NORM_FWD);
 #undef B200_NORM_FWD
@@ -877,11 +904,11 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
   do {                                                                                                                \
     const int groups = (T + NORM_THREADS / TPR - 1) / (NORM_THREADS / TPR);                                           \
     if (grid > groups) grid = groups;                                                                                 \
-    rmsnorm_bwd_kernel<TPR, VPT><<<grid, NORM_THREADS, 0, s>>>(DY, X, W, rstd, DR, DX, dw_partial, T, H);             \
+    launch_dependent(rmsnorm_bwd_kernel<TPR, VPT>, grid, NORM_THREADS, 0, s, DY, X, W, rstd, DR, DX, dw_partial, T, H);             \
   } while (0)
   B200_NORM_DISPATCH(B200_NORM_BWD);
 #undef B200_NORM_BWD
-  colsum_partial_kernel<<<(H + 31) / 32, 256, 0, s>>>(dw_partial, static_cast<bf16*>(dw), grid, H, accumulate_dw);
+  launch_dependent(colsum_partial_kernel, (H + 31) / 32, 256, 0, s, dw_partial, static_cast<bf16*>(dw), grid, H, accumulate_dw);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -893,8 +920,8 @@ int b200_swiglu_fwd(const void* gu, void* out, long long T, int F, void* stream)
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto GU = static_cast<const bf16*>(gu);
   auto O = static_cast<bf16*>(out);
-  if (swiglu_small(T, F)) swiglu_fwd_kernel<unsigned><<<grid, 256, 0, s>>>(GU, O, T, F);
-  else swiglu_fwd_kernel<int64_t><<<grid, 256, 0, s>>>(GU, O, T, F);
+  if (swiglu_small(T, F)) launch_dependent(swiglu_fwd_kernel<unsigned>, grid, 256, 0, s, GU, O, T, F);
+  else launch_dependent(swiglu_fwd_kernel<int64_t>, grid, 256, 0, s, GU, O, T, F);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -903,7 +930,7 @@ int b200_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, in
   b200::ensure_context();
   if (F % 8 || !aligned16(dout, gu, dgu)) return B200_ERR_BAD_ARG;
   auto kern = swiglu_small(T, F) ? swiglu_bwd_kernel<false, unsigned> : swiglu_bwd_kernel<false, int64_t>;
-  kern<<<grid_for(T * F / 8, 256, 64), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(kern, grid_for(T * F / 8, 256, 64), 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<const bf16*>(dout), static_cast<const bf16*>(gu), static_cast<bf16*>(dgu), T, F);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -912,7 +939,7 @@ int b200_swiglu_bwd_interleaved(const void* dout, const void* gu, void* dgu, lon
   b200::ensure_context();
   if (F % 32 || !aligned16(dout, gu, dgu)) return B200_ERR_BAD_ARG;
   auto kern = swiglu_small(T, F) ? swiglu_bwd_kernel<true, unsigned> : swiglu_bwd_kernel<true, int64_t>;
-  kern<<<grid_for(T * F / 8, 256, 64), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(kern, grid_for(T * F / 8, 256, 64), 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<const bf16*>(dout), static_cast<const bf16*>(gu), static_cast<bf16*>(dgu), T, F);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -924,7 +951,7 @@ int b200_rope(void* x, const float* cs, const float* sn, long long T, int nheads
   if (hd % 4 || reinterpret_cast<uintptr_t>(x) % 4 || (T > 1 && pitch % 2) ||
       (reinterpret_cast<uintptr_t>(cs) | reinterpret_cast<uintptr_t>(sn)) % 8)
     return B200_ERR_BAD_ARG;
-  rope_kernel<<<grid_for(T * nheads * (hd / 4), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(rope_kernel, grid_for(T * nheads * (hd / 4), 256), 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<bf16*>(x), cs, sn, T, nheads, hd, pitch, seq, backward ? -1.f : 1.f);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -950,7 +977,7 @@ int b200_rope_qkv(void* qkv, long long pitch, void* q, void* k, void* v, const l
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto kern = wide ? (backward ? rope_qkv_kernel<8, true> : rope_qkv_kernel<8, false>)
                    : (backward ? rope_qkv_kernel<2, true> : rope_qkv_kernel<2, false>);
-  kern<<<grid, 256, 0, s>>>(static_cast<bf16*>(qkv), pitch, w[0], w[1], w[2], cs, sn, T, nq, nkv, hd, seq);
+  launch_dependent(kern, grid, 256, 0, s, static_cast<bf16*>(qkv), pitch, w[0], w[1], w[2], cs, sn, T, nq, nkv, hd, seq);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -966,20 +993,22 @@ int b200_cross_entropy(void* logits, const long long* targets, float* loss, int 
   if (r.ctas) {
     auto kern = r.vpt == 1 ? cross_entropy_row_kernel<1> : r.vpt == 2 ? cross_entropy_row_kernel<2>
               : r.vpt == 4 ? cross_entropy_row_kernel<4> : cross_entropy_row_kernel<8>;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = r.ctas;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = r.ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see dependent_launch.cuh
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(T * r.ctas);
     cfg.blockDim = dim3(CE_ROW_THREADS);
     cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, L, TG, loss, V, static_cast<int64_t>(ld), grad_scale, r.ctas));
     return 0;
   }
-  cross_entropy_two_pass_kernel<<<T, CE_THREADS, 0, st>>>(L, TG, loss, V, ld, grad_scale);
+  launch_dependent(cross_entropy_two_pass_kernel, T, CE_THREADS, 0, st, L, TG, loss, V, ld, grad_scale);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -990,7 +1019,7 @@ int b200_cross_entropy_ctas(int T, int V) { return ce_row(T, V).ctas; }
 int b200_embedding_fwd(const long long* ids, const void* table, void* out, long long T, int H, void* stream) {
   b200::ensure_context();
   if (H % 8 || !aligned16(table, out)) return B200_ERR_BAD_ARG;
-  embedding_fwd_kernel<<<grid_for(T * H / 8, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(embedding_fwd_kernel, grid_for(T * H / 8, 256), 256, 0, static_cast<cudaStream_t>(stream),
       reinterpret_cast<const int64_t*>(ids), static_cast<const bf16*>(table), static_cast<bf16*>(out), T, H);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -999,7 +1028,7 @@ int b200_embedding_bwd(const long long* ids, const void* dout, void* dtable, lon
   b200::ensure_context();
   // pairs of elements, and atomics on them
   if (H % 2 || (reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dtable)) % 4) return B200_ERR_BAD_ARG;
-  embedding_bwd_kernel<<<grid_for(T * H / 2, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(embedding_bwd_kernel, grid_for(T * H / 2, 256), 256, 0, static_cast<cudaStream_t>(stream),
       reinterpret_cast<const int64_t*>(ids), static_cast<const bf16*>(dout), static_cast<bf16*>(dtable), T, H);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -1011,7 +1040,7 @@ int b200_adamw(void* p, void* g, float* m, float* v, float* master, long long n,
   if (n % 8) return B200_ERR_BAD_ARG;
   const float bc1 = 1.f - powf(beta1, static_cast<float>(step));
   const float bc2 = 1.f - powf(beta2, static_cast<float>(step));
-  adamw_kernel<<<grid_for(n / 8, 256, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(adamw_kernel, grid_for(n / 8, 256, 256), 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<bf16*>(p), static_cast<bf16*>(g), m, v, master, n, lr, beta1, beta2, eps, wd, bc1, bc2, grad_scale,
       zero_grad);
   B200_CUDA_OK(cudaGetLastError());
@@ -1021,7 +1050,7 @@ int b200_adamw(void* p, void* g, float* m, float* v, float* master, long long n,
 int b200_sumsq(const void* x, long long n, float* out, void* stream) {
   b200::ensure_context();
   if (n % 8) return B200_ERR_BAD_ARG;
-  sumsq_kernel<<<grid_for(n / 8, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const bf16*>(x), n, out);
+  launch_dependent(sumsq_kernel, grid_for(n / 8, 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const bf16*>(x), n, out);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -25,6 +25,7 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include "dependent_launch.cuh"
 #include "gin_device.cuh"
 #include "host_util.h"
 
@@ -81,6 +82,7 @@ struct RouteArgs {
 };
 
 __global__ void __launch_bounds__(MOE_THREADS) moe_route_kernel(RouteArgs a) {
+  grid_wait();
   __shared__ int32_t hist[MOE_MAX_EXPERTS];
   for (int e = threadIdx.x; e < a.E; e += blockDim.x) hist[e] = 0;
   __syncthreads();
@@ -223,6 +225,7 @@ __device__ __forceinline__ uint4 dequantize8(uint2 q, float scale) {
 // routing included: fp8 95 -> 79 us, bf16 140 -> 120). Four CTAs per SM: with the registers of three the
 // fp8 call took 101 us. local_out adds stores to the call and saves reading the window back.
 __global__ void __launch_bounds__(MOE_THREADS, 4) moe_dispatch_kernel(DispatchArgs a) {
+  grid_wait();
   const GinDevHandle& h = a.h;
   const TokenTeam team(a.team_warps);
   const int lane = threadIdx.x & 31;
@@ -339,6 +342,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_dispatch_kernel(DispatchAr
       }
     }
   }
+  grid_release();
   if (!last_cta_done(a.done)) return;
   // every row of this rank is on its way: tell all ranks, then wait until everybody's rows are here
   if (static_cast<int>(threadIdx.x) < h.nranks) {
@@ -354,6 +358,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_dispatch_kernel(DispatchAr
 __global__ void __launch_bounds__(MOE_THREADS)
     moe_collect_rows_kernel(GinDevHandle h, const int32_t* rows_ptr, size_t recv_off, size_t meta_off, int capacity_rows, int H,
                             int local_in_place, __nv_bfloat16* out) {
+  grid_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int rows = min(*rows_ptr, capacity_rows);
   const int vec = H / 8;
@@ -399,6 +404,7 @@ struct CombineArgs {
 };
 
 __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs a) {
+  grid_wait();
   const GinDevHandle& h = a.h;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int rows = a.expert_offsets[a.experts_local];
@@ -503,6 +509,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
 __global__ void __launch_bounds__(MOE_THREADS)
     moe_combine_wgrad_kernel(const __nv_bfloat16* dout, const __nv_bfloat16* comb, const int32_t* row_of, float* dw, int T,
                              int k, int H) {
+  grid_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int vec = H / 8;
   for (int i = blockIdx.x * warps + warp; i < T * k; i += gridDim.x * warps) {
@@ -551,6 +558,7 @@ __host__ __device__ inline int dequant_pieces(int H) { return (H / 8 + DEQUANT_P
 __global__ void __launch_bounds__(MOE_THREADS)
     fp8_dequant_rows_kernel(const uint8_t* q, const float* scales, __nv_bfloat16* out, const int32_t* rows_ptr, int rows_max,
                             int H, int zero_tail, const MoeMeta* meta, int here) {
+  grid_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int rows = rows_ptr ? min(*rows_ptr, rows_max) : rows_max;
   const int vec = H / 8, groups = H / 128, pieces = dequant_pieces(H);
@@ -626,7 +634,7 @@ int b200_moe_route(int comm, const void* topk_idx, int T, int k, int E, size_t c
               static_cast<unsigned int*>(done), ++g_moe_epoch[comm][0]};
   int grid = (T * k + MOE_THREADS * 8 - 1) / (MOE_THREADS * 8);
   if (grid > 64) grid = 64;
-  moe_route_kernel<<<grid, MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  launch_dependent(moe_route_kernel, grid, MOE_THREADS, 0, static_cast<cudaStream_t>(stream), a);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -654,7 +662,7 @@ int b200_moe_dispatch(int comm, const void* x, const void* topk_idx, const void*
                  static_cast<int32_t*>(local_row), static_cast<__nv_bfloat16*>(local_out), recv_off, scale_off, meta_off, capacity_rows, static_cast<unsigned int*>(done), ++g_moe_epoch[comm][1]};
   const int per_cta = TokenTeam::WARPS / a.team_warps;
   const int cap = sm_count() * 4, grid = (T + per_cta - 1) / per_cta;
-  moe_dispatch_kernel<<<grid < cap ? grid : cap, MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  launch_dependent(moe_dispatch_kernel, grid < cap ? grid : cap, MOE_THREADS, 0, static_cast<cudaStream_t>(stream), a);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -667,7 +675,7 @@ int b200_moe_collect_rows(int comm, const void* rows_ptr, size_t recv_off, size_
   if (!hp || !rows_ptr || !out || H % 8 || capacity_rows <= 0 || recv_off % 16 || meta_off % 16) return B200_ERR_BAD_ARG;
   if (recv_off + 2ull * H * capacity_rows > hp->window_bytes || meta_off + 16ull * capacity_rows > hp->window_bytes)
     return B200_ERR_BAD_ARG;
-  moe_collect_rows_kernel<<<moe_grid(capacity_rows), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(moe_collect_rows_kernel, moe_grid(capacity_rows), MOE_THREADS, 0, static_cast<cudaStream_t>(stream),
       *hp, static_cast<const int32_t*>(rows_ptr), recv_off, meta_off, capacity_rows, H, local_in_place,
       static_cast<__nv_bfloat16*>(out));
   B200_CUDA_OK(cudaGetLastError());
@@ -693,7 +701,7 @@ int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int ex
   B200_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_combine_kernel, MOE_THREADS, 0));
   if (per_sm < 1) return B200_ERR_BAD_ARG;
   if (per_sm > 4) per_sm = 4;
-  moe_combine_kernel<<<sm_count() * per_sm, MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  launch_dependent(moe_combine_kernel, sm_count() * per_sm, MOE_THREADS, 0, static_cast<cudaStream_t>(stream), a);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -701,7 +709,7 @@ int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int ex
 int b200_moe_combine_wgrad(const void* dout, const void* comb, const void* row_of, void* dw, int T, int k, int H, void* stream) {
   ensure_context();
   if (H % 8) return B200_ERR_BAD_ARG;
-  moe_combine_wgrad_kernel<<<moe_grid(T * k), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(moe_combine_wgrad_kernel, moe_grid(T * k), MOE_THREADS, 0, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(comb), static_cast<const int32_t*>(row_of),
       static_cast<float*>(dw), T, k, H);
   B200_CUDA_OK(cudaGetLastError());
@@ -714,7 +722,7 @@ int b200_fp8_dequant_rows(const void* q, const void* scales, void* out, const vo
                           void* stream) {
   ensure_context();
   if (H % 128) return B200_ERR_BAD_ARG;
-  fp8_dequant_rows_kernel<<<moe_grid(static_cast<int64_t>(rows_max) * dequant_pieces(H)), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(fp8_dequant_rows_kernel, moe_grid(static_cast<int64_t>(rows_max) * dequant_pieces(H)), MOE_THREADS, 0, static_cast<cudaStream_t>(stream),
       static_cast<const uint8_t*>(q), static_cast<const float*>(scales), static_cast<__nv_bfloat16*>(out),
       static_cast<const int32_t*>(rows_ptr), rows_max, H, zero_tail, nullptr, 0);
   B200_CUDA_OK(cudaGetLastError());
@@ -733,7 +741,7 @@ int b200_moe_collect_rows_fp8(int comm, const void* rows_ptr, size_t recv_off, s
       meta_off + 16ull * rows > hp->window_bytes)
     return B200_ERR_BAD_ARG;
   const uint8_t* window = static_cast<const uint8_t*>(hp->window[hp->rank]);
-  fp8_dequant_rows_kernel<<<moe_grid(static_cast<int64_t>(rows) * dequant_pieces(H)), MOE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(fp8_dequant_rows_kernel, moe_grid(static_cast<int64_t>(rows) * dequant_pieces(H)), MOE_THREADS, 0, static_cast<cudaStream_t>(stream),
       window + recv_off, reinterpret_cast<const float*>(window + scale_off), static_cast<__nv_bfloat16*>(out),
       static_cast<const int32_t*>(rows_ptr), capacity_rows, H, 1, reinterpret_cast<const MoeMeta*>(window + meta_off), hp->rank);
   B200_CUDA_OK(cudaGetLastError());

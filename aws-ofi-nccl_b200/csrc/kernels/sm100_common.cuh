@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dependent_launch.cuh"
+
 namespace b200 {
 
 // Error codes written to the device status word by kernels in this library.

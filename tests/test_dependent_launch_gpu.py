@@ -1,0 +1,89 @@
+"""Kernels that start while the one before them ends: a chain of them, each reading what the one before has just written into
+buffers that are used again and again, gives the same bits as one that is waited for after every call."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+class _Chain:
+    """Optimizer step, residual norm, gate | up product, SwiGLU, split-K product back, cross entropy and the gradients of the
+    products, all into buffers of its own."""
+
+    def __init__(self, T, H, F):
+        g = torch.Generator(device="cuda").manual_seed(T + H + F)
+
+        def rnd(*s, std=1.0, dtype=torch.bfloat16):
+            return (torch.randn(*s, device="cuda", generator=g) * std).to(dtype)
+
+        self.T, self.H, self.F = T, H, F
+        self.x, self.res, self.w = rnd(T, H), rnd(T, H), rnd(H, std=0.1) + 1
+        self.wgu, self.wdown = rnd(2 * F, H, std=H ** -0.5), rnd(H, F, std=F ** -0.5)
+        self.grad, self.m, self.v = torch.zeros_like(self.wgu), torch.zeros(2 * F, H, device="cuda"), torch.zeros(2 * F, H, device="cuda")
+        self.targets = torch.randint(0, H, (T,), device="cuda", generator=g)
+        self.buf = {k: torch.zeros(*s, device="cuda", dtype=d) for k, (s, d) in {
+            "h": ((T, H), torch.bfloat16), "y": ((T, H), torch.bfloat16), "rstd": ((T,), torch.float32),
+            "gu": ((T, 2 * F), torch.bfloat16), "act": ((T, F), torch.bfloat16), "out": ((T, H), torch.bfloat16),
+            "loss": ((T,), torch.float32), "dact": ((T, F), torch.bfloat16), "dgu": ((T, 2 * F), torch.bfloat16),
+            "dw": ((2 * F, H), torch.bfloat16), "q": ((T, F), torch.uint8), "qs": ((T,), torch.float32)}.items()}
+
+    def steps(self):
+        from aws_ofi_nccl_b200.ops import _lib
+        from aws_ofi_nccl_b200.ops.gemm import gemm
+        from aws_ofi_nccl_b200.ops.llm import adamw_step
+
+        L, b, T, H, F = _lib.load(), self.buf, self.T, self.H, self.F
+
+        def call(name, *args):
+            _lib.check(getattr(L, name)(*[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args], _lib.stream_ptr()), name)
+
+        yield lambda: adamw_step(self.wgu, self.grad, self.m, self.v, None, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8,
+                                 weight_decay=0.1, step=3)
+        yield lambda: call("b200_rmsnorm_fwd", self.x, self.res, b["h"], self.w, b["y"], b["rstd"], T, H, 1e-5)
+        yield lambda: gemm(b["y"], self.wgu, out=b["gu"])
+        yield lambda: call("b200_swiglu_fwd", b["gu"], b["act"], T, F)
+        yield lambda: call("b200_quant_rows_fp8", b["act"], b["q"], b["qs"], T, F, F, F)
+        yield lambda: gemm(b["act"], self.wdown, out=b["out"])
+        yield lambda: call("b200_cross_entropy", b["out"], self.targets, b["loss"], T, H, H, 1.0 / T)
+        yield lambda: gemm(b["out"], self.wdown, b_mn=True, out=b["dact"])
+        yield lambda: call("b200_swiglu_bwd", b["dact"], b["gu"], b["dgu"], T, F)
+        yield lambda: gemm(b["dgu"], b["y"], a_mn=True, b_mn=True, out=b["dw"])
+        yield lambda: self.grad.copy_(b["dw"])   # what the next pass's optimizer step reads
+
+    def run(self, wait):
+        for step in self.steps():
+            step()
+            if wait:
+                torch.cuda.synchronize()
+
+    def results(self):
+        return [t.clone() for t in (self.wgu, self.m, *self.buf.values())]
+
+
+# less than a wave of everything; several waves; a long reduction that is split over clusters
+@pytest.mark.parametrize("T,H,F", [(64, 128, 256), (1000, 1032, 2056), (128, 512, 8192), (4096, 2048, 4096)])
+def test_a_chain_of_kernels_sees_what_the_kernel_before_wrote(T, H, F):
+    waited, chained = _Chain(T, H, F), _Chain(T, H, F)
+    for _ in range(3):
+        waited.run(True)
+    for _ in range(3):
+        chained.run(False)
+    for a, b in zip(waited.results(), chained.results()):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("T,H,F", [(64, 128, 256), (1000, 1032, 2056)])
+def test_a_captured_chain_does_too(T, H, F):
+    waited, captured = _Chain(T, H, F), _Chain(T, H, F)
+    captured.run(False)   # what a first call sets up is no part of a graph
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=stream):
+        captured.run(False)
+    for _ in range(2):
+        graph.replay()
+    for _ in range(3):
+        waited.run(True)
+    torch.cuda.synchronize()
+    for a, b in zip(waited.results(), captured.results()):
+        assert torch.equal(a, b)
