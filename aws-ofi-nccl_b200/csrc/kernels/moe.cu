@@ -25,6 +25,8 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "dependent_launch.cuh"
 #include "gin_device.cuh"
 #include "host_util.h"
@@ -36,6 +38,7 @@ const GinDevHandle* comm_handle(int id);  // collectives.cu
 constexpr int MOE_SIG_BASE = 3072;  // GIN signal slots [3072, 3072 + 3 * 8): phase x source rank
 constexpr int MOE_MAX_EXPERTS = 1024;
 constexpr int MOE_THREADS = 256;
+constexpr int CTAS_PER_SM = 16;   // of a grid that has the work for them, see token_grid
 
 struct MoeMeta {  // one per received row
   int32_t token, slot;
@@ -107,17 +110,41 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_route_kernel(RouteArgs a) {
   const bool ok = moe_wait_all(h, 0, a.epoch);
   const int32_t* mat = reinterpret_cast<const int32_t*>(h.window[h.rank] + a.cnt_off) + (a.epoch & 1) * h.nranks * a.E;
   const int el = a.E / h.nranks;  // experts per rank
-  // totals per expert, then the exclusive prefix over the experts of one owner
-  for (int e = threadIdx.x; e < a.E; e += blockDim.x) {
-    int tot = 0;
-    for (int s = 0; s < h.nranks; ++s) tot += ok ? mat[s * a.E + e] : 0;
-    hist[e] = tot;
+  // Totals per expert and their exclusive prefix over all experts, PER of them to a thread; an owner's experts are neighbours, so
+  // that a prefix among them is a difference. A loop over an expert's predecessors took up to 3 us (256 experts).
+  constexpr int PER = MOE_MAX_EXPERTS / MOE_THREADS, WARPS = MOE_THREADS / 32;
+  __shared__ int32_t before[MOE_MAX_EXPERTS], warp_total[WARPS];
+  int tot[PER], sum = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = threadIdx.x * PER + i;
+    tot[i] = 0;
+    for (int s = 0; s < h.nranks; ++s) tot[i] += ok && e < a.E ? mat[s * a.E + e] : 0;
+    sum += tot[i];
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int scan = sum;   // inclusive over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o *= 2) {
+    const int left = __shfl_up_sync(0xffffffffu, scan, o);
+    if (lane >= o) scan += left;
+  }
+  if (lane == 31) warp_total[warp] = scan;
+  __syncthreads();
+  int at = scan - sum;
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) at += w < warp ? warp_total[w] : 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = threadIdx.x * PER + i;
+    hist[e] = tot[i];
+    before[e] = at;
+    at += tot[i];
   }
   __syncthreads();
   for (int e = threadIdx.x; e < a.E; e += blockDim.x) {
     const int owner_first = (e / el) * el;
-    int base = 0;
-    for (int j = owner_first; j < e; ++j) base += hist[j];
+    const int base = before[e] - before[owner_first];
     int before_me = 0;
     for (int s = 0; s < h.rank; ++s) before_me += ok ? mat[s * a.E + e] : 0;
     a.dest_base[e] = base + before_me;
@@ -364,23 +391,29 @@ __global__ void __launch_bounds__(MOE_THREADS)
   const int vec = H / 8;
   const MoeMeta* meta = reinterpret_cast<const MoeMeta*>(h.window[h.rank] + meta_off);
   const uint4* recv = reinterpret_cast<const uint4*>(h.window[h.rank] + recv_off);
-  for (int r = blockIdx.x * warps + warp; r < capacity_rows; r += gridDim.x * warps) {
-    uint4* dst = reinterpret_cast<uint4*>(out) + static_cast<size_t>(r) * vec;
-    if (r >= rows) {
-      for (int v = lane; v < vec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
-      continue;
-    }
-    if (local_in_place && meta[r].src_rank == h.rank) continue;
-    const uint4* src = recv + static_cast<size_t>(r) * vec;
-    constexpr int U = 4;
-    for (int v0 = lane; v0 < vec; v0 += 32 * U) {
-      uint4 tmp[U];
+  // A warp's lanes look their rows' records up together: one after the other they took 13 us for 32768 rows.
+  const int all_warps = gridDim.x * warps, share = (capacity_rows + all_warps - 1) / all_warps, batch = share < 32 ? share : 32;
+  for (int64_t r0 = static_cast<int64_t>(blockIdx.x * warps + warp) * batch; r0 < capacity_rows; r0 += static_cast<int64_t>(all_warps) * batch) {
+    const int64_t mine = r0 + lane;
+    const bool todo = lane < batch && mine < capacity_rows && !(local_in_place && mine < rows && meta[mine].src_rank == h.rank);
+    for (unsigned left = __ballot_sync(0xffffffffu, todo); left; left &= left - 1) {
+      const int r = static_cast<int>(r0) + __ffs(left) - 1;
+      uint4* dst = reinterpret_cast<uint4*>(out) + static_cast<size_t>(r) * vec;
+      if (r >= rows) {
+        for (int v = lane; v < vec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
+        continue;
+      }
+      const uint4* src = recv + static_cast<size_t>(r) * vec;
+      constexpr int U = 4;
+      for (int v0 = lane; v0 < vec; v0 += 32 * U) {
+        uint4 tmp[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (v0 + 32 * u < vec) tmp[u] = src[v0 + 32 * u];
+        for (int u = 0; u < U; ++u)
+          if (v0 + 32 * u < vec) tmp[u] = src[v0 + 32 * u];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (v0 + 32 * u < vec) dst[v0 + 32 * u] = tmp[u];
+        for (int u = 0; u < U; ++u)
+          if (v0 + 32 * u < vec) dst[v0 + 32 * u] = tmp[u];
+      }
     }
   }
 }
@@ -399,7 +432,8 @@ struct CombineArgs {
   int T, k, H;
   int team_warps;                  // TokenTeam
   __nv_bfloat16* out;              // [T][H]
-  unsigned int* done;
+  unsigned int senders;            // CTAs that send rows to other ranks, no more than run at once
+  unsigned int* done;              // CTAs that have started, and 2^16 for every sender that is through
   uint64_t epoch;
 };
 
@@ -410,7 +444,19 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
   const int rows = a.expert_offsets[a.experts_local];
   const int vec = a.H / 8;
   const MoeMeta* meta = reinterpret_cast<const MoeMeta*>(h.window[h.rank] + a.meta_off);
-  for (int r = blockIdx.x * warps + warp; r < rows; r += gridDim.x * warps) {
+  // The CTAs that start first send, however they are numbered: whoever waits below waits for CTAs that are running.
+  __shared__ unsigned int ticket;
+  const unsigned int all_done = gridDim.x | (a.senders << 16);
+  auto count = [&](unsigned int n) {   // rearmed by whoever counts last
+    const unsigned int was = atomicAdd(a.done, n);
+    if (was + n == all_done) *a.done = 0;
+    return was;
+  };
+  if (threadIdx.x == 0) ticket = count(1) & 0xffffu;
+  __syncthreads();
+  const int cta = static_cast<int>(ticket);
+  const bool sender = ticket < a.senders;
+  for (int r = cta * warps + warp; sender && r < rows; r += a.senders * warps) {
     const MoeMeta m = meta[r];
     if (m.src_rank < 0 || m.src_rank >= h.nranks || m.token < 0 || m.token >= a.T || m.slot < 0 || m.slot >= a.k) {
       if (lane == 0) gin_record_error(h, DEV_ERR_BOUNDS);
@@ -431,9 +477,17 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
         if (v0 + 32 * u < vec) dst[v0 + 32 * u] = tmp[u];
     }
   }
-  // ---- all of this rank's rows are out: signal every source (one CTA does it) ...
-  if (last_cta_done(a.done)) {
-    if (static_cast<int>(threadIdx.x) < h.nranks) {
+  // ---- all of this rank's rows are out: signal every source (the last sender does it) ...
+  if (sender) {
+    __shared__ int is_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      is_last = (count(1u << 16) >> 16) == a.senders - 1;
+      __threadfence();
+    }
+    __syncthreads();
+    if (is_last && static_cast<int>(threadIdx.x) < h.nranks) {
       fence_acq_rel_sys();
       gin_signal(h, threadIdx.x, MOE_SIG_BASE + 2 * GIN_MAX_RANKS + h.rank, 1, GIN_SIGNAL_INC);
     }
@@ -453,7 +507,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
   __shared__ int team_row[TokenTeam::WARPS][MOE_MAX_TOPK];   // row of y, -1: the cell in the window, -2: never sent
   float* slot_w = team_w[team.team];
   int* slot_row = team_row[team.team];
-  for (int t0 = blockIdx.x * team.teams; t0 < a.T; t0 += gridDim.x * team.teams) {
+  for (int t0 = cta * team.teams; t0 < a.T; t0 += gridDim.x * team.teams) {
     const int t = t0 + team.team;
     const bool on = t < a.T;
     team.sync();   // the slots of the token before have been read
@@ -607,10 +661,17 @@ __global__ void __launch_bounds__(MOE_THREADS)
 
 static uint64_t g_moe_epoch[64][3] = {};
 
-static int moe_grid(int64_t work_warps) {
+// CTAs for T tokens, of which one works on per_cta at a time. Four run on an SM; with no more than that the SMs that memory serves
+// last finish last, and with several times as many the others take their work: 4096 x 7168, top-8, fp8 dispatch 147 -> 134 us,
+// combine 262 -> 246, in the backward pass 186 -> 165 and 169 -> 168, the weights' gradient (moe_grid) 98 -> 92 (8 per SM: 146 and
+// 183 for the dispatches, 64: 134 and 166).
+static int token_grid(int T, int per_cta) {
+  return std::min((T + per_cta - 1) / per_cta, sm_count() * CTAS_PER_SM);
+}
+static int moe_grid(int64_t work_warps, int per_sm = 4) {
   const int per_cta = MOE_THREADS / 32;
   const int64_t grid = (work_warps + per_cta - 1) / per_cta;
-  const int cap = sm_count() * 4;
+  const int cap = sm_count() * per_sm;
   return grid > cap ? cap : grid < 1 ? 1 : static_cast<int>(grid);
 }
 
@@ -632,8 +693,8 @@ int b200_moe_route(int comm, const void* topk_idx, int T, int k, int E, size_t c
   RouteArgs a{h, static_cast<const int32_t*>(topk_idx), T, k, E, cnt_off, static_cast<int32_t*>(cnt_local),
               static_cast<int32_t*>(dest_base), static_cast<int32_t*>(expert_offsets), static_cast<int32_t*>(cursor),
               static_cast<unsigned int*>(done), ++g_moe_epoch[comm][0]};
-  int grid = (T * k + MOE_THREADS * 8 - 1) / (MOE_THREADS * 8);
-  if (grid > 64) grid = 64;
+  int grid = (T * k + MOE_THREADS * 2 - 1) / (MOE_THREADS * 2);   // a thread's loads wait for one another
+  if (grid > 128) grid = 128;
   launch_dependent(moe_route_kernel, grid, MOE_THREADS, 0, static_cast<cudaStream_t>(stream), a);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -661,8 +722,7 @@ int b200_moe_dispatch(int comm, const void* x, const void* topk_idx, const void*
                  static_cast<const int32_t*>(dest_base), static_cast<int32_t*>(cursor), static_cast<int32_t*>(row_of),
                  static_cast<int32_t*>(local_row), static_cast<__nv_bfloat16*>(local_out), recv_off, scale_off, meta_off, capacity_rows, static_cast<unsigned int*>(done), ++g_moe_epoch[comm][1]};
   const int per_cta = TokenTeam::WARPS / a.team_warps;
-  const int cap = sm_count() * 4, grid = (T + per_cta - 1) / per_cta;
-  launch_dependent(moe_dispatch_kernel, grid < cap ? grid : cap, MOE_THREADS, 0, static_cast<cudaStream_t>(stream), a);
+  launch_dependent(moe_dispatch_kernel, token_grid(T, per_cta), MOE_THREADS, 0, static_cast<cudaStream_t>(stream), a);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -682,8 +742,8 @@ int b200_moe_collect_rows(int comm, const void* rows_ptr, size_t recv_off, size_
   return 0;
 }
 
-// Collective. Every CTA of this kernel waits for the other ranks, so the grid is limited to what
-// is resident at once.
+// Collective. Every CTA of this kernel waits for the other ranks' rows and for this rank's senders, which are the first CTAs to
+// start: as many as run at once.
 int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int experts_local, size_t meta_off, size_t comb_off,
                      const void* topk_w, const void* row_of, const void* local_row, void* cells_out, int T, int k, int H,
                      void* out, void* done, void* stream) {
@@ -696,12 +756,15 @@ int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int ex
   CombineArgs a{h, static_cast<const __nv_bfloat16*>(y), static_cast<const int32_t*>(expert_offsets), experts_local, meta_off,
                 comb_off, static_cast<const float*>(topk_w), static_cast<const int32_t*>(row_of),
                 static_cast<const int32_t*>(local_row), static_cast<__nv_bfloat16*>(cells_out), T, k, H, TokenTeam::warps_for(T, H),
-                static_cast<__nv_bfloat16*>(out), static_cast<unsigned int*>(done), ++g_moe_epoch[comm][2]};
+                static_cast<__nv_bfloat16*>(out), 0, static_cast<unsigned int*>(done), ++g_moe_epoch[comm][2]};
+  const int per_cta = TokenTeam::WARPS / a.team_warps;
   int per_sm = 0;
   B200_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_combine_kernel, MOE_THREADS, 0));
   if (per_sm < 1) return B200_ERR_BAD_ARG;
   if (per_sm > 4) per_sm = 4;
-  launch_dependent(moe_combine_kernel, sm_count() * per_sm, MOE_THREADS, 0, static_cast<cudaStream_t>(stream), a);
+  a.senders = sm_count() * per_sm;
+  const int grid = std::max(static_cast<int>(a.senders), token_grid(T, per_cta));
+  launch_dependent(moe_combine_kernel, grid, MOE_THREADS, 0, static_cast<cudaStream_t>(stream), a);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -709,7 +772,7 @@ int b200_moe_combine(int comm, const void* y, const void* expert_offsets, int ex
 int b200_moe_combine_wgrad(const void* dout, const void* comb, const void* row_of, void* dw, int T, int k, int H, void* stream) {
   ensure_context();
   if (H % 8) return B200_ERR_BAD_ARG;
-  launch_dependent(moe_combine_wgrad_kernel, moe_grid(T * k), MOE_THREADS, 0, static_cast<cudaStream_t>(stream),
+  launch_dependent(moe_combine_wgrad_kernel, moe_grid(T * k, CTAS_PER_SM), MOE_THREADS, 0, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(comb), static_cast<const int32_t*>(row_of),
       static_cast<float*>(dw), T, k, H);
   B200_CUDA_OK(cudaGetLastError());

@@ -201,3 +201,39 @@ def test_fp8_rows_are_those_of_the_window(comm, T, H, k):
     # weighted rows are scaled and quantised one by one
     ep.dispatch_raw(x, idx, w, fp8=True, use_saved_rows=True, scale_by_weight=True, local_out=own)
     assert torch.equal(own[:n], ep.dequant()[:n])
+
+
+# one expert, an odd number, one per thread and one more, several per thread, as many as there may be; ragged and few tokens
+@pytest.mark.parametrize("E", [1, 3, 256, 257, 700, 1024])
+@pytest.mark.parametrize("T", [1, 1001])
+def test_route_counts_the_rows_of_every_expert(comm, E, T):
+    from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
+
+    ep = ExpertParallel(comm, T, 256, E, 3)
+    for seed in range(2):
+        g = torch.Generator(device="cuda").manual_seed(E + T + seed)
+        idx = torch.randint(-1, E, (T, 3), device="cuda", generator=g, dtype=torch.int32)   # -1 goes nowhere
+        offsets = ep.route(idx)
+        counts = torch.bincount(idx[idx >= 0].long(), minlength=E)
+        assert offsets[0] == 0 and torch.equal(offsets[1:].long(), counts.cumsum(0))
+        assert torch.equal(ep.dest_base.long(), counts.cumsum(0) - counts)
+
+
+# more tokens than CTAs of dispatch, sum and weight gradient at once work on, call after call
+def test_more_tokens_than_a_grid_holds(comm):
+    from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
+
+    T, H, E = 40001, 256, 8
+    ep = ExpertParallel(comm, T, H, E, 1, capacity_factor=1.0)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for _ in range(3):
+        x, dy = (torch.randn(T, H, device="cuda", generator=g).bfloat16() for _ in range(2))
+        x.requires_grad_(True)
+        idx = torch.randint(0, E, (T, 1), device="cuda", generator=g, dtype=torch.int32)
+        w = torch.full((T, 1), 0.5, device="cuda", requires_grad=True)
+        out = ep.combine(ep.dispatch(x, idx, w), w)
+        assert torch.equal(out, x.detach() * 0.5)   # a power of two: nothing is rounded
+        dx, dw = torch.autograd.grad(out, (x, w), dy)
+        want = (dy.double() * x.detach().double()).sum(-1, keepdim=True)
+        mag = (dy.double() * x.detach().double()).abs().sum(-1, keepdim=True)
+        assert torch.equal(dx, dy * 0.5) and ((dw.double() - want).abs() <= H * 2.0 ** -24 * mag).all()
