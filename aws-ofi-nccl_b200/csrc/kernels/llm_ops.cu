@@ -6,15 +6,19 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <type_traits>
+
 #include "b200ops.h"
+#include "cross_entropy_math.cuh"
+#include "cross_entropy_stream.cuh"
 #include "dependent_launch.cuh"
 #include "host_util.h"
 #include "swiglu_math.cuh"
 
 namespace b200 {
 
-using bf16 = __nv_bfloat16;
-using bf162 = __nv_bfloat162;
+int* device_status_word();   // gemm.cu
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -55,23 +59,6 @@ __device__ __forceinline__ float block_max(float v, float* red) {
   }
   __syncthreads();
   return red[0];
-}
-
-struct alignas(16) Bf16x8 {
-  bf162 v[4];
-};
-__device__ __forceinline__ void unpack8(const Bf16x8& p, float (&f)[8]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = __low2float(p.v[i]);
-    f[2 * i + 1] = __high2float(p.v[i]);
-  }
-}
-__device__ __forceinline__ Bf16x8 pack8(const float (&f)[8]) {
-  Bf16x8 p;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) p.v[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-  return p;
 }
 
 // ------------------------------------------------------------------ RMSNorm
@@ -471,60 +458,6 @@ __global__ void __launch_bounds__(256)
 
 // ------------------------------------------------------------------ softmax cross-entropy, forward + backward fused
 // The logits are overwritten with dlogits = (softmax - onehot) * grad_scale; loss[row] = logsumexp - logit[target].
-// Exponentials are powers of two of f * log2(e) - c, one fused multiply-add: c is the maximum times log2(e), rounded, the
-// same for every term, and the loss adds what the rounding left out. Taking the maximum off first is one instruction more, and registers that the
-// row kernel does not have: 69 us for 4096 x 16040, 57 this way. Maxima start below all bf16 but -inf, so that masked elements of that value
-// count as nothing.
-constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
-__device__ __forceinline__ float exp2_approx(float x) {
-  float y;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// From here on a finite maximum's product with log2(e) may overflow (masks are often the lowest bf16). Neighbouring values lie 1e36
-// apart there: e^(f - m) is 1 or 0.
-__device__ __forceinline__ bool huge_max(float m) { return fabsf(m) >= 2e38f && m < INFINITY; }
-__device__ __forceinline__ float exp_base(float m) { return __fmul_rn(m, LOG2E); }
-// A value relative to a huge maximum, as an argument for the base 0
-__device__ __forceinline__ bf16 from_huge(bf16 x, float m) {
-  const float f = __bfloat162float(x);
-  return __float2bfloat16(f == m ? 0.f : f < m ? -INFINITY : f);
-}
-// What a sum relative to the maximum `part` counts relative to m
-__device__ __forceinline__ float exp_share(float part, float m) {
-  const float scale = huge_max(m) ? 1.f : LOG2E;
-  return exp2_approx(__fmul_rn(part, scale) - __fmul_rn(m, scale));
-}
-// The largest of eight values, NaN left aside.
-__device__ __forceinline__ float max8(const Bf16x8& x) {
-  const bf162 m = __hmax2(__hmax2(x.v[0], x.v[1]), __hmax2(x.v[2], x.v[3]));
-  return fmaxf(__low2float(m), __high2float(m));
-}
-__device__ __forceinline__ float exp_sum8(const Bf16x8& x, float c) {
-  float f[8], s = 0.f;
-  unpack8(x, f);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) s += exp2_approx(fmaf(f[j], LOG2E, -c));
-  return s;
-}
-// s: the sum relative to exp_base(m), or to m itself where that is huge
-__device__ __forceinline__ float ce_loss(float m, float s, float target_logit) {
-  return logf(s) + (m - target_logit) + (huge_max(m) ? 0.f : fmaf(m, -LOG2E, exp_base(m)) * LN2);
-}
-// `own`: the target's place among the eight elements, if it is one of them
-__device__ __forceinline__ Bf16x8 ce_gradient8(const Bf16x8& x, float c, float inv, int own, float grad_scale) {
-  float f[8];
-  unpack8(x, f);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) f[j] = exp2_approx(fmaf(f[j], LOG2E, -c)) * inv;
-  if (own >= 0 && own < 8) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (own == j) f[j] -= grad_scale;
-  }
-  return pack8(f);
-}
-
 // Eight elements of a row of V, or as many as are left of it
 __device__ __forceinline__ void zero8(bf16* row, int at, int V) {
   if (at + 8 <= V)
@@ -535,9 +468,8 @@ __device__ __forceinline__ void zero8(bf16* row, int at, int V) {
 
 // A cluster of up to eight CTAs takes a row and keeps it in registers, 8 * VPT elements per thread: all loads of the
 // row are in flight at once, and maximum and sum of the CTAs' parts meet in shared memory. For rows of one CTA, and for
-// few wider ones (ce_row): many are better off with two passes of a CTA each, whose
-// many threads overlap one row's loads with another's stores (2048 x 128256: 294 us in clusters, 245 in two passes).
-// 4096 x 16040 takes 57 us, 97 in two passes; 2048 x 1024 8 and 18; 64 x 128256, in clusters, 13 and 22 (L2 flushed, launches in a graph).
+// few wider ones (ce_row): many stream through shared memory (2048 x 128256: 294 us in clusters, 195 streamed).
+// 4096 x 16040 takes 57 us, 97 in two passes; 2048 x 1024 8 and 18; 64 x 128256, in clusters, 13 and 22.
 constexpr int CE_ROW_THREADS = 256;
 constexpr int CE_ROW_CTAS = 4;   // of an SM
 constexpr int CE_MAX_CLUSTER = 8;
@@ -628,25 +560,31 @@ __global__ void __launch_bounds__(CE_ROW_THREADS, CE_ROW_CTAS)
     for (int i = 0; i < VPT; ++i) *reinterpret_cast<uint4*>(&x[i]) = make_uint4(0, 0, 0, 0);
   }
   const int own = counts ? static_cast<int>(tgt) - first : -1;   // the target's place from this thread's first element on
+  auto store = [&](auto small) {
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int at = first + i * STEP;
-    if (at >= V) break;
-    const Bf16x8 o = ce_gradient8(x[i], c, inv, own - i * STEP, grad_scale);
-    if (at + 8 <= V) {
-      *reinterpret_cast<Bf16x8*>(lr + at) = o;
-    } else {
+    for (int i = 0; i < VPT; ++i) {
+      const int at = first + i * STEP;
+      if (at >= V) break;
+      const Bf16x8 o = ce_gradient8<decltype(small)::value>(x[i], c, inv, own - i * STEP, grad_scale);
+      if (at + 8 <= V) {
+        *reinterpret_cast<Bf16x8*>(lr + at) = o;
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (at + 2 * j < V) lr[at + 2 * j] = o.v[j].x;
-        if (at + 2 * j + 1 < V) lr[at + 2 * j + 1] = o.v[j].y;
+        for (int j = 0; j < 4; ++j) {
+          if (at + 2 * j < V) lr[at + 2 * j] = o.v[j].x;
+          if (at + 2 * j + 1 < V) lr[at + 2 * j + 1] = o.v[j].y;
+        }
       }
     }
-  }
+  };
+  if (small_powers_count(inv))
+    store(std::true_type{});
+  else
+    store(std::false_type{});
   if (cluster > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// One CTA per token row. Pass 1: online max/sum. Pass 2: overwrite the logits. The maximum starts below all bf16 but -inf,
+// One CTA per token row (ce_two_passes). Pass 1: online max/sum. Pass 2: overwrite the logits. The maximum starts below all bf16 but -inf,
 // so that masked elements ahead of the others count as nothing; a branch for them took 16 of 268 us for 2048 x 128256.
 constexpr int CE_THREADS = 1024;
 __global__ void __launch_bounds__(CE_THREADS)
@@ -803,8 +741,8 @@ __global__ void sumsq_kernel(const bf16* __restrict__ x, int64_t n, float* __res
   if (threadIdx.x == 0) atomicAdd(out, s);
 }
 
-// What holds a row of the cross-entropy in registers: CTAs of a cluster with `vpt` vectors per thread, the fewest that can; none where two
-// passes are better or a cluster is too small. One CTA always pays. Clusters use the SMs that two passes leave idle, so they pay for few rows, and for more
+// What holds a row of the cross-entropy in registers: CTAs of a cluster with `vpt` vectors per thread, the fewest that can; none where
+// two passes or the stream are better or a cluster is too small. One CTA always pays. Clusters use the SMs that two passes leave idle, so they pay for few rows, and for more
 // of them the fuller a row makes their registers. Of 240 pairs of 20 widths from 16392 to 131072 and 1 to 296 rows the rule takes clusters for 116, in
 // 0.29 to 1.10 of the time of two passes (1 x 65536 5.7 us, 12.1; 74 x 131072 16.4 and 22.3; 200 x 32768 10.6 and 12.4), and leaves out the slower
 // ones (148 x 65544 23.9 and 15.1, 74 x 32776 10.1 and 8.9, 1 x 16392 5.7 and 4.9); its times are 1.005 of the better ones'.
@@ -824,6 +762,11 @@ static CeRow ce_row(int64_t T, int V) {
   if (ctas > 2) pays = 10 * T * held <= 9 * sms * vecs && T * ctas <= CE_ROW_CTAS * sms;
   return pays ? CeRow{ctas, vpt} : CeRow{0, 0};
 }
+
+// Rows that no registers hold stream through shared memory, but for two rows for an SM of a length that a chunk or two hold: there two
+// CTAs of many threads are ahead (222 x 24576 10.0 us, 10.8 streamed; 296 x 28672 11.7 and 12.8). Everywhere else of 18 numbers of rows from 1
+// to 2048 and 12 widths from 16392 to 200000 the stream takes 0.68 to 1.00 of two passes.
+static bool ce_two_passes(int64_t T, int V) { return V >= 20000 && V < 32768 && T > sm_count() && T <= 2 * sm_count(); }
 
 // Rows move as 16-byte vectors: null (an argument left out) or on a 16-byte boundary.
 template <class... P>
@@ -1008,12 +951,22 @@ int b200_cross_entropy(void* logits, const long long* targets, float* loss, int 
     B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, L, TG, loss, V, static_cast<int64_t>(ld), grad_scale, r.ctas));
     return 0;
   }
-  launch_dependent(cross_entropy_two_pass_kernel, T, CE_THREADS, 0, st, L, TG, loss, V, ld, grad_scale);
+  if (ce_two_passes(T, V)) {
+    launch_dependent(cross_entropy_two_pass_kernel, T, CE_THREADS, 0, st, L, TG, loss, V, ld, grad_scale);
+  } else {
+    static std::atomic<bool> attr_set{false};
+    if (!attr_set.load(std::memory_order_acquire)) {
+      B200_CUDA_OK(cudaFuncSetAttribute(cross_entropy_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CES_SMEM));
+      attr_set.store(true, std::memory_order_release);
+    }
+    launch_dependent(cross_entropy_stream_kernel, T < sm_count() ? T : sm_count(), CES_THREADS, CES_SMEM, st, L, TG, loss, T, V, ld,
+                     grad_scale, device_status_word());
+  }
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
-// CTAs that share a row of that call, 0 for two passes.
+// CTAs that share a row of that call, 0 where a CTA goes over its row twice.
 int b200_cross_entropy_ctas(int T, int V) { return ce_row(T, V).ctas; }
 
 int b200_embedding_fwd(const long long* ids, const void* table, void* out, long long T, int H, void* stream) {

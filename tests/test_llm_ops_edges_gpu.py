@@ -182,6 +182,9 @@ def test_adamw_over_the_whole_grid(n):
     assert ((w - (w0 * (1 - 1e-2 * 0.1) - per_m * em)).abs() <= 4 * ulp * w0.abs() + 64 * ulp * per_m * terms).all()
     assert torch.equal(p, w.bfloat16()) and not g.any()
 
+LOWEST = torch.finfo(torch.bfloat16).min   # the usual value of a mask
+
+
 # a vector, a thread's vectors (one to eight), a cluster of two to eight CTAs and the widest row that it holds, each with
 # one element or vector more; the last is a row for two passes
 @pytest.mark.parametrize("T,V", [(1, 1), (5, 7), (3, 2048), (300, 2049), (4, 4104), (7, 8200), (5, 16384), (40, 16392), (3, 32771),
@@ -217,6 +220,43 @@ def test_cross_entropy(T, V):
     assert (pad[:, V:] == 5).all()
 
 
+# streamed rows: one chunk (24576 elements) and one vector more, all that the ring holds (98304) and one more, whole rings and more a second time; one
+# row, several for a CTA, ragged widths; two rows for an SM in two passes
+@pytest.mark.parametrize("T,V", [(1, 16392), (150, 16401), (700, 24576), (700, 24584), (200, 49153), (300, 32776), (160, 98304), (150, 98312), (2, 131080),
+                                 (149, 196609), (2, 600007), (200, 24576)])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -10])   # small powers count, and do not
+def test_cross_entropy_of_wide_rows(T, V, scale):
+    from aws_ofi_nccl_b200.ops import _lib
+
+    assert _lib.load().b200_cross_entropy_ctas(T, V) == 0
+    g = torch.Generator(device="cuda").manual_seed(T + V)
+    pad = torch.full((T, (V + 7) // 8 * 8 + 8), 5.0, device="cuda").bfloat16()
+    logits = pad[:, :V]
+    logits.copy_(torch.randn(T, V, device="cuda", generator=g) * 3)
+    logits[0, :V // 2] = LOWEST
+    logits[-1, V - 1] = 90.0   # the last element, alone in its sum: the others are small powers
+    targets = torch.randint(0, V, (T,), device="cuda", generator=g)
+    targets[0] = V - 1
+    if T > 2:
+        targets[1] = V
+    counts = targets < V
+    at = targets.clamp_max(V - 1)[:, None]
+    rows = [0, T - 1] + ([1, T // 2] if T > 2 else [])
+    x, loss = logits[rows].double(), torch.full((T,), math.nan, device="cuda")
+    lse = torch.logsumexp(x, -1)
+    want_loss = (lse - x.gather(1, at[rows])[:, 0]) * counts[rows]
+    want = (x - lse[:, None]).exp()
+    want.scatter_add_(1, at[rows], -torch.ones_like(lse)[:, None])
+    want *= counts[rows][:, None] * scale
+    rc = _lib.load().b200_cross_entropy(pad.data_ptr(), targets.data_ptr(), loss.data_ptr(), T, V, pad.stride(0), scale, _lib.stream_ptr())
+    assert rc == 0 and (pad[:, V:] == 5).all() and loss.isfinite().all() and logits.isfinite().all() and (logits[counts] != 0).any(-1).all()
+    # exponentials of arguments up to 110 whose product with log2(e) is rounded to 24 bits, and sums of them; a bf16 has no steps below 2^-133
+    err = 160 * 2.0 ** -24
+    _within(loss[rows], want_loss, err, err * (1 + lse.abs().max()))
+    _within(logits[rows], want, BF + err, scale * err + 2.0 ** -133)
+    assert _lib.read_status() == 0
+
+
 def test_cross_entropy_of_a_row_with_nan_is_nan():
     from aws_ofi_nccl_b200.ops import llm
 
@@ -237,9 +277,6 @@ def _loss_and_gradient(rows, targets):
     rc = _lib.load().b200_cross_entropy(pad.data_ptr(), targets.data_ptr(), loss.data_ptr(), T, V, pad.stride(0), 1.0, _lib.stream_ptr())
     assert rc == 0 and (pad[:, V:] == 5).all()
     return loss, pad[:, :V]
-
-
-LOWEST = torch.finfo(torch.bfloat16).min   # the usual value of a mask
 
 
 # rows of one CTA, of a cluster of two, four and eight, too many of them (two passes), and a wider row than a cluster holds
