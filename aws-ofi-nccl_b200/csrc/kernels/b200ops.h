@@ -15,6 +15,7 @@ int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w,
                      void* stream);
 int b200_embedding_fwd(const long long* ids, const void* table, void* out, long long T, int H, void* stream);
 int b200_embedding_bwd(const long long* ids, const void* dout, void* dtable, long long T, int H, void* stream);
+int b200_cross_entropy(void* logits, const long long* targets, float* loss, int T, int V, long long ld, float grad_scale, void* stream);
 int b200_rmsnorm_bwd_partial_rows();
 int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                      float* dw_partial, void* dw, int accumulate_dw, int T, int H, void* stream);

@@ -368,6 +368,36 @@ struct SwiGLUMLP : public Function<SwiGLUMLP> {
   }
 };
 
+// Mean cross-entropy of a matrix of logits, which are overwritten with its gradient: the backward pass hands them on. In Python this was
+// 60 us of a forward and backward pass, 30 here: a head of 300 x 512 x 4096 takes 97 us for 130, the two-layer model of 256 channels on
+// 256 tokens 860 for 970 (three processes of each in turn, within 5 %).
+struct CrossEntropy : public Function<CrossEntropy> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& logits, const Tensor& targets) {
+    if (logits.dim() != 2) raise(PyExc_ValueError, "the logits are a matrix");
+    const int64_t T = logits.size(0), V = logits.size(1);
+    require(logits.stride(1) == 1, "the logits have contiguous rows");
+    if (T == 0) raise(PyExc_ZeroDivisionError, "the mean of no rows");
+    const Tensor loss = at::empty({T}, logits.options().dtype(at::kFloat));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    check(b200_cross_entropy(logits.data_ptr(), static_cast<const long long*>(targets.data_ptr()), loss.data_ptr<float>(), static_cast<int>(T),
+                             static_cast<int>(V), logits.stride(0), static_cast<float>(1.0 / static_cast<double>(T)), stream()),
+          "cross_entropy");
+    ctx->save_for_backward({logits});
+    ctx->mark_dirty({logits});
+    // nobody differentiates through the overwritten logits: no zero-filled [T, V] gradient for them
+    ctx->set_materialize_grads(false);
+    return {loss.mean(), logits};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return on_engine_thread([&]() -> variable_list {
+      const Tensor dlogits = ctx->get_saved_variables()[0];
+      if (grads[1].defined())
+        raise(PyExc_RuntimeError, "cross_entropy overwrites its logits with their gradient: nothing can be differentiated through them afterwards");
+      return {grads[0].defined() ? dlogits : Tensor(), Tensor()};
+    });
+  }
+};
+
 // q, k (rotated) and v as [B, S, heads, hd] tensors of their own from the fused projection [B*S, (nq+2nkv)*hd]
 struct RopeQKV : public Function<RopeQKV> {
   static void launch(const Tensor& qkv, const Tensor (&part)[3], const Tensor& cos, const Tensor& sin, int64_t S, bool backward) {
@@ -420,6 +450,7 @@ variable_list rmsnorm(const Tensor& x, const c10::optional<Tensor>& res, const T
 Tensor swiglu(const Tensor& gu) { return SwiGLU::apply(gu); }
 Tensor embedding(const Tensor& ids, const Tensor& table) { return Embedding::apply(ids, table); }
 Tensor swiglu_mlp(const Tensor& x, const Tensor& w_gu, const Tensor& w_down) { return SwiGLUMLP::apply(x, w_gu, w_down); }
+variable_list cross_entropy(const Tensor& logits, const Tensor& targets) { return CrossEntropy::apply(logits, targets); }
 variable_list rope_qkv(const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t S, int64_t nq, int64_t nkv,
                        int64_t hd) {
   return RopeQKV::apply(qkv, cos, sin, B, S, nq, nkv, hd);
@@ -467,5 +498,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                                           int64_t nq, int64_t nkv, int64_t hd) {
           return traced_or_direct("b200ops::rope_qkv", rope_qkv, qkv, cos, sin, B, S, nq, nkv, hd);
         }));
+  m.def("cross_entropy", torch::wrap_pybind_function_no_gil(cross_entropy));
   m.def("launches", [] { return g_launches.load(std::memory_order_relaxed); });
 }

@@ -64,7 +64,9 @@ def rope_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, seq: int) -> to
 
 class _CrossEntropy(torch.autograd.Function):
     """Mean token cross-entropy.  The logits tensor is overwritten with its own gradient in the
-    forward pass (one fused kernel), so backward only rescales by the incoming scalar."""
+    forward pass (one fused kernel), so backward only rescales by the incoming scalar.  What ``cross_entropy`` is
+    while torch.jit.trace records it (which refuses it: it overwrites its input), and for programs that clear
+    ``assume_unit_grad``; otherwise it is native."""
 
     @staticmethod
     def forward(ctx, logits, targets):
@@ -94,8 +96,9 @@ class _CrossEntropy(torch.autograd.Function):
 
 
 def cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
-    loss, _ = _CrossEntropy.apply(logits, targets)
-    return loss
+    if torch._C._get_tracing_state() is not None or not getattr(_CrossEntropy, "assume_unit_grad", True):
+        return _CrossEntropy.apply(logits, targets)[0]
+    return _lib.native().cross_entropy(logits, targets)[0]
 
 
 def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:

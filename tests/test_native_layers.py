@@ -312,3 +312,43 @@ def test_the_embedding_adds_its_gradient_up_from_any_view(shape):
         assert torch.equal(got.float(), want + (1 if written else 0))
     traced = torch.jit.trace(llm.embedding, (torch.zeros_like(ids), torch.zeros_like(table)), check_trace=False)
     assert torch.equal(traced(ids, table), out)
+
+
+@pytest.mark.gpu
+def test_the_cross_entropy_is_the_same_inside_and_outside_of_python():
+    """Loss, gradient, what the logits hold, and what is refused."""
+    from aws_ofi_nccl_b200.ops import llm
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    leaf = torch.randn(40, 96, device="cuda", generator=g).bfloat16().requires_grad_(True)
+    targets = torch.randint(0, 96, (40,), device="cuda", generator=g)
+    results = []
+    for fn in (llm.cross_entropy, lambda *a: llm._CrossEntropy.apply(*a)[0]):
+        logits = leaf[:, :72] * 1.0   # any row pitch
+        version = logits._version
+        loss = fn(logits, targets % 72)
+        assert logits._version > version and loss.requires_grad and loss.shape == ()
+        (d,) = torch.autograd.grad(loss * 3, leaf)   # the incoming scalar is taken for one
+        with torch.no_grad():
+            plain = fn(leaf.detach().clone(), targets)
+        assert not plain.requires_grad
+        results.append((loss.detach(), d, logits.detach(), plain))
+        with pytest.raises(ValueError):
+            fn(torch.zeros(8, device="cuda", dtype=torch.bfloat16), targets)
+        with pytest.raises(AssertionError):
+            fn(torch.zeros(96, 40, device="cuda", dtype=torch.bfloat16).T, targets)
+        with pytest.raises(ZeroDivisionError):
+            fn(torch.zeros(0, 96, device="cuda", dtype=torch.bfloat16), targets[:0])
+        with pytest.raises(RuntimeError, match="leaf"):
+            fn(leaf.detach().clone().requires_grad_(True), targets)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.gpu
+def test_a_traced_cross_entropy_is_refused():
+    """torch.jit.trace records no function that overwrites its input."""
+    from aws_ofi_nccl_b200.ops import llm
+
+    targets = torch.arange(6, device="cuda")
+    with pytest.raises(RuntimeError, match="JIT"):
+        torch.jit.trace(lambda x: llm.cross_entropy(x * 1.0, targets), (torch.randn(6, 64, device="cuda").bfloat16(),), check_trace=False)
