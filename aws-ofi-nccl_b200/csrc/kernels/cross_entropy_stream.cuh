@@ -27,11 +27,6 @@ constexpr int CES_SMEM = 1024 + CES_SLOTS * CES_SLOT_BYTES;
 constexpr uint64_t CES_WAIT_LIMIT_NS = 2000000000ull;
 static_assert(CES_SMEM <= 232448, "more than a CTA's shared memory");
 
-__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem),
-               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
-               : "memory");
-}
 // The chunks of this CTA's rows in the order in which they are loaded.
 struct CesWalk {
   int chunks, again;   // of a row: all, and those that are loaded a second time

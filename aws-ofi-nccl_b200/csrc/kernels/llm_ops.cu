@@ -68,6 +68,9 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // 256 / TPR rows, so that a narrow row does not leave most of the CTA idle; each thread holds VPT
 // 16-byte vectors of it.
 constexpr int NORM_THREADS = 256;
+constexpr int NORM_RING_CTAS = 3;   // of an SM, forward; the backward kernel's partial sums are for two
+constexpr int NORM_MAX_SLOTS = 8;
+constexpr uint64_t NORM_WAIT_LIMIT_NS = 2000000000ull;
 
 // Sum over the TPR threads of a row, the same in each. `parity` alternates between consecutive calls:
 // the one barrier of the next call then separates this call's reads from that buffer's next writes.
@@ -150,6 +153,36 @@ __global__ void __launch_bounds__(NORM_THREADS)
   }
 }
 
+// The groups' parts of dw are added up in shared memory, R - 1 rows of TPR * VPT * 8 floats, and make one row of the partial sums.
+template <int TPR, int VPT>
+__device__ __forceinline__ void norm_partial_row(float (&dw_acc)[VPT][8], float* group_dw, float* dw_partial, int H, int lane, int group) {
+  constexpr int R = NORM_THREADS / TPR, ROW = TPR * VPT * 8;
+  if constexpr (R > 1) {
+    if (group > 0) {
+#pragma unroll
+      for (int i = 0; i < VPT; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) group_dw[(group - 1) * ROW + (i * 8 + j) * TPR + lane] = dw_acc[i][j];
+    }
+    __syncthreads();
+    if (group > 0) return;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        for (int q = 0; q < R - 1; ++q) dw_acc[i][j] += group_dw[q * ROW + (i * 8 + j) * TPR + lane];
+  }
+  float* out = dw_partial + static_cast<int64_t>(blockIdx.x) * H;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int idx = lane + i * TPR;
+    if (idx * 8 < H) {
+      reinterpret_cast<float4*>(out)[2 * idx] = make_float4(dw_acc[i][0], dw_acc[i][1], dw_acc[i][2], dw_acc[i][3]);
+      reinterpret_cast<float4*>(out)[2 * idx + 1] = make_float4(dw_acc[i][4], dw_acc[i][5], dw_acc[i][6], dw_acc[i][7]);
+    }
+  }
+}
+
 template <int VPT>
 struct NormRow {
   Bf16x8 dy[VPT], x[VPT], dr[VPT];
@@ -170,7 +203,7 @@ __global__ void __launch_bounds__(NORM_THREADS, 2)
   after_wait(dy, x, w, rstd, dres, dx, dw_partial);
   constexpr int R = NORM_THREADS / TPR;   // rows of a CTA at a time
   __shared__ float red[2][NORM_THREADS / 32];
-  __shared__ float group_dw[R > 1 ? R - 1 : 1][R > 1 ? TPR * VPT * 8 : 1];
+  __shared__ float group_dw[R > 1 ? (R - 1) * TPR * VPT * 8 : 1];
   const int lane = threadIdx.x % TPR, group = threadIdx.x / TPR;
   float dw_acc[VPT][8];
   Bf16x8 wv[VPT];
@@ -248,52 +281,264 @@ __global__ void __launch_bounds__(NORM_THREADS, 2)
     if (AHEAD) cur = next;
   }
   grid_release();
-  if constexpr (R > 1) {
-    if (group > 0) {
-#pragma unroll
-      for (int i = 0; i < VPT; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) group_dw[group - 1][(i * 8 + j) * TPR + lane] = dw_acc[i][j];
+  norm_partial_row<TPR, VPT>(dw_acc, group_dw, dw_partial, H, lane, group);
+}
+
+// ---- The same for many rows: a persistent CTA's rows come through a ring of shared memory, groups of 256 / TPR of them at a time, by bulk
+// copies that one thread issues as soon as a group has been read. With loads into registers nothing of a CTA's next row is in flight
+// while it reduces (forward), or one row (backward): 16384 x 4096 forward 63 -> 48 us (5.6 TB/s), backward 86 -> 79; 4096 x 4096
+// with a residual 26.9 -> 25.3 and 31.5 -> 29.4 with the sum of the partial rows; 1000 x 2048 forward 6.8 -> 5.5. The weight is read once
+// per CTA instead of once per row. A CTA with one group has nothing to read ahead: those are left to the kernels above
+// (256 x 256 backward 5.7 us, 6.4 so), and so are rows of which a ring holds less than three in the backward pass (2048 x 8192 34.6, 35.3).
+struct NormRing {
+  uint32_t ring, bars;       // shared memory: slots, and a barrier for each
+  int slots, slot;
+  uint32_t phase, slot_bytes;
+  int* err_word;
+  volatile int* abort_flag;
+  __device__ __forceinline__ NormRing(uint8_t* smem, uint64_t* bar_words, int* abort_word, int n, uint32_t bytes, int* err)
+      : ring(smem_u32(smem)), bars(smem_u32(bar_words)), slots(n), slot(0), phase(0), slot_bytes(bytes), err_word(err), abort_flag(abort_word) {
+    if (threadIdx.x == 0) {
+      for (int s = 0; s < slots; ++s) mbar_init(bars + 8u * s, 1);
+      *abort_word = 0;
+      fence_barrier_init();
     }
     __syncthreads();
-    if (group > 0) return;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        for (int q = 0; q < R - 1; ++q) dw_acc[i][j] += group_dw[q][(i * 8 + j) * TPR + lane];
   }
-  float* out = dw_partial + static_cast<int64_t>(blockIdx.x) * H;
+  __device__ __forceinline__ uint32_t at() const { return ring + slot * slot_bytes; }
+  // One thread: part `part` of N of a slot, `bytes` of them.
+  template <int N, typename... P>
+  __device__ __forceinline__ void load(int s, uint32_t bytes, const P*... from) const {
+    mbar_expect_tx(bars + 8u * s, bytes * (0 + ... + (from ? 1 : 0)));
+    uint32_t to = ring + s * slot_bytes;
+    ((from ? bulk_load(to, from, bytes, bars + 8u * s) : void(), to += slot_bytes / N), ...);
+  }
+  __device__ __forceinline__ void wait() const {
+    mbar_wait_bounded(bars + 8u * slot, phase, abort_flag, err_word, DEV_ERR_FULL_BAR_TIMEOUT, NORM_WAIT_LIMIT_NS);
+  }
+  __device__ __forceinline__ void next() {
+    if (++slot == slots) {
+      slot = 0;
+      phase ^= 1;
+    }
+  }
+  // After a wait that ran out copies may still be under way.
+  __device__ __forceinline__ void leave() const {
+    __syncthreads();
+    if (*abort_flag) {
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    }
+  }
+};
+__device__ __forceinline__ Bf16x8 ring_vector(uint32_t at) {
+  uint32_t r[4];
+  ld_shared_v4(at, r);
+  return *reinterpret_cast<const Bf16x8*>(r);
+}
+
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(NORM_THREADS, NORM_RING_CTAS)
+    rmsnorm_fwd_ring_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, bf16* __restrict__ h_out, const bf16* __restrict__ w,
+                            bf16* __restrict__ y, float* __restrict__ rstd, int T, int H, float eps, int slots, int* err_word) {
+  constexpr int R = NORM_THREADS / TPR;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ uint64_t bar_words[NORM_MAX_SLOTS];
+  __shared__ int abort_word;
+  __shared__ float red[2][NORM_THREADS / 32];
+  const uint32_t row_bytes = H * 2, part = R * row_bytes;
+  NormRing ring(smem, bar_words, &abort_word, slots, res ? 2 * part : part, err_word);
+  after_wait(x, res, h_out, w, y, rstd);
+  const int lane = threadIdx.x % TPR, group = threadIdx.x / TPR;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * R;
+  int64_t row0 = static_cast<int64_t>(blockIdx.x) * R, ahead = row0;
+  auto load = [&](int s) {
+    if (ahead < T) {
+      const uint32_t bytes = static_cast<uint32_t>(T - ahead < R ? T - ahead : R) * row_bytes;
+      if (res)
+        ring.load<2>(s, bytes, x + ahead * H, res + ahead * H);
+      else
+        ring.load<1>(s, bytes, x + ahead * H);
+    }
+    ahead += stride;
+  };
+  if (threadIdx.x == 0)
+    for (int s = 0; s < slots; ++s) load(s);
+  Bf16x8 wv[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if ((lane + i * TPR) * 8 < H) wv[i] = reinterpret_cast<const Bf16x8*>(w)[lane + i * TPR];
+  for (int parity = 0; row0 < T; row0 += stride, parity ^= 1) {
+    const int64_t row = row0 + group;
+    const bool live = row < T;
+    ring.wait();
+    const uint32_t at = ring.at() + group * row_bytes;
+    Bf16x8 hv[VPT];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int idx = lane + i * TPR;
+      if (live && idx * 8 < H) {
+        hv[i] = ring_vector(at + idx * 16);
+        float f[8];
+        unpack8(hv[i], f);
+        if (res) {
+          float r[8];
+          unpack8(ring_vector(at + part + idx * 16), r);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] += r[j];
+          hv[i] = pack8(f);
+          reinterpret_cast<Bf16x8*>(h_out + row * H)[idx] = hv[i];
+          unpack8(hv[i], f);  // normalise exactly what was stored
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+      }
+    }
+    ss = row_sum<TPR>(ss, red, parity);
+    if constexpr (TPR <= 32) __syncthreads();   // everybody has read the slot
+    if (threadIdx.x == 0) load(ring.slot);
+    ring.next();
+    if (!live) continue;
+    const float r = rsqrtf(ss / H + eps);
+    if (lane == 0 && rstd) rstd[row] = r;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int idx = lane + i * TPR;
+      if (idx * 8 < H) {
+        float f[8], wf[8];
+        unpack8(hv[i], f);
+        unpack8(wv[i], wf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * r * wf[j];
+        reinterpret_cast<Bf16x8*>(y + row * H)[idx] = pack8(f);
+      }
+    }
+  }
+  grid_release();
+  ring.leave();
+}
+
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(NORM_THREADS, 2)
+    rmsnorm_bwd_ring_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
+                            const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
+                            float* __restrict__ dw_partial, int T, int H, int slots, int* err_word) {
+  constexpr int R = NORM_THREADS / TPR;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ uint64_t bar_words[NORM_MAX_SLOTS];
+  __shared__ int abort_word;
+  __shared__ float red[2][NORM_THREADS / 32];
+  const uint32_t row_bytes = H * 2, part = R * row_bytes;
+  NormRing ring(smem, bar_words, &abort_word, slots, dres ? 3 * part : 2 * part, err_word);
+  after_wait(dy, x, w, rstd, dres, dx, dw_partial);
+  const int lane = threadIdx.x % TPR, group = threadIdx.x / TPR;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * R;
+  int64_t row0 = static_cast<int64_t>(blockIdx.x) * R, ahead = row0;
+  auto load = [&](int s) {
+    if (ahead < T) {
+      const uint32_t bytes = static_cast<uint32_t>(T - ahead < R ? T - ahead : R) * row_bytes;
+      if (dres)
+        ring.load<3>(s, bytes, dy + ahead * H, x + ahead * H, dres + ahead * H);
+      else
+        ring.load<2>(s, bytes, dy + ahead * H, x + ahead * H);
+    }
+    ahead += stride;
+  };
+  if (threadIdx.x == 0)
+    for (int s = 0; s < slots; ++s) load(s);
+  float dw_acc[VPT][8];
+  Bf16x8 wv[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int idx = lane + i * TPR;
-    if (idx * 8 < H) {
-      reinterpret_cast<float4*>(out)[2 * idx] = make_float4(dw_acc[i][0], dw_acc[i][1], dw_acc[i][2], dw_acc[i][3]);
-      reinterpret_cast<float4*>(out)[2 * idx + 1] = make_float4(dw_acc[i][4], dw_acc[i][5], dw_acc[i][6], dw_acc[i][7]);
+    if (idx * 8 < H) wv[i] = reinterpret_cast<const Bf16x8*>(w)[idx];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dw_acc[i][j] = 0.f;
+  }
+  float r_next = row0 + group < T ? rstd[row0 + group] : 0.f;
+  for (int parity = 0; row0 < T; row0 += stride, parity ^= 1) {
+    const int64_t row = row0 + group;
+    const bool live = row < T;
+    const float r = r_next;
+    if (row + stride < T) r_next = rstd[row + stride];
+    ring.wait();
+    const uint32_t at = ring.at() + group * row_bytes;
+    Bf16x8 dv[VPT], xv[VPT], ev[VPT];
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int idx = lane + i * TPR;
+      if (live && idx * 8 < H) {
+        dv[i] = ring_vector(at + idx * 16);
+        xv[i] = ring_vector(at + part + idx * 16);
+        if (dres) ev[i] = ring_vector(at + 2 * part + idx * 16);
+        float d[8], xf[8], wf[8];
+        unpack8(dv[i], d);
+        unpack8(xv[i], xf);
+        unpack8(wv[i], wf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          dw_acc[i][j] += d[j] * xf[j] * r;
+          dot += d[j] * wf[j] * xf[j];
+        }
+      }
+    }
+    dot = row_sum<TPR>(dot, red, parity);
+    if constexpr (TPR <= 32) __syncthreads();   // everybody has read the slot
+    if (threadIdx.x == 0) load(ring.slot);
+    ring.next();
+    if (live) {
+      const float c = dot * r * r / H;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int idx = lane + i * TPR;
+        if (idx * 8 < H) {
+          float d[8], xf[8], wf[8], o[8];   // unpacked again: the packed row takes half the registers
+          unpack8(dv[i], d);
+          unpack8(xv[i], xf);
+          unpack8(wv[i], wf);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = r * (d[j] * wf[j] - xf[j] * c);
+          if (dres) {
+            float e[8];
+            unpack8(ev[i], e);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += e[j];
+          }
+          reinterpret_cast<Bf16x8*>(dx + row * H)[idx] = pack8(o);
+        }
+      }
     }
   }
+  grid_release();
+  ring.leave();   // the ring's memory is free: the groups' sums are added up in it
+  float* group_dw = reinterpret_cast<float*>(smem);
+  norm_partial_row<TPR, VPT>(dw_acc, group_dw, dw_partial, H, lane, group);
 }
 
-// dw[h] (+)= sum over partial rows. A CTA takes 32 columns; its eight warps add up every eighth row
-// each, so that a column's rows are not one chain of dependent loads.
-__global__ void __launch_bounds__(256)
+// dw[h] (+)= sum over partial rows. A CTA takes 32 columns; each of its warps adds up every COLSUM_WARPS-th row, so that a column's
+// rows are not one chain of dependent loads: the backward pass of 4096 x 4096
+// takes 29.4 us, 29.9 with eight warps, 37 x 5120 7.0 and 7.5.
+constexpr int COLSUM_WARPS = 32;
+__global__ void __launch_bounds__(32 * COLSUM_WARPS)
     colsum_partial_kernel(const float* __restrict__ partial, bf16* __restrict__ dw, int nrows, int H, int accumulate) {
   after_wait(partial, dw);
   grid_release();
-  __shared__ float part[8][32];
+  __shared__ float part[COLSUM_WARPS][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int h = blockIdx.x * 32 + lane;
   float s = 0.f;
   if (h < H) {
-#pragma unroll 8
-    for (int r = warp; r < nrows; r += 8) s += partial[static_cast<int64_t>(r) * H + h];
+#pragma unroll 10
+    for (int r = warp; r < nrows; r += COLSUM_WARPS) s += partial[static_cast<int64_t>(r) * H + h];
   }
   part[warp][lane] = s;
   __syncthreads();
   if (warp != 0 || h >= H) return;
   s = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) s += part[i][lane];
+  for (int i = 0; i < COLSUM_WARPS; ++i) s += part[i][lane];
   if (accumulate) s += __bfloat162float(dw[h]);
   dw[h] = __float2bfloat16(s);
 }
@@ -785,6 +1030,20 @@ static inline int grid_for(int64_t work_items, int threads, int per_sm = 16) {
   return static_cast<int>(b);
 }
 
+// Slots of `bytes` for each of `ctas` CTAs of an SM (228 KB, of which a CTA's own part takes 1 KB and the kernels' other arrays less than that).
+static int norm_slots(int bytes, int ctas) {
+  const int n = (228 / ctas - 3) * 1024 / bytes;
+  return n < NORM_MAX_SLOTS ? n : NORM_MAX_SLOTS;
+}
+template <auto KERNEL>
+static int norm_smem() {   // once per kernel
+  static std::atomic<bool> set{false};
+  if (set.load(std::memory_order_acquire)) return 0;
+  B200_CUDA_OK(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+  set.store(true, std::memory_order_release);
+  return 0;
+}
+
 // 32-bit indices hold while a grid's last pass, beyond the last item, stays below 2^32. What they gain is their divisions: rotary split of
 // 4096 x 48 x 128 22.9 -> 22.2 us, its backward pass 23.8 -> 22.6, 2048 x 12 x 64 4.6 -> 4.2, the embedding's gradient of 4096 x 4096 28.7 -> 24.8.
 static bool small_index(int64_t items) { return items < (1ll << 31); }
@@ -816,13 +1075,24 @@ int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w,
   if (!aligned16(x, res, h_out, w, y)) return B200_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto X = static_cast<const bf16*>(x);
-  auto R = static_cast<const bf16*>(res);
+  auto RES = static_cast<const bf16*>(res);
   auto HO = static_cast<bf16*>(h_out);
   auto W = static_cast<const bf16*>(w);
   auto Y = static_cast<bf16*>(y);
-#define B200_NORM_FWD(TPR, VPT)                                                              \
-  launch_dependent(rmsnorm_fwd_kernel<TPR, VPT>, (T + NORM_THREADS / TPR - 1) / (NORM_THREADS / TPR), NORM_THREADS, 0, s, X, R, HO, W, Y, \
-                                                                                            rstd, T, H, eps)
+#define B200_NORM_FWD(TPR, VPT)                                                                                              \
+  do {                                                                                                                       \
+    constexpr int R = NORM_THREADS / TPR;                                                                                    \
+    const int groups = (T + R - 1) / R, ctas = sm_count() * NORM_RING_CTAS;                                                  \
+    const int slot = R * H * 2 * (RES ? 2 : 1), slots = norm_slots(slot, NORM_RING_CTAS);                                     \
+    if (groups > ctas) {                                                                                                     \
+      const int rc = norm_smem<rmsnorm_fwd_ring_kernel<TPR, VPT>>();                                                           \
+      if (rc) return rc;                                                                                                     \
+      launch_dependent(rmsnorm_fwd_ring_kernel<TPR, VPT>, ctas, NORM_THREADS, slots * slot, s, X, RES, HO, W, Y, rstd, T, H, eps, slots, \
+                       device_status_word());                                                                                \
+    } else {                                                                                                                 \
+      launch_dependent(rmsnorm_fwd_kernel<TPR, VPT>, groups, NORM_THREADS, 0, s, X, RES, HO, W, Y, rstd, T, H, eps);           \
+    }                                                                                                                        \
+  } while (0)
   B200_NORM_DISPATCH(B200_NORM_FWD);
 #undef B200_NORM_FWD
   B200_CUDA_OK(cudaGetLastError());
@@ -844,15 +1114,24 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
   auto W = static_cast<const bf16*>(w);
   auto DR = static_cast<const bf16*>(dres);
   auto DX = static_cast<bf16*>(dx);
-#define B200_NORM_BWD(TPR, VPT)                                                                                       \
-  do {                                                                                                                \
-    const int groups = (T + NORM_THREADS / TPR - 1) / (NORM_THREADS / TPR);                                           \
-    if (grid > groups) grid = groups;                                                                                 \
-    launch_dependent(rmsnorm_bwd_kernel<TPR, VPT>, grid, NORM_THREADS, 0, s, DY, X, W, rstd, DR, DX, dw_partial, T, H);             \
+#define B200_NORM_BWD(TPR, VPT)                                                                                              \
+  do {                                                                                                                       \
+    constexpr int R = NORM_THREADS / TPR;                                                                                    \
+    const int groups = (T + R - 1) / R;                                                                                      \
+    const int parts = (R - 1) * TPR * VPT * 8 * 4, slot = R * H * 2 * (DR ? 3 : 2), slots = norm_slots(slot, 2);               \
+    if (groups > grid && slots >= 3) {                                                                                       \
+      const int rc = norm_smem<rmsnorm_bwd_ring_kernel<TPR, VPT>>();                                                           \
+      if (rc) return rc;                                                                                                     \
+      launch_dependent(rmsnorm_bwd_ring_kernel<TPR, VPT>, grid, NORM_THREADS, slots * slot > parts ? slots * slot : parts, s, DY, X, W, rstd, \
+                       DR, DX, dw_partial, T, H, slots, device_status_word());                                               \
+    } else {                                                                                                                 \
+      if (grid > groups) grid = groups;                                                                                      \
+      launch_dependent(rmsnorm_bwd_kernel<TPR, VPT>, grid, NORM_THREADS, 0, s, DY, X, W, rstd, DR, DX, dw_partial, T, H);     \
+    }                                                                                                                        \
   } while (0)
   B200_NORM_DISPATCH(B200_NORM_BWD);
 #undef B200_NORM_BWD
-  launch_dependent(colsum_partial_kernel, (H + 31) / 32, 256, 0, s, dw_partial, static_cast<bf16*>(dw), grid, H, accumulate_dw);
+  launch_dependent(colsum_partial_kernel, (H + 31) / 32, 32 * COLSUM_WARPS, 0, s, dw_partial, static_cast<bf16*>(dw), grid, H, accumulate_dw);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }

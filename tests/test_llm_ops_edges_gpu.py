@@ -42,6 +42,18 @@ def test_rmsnorm(T, H, with_res):
         assert torch.equal(got[0], got[2])
 
 
+# more groups of rows than CTAs, whose rows come through a ring: eight to one rows in a group, ragged last groups and widths, one group and a row
+# more than the CTAs take at once, several rounds of the ring
+@pytest.mark.parametrize("T,H", [(20001, 8), (3553, 64), (3553, 256), (7003, 264), (1777, 520), (889, 2048), (445, 2056), (4001, 4096), (445, 4104),
+                                 (1201, 6144), (445, 6152), (1800, 8192)])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_rmsnorm_of_many_rows(T, H, with_res):
+    from aws_ofi_nccl_b200.ops import _lib
+
+    test_rmsnorm(T, H, with_res)
+    assert _lib.read_status() == 0
+
+
 @pytest.mark.parametrize("T,F", [(1, 8), (3, 72), (257, 520), (1000, 2056), (4096, 1376)])
 def test_swiglu(T, F):
     from aws_ofi_nccl_b200.ops import llm
