@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(MOE_THREADS)
         for (int u = 0; u < U; ++u)
           if (v0 + 32 * u < vec) {
             x[u] = a[v0 + 32 * u];
-            y[u] = b[v0 + 32 * u];
+            y[u] = __ldcs(b + v0 + 32 * u);   // the token's gradient is read k times, a cell once: 92 -> 87 us
           }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
