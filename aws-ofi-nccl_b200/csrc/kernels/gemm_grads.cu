@@ -82,16 +82,21 @@ GradsPlan plan_joint(const GradsCall& c) {
 // at the pace of its own pipeline, and joint kernels got 3.8 TB/s there where dx alone gets 5.3 (128 x 4096 x 14336
 // with cold weights 63 us, 58 in two). Of 128 layers (M 16 to 8192, N 64 to 28672, K 64 to 14336, and the 8B model's) the
 // rule takes one launch for 93; the mean of its times is 0.789 of two launches', the faster way's 0.785, and it is never
-// slower by more than 3 % than two. 256 x 768 x 256: 11 us for 20; 1000 x 2568 x 5160 58 for 75; 4096 x 4096 x 4096 158 for 169.
+// slower by more than 3 % than two. Between 129 and 256 rows dx by itself is a single row of tiles as well, and takes longer than the
+// estimate for a product by itself says: of 37 such layers over weights of 64 to 600 MB with N <= 3 K the rule takes one launch for 33; the mean of
+// its times is 0.86 of two launches' and 1.008 of the faster way's, 1.089 with the line that fewer rows have (256 x 8192 x 8192 72 us for
+// 86, 200 x 5120 x 13824 73 and 92, 256 x 6144 x 6144 47 and 59). A longer reduction is a chain that two launches split (136 x 28672 x 4096 126 us, 147 jointly).
+// 256 x 768 x 256: 11 us for 20; 1000 x 2568 x 5160 58 for 75; 4096 x 4096 x 4096 158 for 169.
 bool pays(const GradsCall& c, const GradsPlan& p) {
   if (!pairs_enabled()) return false;
   if (one_wave(c)) return true;
   const bool few_rows = c.M <= GEMM2_BM && 2.0 * c.N * c.K > 64e6;
+  const bool one_pair_row = few_rows && c.M > GEMM_BM && c.N <= 3ll * c.K;   // a row of tiles on CTA pairs in either way
   double alone = pair_tile_clocks(c.N, p.width[0], on_lines(c), p.warps);
-  if (few_rows) alone = std::max(alone, 700.0 * ((c.N + GEMM_BK - 1) / GEMM_BK));
-  const double moved = (few_rows ? 1.25 : 0.8) * (memory_clocks(c.M, c.K, c.N) + memory_clocks(c.N, c.K, c.M));
+  if (few_rows) alone = std::max(alone, (one_pair_row ? 520.0 : 700.0) * ((c.N + GEMM_BK - 1) / GEMM_BK));
+  const double moved = (one_pair_row ? 1.15 : few_rows ? 1.25 : 0.8) * (memory_clocks(c.M, c.K, c.N) + memory_clocks(c.N, c.K, c.M));
   const double joint = std::max({p.clocks, alone, moved}) + LAUNCH_CLOCKS;
-  return joint < product_clocks(c.M, c.K, c.N, c.lddy, c.ldw, true, c.dy, c.w) + product_clocks(c.N, c.K, c.M, c.lddy, c.ldx, true, c.dy, c.x);
+  return joint < (one_pair_row ? 1.08 : 1.0) * (product_clocks(c.M, c.K, c.N, c.lddy, c.ldw, true, c.dy, c.w) + product_clocks(c.N, c.K, c.M, c.lddy, c.ldx, true, c.dy, c.x));
 }
 
 GemmShape product_shape(int rows, int cols, int k, int width) {

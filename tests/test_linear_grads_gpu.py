@@ -73,6 +73,12 @@ def test_linear_layer_takes_the_faster_way(M, N, K, joint):
         _within(wl.grad if buffer is None else wl.main_grad, want_dw, M, mag_dw)
 
 
+@pytest.mark.parametrize("M,N,K,joint", [(200, 6144, 6144, 1), (129, 8192, 8192, 1), (136, 16384, 4096, 0)])
+def test_a_row_of_pair_tiles_takes_the_faster_way(M, N, K, joint):
+    """129 to 256 rows over a weight that L2 does not hold."""
+    test_linear_layer_takes_the_faster_way(M, N, K, joint)
+
+
 def test_only_one_of_the_gradients():
     from aws_ofi_nccl_b200.ops.gemm import linear
 
