@@ -361,6 +361,14 @@ static bool use_pairs(int M, int N, int max_ctas) {
   return pairs_enabled() && M >= 256 && N >= 128 && (max_ctas == 0 || max_ctas >= 2);
 }
 
+// Three rows of 128 x 128 tiles that all run at once, where pairs would compute four rows in wide tiles on two thirds of the SMs: 257 to 384 rows
+// and 4737 to 6272 columns. 384 x 6144 x 4096 19.4 us, 22.4 on pairs; 340 x 5952 x 2816 14.2 and 16.8; 384 x 6208 x 1024 8.3 and 10.4; 300 x
+// 5120 x 13824 51 and 58. Fewer columns fit narrow pair tiles (384 x 4096 x 4096 16.6 us, 18.5 so), more take these two waves.
+static bool three_tile_rows(int M, int N) {
+  const int columns = (N + 127) / 128;
+  return M > 2 * GEMM_BM && M <= 3 * GEMM_BM && 3 * columns <= sm_count() && 2 * columns > sm_count() / 2;
+}
+
 // What a product with bn = 0 runs on: the tile width of the persistent kernel, or a split along K.
 // `a_at`, `b_at`: the operands' addresses (their alignment counts).
 struct GemmChoice {
@@ -488,7 +496,7 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
   using namespace b200;
   if (!gemm_args_ok(A, B, C, M, N, K, lda, ldb, ldc, out_fp32)) return B200_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool pairs = use_pairs(M, N, max_ctas);
+  bool pairs = use_pairs(M, N, max_ctas);
   PairTiles tiles{bn, false};
   if (bn == 0) {
     const GemmChoice g =
@@ -497,6 +505,10 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
       return launch_splitk({A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate}, pairs, g.split, s);
     bn = g.bn;
     tiles = g.tiles;
+    if (pairs && max_ctas == 0 && three_tile_rows(M, N)) {
+      pairs = false;
+      bn = 128;
+    }
   }
   if (pairs && (bn == 256 || bn == 128))
     return gemm_2cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, tiles, max_ctas, s);
@@ -521,6 +533,10 @@ int b200_gemm_plan(int M, int N, int K, long long lda, long long ldb, int* pair,
   *pair = use_pairs(M, N, 0);
   *slices = g.split.slices;
   *bn = g.split.slices > 1 ? 128 : g.bn;
+  if (*pair && *slices == 1 && three_tile_rows(M, N)) {
+    *pair = 0;
+    *bn = 128;
+  }
   return 0;
 }
 

@@ -72,6 +72,18 @@ def test_the_listed_sizes_take_the_path_that_they_are_listed_for():
     assert {_plan(*s)[::2] for s in SPLIT} == {(0, 4), (0, 8), (1, 2), (1, 4)}
 
 
+@pytest.mark.parametrize("M,N,K", [(257, 4744, 200), (384, 6144, 72), (300, 6272, 1032)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_three_rows_of_tiles_that_all_run_at_once(M, N, K, a_mn, b_mn):
+    assert _plan(M, N, K) == (0, 128, 1)
+    test_product_and_accumulation(M, N, K, torch.bfloat16, a_mn, b_mn)
+
+
+@pytest.mark.parametrize("M,N", [(256, 6144), (385, 6144), (384, 4736), (384, 6280)])
+def test_other_rows_and_columns_stay_on_pairs(M, N):
+    assert _plan(M, N, 2048)[0] == 1
+
+
 @pytest.mark.parametrize("M,N,K", [(256, 256, 1024), (512, 1024, 2048), (128, 4096, 1024), (768, 1536, 2048)])
 def test_a_short_reduction_is_not_split(M, N, K):
     """Products that a split made up to 1.4 times slower."""
