@@ -1010,7 +1010,8 @@ static CeRow ce_row(int64_t T, int V) {
 // Rows that no registers hold stream through shared memory, but for two rows for an SM of a length that a chunk or two hold: there two
 // CTAs of many threads are ahead (222 x 24576 10.0 us, 10.8 streamed; 296 x 28672 11.7 and 12.8). Everywhere else of 18 numbers of rows from 1
 // to 2048 and 12 widths from 16392 to 200000 the stream takes 0.68 to 1.00 of two passes.
-static bool ce_two_passes(int64_t T, int V) { return V >= 20000 && V < 32768 && T > sm_count() && T <= 2 * sm_count(); }
+// A row without elements has no chunk to stream.
+static bool ce_two_passes(int64_t T, int V) { return V < 8 || (V >= 20000 && V < 32768 && T > sm_count() && T <= 2 * sm_count()); }
 
 // Rows move as 16-byte vectors: null (an argument left out) or on a 16-byte boundary.
 template <class... P>
@@ -1032,7 +1033,7 @@ static inline int grid_for(int64_t work_items, int threads, int per_sm = 16) {
 
 // Slots of `bytes` for each of `ctas` CTAs of an SM (228 KB, of which a CTA's own part takes 1 KB and the kernels' other arrays less than that).
 static int norm_slots(int bytes, int ctas) {
-  const int n = (228 / ctas - 3) * 1024 / bytes;
+  const int n = bytes > 0 ? (228 / ctas - 3) * 1024 / bytes : 0;
   return n < NORM_MAX_SLOTS ? n : NORM_MAX_SLOTS;
 }
 template <auto KERNEL>
@@ -1084,7 +1085,7 @@ int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w,
     constexpr int R = NORM_THREADS / TPR;                                                                                    \
     const int groups = (T + R - 1) / R, ctas = sm_count() * NORM_RING_CTAS;                                                  \
     const int slot = R * H * 2 * (RES ? 2 : 1), slots = norm_slots(slot, NORM_RING_CTAS);                                     \
-    if (groups > ctas) {                                                                                                     \
+    if (groups > ctas && slots >= 2) {                                                                                       \
       const int rc = norm_smem<rmsnorm_fwd_ring_kernel<TPR, VPT>>();                                                           \
       if (rc) return rc;                                                                                                     \
       launch_dependent(rmsnorm_fwd_ring_kernel<TPR, VPT>, ctas, NORM_THREADS, slots * slot, s, X, RES, HO, W, Y, rstd, T, H, eps, slots, \

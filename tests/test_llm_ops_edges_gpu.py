@@ -269,6 +269,22 @@ def test_cross_entropy_of_wide_rows(T, V, scale):
     assert _lib.read_status() == 0
 
 
+def test_rows_without_elements():
+    """No loss, and no norm: what the entry points did before rows came through rings."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    lib, st = _lib.load(), _lib.stream_ptr()
+    loss, targets = torch.full((3,), 7.0, device="cuda"), torch.zeros(3, device="cuda", dtype=torch.int64)
+    buf = torch.zeros(64, device="cuda")
+    assert lib.b200_cross_entropy(buf.data_ptr(), targets.data_ptr(), loss.data_ptr(), 3, 0, 0, 1.0, st) == 0
+    assert (loss == 0).all()
+    p = buf.data_ptr()
+    rstd = torch.zeros(10000, device="cuda")
+    assert lib.b200_rmsnorm_fwd(p, None, None, p, p, rstd.data_ptr(), 10000, 0, 1e-5, st) == 0
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0
+
+
 def test_cross_entropy_of_a_row_with_nan_is_nan():
     from aws_ofi_nccl_b200.ops import llm
 
