@@ -6,7 +6,8 @@
 // kernel before it, and by the same rule everything before that, has ended and its writes are visible. Behind a kernel that
 // never releases, or anything that is no kernel, such a launch is an ordinary one. What it gains is 2 to 2.5 us between two
 // kernels: forward and both gradients of 128 x 4096 x 14336, three of them, take 82.6 us for 89.6, 1000 x 2568 x 5160 85 for 90
-// (two), SwiGLU of 4096 x 14336 and its gradient 147.6 for 150.2. Kernels that wait for other ranks' tiles are launched ordinarily.
+// (two), SwiGLU of 4096 x 14336 and its gradient 147.6 for 150.2. The products fused with a
+// collective, whose CTAs wait for other ranks' tiles, are launched ordinarily.
 //
 // Where a kernel takes const __restrict__ pointers (or restrict ones that it only reads from) the compiler may move loads through
 // them anywhere, before grid_wait too: such kernels use their pointers as after_wait returns them.

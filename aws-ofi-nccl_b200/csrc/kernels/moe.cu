@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(MOE_THREADS, 4) moe_combine_kernel(CombineArgs
   // A team per token: a wide one reads 4 KiB of each of the token's rows at a time. With a warp per
   // token every row is visited 512 bytes at a time by thousands of warps at once: 4096 tokens x 7168,
   // top-8, one rank took 194 us that way (314 with eight loads in flight per warp instead of four)
-  // and 140 so, before the stores to the window's cells: 215 with them, on average over the forward call,
+  // and 140 so, before the stores to the window's cells: 207 with them, on average over the forward call,
   // which copies the cells out as well, and the backward call, which does not; 299 (and 150 for the copy)
   // when every row was read back from its cell. Four cells' loads are issued together and added in the
   // order of the slots.
@@ -608,7 +608,7 @@ __host__ __device__ inline int dequant_pieces(int H) { return (H / 8 + DEQUANT_P
 // for a whole row. With zero_tail the rows past
 // the last received one are written as zeros, in place of a fill of the whole output before (120 us). With `meta`
 // the rows of rank `here` are in `out` already. Dispatch and combine of 4096 x 7168, top-8, with their gradients on one
-// rank: 889 us, 922 when every row was read back here.
+// rank: 814 us; reading every row back here cost 33 more.
 __global__ void __launch_bounds__(MOE_THREADS)
     fp8_dequant_rows_kernel(const uint8_t* q, const float* scales, __nv_bfloat16* out, const int32_t* rows_ptr, int rows_max,
                             int H, int zero_tail, const MoeMeta* meta, int here) {

@@ -1,5 +1,5 @@
-// The differentiable layers of the training path (linear, embedding, RMSNorm, SwiGLU, SwiGLU MLP, rotary split of
-// the fused projection) as autograd functions in native code: shape checks, output allocation, the calls into
+// The differentiable layers of the training path (linear, embedding, RMSNorm, SwiGLU, SwiGLU MLP, cross-entropy,
+// rotary split of the fused projection) as autograd functions in native code: shape checks, output allocation, the calls into
 // libb200ops.so and the weight-gradient hand-over run without the interpreter. A layer's launches are
 // a few microseconds of device time each at small sizes, and the interpreter's share of a forward and
 // backward call was several times that: a linear layer of 256 x 768 x 256 took 148 us a pass through
