@@ -397,7 +397,13 @@ static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint6
   const bool a_lines = a_low % 128 == 0, b_lines = b_low % 128 == 0;
   const Costs& c = a_lines && b_lines ? ON_LINES[b_mn] : a_lines || b_lines || (a_low | b_low) % 64 == 0 ? BETWEEN[b_mn] : OFF_LINES[b_mn];
   const int64_t rows = (M + GEMM2_BM - 1) / GEMM2_BM;
-  constexpr double GAIN = 1.03;   // a width that is not the plain one has to promise 3 %, halves of the last wave 1 %
+  // A width that is not the plain one has to promise 3 %, halves of the last wave 1 %. From K = 4096 on, with rows on cache lines, 2 % are enough, and
+  // halves behind a single wave cost .64 of one, where behind several the pairs' drift hides some of it. Of 55 such products that
+  // this gives another width none took more than 1.003 of the halves' time, and they took 0.967 on average: 768 x 8192 x 8192 99 -> 89 us,
+  // 433 x 12416 x 10112 0.95, 2403 x 7680 x 11456 416 -> 396; 40 of fp8 (K is half of theirs) 0.98, 1343 x 4608 x 11520 68.1 -> 65.6. A shorter
+  // K gains less and loses up to 3 % as often.
+  const bool long_k = step == 32 && a_lines && b_lines && K >= 4096;
+  const double gain = long_k ? 1.02 : 1.03;
   PairTiles best{bn, false};
   double best_cost = 1e30;
   for (int i = 0; i < 5; i += step / 32) {
@@ -405,14 +411,15 @@ static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint6
     if (width > 128 && N <= width - step) break;   // a narrower one covers the row as well
     if (width % 64 && K < 1024) continue;        // the last 32 columns of a tile leave as vectors, not by TMA: with few k-blocks that counts
     const int64_t tiles = rows * ((N + width - 1) / width);
-    const double cost = static_cast<double>((tiles + units - 1) / units) * c.at[i] * (width == bn ? 1 : GAIN);
+    const double cost = static_cast<double>((tiles + units - 1) / units) * c.at[i] * (width == bn ? 1 : gain);
     if (cost < best_cost) {
       best_cost = cost;
       best = {width, false};
     }
   }
   const int64_t wide = rows * ((N + 255) / 256), last = wide % units;
-  if (wide > units && last > 0 && 2 * last <= units && (static_cast<double>(wide / units) + c.at[0]) * 1.01 <= best_cost) best = {256, true};
+  const double half_wave = long_k && wide / units == 1 ? .64 : c.at[0];
+  if (wide > units && last > 0 && 2 * last <= units && (static_cast<double>(wide / units) + half_wave) * 1.01 <= best_cost) best = {256, true};
   return best;
 }
 static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, uintptr_t a_at, uintptr_t b_at, int max_ctas) {

@@ -273,6 +273,15 @@ def test_tiles_follow_the_waves_that_they_fill(M, N, K, b_mn, want):
     assert _tiles(M, N, K, b_mn) == want
 
 
+@pytest.mark.parametrize("M,N,K,b_mn,want", [
+    (768, 8192, 8192, False, (192, 0)), (768, 8192, 4096, True, (192, 0)), (768, 8192, 4032, False, (256, 1)),
+    (768, 8192, 8200, False, (256, 1)),   # rows off cache lines
+    (2403, 7680, 11456, False, (224, 0)), (2403, 7680, 2304, False, (256, 1))])
+def test_a_long_reduction_halves_fewer_waves(M, N, K, b_mn, want):
+    """Choices that were measured to be the faster ones, on both sides of where they change."""
+    assert _tiles(M, N, K, b_mn) == want
+
+
 @pytest.mark.parametrize("M,N,K", [(4096, 2072, 256), (2304, 3332, 144), (513, 300, 272)])
 def test_fp8_product_on_every_kind_of_tile(M, N, K):
     """A last wave of halves, a ragged width, single tiles."""
