@@ -197,13 +197,17 @@ static int dispatch_major_2cta(const void* A, const void* B, void* C, int M, int
   return launch_gemm_2cta<BN, true, true, OutT, EW>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, tiles, max_ctas, stream);
 }
 
-// The narrow kernel has more stages; tiles of any other width run on the wide one.
+// The narrow kernel has more stages; tiles of any other width run on the wide one. Eight epilogue warps store one tile during the next one's
+// products; where every pair has a single tile there is no next one, and four start sooner: 1504 x 1784 x 96 5.9 -> 5.5 us, 3200 x 1136
+// x 128 6.1 -> 5.9, 4 to 8 % over products of 38 to 74 tiles. Four are slower from three waves on (4096 x 4096 x 128 by 8 %), with two it varies.
 static int gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_mn,
                      int b_mn, int out_fp32, int accumulate, PairTiles tiles, int max_ctas, cudaStream_t s) {
   if (tiles.width == 128)
     return out_fp32 ? dispatch_major_2cta<128, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
                     : dispatch_major_2cta<128, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
-  if (K <= SHORT_K && !out_fp32)
+  const int64_t all = static_cast<int64_t>((M + GEMM2_BM - 1) / GEMM2_BM) * ((N + tiles.width - 1) / tiles.width);
+  const int pairs = (max_ctas > 0 && max_ctas < sm_count() ? max_ctas : sm_count()) / 2;
+  if (K <= SHORT_K && !out_fp32 && all > pairs)
     return dispatch_major_2cta<256, __nv_bfloat16, 8>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
   return out_fp32 ? dispatch_major_2cta<256, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
                   : dispatch_major_2cta<256, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);

@@ -253,6 +253,24 @@ def test_every_tile_width_and_the_halved_last_wave(width, halves, out_dtype, a_m
         assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
 
 
+@pytest.mark.parametrize("K", [8, 192, 200])
+@pytest.mark.parametrize("M,N", [(500, 37 * 256), (512, 37 * 256 + 8), (1, 8)])
+def test_a_tile_for_every_pair_and_one_more(M, N, K):
+    """74 wide tiles, as many as there are pairs of CTAs, then 76 of them, and a single one: the epilogue's warps differ."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    ll, vp = ctypes.c_longlong, ctypes.c_void_p
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    pad = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    rc = _lib.load().b200_gemm_bf16_tiles(vp(a.data_ptr()), vp(b.data_ptr()), vp(pad.data_ptr()), M, N, K, ll(K), ll(K), ll(N + 8),
+                                          0, 0, 0, 0, 256, 0, vp(_lib.stream_ptr()))
+    assert rc == 0
+    ref, mag = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
+    # fp32 sums of K exact products in any order, one rounding of the output
+    assert ((pad[:M, :N].double() - ref).abs() <= K * 2.0 ** -24 * mag + 2.0 ** -8 * ref.abs()).all()
+    assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
+
+
 def _tiles(M, N, K, b_mn=False):
     """(width, halves) that the automatic choice runs on, for operands with contiguous rows."""
     from aws_ofi_nccl_b200.ops import _lib
