@@ -14,8 +14,8 @@ struct PairTiles {
 };
 
 // Up to this K a tile's stores take longer than its products, and eight epilogue warps are worth the stage that their
-// staging area costs: 4096 x 14336 of K = 128 takes 31 us in wide tiles, 35 with four warps; at K = 256 both take 37 to
-// 39, at 320 four warps are ahead (39 and 47).
+// staging area costs, where a pair has several tiles: 4096 x 14336 of K = 128 takes 26.6 us in wide tiles, 29.8 with four warps, of K = 192
+// 29.7 and 30.2; at K = 256 four are ahead (32.2, 33.1 with eight), over 40 products of K 200 to 256 by 2.5 %.
 constexpr int SHORT_K = 192;
 
 // Whether products may run on CTA pairs at all (B200_GEMM_2CTA).
