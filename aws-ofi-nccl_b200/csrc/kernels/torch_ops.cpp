@@ -107,20 +107,22 @@ PyObject* name_written() {
   return name;
 }
 
+// An attribute, or nothing where there is none; needs the interpreter lock.
+py::object attribute(const py::object& of, PyObject* name) {
+  PyObject* v = PyObject_GetAttr(of.ptr(), name);
+  if (!v) {
+    if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw py::error_already_set();
+    PyErr_Clear();
+  }
+  return py::reinterpret_steal<py::object>(v);
+}
+
 // Runs produce(out, accumulate) into weight.main_grad when the parameter has one (and returns an
 // undefined tensor), else into a new tensor of the weight's shape.
 template <class Produce>
 Tensor write_param_grad(const Tensor& weight, Produce produce) {
   Tensor main;
   bool accumulate = false;
-  auto attribute = [](const py::object& of, PyObject* name) {
-    PyObject* v = PyObject_GetAttr(of.ptr(), name);
-    if (!v) {
-      if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw py::error_already_set();
-      PyErr_Clear();
-    }
-    return py::reinterpret_steal<py::object>(v);
-  };
   {
     py::gil_scoped_acquire gil;
     static PyObject* const kMain = interned("main_grad");
@@ -368,6 +370,19 @@ struct SwiGLUMLP : public Function<SwiGLUMLP> {
   }
 };
 
+// Whether the gradient that comes into the cross-entropy's backward pass is taken for one: `assume_unit_grad` of the Python class, which a
+// program may clear at any time before the backward pass.
+bool unit_grad_assumed() {
+  py::gil_scoped_acquire gil;
+  static PyObject* const module = py::module_::import("aws_ofi_nccl_b200.ops.llm").release().ptr();
+  static PyObject *const cls_name = interned("_CrossEntropy"), *const flag_name = interned("assume_unit_grad");
+  const py::object cls = attribute(py::reinterpret_borrow<py::object>(module), cls_name);
+  const py::object flag = cls ? attribute(cls, flag_name) : py::object();
+  const int truth = flag ? PyObject_IsTrue(flag.ptr()) : 1;
+  if (truth < 0) throw py::error_already_set();
+  return truth == 1;
+}
+
 // Mean cross-entropy of a matrix of logits, which are overwritten with its gradient: the backward pass hands them on. In Python this was
 // 60 us of a forward and backward pass, 30 here: a head of 300 x 512 x 4096 takes 97 us for 130, the two-layer model of 256 channels on
 // 256 tokens 860 for 970 (three processes of each in turn, within 5 %).
@@ -393,7 +408,9 @@ struct CrossEntropy : public Function<CrossEntropy> {
       const Tensor dlogits = ctx->get_saved_variables()[0];
       if (grads[1].defined())
         raise(PyExc_RuntimeError, "cross_entropy overwrites its logits with their gradient: nothing can be differentiated through them afterwards");
-      return {grads[0].defined() ? dlogits : Tensor(), Tensor()};
+      if (!grads[0].defined()) return {Tensor(), Tensor()};   // the loss was not differentiated
+      // the gradient is one in a training loop: no pass over all logits for it
+      return {unit_grad_assumed() ? dlogits : dlogits * grads[0], Tensor()};
     });
   }
 };

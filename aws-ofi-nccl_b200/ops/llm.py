@@ -63,10 +63,9 @@ def rope_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, seq: int) -> to
 
 
 class _CrossEntropy(torch.autograd.Function):
-    """Mean token cross-entropy.  The logits tensor is overwritten with its own gradient in the
-    forward pass (one fused kernel), so backward only rescales by the incoming scalar.  What ``cross_entropy`` is
-    while torch.jit.trace records it (which refuses it: it overwrites its input), and for programs that clear
-    ``assume_unit_grad``; otherwise it is native."""
+    """What ``cross_entropy`` is while torch.jit.trace records it (which refuses it: it overwrites its input); otherwise it is native.
+    ``assume_unit_grad``, which the native one reads as well when its backward pass runs, says whether the incoming scalar is
+    taken for one; cleared, the logits' gradient is multiplied by it."""
 
     @staticmethod
     def forward(ctx, logits, targets):
@@ -96,7 +95,11 @@ class _CrossEntropy(torch.autograd.Function):
 
 
 def cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
-    if torch._C._get_tracing_state() is not None or not getattr(_CrossEntropy, "assume_unit_grad", True):
+    """Mean token cross-entropy of a [rows, classes] matrix. The logits are overwritten with the gradient of the loss in the forward
+    pass (one fused kernel) and the backward pass hands them on as they are: it takes the gradient that comes in for one, so
+    ``(loss / n).backward()`` gives the gradients of ``loss``. A program that scales or weights its loss clears
+    ``_CrossEntropy.assume_unit_grad`` before the backward pass; the gradient is then multiplied, a pass over all logits."""
+    if torch._C._get_tracing_state() is not None:
         return _CrossEntropy.apply(logits, targets)[0]
     return _lib.native().cross_entropy(logits, targets)[0]
 

@@ -345,6 +345,26 @@ def test_the_cross_entropy_is_the_same_inside_and_outside_of_python():
 
 
 @pytest.mark.gpu
+def test_the_cross_entropy_reads_its_switch_in_the_backward_pass(monkeypatch):
+    """Cleared between the passes, the incoming scalar counts; set again before the backward pass, it does not."""
+    from aws_ofi_nccl_b200.ops import llm
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    leaf = torch.randn(40, 96, device="cuda", generator=g).bfloat16().requires_grad_(True)
+    targets = torch.randint(0, 96, (40,), device="cuda", generator=g)
+
+    def gradient(before, between):
+        monkeypatch.setattr(llm._CrossEntropy, "assume_unit_grad", before, raising=False)
+        loss = llm.cross_entropy(leaf * 1.0, targets)
+        monkeypatch.setattr(llm._CrossEntropy, "assume_unit_grad", between, raising=False)
+        return torch.autograd.grad(loss * 4, leaf)[0]   # a power of two: nothing is rounded
+
+    unit = gradient(True, True)
+    assert torch.equal(gradient(True, False), unit * 4) and torch.equal(gradient(False, False), unit * 4)
+    assert torch.equal(gradient(False, True), unit)
+
+
+@pytest.mark.gpu
 def test_a_traced_cross_entropy_is_refused():
     """What torch.jit.trace records of a function that overwrites its input does not run."""
     from aws_ofi_nccl_b200.ops import llm
