@@ -17,6 +17,7 @@
 #include <torch/library.h>
 
 #include <atomic>
+#include <climits>
 
 #include "b200ops.h"
 
@@ -392,6 +393,11 @@ struct CrossEntropy : public Function<CrossEntropy> {
     const int64_t T = logits.size(0), V = logits.size(1);
     require(logits.stride(1) == 1, "the logits have contiguous rows");
     if (T == 0) raise(PyExc_ZeroDivisionError, "the mean of no rows");
+    require(bf16_cuda(logits), "the logits are a bfloat16 CUDA tensor");
+    require(targets.scalar_type() == at::kLong && targets.is_contiguous() && targets.numel() >= T &&
+                (targets.device() == logits.device() || targets.is_pinned()),
+            "the targets are contiguous 64-bit integers that the GPU can read, one for every row");
+    require(T <= INT_MAX && V <= INT_MAX, "rows and columns are numbers of 32 bits");
     const Tensor loss = at::empty({T}, logits.options().dtype(at::kFloat));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     check(b200_cross_entropy(logits.data_ptr(), static_cast<const long long*>(targets.data_ptr()), loss.data_ptr<float>(), static_cast<int>(T),

@@ -71,9 +71,13 @@ class _CrossEntropy(torch.autograd.Function):
     def forward(ctx, logits, targets):
         T, V = logits.shape
         assert logits.stride(1) == 1
+        scale = 1.0 / T
+        assert logits.is_cuda and logits.dtype == torch.bfloat16
+        assert (targets.dtype == torch.int64 and targets.is_contiguous() and targets.numel() >= T
+                and (targets.device == logits.device or targets.is_pinned()))
         loss = torch.empty(T, device=logits.device, dtype=torch.float32)
         _lib.check(_lib.load().b200_cross_entropy(logits.data_ptr(), targets.data_ptr(), loss.data_ptr(), T, V,
-                                                  logits.stride(0), 1.0 / T, _lib.stream_ptr()), "cross_entropy")
+                                                  logits.stride(0), scale, _lib.stream_ptr()), "cross_entropy")
         ctx.save_for_backward(logits)
         ctx.mark_dirty(logits)
         # nobody differentiates through the overwritten logits: no zero-filled [T, V] gradient for them

@@ -344,6 +344,35 @@ def test_the_cross_entropy_is_the_same_inside_and_outside_of_python():
     assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
+def _cross_entropies():
+    from aws_ofi_nccl_b200.ops import llm
+
+    return llm.cross_entropy, lambda *a: llm._CrossEntropy.apply(*a)[0]
+
+
+def test_the_cross_entropy_refuses_what_its_kernel_cannot_read():
+    """Nothing here is on a GPU; what lies on one is tested below."""
+    targets = torch.zeros(4, dtype=torch.int64)
+    for fn in _cross_entropies():
+        for logits in (torch.zeros(4, 16, dtype=torch.bfloat16), torch.zeros(4, 16)):
+            with pytest.raises(AssertionError):
+                fn(logits, targets)
+
+
+@pytest.mark.gpu
+def test_the_cross_entropy_refuses_other_types_and_targets():
+    """Before anything is launched: the logits stay as they are."""
+    logits, targets = torch.ones(8, 16, device="cuda").bfloat16(), torch.arange(8, device="cuda")
+    for fn in _cross_entropies():
+        for x, t in ((logits.float(), targets), (logits.half(), targets), (logits, targets.int()), (logits, targets.float()),
+                     (logits, targets[:7]), (logits, torch.arange(16, device="cuda")[::2]), (logits, targets.cpu())):
+            with pytest.raises(AssertionError):
+                fn(x, t)
+            assert (x == 1).all()
+        for t in (targets.view(2, 4), torch.arange(9, device="cuda"), targets.cpu().pin_memory()):   # one for every row
+            assert fn(logits.clone(), t).isfinite()
+
+
 @pytest.mark.gpu
 def test_the_cross_entropy_reads_its_switch_in_the_backward_pass(monkeypatch):
     """Cleared between the passes, the incoming scalar counts; set again before the backward pass, it does not."""
