@@ -108,12 +108,8 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if ((rc = make_tmap_out<OutT>(&tmC, C, M, N, ldc))) return rc;
   GemmShape shape{M, N, K, (M + GEMM_BM - 1) / GEMM_BM, (N + BN - 1) / BN};
   shape.group_m = gemm_group_m(BN);
-  auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, OutT>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL_EPI));
-    attr_set = true;
-  }
+  constexpr auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, OutT>;
+  if ((rc = allow_smem<kern>(GemmSmem<BN>::TOTAL_EPI))) return rc;
   int grid = shape.tiles_m * shape.tiles_n;
   int cap = sm_count();
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
@@ -176,12 +172,8 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
     rc = make_tmap_2d(&tmB, B, K, N, ldb, GEMM_BK, 64, 2, true);
   if (rc) return rc;
   if ((rc = make_tmap_out<OutT>(&tmC, C, M, N, ldc))) return rc;
-  auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, OutT, EW>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL_EPI));
-    attr_set = true;
-  }
+  constexpr auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, OutT, EW>;
+  if ((rc = allow_smem<kern>(S::TOTAL_EPI))) return rc;
   int* err = device_status_word();
   launch_dependent(kern, grid, S::THREADS, S::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
@@ -237,12 +229,8 @@ static int launch_gemm_fp8(const void* A, const void* B, const float* a_scale, c
   rc = make_tmap_2d(&tmB, B, N, K, ldb, shape.b_box, 2 * GEMM_BK, 1, true);
   if (rc) return rc;
   if ((rc = make_tmap_out<__nv_bfloat16>(&tmC, C, M, N, ldc))) return rc;
-  auto kern = gemm_fp8_2cta_kernel<BN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
-    attr_set = true;
-  }
+  constexpr auto kern = gemm_fp8_2cta_kernel<BN>;
+  if ((rc = allow_smem<kern>(Gemm2Smem<BN>::TOTAL_EPI))) return rc;
   launch_dependent(kern, grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<__nv_bfloat16*>(C), ldc, a_scale, b_scale,
                                                                      shape, device_status_word());
   B200_CUDA_OK(cudaGetLastError());

@@ -1,6 +1,5 @@
 // The gradients of a linear layer: one launch for both products or one for each, and the plan that decides.
 #include <algorithm>
-#include <atomic>
 
 #include "b200ops.h"
 #include "gemm_grads.cuh"
@@ -135,12 +134,8 @@ int launch(const GradsCall& c, const GradsPlan& p, cudaStream_t stream) {
   a.accumulate = c.accumulate;
   a.first = p.first;
   a.fill = p.fill;
-  auto kern = gemm_grads_kernel<EW>;
-  static std::atomic<bool> attr_set{false};
-  if (!attr_set.load(std::memory_order_acquire)) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL_EPI));
-    attr_set.store(true, std::memory_order_release);
-  }
+  constexpr auto kern = gemm_grads_kernel<EW>;
+  if ((rc = allow_smem<kern>(S::TOTAL_EPI))) return rc;
   const int pairs = sm_count() / 2;
   const int grid = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
   launch_dependent(kern, grid, S::THREADS, S::TOTAL_EPI, stream, rows, cols, w, x, dx, dw, a, device_status_word());

@@ -40,12 +40,8 @@ int launch(const SplitkCall& c, int slices, cudaStream_t stream) {
             : make_tmap_2d(&tmB, c.B, c.N, c.K, c.ldb, PAIR ? BN / 2 : BN, GEMM_BK, 2, true);
   if (rc) return rc;
   GemmShape shape{c.M, c.N, c.K, (c.M + BM - 1) / BM, (c.N + BN - 1) / BN};
-  auto kern = gemm_splitk_kernel<PAIR, A_MN, B_MN, OutT>;
-  static std::atomic<bool> attr_set{false};
-  if (!attr_set.load(std::memory_order_acquire)) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitkSmem<PAIR>::TOTAL));
-    attr_set.store(true, std::memory_order_release);
-  }
+  constexpr auto kern = gemm_splitk_kernel<PAIR, A_MN, B_MN, OutT>;
+  if ((rc = allow_smem<kern>(SplitkSmem<PAIR>::TOTAL))) return rc;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = config<PAIR>(attr, shape.tiles_m * shape.tiles_n, slices, stream);
   B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, static_cast<OutT*>(c.C), static_cast<int64_t>(c.ldc), shape, slices,
@@ -68,7 +64,7 @@ int resident_clusters(int log2_slices) {
   static std::atomic<int> known[4] = {{-1}, {-1}, {-1}, {-1}};
   int n = known[log2_slices].load(std::memory_order_relaxed);
   if (n >= 0) return n;
-  auto kern = gemm_splitk_kernel<PAIR, false, false, __nv_bfloat16>;
+  constexpr auto kern = gemm_splitk_kernel<PAIR, false, false, __nv_bfloat16>;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = config<PAIR>(attr, 1, 1 << log2_slices, nullptr);
   n = 0;

@@ -64,8 +64,8 @@ static int launch_swiglu(const void* x, const void* w, void* gu, void* act, int 
   if ((rc = make_tmap_2d(&tmGate, g, M, F, 2 * static_cast<uint64_t>(F), 32, 64, 2, true))) return rc;
   if ((rc = make_tmap_2d(&tmUp, g + F, M, F, 2 * static_cast<uint64_t>(F), 32, 64, 2, true))) return rc;
   if ((rc = make_tmap_2d(&tmAct, act, M, F, F, 32, 64, 2, true))) return rc;
-  auto kern = gemm_swiglu_kernel<BN>;
-  B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem<BN>::TOTAL_EPI));
+  constexpr auto kern = gemm_swiglu_kernel<BN>;
+  if ((rc = allow_smem<kern>(Gemm2Smem<BN>::TOTAL_EPI))) return rc;
   launch_dependent(kern, grid, GEMM_THREADS, Gemm2Smem<BN>::TOTAL_EPI, stream, tmA, tmB, tmGate, tmUp, tmAct, shape, F, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
   return 0;
@@ -85,8 +85,8 @@ static int launch_swiglu_bwd(const void* dy, const void* w, const void* gu, void
     const __nv_bfloat16* base = static_cast<const __nv_bfloat16*>(i < 2 ? gu : dgu) + (i & 1) * F;
     if ((rc = make_tmap_2d(&tm[i], base, M, F, 2 * static_cast<uint64_t>(F), 32, 64, 2, true))) return rc;
   }
-  auto kern = gemm_swiglu_bwd_kernel<BN>;
-  B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL_EPI));
+  constexpr auto kern = gemm_swiglu_bwd_kernel<BN>;
+  if ((rc = allow_smem<kern>(S::TOTAL_EPI))) return rc;
   launch_dependent(kern, grid, S::THREADS, S::TOTAL_EPI, stream, tmA, tmB, tm[0], tm[1], tm[2], tm[3], shape, device_status_word());
   B200_CUDA_OK(cudaGetLastError());
   return 0;

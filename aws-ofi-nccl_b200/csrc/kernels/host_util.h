@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include "per_device.h"
+
 namespace b200 {
 
 #define B200_CUDA_OK(expr)                                                                      \
@@ -93,6 +95,19 @@ inline void ensure_context() {
 
 // Per-device status word that kernels write on a bounded-wait timeout. Allocated once per device.
 int* device_status_word();
+
+// Lets KERNEL have `bytes` of dynamic shared memory on the current device, and returns 0 on success. The runtime keeps that limit for each device by
+// itself. `bytes` is the same in every call for a KERNEL.
+template <auto KERNEL>
+int allow_smem(int bytes) {
+  static OncePerDevice once;
+  int dev = -1;
+  B200_CUDA_OK(cudaGetDevice(&dev));
+  return once.run(dev, [&]() -> int {
+    B200_CUDA_OK(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    return 0;
+  });
+}
 
 inline int sm_count() {
   static int n[16] = {0};

@@ -6,7 +6,6 @@
 #include <float.h>
 #include <stdint.h>
 
-#include <atomic>
 #include <type_traits>
 
 #include "b200ops.h"
@@ -1031,18 +1030,11 @@ static inline int grid_for(int64_t work_items, int threads, int per_sm = 16) {
   return static_cast<int>(b);
 }
 
+constexpr int NORM_RING_SMEM = 112 * 1024;   // what a ring takes at most
 // Slots of `bytes` for each of `ctas` CTAs of an SM (228 KB, of which a CTA's own part takes 1 KB and the kernels' other arrays less than that).
 static int norm_slots(int bytes, int ctas) {
   const int n = bytes > 0 ? (228 / ctas - 3) * 1024 / bytes : 0;
   return n < NORM_MAX_SLOTS ? n : NORM_MAX_SLOTS;
-}
-template <auto KERNEL>
-static int norm_smem() {   // once per kernel
-  static std::atomic<bool> set{false};
-  if (set.load(std::memory_order_acquire)) return 0;
-  B200_CUDA_OK(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
-  set.store(true, std::memory_order_release);
-  return 0;
 }
 
 // 32-bit indices hold while a grid's last pass, beyond the last item, stays below 2^32. What they gain is their divisions: rotary split of
@@ -1086,7 +1078,7 @@ int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w,
     const int groups = (T + R - 1) / R, ctas = sm_count() * NORM_RING_CTAS;                                                  \
     const int slot = R * H * 2 * (RES ? 2 : 1), slots = norm_slots(slot, NORM_RING_CTAS);                                     \
     if (groups > ctas && slots >= 2) {                                                                                       \
-      const int rc = norm_smem<rmsnorm_fwd_ring_kernel<TPR, VPT>>();                                                           \
+      const int rc = allow_smem<rmsnorm_fwd_ring_kernel<TPR, VPT>>(NORM_RING_SMEM);                                                         \
       if (rc) return rc;                                                                                                     \
       launch_dependent(rmsnorm_fwd_ring_kernel<TPR, VPT>, ctas, NORM_THREADS, slots * slot, s, X, RES, HO, W, Y, rstd, T, H, eps, slots, \
                        device_status_word());                                                                                \
@@ -1121,7 +1113,7 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
     const int groups = (T + R - 1) / R;                                                                                      \
     const int parts = (R - 1) * TPR * VPT * 8 * 4, slot = R * H * 2 * (DR ? 3 : 2), slots = norm_slots(slot, 2);               \
     if (groups > grid && slots >= 3) {                                                                                       \
-      const int rc = norm_smem<rmsnorm_bwd_ring_kernel<TPR, VPT>>();                                                           \
+      const int rc = allow_smem<rmsnorm_bwd_ring_kernel<TPR, VPT>>(NORM_RING_SMEM);                                                         \
       if (rc) return rc;                                                                                                     \
       launch_dependent(rmsnorm_bwd_ring_kernel<TPR, VPT>, grid, NORM_THREADS, slots * slot > parts ? slots * slot : parts, s, DY, X, W, rstd, \
                        DR, DX, dw_partial, T, H, slots, device_status_word());                                               \
@@ -1240,11 +1232,8 @@ int b200_cross_entropy(void* logits, const long long* targets, float* loss, int 
   if (ce_two_passes(T, V)) {
     launch_dependent(cross_entropy_two_pass_kernel, T, CE_THREADS, 0, st, L, TG, loss, V, ld, grad_scale);
   } else {
-    static std::atomic<bool> attr_set{false};
-    if (!attr_set.load(std::memory_order_acquire)) {
-      B200_CUDA_OK(cudaFuncSetAttribute(cross_entropy_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CES_SMEM));
-      attr_set.store(true, std::memory_order_release);
-    }
+    const int rc = allow_smem<cross_entropy_stream_kernel>(CES_SMEM);
+    if (rc) return rc;
     launch_dependent(cross_entropy_stream_kernel, T < sm_count() ? T : sm_count(), CES_THREADS, CES_SMEM, st, L, TG, loss, T, V, ld,
                      grad_scale, device_status_word());
   }
