@@ -10,6 +10,7 @@
 #include <cuda_fp8.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "b200ops.h"
 #include "gemm_epilogues.cuh"
@@ -21,16 +22,20 @@
 
 namespace b200 {
 
+// Part of the library's image, zero when that is loaded: a first call may come while a stream is being captured, where nothing may be
+// allocated or set, and from several threads at once.
+__device__ int g_status_word;
+
 int* device_status_word() {
-  static int* words[16] = {nullptr};
-  int dev = 0;
+  static std::atomic<int*> words[64];
+  int dev = -1;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16) dev = 0;
-  if (!words[dev]) {
-    if (cudaMalloc(&words[dev], 256) != cudaSuccess) return nullptr;
-    cudaMemset(words[dev], 0, 256);
-  }
-  return words[dev];
+  const bool known = dev >= 0 && dev < 64;
+  if (int* w = known ? words[dev].load(std::memory_order_acquire) : nullptr) return w;
+  void* w = nullptr;
+  if (cudaGetSymbolAddress(&w, g_status_word) != cudaSuccess) return nullptr;
+  if (known) words[dev].store(static_cast<int*>(w), std::memory_order_release);
+  return static_cast<int*>(w);
 }
 
 // C as the epilogues store it: boxes of 32 rows x 128 bytes. A store clips a row at 16 bytes, not at an

@@ -93,7 +93,7 @@ inline void ensure_context() {
   }
 }
 
-// Per-device status word that kernels write on a bounded-wait timeout. Allocated once per device.
+// Status word of the current device, which kernels write when a bounded wait gives up.
 int* device_status_word();
 
 // Lets KERNEL have `bytes` of dynamic shared memory on the current device, and returns 0 on success. The runtime keeps that limit for each device by

@@ -1,5 +1,9 @@
 """Kernels that start while the one before them ends: a chain of them, each reading what the one before has just written into
 buffers that are used again and again, gives the same bits as one that is waited for after every call."""
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -87,3 +91,37 @@ def test_a_captured_chain_does_too(T, H, F):
     torch.cuda.synchronize()
     for a, b in zip(waited.results(), captured.results()):
         assert torch.equal(a, b)
+
+
+FIRST_CALL = """
+import torch
+from aws_ofi_nccl_b200.ops import _lib
+from aws_ofi_nccl_b200.ops.gemm import gemm
+bf = dict(device="cuda", dtype=torch.bfloat16)
+x, y, w, rstd = torch.ones(%(T)d, %(W)d, **bf), torch.zeros(%(T)d, %(W)d, **bf), torch.ones(%(W)d, **bf), torch.zeros(%(T)d, device="cuda")
+targets, loss, sq = torch.zeros(%(T)d, device="cuda", dtype=torch.int64), torch.zeros(%(T)d, device="cuda"), torch.zeros(%(T)d, %(T)d, **bf)
+lib, p = _lib.load(), lambda t: t.data_ptr()
+calls = {
+    "norm": lambda s: lib.b200_rmsnorm_fwd(p(x), None, None, p(w), p(y), p(rstd), %(T)d, %(W)d, 0.0, s),
+    "cross_entropy": lambda s: lib.b200_cross_entropy(p(x), p(targets), p(loss), %(T)d, %(W)d, %(W)d, 1.0, s),
+    "product": lambda s: int(gemm(x, x, out=sq) is not sq),
+}
+torch.cuda.synchronize()
+stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph, stream=stream):
+    assert calls["%(name)s"](stream.cuda_stream) == 0
+graph.replay()
+torch.cuda.synchronize()
+result = {"norm": y, "cross_entropy": loss, "product": sq}["%(name)s"]
+want = {"norm": 1.0, "cross_entropy": torch.tensor(%(W)d, dtype=torch.float64).log().item(), "product": %(W)d}["%(name)s"]
+assert ((result.double() - want).abs() <= 2.0 ** -8 * want).all(), result
+assert _lib.read_status() == 0
+"""
+
+
+# rows that come through rings of shared memory, and a product
+@pytest.mark.parametrize("name,T,W", [("norm", 2400, 8192), ("cross_entropy", 300, 32776), ("product", 512, 256)])
+def test_a_process_whose_first_call_is_captured(name, T, W):
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL % {"name": name, "T": T, "W": W}], capture_output=True, text=True, timeout=300,
+                       cwd=Path(__file__).resolve().parent.parent)
+    assert r.returncode == 0, r.stderr[-3000:]
