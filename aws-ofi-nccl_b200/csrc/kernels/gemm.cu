@@ -95,6 +95,10 @@ void plan_walk(GemmShape& s, int elem_bytes) {
   }
 }
 
+// max_ctas keeps SMs free for other streams. Such a product is launched when the kernel before it has ended, and releases none before it ends itself: the
+// CTAs of a dependent, which come up wherever there is room, would hold those SMs.
+static bool keeps_room(int max_ctas) { return max_ctas > 0 && max_ctas < sm_count(); }
+
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
                        int64_t ldc, int accumulate, int max_ctas, cudaStream_t stream) {
@@ -116,11 +120,11 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   constexpr auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, OutT>;
   if ((rc = allow_smem<kern>(GemmSmem<BN>::TOTAL_EPI))) return rc;
   int grid = shape.tiles_m * shape.tiles_n;
-  int cap = sm_count();
-  if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
+  shape.keep_room = keeps_room(max_ctas);
+  const int cap = shape.keep_room ? max_ctas : sm_count();
   if (grid > cap) grid = cap;
   int* err = device_status_word();
-  launch_dependent(kern, grid, GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
+  launch_after(!shape.keep_room, kern, grid, GEMM_THREADS, GemmSmem<BN>::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -162,9 +166,8 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
   CUtensorMap tmA, tmB, tmC;
   int rc;
   GemmShape shape{M, N, K, 0, 0};
-  int cap = sm_count();
-  if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
-  const int grid = pair_grid(shape, tiles, BN, cap);
+  shape.keep_room = keeps_room(max_ctas);
+  const int grid = pair_grid(shape, tiles, BN, shape.keep_room ? max_ctas : sm_count());
   // every CTA loads 128 rows of A and its half of the tile's rows of B per k-block
   if (!A_MN)
     rc = make_tmap_2d(&tmA, A, M, K, lda, 128, GEMM_BK, 2, true);
@@ -180,7 +183,7 @@ static int launch_gemm_2cta(const void* A, const void* B, void* C, int M, int N,
   constexpr auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, OutT, EW>;
   if ((rc = allow_smem<kern>(S::TOTAL_EPI))) return rc;
   int* err = device_status_word();
-  launch_dependent(kern, grid, S::THREADS, S::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
+  launch_after(!shape.keep_room, kern, grid, S::THREADS, S::TOTAL_EPI, stream, tmA, tmB, tmC, static_cast<OutT*>(C), ldc, shape, accumulate, err);
   B200_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -203,7 +206,7 @@ static int gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K,
     return out_fp32 ? dispatch_major_2cta<128, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
                     : dispatch_major_2cta<128, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
   const int64_t all = static_cast<int64_t>((M + GEMM2_BM - 1) / GEMM2_BM) * ((N + tiles.width - 1) / tiles.width);
-  const int pairs = (max_ctas > 0 && max_ctas < sm_count() ? max_ctas : sm_count()) / 2;
+  const int pairs = (keeps_room(max_ctas) ? max_ctas : sm_count()) / 2;
   if (K <= SHORT_K && !out_fp32 && all > pairs)
     return dispatch_major_2cta<256, __nv_bfloat16, 8>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
   return out_fp32 ? dispatch_major_2cta<256, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)

@@ -41,6 +41,7 @@ struct GemmShape {
   int n_rot = 0;       // tile_n = (raw + n_rot) % tiles_n
   int group_m = 0;     // default order only: M tiles are walked in groups of this many (0 = all)
   int one_group = 0;   // 1: all M tiles are one group, whatever group_m says (plan_walk)
+  int keep_room = 0;   // 1: no CTA of the next kernel comes up on the SMs that this one leaves free
   // CTA pairs only, see TileSpan:
   int bn = 0;               // columns of a tile (0 = the kernel's BN)
   int halve_from = 1 << 30; // tiles from this number on are computed as two halves
@@ -173,7 +174,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
           }
         }
       }
-      grid_release();   // what is left are the last stages' products and the last stores
+      if (!shape.keep_room) grid_release();   // what is left are the last stages' products and the last stores
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer

@@ -235,7 +235,7 @@ __device__ __forceinline__ void gemm_mainloop_2cta(const CUtensorMap* tmA, const
           }
         }
       }
-      grid_release();   // what is left are the last stages' products and the last stores
+      if (!shape.keep_room) grid_release();   // what is left are the last stages' products and the last stores
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)

@@ -1,5 +1,6 @@
 """Kernels that start while the one before them ends: a chain of them, each reading what the one before has just written into
 buffers that are used again and again, gives the same bits as one that is waited for after every call."""
+import ctypes
 import subprocess
 import sys
 from pathlib import Path
@@ -125,3 +126,62 @@ def test_a_process_whose_first_call_is_captured(name, T, W):
     r = subprocess.run([sys.executable, "-c", FIRST_CALL % {"name": name, "T": T, "W": W}], capture_output=True, text=True, timeout=300,
                        cwd=Path(__file__).resolve().parent.parent)
     assert r.returncode == 0, r.stderr[-3000:]
+
+
+def _programmatic(calls):
+    """Of kernels captured one after the other: whether each after the first may come up before the one before it has ended."""
+    graph, stream = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=stream):
+        for call in calls:
+            call()
+    driver, raw, n = ctypes.CDLL("libcuda.so.1"), ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(len(calls))
+    start, to, data = (ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)(), (ctypes.c_uint8 * 8 * n.value)()
+    assert driver.cuGraphGetEdges_v2(raw, start, to, data, ctypes.byref(n)) == 0 and n.value == len(calls) - 1
+    after = {a: (b, kind[2] == 1) for a, b, kind in zip(start, to, data) if a}   # ports of both ends, then the edge's type
+    at, = set(after) - {b for b, _ in after.values()}
+    out = []
+    while at in after:
+        at, early = after[at]
+        out.append(early)
+    return out
+
+
+@pytest.mark.parametrize("M,N", [(512, 1024), (128, 512)])   # CTA pairs, single CTAs
+def test_a_product_that_leaves_room_is_launched_when_the_kernel_before_has_ended(M, N):
+    from aws_ofi_nccl_b200.ops.gemm import gemm
+
+    a, b, out = (torch.zeros(*s, device="cuda", dtype=torch.bfloat16) for s in ((M, 256), (N, 256), (M, N)))
+    product = [lambda c=c: gemm(a, b, out=out, max_ctas=c) for c in (0, 0, 100, 100, 2, 148, 0)]
+    product[0]()   # what a first call sets up
+    assert _programmatic(product) == [True, False, False, False, True, True]
+
+
+def test_room_that_a_product_leaves_is_there_for_another_stream():
+    """Products on 74 SMs beside a chain of products that leaves these free take about as long as by themselves (16 us, 72 beside
+    a chain that leaves none)."""
+    from aws_ofi_nccl_b200.ops.gemm import gemm
+
+    big, small = (torch.randn(n, n, device="cuda").bfloat16() for n in (2048, 1024))
+    outs = [torch.empty_like(big), torch.empty_like(small)]
+    chain, side = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def times(products):
+        events = [[torch.cuda.Event(enable_timing=True) for _ in range(2)] for _ in range(40)]
+        torch.cuda._sleep(4_000_000)   # everything is queued before anything runs
+        for s in (chain, side):
+            s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(chain):
+            for _ in range(products):
+                gemm(big, big, out=outs[0], max_ctas=74)
+        with torch.cuda.stream(side):
+            for begin, end in events:
+                begin.record()
+                gemm(small, small, out=outs[1], max_ctas=74)
+                end.record()
+        torch.cuda.synchronize()
+        return sorted(b.elapsed_time(e) for b, e in events)
+
+    times(1)
+    alone, beside = times(0), times(60)
+    assert beside[20] < 2 * alone[20] and beside[-1] < 3 * alone[20]
+    assert all(torch.equal(o, gemm(x, x)) for o, x in zip(outs, (big, small)))
