@@ -285,10 +285,9 @@ __global__ void __launch_bounds__(NORM_THREADS, 2)
 
 // ---- The same for many rows: a persistent CTA's rows come through a ring of shared memory, groups of 256 / TPR of them at a time, by bulk
 // copies that one thread issues as soon as a group has been read. With loads into registers nothing of a CTA's next row is in flight
-// while it reduces (forward), or one row (backward): 16384 x 4096 forward 63 -> 48 us (5.6 TB/s), backward 86 -> 79; 4096 x 4096
-// with a residual 26.9 -> 25.3 and 31.5 -> 29.4 with the sum of the partial rows; 1000 x 2048 forward 6.8 -> 5.5. The weight is read once
-// per CTA instead of once per row. A CTA with one group has nothing to read ahead: those are left to the kernels above
-// (256 x 256 backward 5.7 us, 6.4 so), and so are rows of which a ring holds less than three in the backward pass (2048 x 8192 34.6, 35.3).
+// while it reduces (forward), or one row (backward): 16384 x 4096 forward 62 -> 48 us (5.6 TB/s), backward 86 -> 77; 4096 x 4096
+// with a residual 27.0 -> 26.0 and 31.7 -> 29.9 with the sum of the partial rows. The weight is read once
+// per CTA instead of once per row. What it costs is a barrier of the CTA for every group: norm_ring_slots has where that pays.
 struct NormRing {
   uint32_t ring, bars;       // shared memory: slots, and a barrier for each
   int slots, slot;
@@ -1037,6 +1036,38 @@ static int norm_slots(int bytes, int ctas) {
   return n < NORM_MAX_SLOTS ? n : NORM_MAX_SLOTS;
 }
 
+// Slots of the ring that T rows of H elements come through, of 256 / tpr rows each, or none where the kernels without one are as fast. A CTA with one group
+// has nothing to read ahead. The lines below lie between those of 1394 pairs of times (330 to 262144 rows of 54 widths from 8 to 8192, up to 2^27
+// elements, both kernels in one process, memory cold) where the ring gains and those where it loses, 0.75 to 1.5 of the time:
+// - a group of a few hundred elements costs more in its barrier than in its loads (65536 x 64 forward 15.1 us for 12.9, backward 31.6 for 25.2);
+// - a ring has to turn some times to gain (1500 x 2048 forward 5.3 for 4.6, 16384 x 2048 28 for 33), and rows that leave a quarter of the
+//   threads' registers empty or more are bound by their groups' latency, which a ring makes longer (12000 x 2304 backward 64 us for 59);
+// - with a residual many rows are bound by memory, and a ring's are slower there (4096 x 4096 26.0 for 27.0, 16384 x 4096 100 for 94) but for rows
+//   that fill half of the threads (65536 x 1032 96 for 108);
+// - backward rows wider than 4096 are not loaded ahead without a ring (4096 x 5120 34 for 41), narrower ones are (16384 x 2048 43 for 48, 4096 x 2048
+//   17.9 for 17.1), and a fourth vector of a thread costs both more.
+// What the rule takes is 1.002 of the better one's time on average forward, 1.003 with a residual, 1.001 and 1.002 backward, and at worst 1.09 (2200 x 1000); no rings
+// would be 1.02 to 1.06, rings wherever there are two groups for a CTA 1.04 to 1.06. At 888 other sizes, which it was not drawn by, it is 1.005, 1.006, 1.001 and
+// 1.003, at worst 1.12 (500 x 3400 with a residual 6.1 us for 5.5), no rings 1.02 to 1.06.
+static int norm_ring_slots(int64_t T, int H, int tpr, int vpt, bool res, bool backward) {
+  const int rows = NORM_THREADS / tpr, per_sm = backward ? 2 : NORM_RING_CTAS, room = tpr * vpt * 8;   // elements that a group's registers hold of a row
+  const int slots = norm_slots(rows * H * 2 * (1 + backward + res), per_sm);
+  if ((T + rows - 1) / rows <= sm_count() * per_sm || slots < (backward ? 3 : 2)) return 0;
+  const int64_t millions = T * H / 1000000;
+  const bool full = 8 * H >= 7 * room, half = 16 * H <= 9 * room;
+  bool pays;
+  if (backward)
+    pays = H > 6144 ? millions >= (full ? 8 : 20) : H > 4096 ? true : full ? H >= 512 && millions >= (H < 896 ? 25 : 16)
+                                                                            : H >= 640 && 16 * H >= 11 * room && millions >= 50;
+  else if (!res)
+    pays = H >= 256 && millions >= (H > 2048 && H <= 4096 ? 16 : 6);
+  else if (H > 4096)
+    pays = millions >= 5 && millions < 20;
+  else
+    pays = full ? H >= 448 && millions < 20 : H >= 256 && half && millions >= 16;
+  return pays ? slots : 0;
+}
+
 // 32-bit indices hold while a grid's last pass, beyond the last item, stays below 2^32. What they gain is their divisions: rotary split of
 // 4096 x 48 x 128 22.9 -> 22.2 us, its backward pass 23.8 -> 22.6, 2048 x 12 x 64 4.6 -> 4.2, the embedding's gradient of 4096 x 4096 28.7 -> 24.8.
 static bool small_index(int64_t items) { return items < (1ll << 31); }
@@ -1075,21 +1106,29 @@ int b200_rmsnorm_fwd(const void* x, const void* res, void* h_out, const void* w,
 #define B200_NORM_FWD(TPR, VPT)                                                                                              \
   do {                                                                                                                       \
     constexpr int R = NORM_THREADS / TPR;                                                                                    \
-    const int groups = (T + R - 1) / R, ctas = sm_count() * NORM_RING_CTAS;                                                  \
-    const int slot = R * H * 2 * (RES ? 2 : 1), slots = norm_slots(slot, NORM_RING_CTAS);                                     \
-    if (groups > ctas && slots >= 2) {                                                                                       \
-      const int rc = allow_smem<rmsnorm_fwd_ring_kernel<TPR, VPT>>(NORM_RING_SMEM);                                                         \
+    const int slots = norm_ring_slots(T, H, TPR, VPT, RES, false);                                                           \
+    if (slots) {                                                                                                             \
+      const int rc = allow_smem<rmsnorm_fwd_ring_kernel<TPR, VPT>>(NORM_RING_SMEM);                                          \
       if (rc) return rc;                                                                                                     \
-      launch_dependent(rmsnorm_fwd_ring_kernel<TPR, VPT>, ctas, NORM_THREADS, slots * slot, s, X, RES, HO, W, Y, rstd, T, H, eps, slots, \
-                       device_status_word());                                                                                \
+      launch_dependent(rmsnorm_fwd_ring_kernel<TPR, VPT>, sm_count() * NORM_RING_CTAS, NORM_THREADS,                         \
+                       slots * R * H * 2 * (RES ? 2 : 1), s, X, RES, HO, W, Y, rstd, T, H, eps, slots, device_status_word());\
     } else {                                                                                                                 \
-      launch_dependent(rmsnorm_fwd_kernel<TPR, VPT>, groups, NORM_THREADS, 0, s, X, RES, HO, W, Y, rstd, T, H, eps);           \
+      launch_dependent(rmsnorm_fwd_kernel<TPR, VPT>, (T + R - 1) / R, NORM_THREADS, 0, s, X, RES, HO, W, Y, rstd, T, H, eps);\
     }                                                                                                                        \
   } while (0)
   B200_NORM_DISPATCH(B200_NORM_FWD);
 #undef B200_NORM_FWD
   B200_CUDA_OK(cudaGetLastError());
   return 0;
+}
+
+// Whether the rows of those calls come through a ring of shared memory.
+int b200_rmsnorm_ring(int T, int H, int with_res, int backward) {
+  b200::ensure_context();
+  if (H % 8 || H > NORM_THREADS * 8 * 4) return 0;
+#define B200_NORM_RING(TPR, VPT) return norm_ring_slots(T, H, TPR, VPT, with_res, backward) > 0
+  B200_NORM_DISPATCH(B200_NORM_RING);
+#undef B200_NORM_RING
 }
 
 // Number of fp32 rows the caller must provide in dw_partial.
@@ -1110,16 +1149,17 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
 #define B200_NORM_BWD(TPR, VPT)                                                                                              \
   do {                                                                                                                       \
     constexpr int R = NORM_THREADS / TPR;                                                                                    \
-    const int groups = (T + R - 1) / R;                                                                                      \
-    const int parts = (R - 1) * TPR * VPT * 8 * 4, slot = R * H * 2 * (DR ? 3 : 2), slots = norm_slots(slot, 2);               \
-    if (groups > grid && slots >= 3) {                                                                                       \
-      const int rc = allow_smem<rmsnorm_bwd_ring_kernel<TPR, VPT>>(NORM_RING_SMEM);                                                         \
+    const int slots = norm_ring_slots(T, H, TPR, VPT, DR, true);                                                             \
+    if (slots) {                                                                                                             \
+      const int ring = slots * R * H * 2 * (DR ? 3 : 2), parts = (R - 1) * TPR * VPT * 8 * 4;                                \
+      const int rc = allow_smem<rmsnorm_bwd_ring_kernel<TPR, VPT>>(NORM_RING_SMEM);                                          \
       if (rc) return rc;                                                                                                     \
-      launch_dependent(rmsnorm_bwd_ring_kernel<TPR, VPT>, grid, NORM_THREADS, slots * slot > parts ? slots * slot : parts, s, DY, X, W, rstd, \
-                       DR, DX, dw_partial, T, H, slots, device_status_word());                                               \
+      launch_dependent(rmsnorm_bwd_ring_kernel<TPR, VPT>, grid, NORM_THREADS, ring > parts ? ring : parts, s, DY, X, W, rstd, DR, DX,\
+                       dw_partial, T, H, slots, device_status_word());                                                       \
     } else {                                                                                                                 \
+      const int groups = (T + R - 1) / R;                                                                                    \
       if (grid > groups) grid = groups;                                                                                      \
-      launch_dependent(rmsnorm_bwd_kernel<TPR, VPT>, grid, NORM_THREADS, 0, s, DY, X, W, rstd, DR, DX, dw_partial, T, H);     \
+      launch_dependent(rmsnorm_bwd_kernel<TPR, VPT>, grid, NORM_THREADS, 0, s, DY, X, W, rstd, DR, DX, dw_partial, T, H);    \
     }                                                                                                                        \
   } while (0)
   B200_NORM_DISPATCH(B200_NORM_BWD);

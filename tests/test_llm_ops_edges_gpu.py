@@ -42,8 +42,7 @@ def test_rmsnorm(T, H, with_res):
         assert torch.equal(got[0], got[2])
 
 
-# more groups of rows than CTAs, whose rows come through a ring: eight to one rows in a group, ragged last groups and widths, one group and a row
-# more than the CTAs take at once, several rounds of the ring
+# more groups of rows than CTAs: eight to one rows in a group, ragged last groups and widths, one group and a row more than the CTAs take at once
 @pytest.mark.parametrize("T,H", [(20001, 8), (3553, 64), (3553, 256), (7003, 264), (1777, 520), (889, 2048), (445, 2056), (4001, 4096), (445, 4104),
                                  (1201, 6144), (445, 6152), (1800, 8192)])
 @pytest.mark.parametrize("with_res", [False, True])
@@ -51,6 +50,22 @@ def test_rmsnorm_of_many_rows(T, H, with_res):
     from aws_ofi_nccl_b200.ops import _lib
 
     test_rmsnorm(T, H, with_res)
+    assert _lib.read_status() == 0
+
+
+# rows that come through a ring of shared memory, forward, backward or both: eight to one rows in a group, ragged last groups and widths, every layout
+# of a row, the fewest rows that take it, several rounds of the ring
+@pytest.mark.parametrize("T,H,with_res,forward,backward", [
+    (23441, 256, 0, 1, 0), (22729, 264, 0, 1, 0), (63551, 264, 1, 1, 0), (11721, 512, 0, 1, 0), (4003, 512, 1, 1, 0), (65537, 512, 0, 1, 1),
+    (11539, 520, 0, 1, 0), (3553, 448, 1, 1, 0), (27779, 576, 1, 1, 0), (5861, 1024, 0, 1, 0), (16385, 1024, 1, 1, 1), (16257, 1032, 1, 1, 0), (72675, 704, 1, 0, 1), (16001, 1000, 0, 1, 1), (62501, 800, 0, 1, 1),
+    (2931, 2048, 0, 1, 0), (8193, 2048, 1, 1, 1), (7783, 2056, 0, 1, 0), (16667, 3000, 1, 0, 1), (5571, 3592, 1, 0, 1), (4097, 4096, 0, 1, 1), (4097, 4096, 1, 1, 1),
+    (445, 4096, 1, 1, 0), (297, 4104, 0, 0, 1), (1463, 4104, 0, 1, 1), (1220, 4104, 1, 1, 1), (297, 6144, 1, 0, 1), (977, 6144, 0, 1, 1),
+    (2728, 6152, 1, 1, 0), (3252, 6152, 1, 0, 1), (1115, 7176, 0, 1, 1), (733, 8192, 0, 1, 0), (611, 8192, 1, 1, 0), (2049, 8192, 0, 1, 1)])
+def test_rmsnorm_through_rings(T, H, with_res, forward, backward):
+    from aws_ofi_nccl_b200.ops import _lib
+
+    assert [_lib.load().b200_rmsnorm_ring(T, H, with_res, b) for b in (0, 1)] == [forward, backward]
+    test_rmsnorm(T, H, bool(with_res))
     assert _lib.read_status() == 0
 
 

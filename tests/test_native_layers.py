@@ -126,6 +126,19 @@ def test_rows_of_the_cross_entropy_take_the_faster_way(T, V, ctas):
     assert _lib.load().b200_cross_entropy_ctas(T, V) == ctas
 
 
+@pytest.mark.parametrize("T,H,with_res,backward,ring", [
+    (65536, 64, 0, 0, 0), (65536, 64, 0, 1, 0), (262144, 192, 1, 0, 0), (8192, 128, 0, 0, 0), (65536, 256, 0, 0, 1), (20000, 256, 0, 0, 0), (65536, 256, 0, 1, 0),
+    (1500, 2048, 0, 0, 0), (8192, 2048, 0, 0, 1), (3000, 3072, 0, 0, 0), (8192, 3072, 0, 0, 1), (4096, 4096, 1, 0, 1), (16384, 4096, 1, 0, 0), (16384, 4096, 0, 0, 1),
+    (4096, 640, 1, 0, 0), (65536, 520, 1, 0, 1), (900, 3072, 1, 0, 0), (1500, 5120, 1, 0, 1), (600, 8192, 1, 0, 0),
+    (4096, 2048, 0, 1, 0), (16384, 2048, 0, 1, 1), (16384, 2056, 0, 1, 0), (4096, 4096, 1, 1, 1), (4096, 5120, 0, 1, 1), (296, 4104, 0, 1, 0), (297, 4104, 0, 1, 1),
+    (1500, 6152, 0, 1, 0), (4096, 8192, 0, 1, 1), (4096, 8192, 1, 1, 0), (0, 4096, 0, 0, 0), (1000000, 0, 0, 0, 0), (1000000, 0, 0, 1, 0)])
+def test_rows_of_a_norm_take_the_faster_way(T, H, with_res, backward, ring):
+    """Whether they come through a ring, as measured on 148 SMs on both sides of where that changes."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    assert _lib.load().b200_rmsnorm_ring(T, H, with_res, backward) == ring
+
+
 def test_the_embedding_refuses_what_its_kernel_cannot_read():
     """Nothing here is on a GPU; what lies on one is tested below."""
     from aws_ofi_nccl_b200.ops import llm
