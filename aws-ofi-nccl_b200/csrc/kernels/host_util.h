@@ -97,9 +97,10 @@ inline void ensure_context() {
 int* device_status_word();
 
 // Lets KERNEL have `bytes` of dynamic shared memory on the current device, and returns 0 on success. The runtime keeps that limit for each device by
-// itself. `bytes` is the same in every call for a KERNEL.
+// itself. `bytes` is the same in every call for a KERNEL. Static: the linker would give two copies of this library in one process a single `once`
+// otherwise, though each has kernels of its own.
 template <auto KERNEL>
-int allow_smem(int bytes) {
+static int allow_smem(int bytes) {
   static OncePerDevice once;
   int dev = -1;
   B200_CUDA_OK(cudaGetDevice(&dev));

@@ -1,6 +1,7 @@
 """Kernels that start while the one before them ends: a chain of them, each reading what the one before has just written into
 buffers that are used again and again, gives the same bits as one that is waited for after every call."""
 import ctypes
+import shutil
 import subprocess
 import sys
 from pathlib import Path
@@ -126,6 +127,20 @@ def test_a_process_whose_first_call_is_captured(name, T, W):
     r = subprocess.run([sys.executable, "-c", FIRST_CALL % {"name": name, "T": T, "W": W}], capture_output=True, text=True, timeout=300,
                        cwd=Path(__file__).resolve().parent.parent)
     assert r.returncode == 0, r.stderr[-3000:]
+
+
+def test_two_copies_of_the_library_in_one_process(tmp_path):
+    """Each raises the limits of its own kernels."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    copy = tmp_path / "copy.so"
+    shutil.copyfile(_lib.lib_path(), copy)
+    second, ll, vp = ctypes.CDLL(str(copy)), ctypes.c_longlong, lambda t: ctypes.c_void_p(t.data_ptr())
+    x = torch.ones(512, 256, device="cuda", dtype=torch.bfloat16)
+    for lib in (_lib.load(), second):
+        out = torch.zeros(512, 512, device="cuda", dtype=torch.bfloat16)
+        assert lib.b200_gemm_bf16(vp(x), vp(x), vp(out), 512, 512, 256, ll(256), ll(256), ll(512), 0, 0, 0, 0, 0, 0, ctypes.c_void_p(_lib.stream_ptr())) == 0
+        assert (out == 256).all()
 
 
 def _programmatic(calls):
