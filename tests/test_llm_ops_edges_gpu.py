@@ -209,6 +209,16 @@ def test_adamw_over_the_whole_grid(n):
     assert ((w - (w0 * (1 - 1e-2 * 0.1) - per_m * em)).abs() <= 4 * ulp * w0.abs() + 64 * ulp * per_m * terms).all()
     assert torch.equal(p, w.bfloat16()) and not g.any()
 
+# a vector, a CTA's vectors and one more, more than the largest grid takes at once
+@pytest.mark.parametrize("T,H", [(1, 8), (256, 8), (257, 8), (5, 4104), (9700, 8192)])
+def test_embedding(T, H):
+    from aws_ofi_nccl_b200.ops import llm
+
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    table, ids = torch.randn(50, H, device="cuda", generator=g).bfloat16(), torch.randint(0, 50, (T,), device="cuda", generator=g)
+    assert torch.equal(llm.embedding(ids, table), table[ids])
+
+
 LOWEST = torch.finfo(torch.bfloat16).min   # the usual value of a mask
 
 
