@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
     rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, bf16* __restrict__ h_out,
                        const bf16* __restrict__ w, bf16* __restrict__ y, float* __restrict__ rstd, int T, int H, float eps) {
   after_wait(x, res, h_out, w, y, rstd);
-  grid_release();
+  grid_release_at_start<VPT == 1 ? 8 : VPT == 2 ? 6 : 4>();
   __shared__ float red[2][NORM_THREADS / 32];
   const int lane = threadIdx.x % TPR;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (NORM_THREADS / TPR) + threadIdx.x / TPR;
@@ -557,7 +557,7 @@ __device__ __forceinline__ void store_stream(Bf16x8* p, const Bf16x8& v) {
 template <typename Index>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, int64_t T, int F) {
   after_wait(gu, out);
-  grid_release();
+  grid_release_at_start<8>();
   const Index nvec = static_cast<Index>(T * F / 8), fv = F / 8;
   for (Index k = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; k < nvec; k += static_cast<Index>(gridDim.x) * blockDim.x) {
     const Index t = k / fv, c = k - t * fv;
@@ -578,7 +578,7 @@ template <bool INTERLEAVED, typename Index>
 __global__ void __launch_bounds__(256)
     swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu, int64_t T, int F) {
   after_wait(dout, gu, dgu);
-  grid_release();
+  grid_release_at_start<6>();
   const Index nvec = static_cast<Index>(T * F / 8), fv = F / 8;
   for (Index k = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; k < nvec; k += static_cast<Index>(gridDim.x) * blockDim.x) {
     int64_t gi, ui;
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(256)
 __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn, int64_t T,
                             int nheads, int hd, int64_t pitch, int seq, float sign) {
   after_wait(x, cs, sn);
-  grid_release();
+  grid_release_at_start<8>();
   const int half = hd / 2;
   const int64_t total = T * nheads * (half / 2);  // each thread rotates two adjacent pairs (bf162 loads)
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(256)
     rope_qkv_kernel(bf16* __restrict__ qkv, int64_t pitch, HeadsView q, HeadsView k, HeadsView v, const float* __restrict__ cs,
                     const float* __restrict__ sn, int64_t T, int nq, int nkv, int hd, int seq) {
   after_wait(qkv, cs, sn);
-  grid_release();
+  grid_release_at_start<6>();
   using Vec = Bf16Vec<V>;
   const int half = hd / 2;
   const Index per_head = half / V, heads = nq + 2 * nkv;
@@ -929,7 +929,7 @@ __global__ void adamw_kernel(bf16* __restrict__ p, bf16* __restrict__ g, float* 
                              float* __restrict__ master, int64_t n, float lr, float beta1, float beta2, float eps,
                              float wd, float bc1, float bc2, float grad_scale, int zero_grad) {
   after_wait(p, g, m, v, master);
-  grid_release();
+  grid_release_at_start<4>();
   const int64_t nvec = n / 8;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < nvec;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
