@@ -82,11 +82,14 @@ int gemm_group_m(int bn) {
 // tiles first) 4096 x 14336 x 4096 364 for 371, 8192 x 16384 x 2048 417 for 429, the fp8 product 4096 x 14336 x 4096 with its
 // quantiser 205 for 211. An operand of 34 MB stays; with 50 MB (6144 x 16384 x 4096, 5120 x 13824 x 5120) products took up to 2 %
 // longer so, with 67 MB 6 %: the two halves of L2 each hold what their own SMs read. Operands of no more tiles than a group are
-// walked whole by the groups (28672 x 2048 x 1024: N tiles first 105 us, 103 in groups).
+// walked whole by the groups (28672 x 2048 x 1024: N tiles first 105 us, 103 in groups). Where both operands are small both stay, and nothing is left to gain:
+// over 623 such products the walk takes 0.995 of the time of groups on average, but 0.85 to 1.21 with how their stores fall, short reductions above all
+// (5632 x 3592 x 352 with SwiGLU 54 us for 44, fp8 6656 x 8704 x 416 60 for 52); with a larger operand beyond 15 MB 0.990 over 284, and at most 1.03 but for one.
 void plan_walk(GemmShape& s, int elem_bytes) {
-  constexpr int64_t ROOM = 40000000;
+  constexpr int64_t ROOM = 40000000, BOTH_STAY = 15000000;
   if (group_m_override() >= 0) return;
   const int64_t a = static_cast<int64_t>(s.M) * s.K * elem_bytes, b = static_cast<int64_t>(s.N) * s.K * elem_bytes;
+  if (a <= BOTH_STAY && b <= BOTH_STAY) return;
   if (a <= b && a <= ROOM && s.tiles_m > s.group_m) {
     s.one_group = 1;
     s.m_major = 0;

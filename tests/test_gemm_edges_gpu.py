@@ -41,8 +41,10 @@ def test_product_and_accumulation(M, N, K, out_dtype, a_mn, b_mn):
     assert (pad[M:] == 7).all() and (pad[:, N:] == 7).all()
 
 
-# all M tiles of a column before the next column; all N tiles of a row before the next row; the last wave halved or not
-@pytest.mark.parametrize("M,N,K", [(2504, 2632, 72), (2632, 2504, 72), (2312, 4104, 200), (4104, 2312, 200)])
+# groups of M tiles where both operands are small; beside a larger one all M tiles of a column before the next column, or all N tiles of a row before the
+# next row; the last wave halved or not
+@pytest.mark.parametrize("M,N,K", [(2504, 2632, 72), (2632, 2504, 72), (2312, 4104, 200), (4104, 2312, 200), (2504, 15008, 520), (15008, 2504, 520),
+                                   (2312, 8200, 1000), (8200, 2312, 1000)])
 @pytest.mark.parametrize("b_mn", [False, True])
 def test_every_tile_is_computed_in_either_order_of_tiles(M, N, K, b_mn):
     from aws_ofi_nccl_b200.ops.gemm import gemm
