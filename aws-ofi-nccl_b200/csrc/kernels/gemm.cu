@@ -203,14 +203,16 @@ static int dispatch_major_2cta(const void* A, const void* B, void* C, int M, int
 // The narrow kernel has more stages; tiles of any other width run on the wide one. Eight epilogue warps store one tile during the next one's
 // products; where every pair has a single tile there is no next one, and four start sooner: 1504 x 1784 x 96 5.9 -> 5.5 us, 3200 x 1136
 // x 128 6.1 -> 5.9, 4 to 8 % over products of 38 to 74 tiles. Four are slower from three waves on (4096 x 4096 x 128 by 8 %), with two it varies.
+static int epilogue_warps(int M, int N, int K, int width, int out_fp32, int ctas) {
+  const int64_t tiles = static_cast<int64_t>((M + GEMM2_BM - 1) / GEMM2_BM) * ((N + width - 1) / width);
+  return width > 128 && K <= SHORT_K && !out_fp32 && tiles > ctas / 2 ? 8 : 4;
+}
 static int gemm_2cta(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_mn,
                      int b_mn, int out_fp32, int accumulate, PairTiles tiles, int max_ctas, cudaStream_t s) {
   if (tiles.width == 128)
     return out_fp32 ? dispatch_major_2cta<128, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
                     : dispatch_major_2cta<128, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
-  const int64_t all = static_cast<int64_t>((M + GEMM2_BM - 1) / GEMM2_BM) * ((N + tiles.width - 1) / tiles.width);
-  const int pairs = (keeps_room(max_ctas) ? max_ctas : sm_count()) / 2;
-  if (K <= SHORT_K && !out_fp32 && all > pairs)
+  if (epilogue_warps(M, N, K, tiles.width, out_fp32, keeps_room(max_ctas) ? max_ctas : sm_count()) == 8)
     return dispatch_major_2cta<256, __nv_bfloat16, 8>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
   return out_fp32 ? dispatch_major_2cta<256, float>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s)
                   : dispatch_major_2cta<256, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, tiles, max_ctas, s);
@@ -366,15 +368,18 @@ static bool use_pairs(int M, int N, int max_ctas) {
 
 // Three rows of 128 x 128 tiles that all run at once, where pairs would compute four rows in wide tiles on two thirds of the SMs: 257 to 384 rows
 // and 4737 to 6272 columns. 384 x 6144 x 4096 19.4 us, 22.4 on pairs; 340 x 5952 x 2816 14.2 and 16.8; 384 x 6208 x 1024 8.3 and 10.4; 300 x
-// 5120 x 13824 51 and 58. Fewer columns fit narrow pair tiles (384 x 4096 x 4096 16.6 us, 18.5 so), more take these two waves.
+// 5120 x 13824 51 and 58. Fewer columns fit narrow pair tiles (384 x 4096 x 4096 16.6 us, 18.5 so), more take these two waves. A k-block takes THREE_ROWS_KBLOCK
+// clocks there.
+constexpr double THREE_ROWS_KBLOCK = 395;
 static bool three_tile_rows(int M, int N) {
   const int columns = (N + 127) / 128;
   return M > 2 * GEMM_BM && M <= 3 * GEMM_BM && 3 * columns <= sm_count() && 2 * columns > sm_count() / 2;
 }
 
-// What a product with bn = 0 runs on: the tile width of the persistent kernel, or a split along K.
+// What a product with bn = 0 runs on: CTA pairs or single CTAs, the tile width of the persistent kernel, or a split along K.
 // `a_at`, `b_at`: the operands' addresses (their alignment counts).
 struct GemmChoice {
+  bool pairs;
   int bn;            // the plain width that fits better, 128 or 256
   PairTiles tiles;   // on CTA pairs: what the product runs on
   SplitkPlan split;
@@ -425,8 +430,11 @@ static PairTiles fit_tiles(int M, int N, int K, bool b_mn, uint64_t a_low, uint6
   if (wide > units && last > 0 && 2 * last <= units && (static_cast<double>(wide / units) + half_wave) * 1.01 <= best_cost) best = {256, true};
   return best;
 }
-static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, uintptr_t a_at, uintptr_t b_at, int max_ctas) {
+// three_rows: whether three_tile_rows may have it.
+static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, uintptr_t a_at, uintptr_t b_at, int max_ctas,
+                              bool three_rows = true) {
   const bool pairs = use_pairs(M, N, max_ctas);
+  const auto split_on = [&](int width) { return max_ctas == 0 ? plan_splitk(M, N, K, pairs, width) : SplitkPlan{1}; };
   int bn;
   PairTiles tiles{};
   // Wider tiles re-read A less; fall back to the narrower tile when that fills the SMs better.
@@ -458,12 +466,14 @@ static GemmChoice choose_gemm(int M, int N, int K, int64_t lda, int64_t ldb, boo
     // Narrow tiles that need no more waves are done sooner: 16 x 624 x 256 8 us, 10 in wide ones. The split is weighed against the
     // width above all the same, which its model was fitted to: against narrow tiles it would leave 24 x 560 x 2032 whole (12.8 us, 8.5 split).
     if (w256 == w128) {
-      const SplitkPlan split = max_ctas == 0 ? plan_splitk(M, N, K, false, bn) : SplitkPlan{1};
-      return split.slices > 1 ? GemmChoice{bn, tiles, split} : GemmChoice{128, tiles, max_ctas == 0 ? plan_splitk(M, N, K, false, 128) : split};
+      const SplitkPlan split = split_on(bn);
+      return split.slices > 1 ? GemmChoice{false, bn, tiles, split} : GemmChoice{false, 128, tiles, split_on(128)};
     }
   }
   // Few tiles and a long K: the chip is filled by splitting K over clusters.
-  return {bn, tiles, max_ctas == 0 ? plan_splitk(M, N, K, pairs, bn) : SplitkPlan{1}};
+  const SplitkPlan split = split_on(bn);
+  if (pairs && max_ctas == 0 && split.slices == 1 && three_rows && three_tile_rows(M, N)) return {false, 128, {}, split};
+  return {pairs, bn, tiles, split};
 }
 
 double product_clocks(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, const void* A, const void* B) {
@@ -472,13 +482,16 @@ double product_clocks(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, 
   const double floor = memory_clocks(M, N, K);
   // what the split model was fitted to had slower waits
   if (g.split.slices > 1) return std::max((g.split.clocks - LAUNCH_CLOCKS) * 0.7, floor) + LAUNCH_CLOCKS;
-  if (!use_pairs(M, N, 0)) return std::max((g.split.clocks - LAUNCH_CLOCKS) * 0.8, floor) + LAUNCH_CLOCKS;
+  if (!g.pairs) {
+    const double tiles = use_pairs(M, N, 0) ? (K + GEMM_BK - 1) / GEMM_BK * THREE_ROWS_KBLOCK : (g.split.clocks - LAUNCH_CLOCKS) * 0.8;
+    return std::max(tiles, floor) + LAUNCH_CLOCKS;
+  }
   const bool lines = (a_at | b_at | static_cast<uint64_t>(lda | ldb) * 2) % 128 == 0;
   const int64_t rows = (M + GEMM2_BM - 1) / GEMM2_BM, units = sm_count() / 2;
   double best = 1e30;
   for (int width = 128; width <= 256; width += 64) {
     const int64_t tiles = rows * ((N + width - 1) / width);
-    best = std::min(best, static_cast<double>((tiles + units - 1) / units) * pair_tile_clocks(K, width, lines, K <= SHORT_K ? 8 : 4));
+    best = std::min(best, static_cast<double>((tiles + units - 1) / units) * pair_tile_clocks(K, width, lines, epilogue_warps(M, N, K, width, 0, sm_count())));
   }
   return std::max(best, floor) + LAUNCH_CLOCKS;
 }
@@ -486,7 +499,7 @@ double product_clocks(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, 
 bool runs_on_pairs(int M, int N, int K, int64_t lda, int64_t ldb, bool b_mn, const void* A, const void* B, PairTiles* tiles) {
   if (!use_pairs(M, N, 0)) return false;
   const uintptr_t a_at = reinterpret_cast<uintptr_t>(A), b_at = reinterpret_cast<uintptr_t>(B);
-  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, b_mn, a_at, b_at, 0);
+  const GemmChoice g = choose_gemm(M, N, K, lda, ldb, b_mn, a_at, b_at, 0, false);
   if (g.split.slices > 1) return false;
   *tiles = fit_tiles(M, N, K, b_mn, a_at | (static_cast<uint64_t>(lda) * 2), b_at | (static_cast<uint64_t>(ldb) * 2), sm_count() / 2,
                      g.bn, 128);
@@ -506,19 +519,16 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, l
   using namespace b200;
   if (!gemm_args_ok(A, B, C, M, N, K, lda, ldb, ldc, out_fp32)) return B200_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  bool pairs = use_pairs(M, N, max_ctas);
+  bool pairs = use_pairs(M, N, max_ctas);   // of a width that the caller chose
   PairTiles tiles{bn, false};
   if (bn == 0) {
     const GemmChoice g =
         choose_gemm(M, N, K, lda, ldb, b_mn != 0, reinterpret_cast<uintptr_t>(A), reinterpret_cast<uintptr_t>(B), max_ctas);
+    pairs = g.pairs;
     if (g.split.slices > 1)
       return launch_splitk({A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate}, pairs, g.split, s);
     bn = g.bn;
     tiles = g.tiles;
-    if (pairs && max_ctas == 0 && three_tile_rows(M, N)) {
-      pairs = false;
-      bn = 128;
-    }
   }
   if (pairs && (bn == 256 || bn == 128))
     return gemm_2cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, tiles, max_ctas, s);
@@ -540,13 +550,9 @@ int b200_gemm_plan(int M, int N, int K, long long lda, long long ldb, int* pair,
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || !pair || !bn || !slices) return B200_ERR_BAD_ARG;
   const GemmChoice g = choose_gemm(M, N, K, lda, ldb, false, 0, 0, 0);
-  *pair = use_pairs(M, N, 0);
+  *pair = g.pairs;
   *slices = g.split.slices;
   *bn = g.split.slices > 1 ? 128 : g.bn;
-  if (*pair && *slices == 1 && three_tile_rows(M, N)) {
-    *pair = 0;
-    *bn = 128;
-  }
   return 0;
 }
 
@@ -555,8 +561,9 @@ int b200_gemm_plan(int M, int N, int K, long long lda, long long ldb, int* pair,
 int b200_gemm_tiles(int M, int N, int K, long long lda, long long ldb, int b_mn, int* width, int* halves) {
   b200::ensure_context();
   using namespace b200;
-  if (M <= 0 || N <= 0 || K <= 0 || !width || !halves || !use_pairs(M, N, 0)) return B200_ERR_BAD_ARG;
+  if (M <= 0 || N <= 0 || K <= 0 || !width || !halves) return B200_ERR_BAD_ARG;
   const GemmChoice g = choose_gemm(M, N, K, lda, ldb, b_mn != 0, 0, 0, 0);
+  if (!g.pairs) return B200_ERR_BAD_ARG;
   *width = g.tiles.width;
   *halves = g.tiles.halves;
   return 0;

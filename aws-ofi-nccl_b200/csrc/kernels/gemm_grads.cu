@@ -80,8 +80,10 @@ GradsPlan plan_joint(const GradsCall& c) {
 // over clusters, and for few rows through a weight that L2 does not hold: a single row of tiles takes the weight from memory
 // at the pace of its own pipeline, and joint kernels got 3.8 TB/s there where dx alone gets 5.3 (128 x 4096 x 14336
 // with cold weights 63 us, 58 in two). Of 128 layers (M 16 to 8192, N 64 to 28672, K 64 to 14336, and the 8B model's) the
-// rule takes one launch for 93; the mean of its times is 0.789 of two launches', the faster way's 0.785, and it is never
-// slower by more than 3 % than two. Between 129 and 256 rows dx by itself is a single row of tiles as well, and takes longer than the
+// rule took one launch for 93; the mean of its times was 0.789 of two launches', the faster way's 0.785. Since the second of two launches comes up
+// while the first one ends (EARLY clocks), of 920 layers (M 16 to 8192, most of them 16 to 384, N 64 to 28672, K 64 to 14336) it takes one for 753 where
+// 743 would be faster so; the mean of its times is 1.004 of the faster way's, 1.002 over 315 layers of 257 to 384 rows, and 34 are slower by
+// more than 3 % (192 x 9408 x 1984 44 us for 31, 88 x 8320 x 3072 42 and 33). Between 129 and 256 rows dx by itself is a single row of tiles as well, and takes longer than the
 // estimate for a product by itself says: of 37 such layers over weights of 64 to 600 MB with N <= 3 K the rule takes one launch for 33; the mean of
 // its times is 0.86 of two launches' and 1.008 of the faster way's, 1.089 with the line that fewer rows have (256 x 8192 x 8192 72 us for
 // 86, 200 x 5120 x 13824 73 and 92, 256 x 6144 x 6144 47 and 59). A longer reduction is a chain that two launches split (136 x 28672 x 4096 126 us, 147 jointly).
@@ -94,7 +96,8 @@ bool pays(const GradsCall& c, const GradsPlan& p) {
   double alone = pair_tile_clocks(c.N, p.width[0], on_lines(c), p.warps);
   if (few_rows) alone = std::max(alone, (one_pair_row ? 520.0 : 700.0) * ((c.N + GEMM_BK - 1) / GEMM_BK));
   const double moved = (one_pair_row ? 1.15 : few_rows ? 1.25 : 0.8) * (memory_clocks(c.M, c.K, c.N) + memory_clocks(c.N, c.K, c.M));
-  const double joint = std::max({p.clocks, alone, moved}) + LAUNCH_CLOCKS;
+  constexpr double EARLY = 4000;
+  const double joint = std::max({p.clocks, alone, moved}) + LAUNCH_CLOCKS + EARLY;
   return joint < (one_pair_row ? 1.08 : 1.0) * (product_clocks(c.M, c.K, c.N, c.lddy, c.ldw, true, c.dy, c.w) + product_clocks(c.N, c.K, c.M, c.lddy, c.ldx, true, c.dy, c.x));
 }
 

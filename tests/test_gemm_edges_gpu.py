@@ -86,6 +86,18 @@ def test_other_rows_and_columns_stay_on_pairs(M, N):
     assert _plan(M, N, 2048)[0] == 1
 
 
+def test_products_on_single_ctas_have_no_pair_tiles():
+    """Nor do they change what SwiGLU's products run on, whose epilogues need the sums in 32 bits."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    lib, ll, vp = _lib.load(), ctypes.c_longlong, ctypes.c_void_p
+    w, h = ctypes.c_int(), ctypes.c_int()
+    for M, N, want in ((300, 6144, 10001), (256, 6144, 0), (385, 6144, 0), (128, 6144, 10001)):
+        assert lib.b200_gemm_tiles(M, N, 2048, ll(2048), ll(2048), 0, ctypes.byref(w), ctypes.byref(h)) == want
+    assert lib.b200_gemm_swiglu_launches(vp(4096), vp(4096), 300, 3072, 2048, ll(2048)) == 1
+    assert lib.b200_gemm_swiglu_bwd_launches(vp(4096), vp(4096), 300, 6144, 2048, ll(6144)) == 1
+
+
 @pytest.mark.parametrize("M,N,K", [(256, 256, 1024), (512, 1024, 2048), (128, 4096, 1024), (768, 1536, 2048)])
 def test_a_short_reduction_is_not_split(M, N, K):
     """Products that a split made up to 1.4 times slower."""

@@ -79,6 +79,12 @@ def test_a_row_of_pair_tiles_takes_the_faster_way(M, N, K, joint):
     test_linear_layer_takes_the_faster_way(M, N, K, joint)
 
 
+@pytest.mark.parametrize("M,N,K,joint", [(144, 7488, 1280, 0), (64, 4800, 448, 0), (340, 5952, 2816, 1), (128, 2048, 1024, 1)])
+def test_two_launches_overlap_where_that_is_the_faster_way(M, N, K, joint):
+    """The second one comes up while the first one ends; rows and columns that single CTAs take, and a K that four warps store."""
+    test_linear_layer_takes_the_faster_way(M, N, K, joint)
+
+
 def test_only_one_of_the_gradients():
     from aws_ofi_nccl_b200.ops.gemm import linear
 
