@@ -3,6 +3,7 @@
 ``Trainer.step(ids_host, labels_host)`` runs one full optimizer step — host-to-device copy of the
 batch from pinned memory, forward, backward (with the gradient all-reduce of a data-parallel job
 overlapped behind it), fused AdamW — and returns the loss as a Python float (device-to-host read).
+Waits in kernels are bounded; where one gave up, the step raises instead.
 """
 from __future__ import annotations
 
@@ -11,6 +12,7 @@ import dataclasses
 import torch
 
 from ..models.llama import Llama, LlamaConfig
+from ..ops import _lib
 from ..ops import llm as llm_ops
 
 
@@ -83,8 +85,11 @@ class Trainer:
             self._labels_dev = torch.empty(labels_host.shape, device=self.device, dtype=torch.int64)
         self._ids_dev.copy_(ids_host, non_blocking=True)
         self._labels_dev.copy_(labels_host, non_blocking=True)
-        loss = self.step_device(self._ids_dev, self._labels_dev)
-        return float(loss.item())
+        loss = float(self.step_device(self._ids_dev, self._labels_dev).item())
+        status = _lib.read_status()
+        if status != 0:
+            raise _lib.B200OpsError(f"a wait in a kernel gave up (status {status}): the parameters may be wrong from this step on")
+        return loss
 
     def launches_per_step(self) -> int:
         """Number of this library's kernels launched by one step (GEMMs + bandwidth kernels)."""

@@ -65,3 +65,22 @@ def test_native_layers_are_rebuilt_for_another_torch_or_header(tmp_path, monkeyp
     os.utime(out, (0, header.stat().st_mtime - 1))
     build.build_torch_ops()
     assert len(runs) == 2                              # a signature may have changed
+
+
+def test_a_step_whose_kernels_gave_up_on_a_wait_raises(monkeypatch):
+    """The status that the kernels leave, read behind the loss; a clean step returns that."""
+    import pytest
+    import torch
+
+    from aws_ofi_nccl_b200.ops import _lib
+    from aws_ofi_nccl_b200.parallel.engine import Trainer
+
+    trainer = Trainer.__new__(Trainer)
+    trainer.device, trainer._ids_dev, trainer.step_device = torch.device("cpu"), None, lambda ids, labels: torch.tensor(1.5)
+    batch = torch.zeros(2, 4, dtype=torch.int64)
+    status = [0]
+    monkeypatch.setattr(_lib, "read_status", lambda: status[0])
+    assert trainer.step(batch, batch) == 1.5
+    status[0] = 7
+    with pytest.raises(_lib.B200OpsError, match="status 7"):
+        trainer.step(batch, batch)
