@@ -95,6 +95,111 @@ def test_a_captured_chain_does_too(T, H, F):
         assert torch.equal(a, b)
 
 
+class _Layers:
+    """Embedding, residual norm, projection, rotary split, a wide head's cross entropy, and what leads back from there: rotary split, projection, norm
+    with its weight's gradient, embedding. No id comes twice, so that the table's gradient is the same every time."""
+
+    def __init__(self, T, heads, hd, V):
+        g = torch.Generator(device="cuda").manual_seed(T + heads + V)
+        bf, f32 = torch.bfloat16, torch.float32
+
+        def rnd(*s, std=1.0):
+            return (torch.randn(*s, device="cuda", generator=g) * std).to(bf)
+
+        H, P = heads * hd, (heads + 2) * hd
+        self.T, self.heads, self.hd, self.V, self.H, self.P = T, heads, hd, V, H, P
+        self.ids, self.targets = torch.randperm(2 * T, device="cuda", generator=g)[:T], torch.randint(0, V, (T,), device="cuda", generator=g)
+        self.table, self.res, self.w = rnd(2 * T, H), rnd(T, H), rnd(H, std=0.1) + 1
+        self.wqkv, self.head = rnd(P, H, std=H ** -0.5), rnd(V, H, std=H ** -0.5)
+        self.cos, self.sin = torch.rand(T, hd // 2, device="cuda", generator=g), torch.rand(T, hd // 2, device="cuda", generator=g)
+        self.buf = {k: torch.zeros(*shape, device="cuda", dtype=d) for k, (shape, d) in {
+            "x": ((T, H), bf), "h": ((T, H), bf), "y": ((T, H), bf), "rstd": ((T,), f32), "qkv": ((T, P), bf), "q": ((T, H), bf), "k": ((T, hd), bf),
+            "v": ((T, hd), bf), "logits": ((T, V), bf), "loss": ((T,), f32), "dy": ((T, H), bf), "dqkv": ((T, P), bf), "dn": ((T, H), bf),
+            "dx": ((T, H), bf), "dw": ((H,), bf), "dtable": ((2 * T, H), bf)}.items()}
+
+    def steps(self):
+        from aws_ofi_nccl_b200.ops import _lib
+        from aws_ofi_nccl_b200.ops.gemm import gemm
+
+        L, b, T, H = _lib.load(), self.buf, self.T, self.H
+        partial = self.buf.setdefault("partial", torch.zeros(L.b200_rmsnorm_bwd_partial_rows(), H, device="cuda"))
+        strides = (ctypes.c_longlong * 9)(*[n for row in (H, self.hd, self.hd) for n in (0, row, self.hd)])
+
+        def call(name, *args):
+            fn = getattr(L, name)
+            _lib.check(fn(*[ctypes.c_void_p(a.data_ptr()) if isinstance(a, torch.Tensor) else a for a in args], ctypes.c_void_p(_lib.stream_ptr())), name)
+
+        def rope(qkv, backward):
+            call("b200_rope_qkv", qkv, ctypes.c_longlong(self.P), b["q"], b["k"], b["v"], strides, self.cos, self.sin, ctypes.c_longlong(T), self.heads, 1, self.hd, T, backward)
+
+        yield lambda: call("b200_embedding_fwd", self.ids, self.table, b["x"], T, H)
+        yield lambda: call("b200_rmsnorm_fwd", b["x"], self.res, b["h"], self.w, b["y"], b["rstd"], T, H, 1e-5)
+        yield lambda: gemm(b["y"], self.wqkv, out=b["qkv"])
+        yield lambda: rope(b["qkv"], 0)
+        yield lambda: gemm(b["y"], self.head, out=b["logits"])
+        yield lambda: call("b200_cross_entropy", b["logits"], self.targets, b["loss"], T, self.V, self.V, 1.0)
+        yield lambda: gemm(b["logits"], self.head, b_mn=True, out=b["dy"])
+        yield lambda: rope(b["dqkv"], 1)
+        yield lambda: gemm(b["dqkv"], self.wqkv, b_mn=True, out=b["dn"])
+        yield lambda: call("b200_rmsnorm_bwd", b["dn"], b["h"], self.w, b["rstd"], b["dy"], b["dx"], partial, b["dw"], 0, T, H)
+        yield lambda: call("b200_embedding_bwd", self.ids, b["dx"], b["dtable"], T, H)
+        yield lambda: self.table.copy_(b["dtable"])   # what the next pass looks up
+
+    run = _Chain.run
+
+    def run_on(self, streams):
+        """Each kernel on the other stream than the one before, behind it and behind the one before that."""
+        streams[1].wait_stream(streams[0])
+        for i, step in enumerate(self.steps()):
+            here, other = streams[i % 2], streams[1 - i % 2]
+            here.wait_stream(other)
+            with torch.cuda.stream(here):
+                step()
+        streams[0].wait_stream(streams[1])
+
+    def results(self):
+        return [t.clone() for t in (self.table, *self.buf.values())]
+
+
+# tokens that fill no wave; norms through rings and streamed rows of the head
+LAYERS = [(64, 4, 64, 1000), (1000, 16, 128, 2056), (300, 4, 128, 32776)]
+
+
+@pytest.mark.parametrize("T,heads,hd,V", LAYERS)
+def test_a_chain_of_layers_does_too(T, heads, hd, V):
+    waited, chained = _Layers(T, heads, hd, V), _Layers(T, heads, hd, V)
+    for _ in range(3):
+        waited.run(True)
+    for _ in range(3):
+        chained.run(False)
+    for a, b in zip(waited.results(), chained.results()):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("T,heads,hd,V", LAYERS)
+def test_and_a_chain_over_two_streams(T, heads, hd, V, captured):
+    """A kernel behind one on its own stream and one on another waits for both."""
+    waited, chained = _Layers(T, heads, hd, V), _Layers(T, heads, hd, V)
+    for _ in range(3):
+        waited.run(True)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    if captured:
+        chained.run(False)   # what a first call sets up is no part of a graph
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=streams[0]):
+            chained.run_on(streams)
+        for _ in range(2):
+            graph.replay()
+    else:
+        for _ in range(3):
+            chained.run_on(streams)
+    torch.cuda.synchronize()
+    for a, b in zip(waited.results(), chained.results()):
+        assert torch.equal(a, b)
+
+
 FIRST_CALL = """
 import torch
 from aws_ofi_nccl_b200.ops import _lib

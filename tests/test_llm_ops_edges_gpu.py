@@ -294,6 +294,32 @@ def test_cross_entropy_of_wide_rows(T, V, scale):
     assert _lib.read_status() == 0
 
 
+# one chunk, two, all that the ring holds; one, two and four more that come a second time
+@pytest.mark.parametrize("V", [16392, 32776, 98304, 98312, 131080, 180232])
+def test_every_row_of_a_cta_of_the_streamed_cross_entropy(V):
+    """Rows that follow one another through a CTA's ring: the slots that a row begins with change from row to row."""
+    from aws_ofi_nccl_b200.ops import _lib
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    T = 5 * sms + 3   # six rows for CTAs 0 to 2, five for the others
+    assert _lib.load().b200_cross_entropy_ctas(T, V) == 0
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = torch.empty(T, V, device="cuda", dtype=torch.bfloat16).normal_(0, 3, generator=g)
+    targets = torch.randint(0, V, (T,), device="cuda", generator=g)
+    rows = torch.tensor([r for cta in (0, 2, 3, sms - 1) for r in range(cta, T, sms)], device="cuda")
+    x, at = logits[rows].double(), targets[rows][:, None]
+    lse = torch.logsumexp(x, -1)
+    want_loss, want = lse - x.gather(1, at)[:, 0], (x - lse[:, None]).exp()
+    want.scatter_add_(1, at, -torch.ones_like(lse)[:, None])
+    loss = torch.full((T,), math.nan, device="cuda")
+    assert _lib.load().b200_cross_entropy(logits.data_ptr(), targets.data_ptr(), loss.data_ptr(), T, V, V, 1.0, _lib.stream_ptr()) == 0
+    # as above: arguments up to 40 whose product with log2(e) is rounded to 24 bits, and sums of their powers
+    err = 160 * 2.0 ** -24
+    _within(loss[rows], want_loss, err, err * (1 + lse.abs().max()))
+    _within(logits[rows], want, BF + err, err + 2.0 ** -133)
+    assert _lib.read_status() == 0
+
+
 def test_rows_without_elements():
     """No loss, and no norm: what the entry points did before rows came through rings."""
     from aws_ofi_nccl_b200.ops import _lib

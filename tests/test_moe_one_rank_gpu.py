@@ -237,3 +237,47 @@ def test_more_tokens_than_a_grid_holds(comm):
         want = (dy.double() * x.detach().double()).sum(-1, keepdim=True)
         mag = (dy.double() * x.detach().double()).abs().sum(-1, keepdim=True)
         assert torch.equal(dx, dy * 0.5) and ((dw.double() - want).abs() <= H * 2.0 ** -24 * mag).all()
+
+
+# fewer tokens than an SM's CTAs take, more than one grid holds
+@pytest.mark.parametrize("T", [50, 9001])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_dispatch_and_combine_between_products(comm, T, fp8):
+    """Kernels that come up while the one before ends: products that make the rows, take them and give them back, pass after pass without a wait,
+    give the same bits as with one after every call."""
+    from aws_ofi_nccl_b200.ops.gemm import gemm
+    from aws_ofi_nccl_b200.parallel.expert_parallel import ExpertParallel
+
+    H, E = 256, 8
+    ep = ExpertParallel(comm, T, H, E, 1, capacity_factor=1.0)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x0 = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    w1, w2 = ((torch.randn(H, H, device="cuda", generator=g) * H ** -0.5).bfloat16() for _ in range(2))
+    idx = torch.randint(0, E, (T, 1), device="cuda", generator=g, dtype=torch.int32)
+    weights = torch.rand(T, 1, device="cuda", generator=g)
+
+    def passes(wait):
+        x, outs = x0.clone(), []
+
+        def done():
+            if wait:
+                torch.cuda.synchronize()
+
+        for _ in range(3):
+            sent = gemm(x, w1)
+            done()
+            rows = ep.dispatch(sent, idx, weights, fp8)
+            done()
+            made = gemm(rows, w2)
+            done()
+            back = ep.combine(made, weights)
+            done()
+            x = gemm(back, w1)
+            done()
+            outs += [sent, back, x]
+        return outs
+
+    with torch.no_grad():
+        want, got = passes(True), passes(False)
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
