@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(CE_ROW_THREADS, CE_ROW_CTAS)
     cross_entropy_row_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ targets, float* __restrict__ loss, int V,
                              int64_t ld, float grad_scale, int cluster) {
   after_wait(logits, targets, loss);
-  grid_release();
+  grid_release_at_start<CE_ROW_CTAS>();
   __shared__ float red[32];
   __shared__ float2 part;   // maximum of this CTA's elements, sum of their exponentials relative to it
   const int rank = static_cast<int>(blockIdx.x) % cluster;
@@ -1006,10 +1006,10 @@ static CeRow ce_row(int64_t T, int V) {
   return pays ? CeRow{ctas, vpt} : CeRow{0, 0};
 }
 
-// Rows that no registers hold stream through shared memory, but for two rows for an SM of a length that a chunk or two hold: there two
-// CTAs of many threads are ahead (222 x 24576 10.0 us, 10.8 streamed; 296 x 28672 11.7 and 12.8). Everywhere else of 18 numbers of rows from 1
-// to 2048 and 12 widths from 16392 to 200000 the stream takes 0.68 to 1.00 of two passes.
-// A row without elements has no chunk to stream.
+// Rows that no registers hold stream through shared memory, but for two rows for an SM of about a chunk's length (24576 elements), where two
+// CTAs of many threads are ahead. The lines are fitted to 64 pairs of times (149 to 296 rows of 18000 to 32760): 240 x 24576 10.0 us, 10.7 streamed, 240 x 28672 11.1
+// and 12.3; at 20000 to 22000 both are within 3 %, below 20000 and from 32768 on the stream is the faster one. Everywhere else of 18 numbers of rows from 1
+// to 2048 and 12 widths from 16392 to 200000 the stream takes 0.68 to 1.00 of two passes. A row without elements has no chunk to stream.
 static bool ce_two_passes(int64_t T, int V) { return V < 8 || (V >= 20000 && V < 32768 && T > sm_count() && T <= 2 * sm_count()); }
 
 // Rows move as 16-byte vectors: null (an argument left out) or on a 16-byte boundary.
