@@ -94,7 +94,7 @@ struct AgGemmArgs {
   uint32_t epoch;
 };
 
-// Untiled bulk copies (no multicast): global -> shared with an mbarrier, shared -> global in a bulk group.
+// An untiled bulk copy from shared to global memory, in a bulk group (bulk_load is the other way).
 __device__ __forceinline__ void bulk_store(void* dst, uint32_t src_smem, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src_smem), "r"(bytes)
                : "memory");
