@@ -10,7 +10,8 @@
 // collective, whose CTAs wait for other ranks' tiles, are launched ordinarily.
 //
 // Where a kernel takes const __restrict__ pointers (or restrict ones that it only reads from) the compiler may move loads through
-// them anywhere, before grid_wait too: such kernels use their pointers as after_wait returns them.
+// them anywhere, before grid_wait too: such kernels use their pointers as after_wait returns them. What it then knows of them no longer is that stores leave
+// the loads alone: a loop's loads are no longer batched across its stores.
 //
 // grid_release stands near the end of a kernel's work, or at the start of kernels of several waves, where the last CTA to start
 // is what counts: from then on CTAs of the next kernel hold what room there is on an SM,
